@@ -357,9 +357,10 @@ def run(state):
     if kind in ("mlm", "lm", "resnet"):
         engine = state["engine"]
         loss = engine.replay(state["batch"])
-        if kind == "resnet":     # twenty 16-bit convolutions under ReLUs leave a tenth of the gradients to rounding: the updated state is what can be compared
-            return {"loss": loss, "params": engine.flat.params, "buffers": state["buffers"]}
-        return {"loss": loss, "grads": engine.flat.grads, "params": engine.flat.params}
+        # The updated weights are what is compared. Gradients are an intermediate here, and a poor yardstick: those of the key biases are
+        # zero but for rounding, and twenty 16-bit convolutions under ReLUs leave a tenth of a filter's gradient to rounding.
+        out = {"loss": loss, "params": engine.flat.params}
+        return dict(out, buffers=state["buffers"]) if kind == "resnet" else out
     if kind == "encode":
         if case["captured"]:
             state["replay"].replay()
@@ -472,7 +473,7 @@ def _exact_training(case, seed):
     if sgd:
         # (nor are the running statistics in: sixteen means near zero are as near as the order of their sums happens to bring them)
         return {"loss": None, "params": _slots(case, w), "buffers": None}
-    return {"loss": None, "grads": _slots(case, grads), "params": _slots(case, w)}
+    return {"loss": None, "params": _slots(case, w)}
 
 
 def exact(case, seed):
@@ -523,14 +524,14 @@ def work(case):
         if kind == "encode":
             return {"bytes": 2.0 * (n - case["vocab"] * h) + T * (2.0 * h + 2.0 * h + 32), "flops": body}
         head = 2.0 * T * h * case["vocab"] if kind == "lm" else 0.15 * T * (2.0 * h * case["vocab"] + 2.0 * h * h)
-        # AdamW reads and writes the weights and both moments (24 bytes a weight); the gradients are an output too
-        return {"bytes": 28.0 * n + 40.0 * T, "flops": 3.0 * (body + head)}
+        # AdamW reads and writes the weights and both moments: 24 bytes a weight
+        return {"bytes": 24.0 * n + 40.0 * T, "flops": 3.0 * (body + head)}
     if kind == "resnet":
         macs, side = 27 * 16 * 1024, 32
         for _, ci, co, stride in _blocks():
             side //= stride
             macs += side * side * (9 * ci * co + 9 * co * co + (ci * co if ci != co else 0))
-        return {"bytes": 20.0 * n + case["batch"] * (3 * 1024 * 4.0 + 8), "flops": 6.0 * case["batch"] * macs}
+        return {"bytes": 16.0 * n + case["batch"] * (3 * 1024 * 4.0 + 8), "flops": 6.0 * case["batch"] * macs}
     if kind == "attention":
         e = case["batch"] * case["heads"] * case["seq"] * 64
         return {"bytes": 2.0 * 8 * e, "flops": 12.0 * e * case["seq"] * (0.5 if case["causal"] else 1.0)}
@@ -541,10 +542,13 @@ def work(case):
 
 
 def tolerance(case):
-    """Measured against `exact`: gradients of 1 to 12 bf16 layers are 0.006 to 0.0125 off, encoder outputs 0.0085, attention 0.0024, one
-    rounding to bf16 0.0017, 32-bit softmax and LayerNorm below 1e-6."""
+    """Measured against `exact`: weights after a step of AdamW are 0.00005 to 0.00013 off (their update is 0.005 to 0.015 of their norm) and
+    0.018 of the root mean square at most, weights after a step of SGD 0.0008 to 0.004, encoder outputs 0.0085, attention 0.0024, one rounding
+    to bf16 0.0017, 32-bit softmax and LayerNorm below 1e-6."""
     kind = case["kind"]
-    if kind in ("mlm", "lm", "resnet", "encode"):
+    if kind in ("mlm", "lm"):
+        return {"rel": 0.0006, "max": 0.08}
+    if kind in ("resnet", "encode"):
         return {"rel": 0.03}
     if kind == "attention":
         return {"rel": 0.01}
