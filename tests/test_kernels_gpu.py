@@ -289,6 +289,45 @@ def test_attention_fwd_bwd(C, B, H, S, causal, use_mask):
         assert err < 0.06 * max(1.0, g.abs().max().item()), (i, err, g.abs().max().item())
 
 
+@pytest.mark.parametrize("B,H,S,causal,use_mask", [(1, 1, 129, True, False), (2, 3, 131, False, True), (1, 2, 255, True, True), (3, 1, 257, False, False),
+                                                   (1, 4, 509, False, True), (2, 2, 641, True, False), (9, 20, 129, False, False), (1, 1, 2050, True, False)])
+def test_attention_several_key_blocks(C, B, H, S, causal, use_mask):
+    """Sizes at the edges of the 128-row blocks, against 64-bit attention. Inputs and outputs are rounded to bf16 (2^-9 relative each), and so
+    are the probabilities and their gradients inside; four such roundings in root-sum-square are 2^-8 of a result's norm."""
+    torch.manual_seed(11)
+    qkv = torch.randn(B, S, 3, H, 64, device="cuda").bfloat16()
+    q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
+    mask = None
+    if use_mask:
+        mask = torch.zeros(B, S, device="cuda")
+        mask[:, S // 3:] = -1e4
+        mask[0] = 0.0
+    C.clear_status(0)
+    o, lse = C.attn_fwd(q, k, v, mask, 0.125, causal)
+    do = torch.randn(B, S, H, 64, device="cuda").bfloat16()
+    dqkv = C.attn_bwd(q, k, v, o, do, lse, mask, 0.125, causal)
+    torch.cuda.synchronize()
+    assert C.read_status(0) == 0
+    ref_in = [t.double().requires_grad_(True) for t in (q, k, v)]
+    ref = _attn_ref(*ref_in, None if mask is None else mask.double(), 0.125, causal)
+    ref.backward(do.double())
+    assert ((o.double() - ref).norm() / ref.norm()).item() < 2 ** -8
+    for i, t in enumerate(ref_in):
+        assert ((dqkv[:, :, i].double() - t.grad).norm() / t.grad.norm()).item() < 2 ** -7, i     # through P and dS both
+
+
+def test_attention_several_key_blocks_dropout(C):
+    """O is linear in V for fixed probabilities, so <dO, O> = <dV, V> exactly if and only if backward drops what forward dropped."""
+    torch.manual_seed(12)
+    qkv = torch.randn(2, 300, 3, 2, 64, device="cuda").bfloat16()
+    q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
+    o, lse = C.attn_fwd(q, k, v, None, 0.125, False, 0.25, 77)
+    do = o.detach().clone()             # every term of <dO, O> positive: no cancellation, a relative bound of two roundings holds
+    dqkv = C.attn_bwd(q, k, v, o, do, lse, None, 0.125, False, 0.25, 77)
+    a, b = (do.double() * o.double()).sum().item(), (dqkv[:, :, 2].double() * v.double()).sum().item()
+    assert abs(a - b) < 2 ** -7 * abs(a), (a, b)
+
+
 def test_attention_dropout_statistics(C):
     torch.manual_seed(6)
     B, H, S, D = 2, 2, 128, 64
