@@ -179,6 +179,38 @@ def test_softmax_ce(C, dtype, rows, V, pad):
     assert cinv[0].item() == (tgt != -100).sum().item()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,V,offset", [(9, 1, 0), (33, 37, 0), (17, 2049, 1), (21, 4097, 3), (1000, 100, 0), (500, 30522, 0), (3, 50001, 1)])
+def test_softmax_ce_row_alignments(C, dtype, rows, V, offset):
+    """Contiguous rows of any length, i.e. of every alignment, starting off a 16-byte boundary too; some values -inf, as masks leave
+    them; the gradient in a buffer of its own and in place. One rounding of the gradient to its type (2^-8 for bf16), whose largest value is
+    1 / rows; sums in another order where the two buffers are aligned differently."""
+    torch.manual_seed(13)
+    flat = torch.randn(rows * V + offset, device="cuda").to(dtype) * 3
+    logits = flat[offset:].view(rows, V)
+    tgt = torch.randint(0, V, (rows,), device="cuda")
+    if V > 8:
+        logits[:, : V // 2] = float("-inf")
+        tgt = tgt % (V - V // 2) + V // 2
+    tgt[1::5] = -100
+    lr = logits.double().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(lr, tgt, ignore_index=-100)
+    ref.backward()
+    n = int((tgt != -100).sum())
+    tol = (2 ** -8 if dtype == torch.bfloat16 else 2 ** -20) / n
+    loss, dl, _ = C.softmax_ce(logits, tgt, -100, True, False)
+    assert abs(loss.item() - ref.item()) < 1e-5 * max(1.0, abs(ref.item()))
+    assert (dl.double() - lr.grad).abs().max().item() <= tol
+    scaled = dl.clone()
+    C.scale_rows(scaled, torch.ones(1, device="cuda"))
+    assert torch.equal(scaled, dl)
+    C.scale_rows(scaled, torch.full((1,), 0.3, device="cuda"))
+    assert (scaled.double() - 0.3 * dl.double()).abs().max().item() <= tol
+    loss2, dl2, _ = C.softmax_ce(logits, tgt, -100, True, True)
+    assert dl2.data_ptr() == logits.data_ptr() and (dl2.double() - lr.grad).abs().max().item() <= tol
+    assert abs(loss2.item() - ref.item()) < 1e-5 * max(1.0, abs(ref.item()))
+
+
 def test_adam_matches_reference(C):
     n = 100003
     torch.manual_seed(4)
