@@ -22,6 +22,9 @@ struct VecIO<float> {
   __device__ static void store(float* p, const float (&v)[4]) {
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
   }
+  __device__ static void unpack(const uint4& raw, float (&v)[4]) {
+    v[0] = __uint_as_float(raw.x); v[1] = __uint_as_float(raw.y); v[2] = __uint_as_float(raw.z); v[3] = __uint_as_float(raw.w);
+  }
   __device__ static float get(const float* p) { return *p; }
   __device__ static void put(float* p, float v) { *p = v; }
 };
@@ -30,7 +33,10 @@ template <>
 struct VecIO<__nv_bfloat16> {
   static constexpr int kVec = 8;
   __device__ static void load(const __nv_bfloat16* p, float (&v)[8]) {
-    uint4 raw = *reinterpret_cast<const uint4*>(p);
+    const uint4 raw = *reinterpret_cast<const uint4*>(p);      // one 16-byte load: through a reference it would become four
+    unpack(raw, v);
+  }
+  __device__ static void unpack(const uint4& raw, float (&v)[8]) {
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -82,6 +88,11 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
   float r = (lane < nwarps) ? scratch[lane] : -INFINITY;
   r = warp_max(r);
   return r;
+}
+
+// Four consecutive fp32 added to a 16-byte aligned address, without reading it back.
+__device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
 // Philox-4x32-10: 4 uniform 32-bit words per (key, counter).

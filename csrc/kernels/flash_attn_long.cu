@@ -85,10 +85,6 @@ struct BwdTiles {
   __device__ bool last() const { return it == n - 1; }
 };
 
-__device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
-  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
 // Per query row: D = dot(dO, O) into the first word of the row's dQ slot (overwritten by attn_dq_kernel at the end), and the
 // row's share of the dQ scratch zeroed. Eight lanes per row, rows of one (batch, head) consecutive.
 __global__ void __launch_bounds__(256) attn_bwd_pre_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
