@@ -88,6 +88,30 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& out, bool a_mn, bool b_mn, c
   check(rc, "fb_gemm_bf16");
 }
 
+// out[:, g * N : (g + 1) * N] = a b_g^T + bias_g: up to three [N, K] weights of one layout over one input.
+void gemm_grouped(const Tensor& a, const std::vector<Tensor>& bs, Tensor& out, const std::vector<Tensor>& biases) {
+  want_cuda(a, "a");
+  c10::cuda::CUDAGuard guard(a.device());
+  TORCH_CHECK(!bs.empty() && bs.size() <= 3 && (biases.empty() || biases.size() == bs.size()), "one to three products, a bias for each or for none");
+  TORCH_CHECK(is_bf16(a) && is_bf16(out) && a.dim() == 2 && out.dim() == 2 && a.stride(1) == 1 && out.stride(1) == 1, "bf16 [rows, cols] with unit inner stride");
+  const int64_t M = a.size(0), K = a.size(1), N = bs[0].size(0), G = static_cast<int64_t>(bs.size());
+  TORCH_CHECK(out.size(0) == M && out.size(1) == N * G, "output shape mismatch");
+  const void* b[3] = {};
+  const void* bias[3] = {};
+  for (int64_t g = 0; g < G; ++g) {
+    TORCH_CHECK(bs[g].is_cuda() && is_bf16(bs[g]) && bs[g].dim() == 2 && bs[g].size(0) == N && bs[g].size(1) == K && bs[g].stride(1) == 1 &&
+                bs[g].stride(0) == bs[0].stride(0), "weights must be bf16 [N, K] of one layout");
+    b[g] = bs[g].data_ptr();
+    if (biases.empty()) continue;
+    TORCH_CHECK(biases[g].is_cuda() && biases[g].numel() == N && biases[g].is_contiguous() && biases[g].scalar_type() == biases[0].scalar_type() &&
+                (is_bf16(biases[g]) || biases[g].scalar_type() == at::kFloat), "biases must be [N] of one type, fp32 or bf16");
+    bias[g] = biases[g].data_ptr();
+  }
+  check(fb_gemm_bf16_grouped(a.data_ptr(), b, out.data_ptr(), (int)M, (int)N, (int)K, (int)G, a.stride(0), bs[0].stride(0), out.stride(0), bias,
+                             !biases.empty() && biases[0].scalar_type() == at::kFloat, status_word(a.get_device()).data_ptr<int>(), stream_of(a)),
+        "fb_gemm_bf16_grouped");
+}
+
 int gemm_pick_config(int M, int N, int K, int split_k) { return fb_gemm_pick_config(M, N, K, split_k); }
 
 // Bounds-check record of the debug build (FLODL_BOUNDS_CHECK): one host-mapped int[4] = {site, index, limit, 0}.
@@ -134,16 +158,28 @@ std::vector<Tensor> layernorm_fwd(const Tensor& x, const OptTensor& residual, co
   const int64_t cols = x.size(-1);
   const int64_t rows = x.numel() / cols;
   if (residual.has_value()) TORCH_CHECK(residual->is_contiguous() && residual->scalar_type() == x.scalar_type() && residual->numel() == x.numel());
-  if (gamma.has_value()) want_f32(*gamma, "gamma");
-  if (beta.has_value()) want_f32(*beta, "beta");
+  // both parameters in bf16, or both in fp32
+  const Tensor* param = gamma.has_value() ? &*gamma : beta.has_value() ? &*beta : nullptr;
+  const bool p16 = param && is_bf16(*param);
+  for (const OptTensor* t : {&gamma, &beta}) {
+    if (!t->has_value()) continue;
+    if (!p16) {
+      want_f32(**t, "gamma / beta");
+      continue;
+    }
+    TORCH_CHECK((*t)->is_cuda() && is_bf16(**t) && (*t)->is_contiguous(), "gamma and beta must be of one type");
+  }
   Tensor y = torch::empty_like(x);
   Tensor pre = want_pre ? torch::empty_like(x) : Tensor();
   auto fopts = torch::dtype(torch::kFloat).device(x.device());
   Tensor mean = torch::empty({rows}, fopts), rstd = torch::empty({rows}, fopts);
-  int rc = fb_layernorm_fwd(x.data_ptr(), ptr<const void>(residual), ptr<const float>(gamma), ptr<const float>(beta),
-                            y.data_ptr(), want_pre ? pre.data_ptr() : nullptr, mean.data_ptr<float>(),
-                            rstd.data_ptr<float>(), (int)rows, (int)cols, (float)eps, (float)p_drop, seed, seed_ptr(seed_dev), is_bf16(x),
-                            stream_of(x));
+  void* pre_ptr = want_pre ? pre.data_ptr() : nullptr;
+  int rc = p16 ? fb_layernorm_fwd_p16(x.data_ptr(), ptr<const void>(residual), ptr<const void>(gamma), ptr<const void>(beta), y.data_ptr(), pre_ptr,
+                                      mean.data_ptr<float>(), rstd.data_ptr<float>(), (int)rows, (int)cols, (float)eps, (float)p_drop, seed, seed_ptr(seed_dev),
+                                      is_bf16(x), stream_of(x))
+               : fb_layernorm_fwd(x.data_ptr(), ptr<const void>(residual), ptr<const float>(gamma), ptr<const float>(beta), y.data_ptr(), pre_ptr,
+                                  mean.data_ptr<float>(), rstd.data_ptr<float>(), (int)rows, (int)cols, (float)eps, (float)p_drop, seed, seed_ptr(seed_dev),
+                                  is_bf16(x), stream_of(x));
   check(rc, "fb_layernorm_fwd");
   return {y, pre, mean, rstd};
 }
@@ -612,6 +648,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("bias") = py::none(), py::arg("epi") = 0, py::arg("aux") = py::none(), py::arg("alpha") = py::none(),
         py::arg("accumulate") = false, py::arg("split_k") = 1, py::arg("config") = -1, py::arg("ts") = py::none(),
         py::arg("m_dyn") = py::none(), py::arg("k_dyn") = py::none());
+  m.def("gemm_grouped", &gemm_grouped);
   m.def("gemm_pick_config", &gemm_pick_config);
   m.def("read_status", &read_status);
   m.def("bounds_check_build", &bounds_check_build);

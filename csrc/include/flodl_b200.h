@@ -75,6 +75,9 @@ int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, int N, int K,
                      void* aux, long long ldaux, const float* alpha, int accumulate, int split_k, int config,
                      int* status, long long* ts, const int* m_dyn, const int* k_dyn, void* stream);
 int fb_gemm_pick_config(int M, int N, int K, int split_k);
+/* C[:, g*N:(g+1)*N] = A B_g^T + bias_g for up to three K-major B's [N, K] of one leading dimension (QKV projections). */
+int fb_gemm_bf16_grouped(const void* A, const void* const* B, void* C, int M, int N, int K, int groups, long long lda, long long ldb, long long ldc,
+                         const void* const* bias, int bias_fp32, int* status, void* stream);
 
 /* ---- attention ----------------------------------------------------------------------------- */
 /* q,k,v,o,do,dq,dk,dv: bf16 [B, S, H, 64] with the given element strides for (batch, seq, head);
@@ -91,6 +94,10 @@ int fb_attn_bwd(const void* q, const void* k, const void* v, const void* o, cons
 
 /* ---- normalisation / activation / loss ----------------------------------------------------- */
 int fb_layernorm_fwd(const void* x, const void* residual, const float* gamma, const float* beta, void* y,
+                     void* pre_out, float* mean, float* rstd, int rows, int cols, float eps, float p_drop,
+                     unsigned long long seed, const unsigned long long* seed_dev, int is_bf16, void* stream);
+/* The same with bf16 gamma / beta. */
+int fb_layernorm_fwd_p16(const void* x, const void* residual, const void* gamma, const void* beta, void* y,
                      void* pre_out, float* mean, float* rstd, int rows, int cols, float eps, float p_drop,
                      unsigned long long seed, const unsigned long long* seed_dev, int is_bf16, void* stream);
 int fb_layernorm_bwd_grid(int rows);

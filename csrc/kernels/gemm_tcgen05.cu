@@ -46,6 +46,12 @@
 
 namespace fb {
 
+// gemm_small.cu
+int gemm_small_split(int M, int N, int K);
+bool gemm_small_aligned(int N, const void* C, long long ldc, const void* aux, long long ldaux);
+int gemm_small(const void* A, const void* const* B, void* C, int M, int group, int groups, int K, long long lda, long long ldb, long long ldc, int b_mn,
+               const void* const* bias, int bias_fp32, int epi, void* aux, long long ldaux, const float* alpha, int split, int* status, cudaStream_t stream);
+
 constexpr int BM = 128;  // rows of the tile held by ONE CTA
 constexpr int BK = 64;   // K per stage = one 128-byte swizzle row of bf16
 constexpr int kEpiWarps = 8;
@@ -865,6 +871,10 @@ extern "C" int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, in
   if (split_k > 1 && !c_fp32) return -2;
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
   if (config < 0) {
+    // few output tiles, plain bf16 result: the cluster split (gemm_small.cu)
+    if (!c_fp32 && !a_mn && !accumulate && split_k == 1 && !m_dyn && !k_dyn && !ts && gemm_small_aligned(N, C, ldc, aux, ldaux))
+      if (const int split = gemm_small_split(M, N, K))
+        return gemm_small(A, &B, C, M, N, 1, K, lda, ldb, ldc, b_mn, &bias, bias_fp32, epi, aux, ldaux, alpha, split, status, stream);
     config = fb_gemm_pick_config(M, N, K, split_k);
     if (config == 5 && b_mn) config = 0;          // 256x192 pair tiles need a K-major B
   }
@@ -917,4 +927,26 @@ extern "C" int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, in
     case 5: return launch_gemm<2, 192>(ta, tb, tc, tx, p, stream);
     default: return launch_gemm<1, 64>(ta, tb, tc, tx, p, stream);
   }
+}
+
+// C[:, g * N : (g + 1) * N] = A B_g^T + bias_g for `groups` (at most three) K-major B's of one shape and leading dimension: one launch where
+// the products are small together, else one after the other. bias: null, or an array with an entry (null or [N]) per product.
+extern "C" int fb_gemm_bf16_grouped(const void* A, const void* const* B, void* C, int M, int N, int K, int groups, long long lda, long long ldb, long long ldc,
+                                    const void* const* bias, int bias_fp32, int* status, void* stream_) {
+  using namespace fb;
+  if (M <= 0 || N <= 0 || K <= 0 || groups <= 0) return 0;
+  if (groups > 3) return -2;
+  const void* none[3] = {nullptr, nullptr, nullptr};
+  if (!bias) bias = none;
+  bool aligned = lda % 8 == 0 && ldb % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && N % 64 == 0 && gemm_small_aligned(N, C, ldc, nullptr, 0);
+  for (int g = 0; g < groups; ++g) aligned = aligned && (reinterpret_cast<uintptr_t>(B[g]) & 15) == 0;
+  const int split = aligned ? gemm_small_split(M, N * groups, K) : 0;
+  if (split)
+    return gemm_small(A, B, C, M, N, groups, K, lda, ldb, ldc, 0, bias, bias_fp32, FB_EPI_NONE, nullptr, 0, nullptr, split, status, static_cast<cudaStream_t>(stream_));
+  for (int g = 0; g < groups; ++g) {
+    const int r = fb_gemm_bf16(A, B[g], static_cast<__nv_bfloat16*>(C) + static_cast<long long>(g) * N, M, N, K, lda, ldb, ldc, 0, 0, 0, bias[g], bias_fp32, FB_EPI_NONE,
+                               nullptr, 0, nullptr, 0, 1, -1, status, stream_);
+    if (r) return r;
+  }
+  return 0;
 }

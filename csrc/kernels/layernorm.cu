@@ -39,10 +39,32 @@ __device__ __forceinline__ void load_f32_vec(const float* __restrict__ p, int of
   }
 }
 
-template <typename T, int VPL>
+// The same for bf16 parameters (a model cast to bf16 for inference): one conversion here instead of a cast launch per parameter.
+template <int N>
+__device__ __forceinline__ void load_f32_vec(const __nv_bfloat16* __restrict__ p, int off, float fill, float (&out)[N]) {
+  static_assert(N == 4 || N == 8, "");
+  if (!p) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) out[j] = fill;
+  } else if ((reinterpret_cast<uintptr_t>(p) & (2 * N - 1)) == 0) {
+    if constexpr (N == 8) {
+      const uint4 q = __ldg(reinterpret_cast<const uint4*>(p + off));
+      VecIO<__nv_bfloat16>::unpack(q, out);
+    } else {
+      const uint2 q = __ldg(reinterpret_cast<const uint2*>(p + off));
+      const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.y));
+      out[0] = a.x; out[1] = a.y; out[2] = b.x; out[3] = b.y;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; ++j) out[j] = __bfloat162float(p[off + j]);
+  }
+}
+
+template <typename T, int VPL, typename P>
 __global__ void __launch_bounds__(kLnWarps * 32)
-ln_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const float* __restrict__ gamma,
-              const float* __restrict__ beta, T* __restrict__ y, T* __restrict__ pre_out,
+ln_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const P* __restrict__ gamma,
+              const P* __restrict__ beta, T* __restrict__ y, T* __restrict__ pre_out,
               float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols, float eps,
               float p_drop, uint64_t seed_in, const unsigned long long* __restrict__ seed_dev) {
   pdl_entry();
@@ -266,12 +288,12 @@ ln_bwd_finalize_kernel(const float* __restrict__ partial, float* __restrict__ dg
   }
 }
 
-template <typename T, int VPL>
-static int ln_fwd_launch(const void* x, const void* res, const float* gamma, const float* beta, void* y,
+template <typename T, int VPL, typename P>
+static int ln_fwd_launch(const void* x, const void* res, const P* gamma, const P* beta, void* y,
                          void* pre, float* mean, float* rstd, int rows, int cols, float eps, float p,
                          uint64_t seed, const unsigned long long* seed_dev, cudaStream_t st) {
   const int grid = (rows + kLnWarps - 1) / kLnWarps;
-  launch_pdl(ln_fwd_kernel<T, VPL>, dim3(grid), dim3(kLnWarps * 32), 0, st, static_cast<const T*>(x), static_cast<const T*>(res), gamma, beta, static_cast<T*>(y),
+  launch_pdl(ln_fwd_kernel<T, VPL, P>, dim3(grid), dim3(kLnWarps * 32), 0, st, static_cast<const T*>(x), static_cast<const T*>(res), gamma, beta, static_cast<T*>(y),
       static_cast<T*>(pre), mean, rstd, rows, cols, eps, p, seed, seed_dev);
   return static_cast<int>(cudaGetLastError());
 }
@@ -287,40 +309,57 @@ static int ln_bwd_launch(const void* dy, const void* pre, const float* mean, con
 
 }  // namespace fb
 
-#define FB_LN_DISPATCH(FN, ...)                                                     \
+// FN<T, VPL> or FN<T, VPL, P> for the row's type and length; PARAM is FB_LN_PARAM(P) or empty.
+#define FB_LN_DISPATCH(FN, PARAM, ...)                                              \
   do {                                                                              \
     const int vec = is_bf16 ? 8 : 4;                                                \
     const int vpl = (cols / vec + 31) / 32;                                         \
     if (is_bf16) {                                                                  \
       switch (vpl) {                                                                \
-        case 1: return fb::FN<__nv_bfloat16, 1>(__VA_ARGS__);                       \
-        case 2: return fb::FN<__nv_bfloat16, 2>(__VA_ARGS__);                       \
-        case 3: return fb::FN<__nv_bfloat16, 3>(__VA_ARGS__);                       \
-        case 4: return fb::FN<__nv_bfloat16, 4>(__VA_ARGS__);                       \
+        case 1: return fb::FN<__nv_bfloat16, 1 PARAM>(__VA_ARGS__);                 \
+        case 2: return fb::FN<__nv_bfloat16, 2 PARAM>(__VA_ARGS__);                 \
+        case 3: return fb::FN<__nv_bfloat16, 3 PARAM>(__VA_ARGS__);                 \
+        case 4: return fb::FN<__nv_bfloat16, 4 PARAM>(__VA_ARGS__);                 \
         default: return -4;                                                         \
       }                                                                             \
     } else {                                                                        \
       switch (vpl) {                                                                \
-        case 1: return fb::FN<float, 1>(__VA_ARGS__);                               \
-        case 2: return fb::FN<float, 2>(__VA_ARGS__);                               \
-        case 3: return fb::FN<float, 3>(__VA_ARGS__);                               \
-        case 4: return fb::FN<float, 4>(__VA_ARGS__);                               \
-        case 5: case 6: return fb::FN<float, 6>(__VA_ARGS__);                       \
-        case 7: case 8: return fb::FN<float, 8>(__VA_ARGS__);                       \
+        case 1: return fb::FN<float, 1 PARAM>(__VA_ARGS__);                         \
+        case 2: return fb::FN<float, 2 PARAM>(__VA_ARGS__);                         \
+        case 3: return fb::FN<float, 3 PARAM>(__VA_ARGS__);                         \
+        case 4: return fb::FN<float, 4 PARAM>(__VA_ARGS__);                         \
+        case 5: case 6: return fb::FN<float, 6 PARAM>(__VA_ARGS__);                 \
+        case 7: case 8: return fb::FN<float, 8 PARAM>(__VA_ARGS__);                 \
         default: return -4;                                                         \
       }                                                                             \
     }                                                                               \
   } while (0)
+#define FB_LN_PARAM(P) , P
 
 extern "C" int fb_layernorm_max_cols(int is_bf16) { return 1024; }
+
+namespace {
+template <typename P>
+int layernorm_fwd(const void* x, const void* residual, const P* gamma, const P* beta, void* y, void* pre_out, float* mean, float* rstd, int rows, int cols,
+                  float eps, float p_drop, unsigned long long seed, const unsigned long long* seed_dev, int is_bf16, void* stream) {
+  if (rows <= 0) return 0;
+  if (cols % (is_bf16 ? 8 : 4) || cols > 1024) return -4;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  FB_LN_DISPATCH(ln_fwd_launch, FB_LN_PARAM(P), x, residual, gamma, beta, y, pre_out, mean, rstd, rows, cols, eps, p_drop, seed, seed_dev, st);
+}
+}  // namespace
 
 extern "C" int fb_layernorm_fwd(const void* x, const void* residual, const float* gamma, const float* beta,
                                 void* y, void* pre_out, float* mean, float* rstd, int rows, int cols,
                                 float eps, float p_drop, unsigned long long seed, const unsigned long long* seed_dev, int is_bf16, void* stream) {
-  if (rows <= 0) return 0;
-  if (cols % (is_bf16 ? 8 : 4) || cols > 1024) return -4;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  FB_LN_DISPATCH(ln_fwd_launch, x, residual, gamma, beta, y, pre_out, mean, rstd, rows, cols, eps, p_drop, seed, seed_dev, st);
+  return layernorm_fwd(x, residual, gamma, beta, y, pre_out, mean, rstd, rows, cols, eps, p_drop, seed, seed_dev, is_bf16, stream);
+}
+
+extern "C" int fb_layernorm_fwd_p16(const void* x, const void* residual, const void* gamma, const void* beta,
+                                    void* y, void* pre_out, float* mean, float* rstd, int rows, int cols,
+                                    float eps, float p_drop, unsigned long long seed, const unsigned long long* seed_dev, int is_bf16, void* stream) {
+  return layernorm_fwd(x, residual, static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), y, pre_out, mean, rstd, rows, cols, eps,
+                       p_drop, seed, seed_dev, is_bf16, stream);
 }
 
 // One resident wave: the backward kernel keeps its dgamma / dbeta partial sums in registers (about
@@ -347,7 +386,7 @@ extern "C" int fb_layernorm_bwd(const void* dy, const void* pre, const float* me
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int grid = fb_layernorm_bwd_grid(rows);
   auto run = [&]() -> int {
-    FB_LN_DISPATCH(ln_bwd_launch, dy, pre, mean, rstd, gamma, dpre, dx_drop, partial, grid, rows, cols, p_drop, seed, seed_dev, st);
+    FB_LN_DISPATCH(ln_bwd_launch, , dy, pre, mean, rstd, gamma, dpre, dx_drop, partial, grid, rows, cols, p_drop, seed, seed_dev, st);
   };
   int r = run();
   if (r) return r;

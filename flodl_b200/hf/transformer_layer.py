@@ -129,8 +129,7 @@ class TransformerLayer(Module):
             fw, fb = self._fused
             if fb is not None:
                 return _ops.linear(x, fw, fb).view(B, S, 3, Hn, D)
-        q, k, v = (_ops.linear(x, w, b).view(B, S, Hn, D) for w, b in zip(ws, bs))
-        return torch.stack((q, k, v), dim=2)
+        return _ops.packed_linear(x, ws, bs).view(B, S, 3, Hn, D)
 
     def forward_impl(self, x: Variable, attention_mask: Optional[Variable]) -> Variable:
         c = self.cfg

@@ -59,7 +59,7 @@ class DecoderBlock(Module):
                 self._fused = (fw, fb) if fw is not None and fb is not None else (ws[0], None)
             if self._fused[1] is not None:
                 return _ops.linear(h, self._fused[0], self._fused[1]).view(B, S, 3, H, D)
-        return torch.stack([_ops.linear(h, w, b).view(B, S, H, D) for w, b in zip(ws, bs)], dim=2)
+        return _ops.packed_linear(h, ws, bs).view(B, S, 3, H, D)
 
     def forward_pair(self, delta, stream):
         """`delta` is the previous sub-layer output not yet added to the residual `stream` (or None)."""

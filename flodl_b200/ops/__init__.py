@@ -25,6 +25,7 @@ from .core import (  # noqa: F401
     linear_cross_entropy,
     native_enabled,
     next_seed,
+    packed_linear,
     seed_state,
     set_native,
 )

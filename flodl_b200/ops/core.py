@@ -136,6 +136,14 @@ def _native_ok(x: torch.Tensor) -> bool:
     return n <= 0 or x.numel() >= n or torch.cuda.is_current_stream_capturing()
 
 
+def _plain_call(*tensors) -> bool:
+    """Whether nothing follows the call: no gradient is recorded, in either mode, and no transform or trace looks on. The kernels may
+    then be launched without an autograd function around them, and need not save what only a backward pass would read."""
+    if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors):
+        return False
+    return torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None and not torch.jit.is_tracing()
+
+
 def _round_up(n: int, m: int) -> int:
     return (n + m - 1) // m * m
 
@@ -338,6 +346,16 @@ class _LinearFn(torch.autograd.Function):
         return dx, dw, db, None
 
 
+def _project(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], act: Optional[str]) -> torch.Tensor:
+    """act(x W^T + b) alone: the pre-activation stays in the epilogue's registers."""
+    N, K = w.shape
+    x2 = _as_operand(x.reshape(-1, K))
+    out = _new_rows(x2.shape[0], N, BF16, x.device)
+    _C().gemm(x2, _as_operand(_shadow(w)), out, False, False, bias=None if b is None else b.detach(), epi=_EPI[act])
+    _launched()
+    return out.view(*x.shape[:-1], N)
+
+
 def _gemm_eligible(x: torch.Tensor, w: torch.Tensor) -> bool:
     if not _native_ok(x) or w.dim() != 2:
         return False
@@ -352,6 +370,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if _gemm_eligible(x, weight):
         if x.dtype != BF16:
             x = x.to(BF16)
+        if _plain_call(x, weight, bias):
+            return _project(x, weight, bias, activation)
         return _LinearFn.apply(x, weight, bias, activation)
     w = weight if weight.dtype == x.dtype else weight.to(x.dtype)
     b = bias if bias is None or bias.dtype == x.dtype else bias.to(x.dtype)
@@ -361,6 +381,26 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     elif activation == "gelu_tanh":
         y = F.gelu(y, approximate="tanh")
     return y
+
+
+def packed_linear(x: torch.Tensor, weights, biases) -> torch.Tensor:
+    """`[..., G, N]`: up to three projections of one input side by side, as attention takes them. Without autograd the GEMMs write
+    straight into the packed tensor (one launch where they are small); else `stack` of `linear`s."""
+    same = len({(w.shape, w.dtype) for w in weights}) == 1 and len({(None if b is None else b.dtype) for b in biases}) == 1
+    if not same or len(weights) > 3 or weights[0].dim() != 2 or not _gemm_eligible(x, weights[0]) or not _plain_call(x, *weights, *biases):
+        return torch.stack([linear(x, w, b) for w, b in zip(weights, biases)], dim=-2)
+    N, K = weights[0].shape
+    ws = [_as_operand(_shadow(w)) for w in weights]
+    bs = [] if biases[0] is None else [b.detach().contiguous() if b.dtype in (BF16, torch.float32) else b.detach().float() for b in biases]
+    if len({w.stride() for w in ws}) != 1 or N % 8:
+        return torch.stack([linear(x, w, b) for w, b in zip(weights, biases)], dim=-2)
+    if x.dtype != BF16:
+        x = x.to(BF16)
+    x2 = _as_operand(x.reshape(-1, K))
+    out = torch.empty(x2.shape[0], len(ws) * N, dtype=BF16, device=x.device)
+    _C().gemm_grouped(x2, ws, out, bs)
+    _launched()
+    return out.view(*x.shape[:-1], len(ws), N)
 
 
 # ------------------------------------------------------------------------------------ feed-forward
@@ -419,11 +459,21 @@ def feed_forward(x, w1, b1, w2, b2, activation: str = "gelu"):
     if _gemm_eligible(x, w1) and w1.shape[0] % 8 == 0:
         if x.dtype != BF16:
             x = x.to(BF16)
+        if _plain_call(x, w1, b1, w2, b2):
+            return _project(_project(x, w1, b1, activation), w2, b2, None)
         return _FeedForwardFn.apply(x, w1, b1, w2, b2, activation)
     return linear(linear(x, w1, b1, activation), w2, b2)
 
 
 # -------------------------------------------------------------------------------------- LayerNorm
+def _norm_params(gamma, beta):
+    """Gain and shift as the kernel takes them: both bf16 as they are, otherwise both fp32."""
+    given = [t for t in (gamma, beta) if t is not None]
+    if given and all(t.dtype == BF16 and t.is_contiguous() for t in given):
+        return (None if gamma is None else gamma.detach()), (None if beta is None else beta.detach())
+    return _f32(gamma), _f32(beta)
+
+
 class _LayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, residual, gamma, beta, eps, p_drop, seed):
@@ -432,7 +482,7 @@ class _LayerNormFn(torch.autograd.Function):
         rc = None if residual is None else residual.contiguous()
         want_pre = rc is not None or p_drop > 0.0
         sd = seed_state(x.device) if p_drop > 0.0 else None
-        y, pre, mean, rstd = C.layernorm_fwd(xc, rc, _f32(gamma), _f32(beta), eps, p_drop, seed, want_pre, sd)
+        y, pre, mean, rstd = C.layernorm_fwd(xc, rc, *_norm_params(gamma, beta), eps, p_drop, seed, want_pre, sd)
         _launched()
         ctx.set_materialize_grads(False)
         ctx.save_for_backward(pre if want_pre else xc, mean, rstd)
@@ -491,6 +541,12 @@ def layer_norm(x, gamma=None, beta=None, eps: float = 1e-5, residual=None, p_dro
     Counterpart of `autograd::layer_norm` (flodl/src/autograd/ops.rs:625-637)."""
     p = p_drop if training else 0.0
     if _ln_eligible(x) and (residual is None or residual.dtype == x.dtype):
+        if not return_pre and _plain_call(x, gamma, beta, residual):      # the pre-normalisation sum is not written out
+            sd = seed_state(x.device) if p > 0 else None
+            y = _C().layernorm_fwd(x.contiguous(), None if residual is None else residual.contiguous(), *_norm_params(gamma, beta), float(eps), float(p),
+                                   next_seed() if p > 0 else 0, False, sd)[0]
+            _launched()
+            return y
         y, pre = _LayerNormFn.apply(x, residual, gamma, beta, float(eps), float(p), next_seed() if p > 0 else 0)
         if pre.numel() == 0 and x.numel() != 0:
             pre = x

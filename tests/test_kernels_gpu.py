@@ -104,6 +104,38 @@ def test_gemm_fp32_out_accumulate_splitk_alpha(C):
     assert (out3 - 0.25 * ref).abs().max().item() < 0.02 * ref.abs().max().item()
 
 
+@pytest.mark.parametrize("M,N,K,b_mn,epi", [(1, 768, 768, False, 0), (77, 768, 3072, False, 0), (77, 3072, 768, False, 1), (128, 64, 64, True, 0), (129, 68, 72, False, 3),
+                                            (300, 128, 520, True, 2), (512, 512, 128, True, 4), (130, 60, 4096, False, 0)])
+def test_gemm_few_tiles(C, M, N, K, b_mn, epi):
+    """Products of few output tiles, which the dispatch gives to the kernel that splits K over a cluster: edges of tiles and of the split, both
+    layouts of B, every epilogue, strided output. Against 64 bits: the output carries one rounding to bf16 (2^-8 at most), GELU' is taken of a
+    stored, rounded value, the fast GELU adds 6e-5 absolute; in norm all of it stays below one such rounding."""
+    torch.manual_seed(15)
+    a = torch.randn(M, K + 8, device="cuda").bfloat16()[:, :K]
+    b = (torch.randn(N, K, device="cuda") / math.sqrt(K)).bfloat16()
+    bm = b.t().contiguous() if b_mn else b
+    bias = torch.randn(N, device="cuda") if epi in (0, 1, 3) else None
+    out = torch.zeros(M, N + 4, device="cuda").bfloat16()
+    aux = torch.randn(M, N, device="cuda").bfloat16()
+    alpha = torch.tensor([0.5], device="cuda") if epi == 0 else None
+    C.clear_status(0)
+    C.gemm(a, bm, out[:, :N], False, b_mn, bias=bias, epi=epi, aux=aux if epi else None, alpha=alpha)
+    torch.cuda.synchronize()
+    assert C.read_status(0) == 0
+    pre = a.double() @ b.double().t() * (0.5 if epi == 0 else 1.0) + (0 if bias is None else bias.double())
+    gelu = lambda x: torch.nn.functional.gelu(x, approximate="tanh" if epi > 2 else "none")
+    if epi in (0, 1, 3):
+        ref = pre if epi == 0 else gelu(pre)
+        if epi:
+            assert ((aux.double() - pre).norm() / pre.norm()).item() < 2 ** -8
+    else:
+        x = aux.double().requires_grad_(True)
+        gelu(x).backward(pre)
+        ref = x.grad
+    assert ((out[:, :N].double() - ref).norm() / ref.norm()).item() < 2 ** -8
+    assert torch.all(out[:, N:] == 0)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("cols", [768, 512, 16 * 8, 1024])
 def test_layernorm_fwd_bwd(C, dtype, cols):
@@ -656,3 +688,39 @@ def test_bounds_checked_debug_build_records_instead_of_faulting():
     env = dict(os.environ, FLODL_B200_BOUNDS_CHECK="1")
     res = subprocess.run([sys.executable, os.path.join(here, "_bounds_worker.py")], capture_output=True, text=True, timeout=900, env=env)
     assert res.returncode == 0 and "BOUNDS_OK" in res.stdout, res.stdout[-2000:] + res.stderr[-3000:]
+
+
+@pytest.mark.parametrize("rows,N,K,bias,dtype,order", [(77, 128, 256, "bf16", "bf16", "rows"), (1, 64, 64, None, "bf16", "rows"), (1500, 192, 128, "fp32", "fp32", "rows"),
+                                                      (200, 72, 40, "bf16", "bf16", "columns"), (130, 128, 64, "fp32", "bf16", "strided")])
+def test_packed_linear_without_gradients(C, rows, N, K, bias, dtype, order):
+    """The grouped projections against the general path (one `linear` each under autograd, stacked), over sizes that take one launch and sizes
+    that take three, input orders, and types. The same products in another order of summation: one rounding to bf16 apart."""
+    from flodl_b200 import nn, ops
+    from flodl_b200.ops import core
+    torch.manual_seed(16)
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    x = torch.randn(rows, K, device="cuda").to(dt)
+    if order == "columns":
+        x = x.t().contiguous().t()
+    elif order == "strided":
+        x = torch.cat((x, x), 1)[:, K:]
+    ws = [(torch.randn(N, K, device="cuda") / math.sqrt(K)).to(dt).requires_grad_() for _ in range(3)]
+    bt = {"bf16": torch.bfloat16, "fp32": torch.float32}.get(bias)
+    bs = [None if bias is None else torch.randn(N, device="cuda").to(bt).requires_grad_() for _ in range(3)]
+    was = core.eager_min_numel()
+    core.set_eager_min_numel(0)
+    try:
+        with nn.AutocastGuard(torch.bfloat16):
+            want = ops.packed_linear(x, ws, bs)
+            with torch.no_grad():
+                got = ops.packed_linear(x, ws, bs)
+                ffn = ops.feed_forward(x, ws[0], bs[0], torch.eye(N, device="cuda").to(dt), None)
+                norm = ops.layer_norm(got[:, 0], torch.ones(N, device="cuda").to(dt), torch.zeros(N, device="cuda").to(dt), residual=got[:, 1])
+            ref = ops.layer_norm(want[:, 0], torch.ones(N, device="cuda"), torch.zeros(N, device="cuda"), residual=want[:, 1])
+    finally:
+        core.set_eager_min_numel(was)
+    assert want.requires_grad and not got.requires_grad and got.shape == want.shape == (rows, 3, N) and got.dtype == want.dtype
+    close = lambda a, b, u: ((a.double() - b.double()).norm() / b.double().norm()).item() < u
+    assert close(got, want, 2 ** -8) and close(norm, ref, 2 ** -7)
+    act = torch.nn.functional.gelu(want[:, 0].detach().double())
+    assert close(ffn, act, 2 ** -7)

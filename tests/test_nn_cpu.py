@@ -352,3 +352,20 @@ def test_no_grad_context():
     with no_grad():
         y = x.mul_scalar(2.0)
     assert not y.t.requires_grad
+
+
+def test_plain_call_sees_every_onlooker():
+    """The kernels are called without an autograd function around them only where nothing would miss it."""
+    from flodl_b200.ops.core import _plain_call
+    import torch.autograd.forward_ad as fwad
+    a, w = torch.ones(2, 2), torch.ones(2, 2, requires_grad=True)
+    assert _plain_call(a) and _plain_call(a, None) and not _plain_call(a, w)
+    with torch.no_grad():
+        assert _plain_call(a, w)
+        seen = []
+        torch.func.vmap(lambda t: (seen.append(_plain_call(t)), t)[1])(a)
+        torch.func.grad(lambda t: (seen.append(_plain_call(t)), t.sum())[1])(a)
+        with fwad.dual_level():
+            seen.append(_plain_call(fwad.make_dual(a, a)))
+        torch.jit.trace(lambda t: (seen.append(_plain_call(t)), t * 2)[1], (a,), check_trace=False)
+        assert seen == [False] * 4
