@@ -162,6 +162,31 @@ def test_layernorm_fwd_bwd(C, dtype, cols):
     assert (db - br.grad).abs().max().item() < 1e-2 * max(1.0, br.grad.abs().max().item())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,cols", [(1, 256), (3, 264), (5000, 768), (4099, 1016), (20001, 320)])
+def test_layernorm_rows_per_warp(C, dtype, rows, cols):
+    """From fewer rows than warps to several rows per warp, columns that leave lanes idle; parameter gradients written and accumulated.
+    Element-wise results carry one rounding to their type (2^-8 for bf16); the parameter gradients are 32-bit sums over the stored `pre`."""
+    torch.manual_seed(14)
+    x, r, dy = (torch.randn(rows, cols, device="cuda").to(dtype) for _ in range(3))
+    g, b = torch.randn(cols, device="cuda"), torch.randn(cols, device="cuda")
+    y, pre, mean, rstd = C.layernorm_fwd(x, r, g, b, 1e-5, 0.0, 0, True)
+    leaves = [pre.double().requires_grad_(True), g.double().requires_grad_(True), b.double().requires_grad_(True)]
+    ref = torch.nn.functional.layer_norm(leaves[0], (cols,), leaves[1], leaves[2], 1e-5)
+    ref.backward(dy.double())
+    unit = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -18
+    close = lambda got, want, u: ((got.double() - want).norm() / want.norm().clamp_min(1e-30)).item() < u
+    # y, mean and rstd are made from the unrounded sum, the reference from the stored one: another rounding
+    assert close(y, ref.detach(), 2 * unit)
+    dpre, _, dg, db = C.layernorm_bwd(dy, pre, mean, rstd, g, 0.0, 0, False, True, None, None)
+    acc_g, acc_b = torch.ones(cols + 1, device="cuda")[1:], torch.ones(cols, device="cuda")      # one off a 16-byte boundary
+    dpre2, _, _, _ = C.layernorm_bwd(dy, pre, mean, rstd, g, 0.0, 0, False, True, acc_g, acc_b)
+    assert torch.equal(dpre, dpre2) and close(dpre, leaves[0].grad, 2 * unit)
+    assert close(dg, leaves[1].grad, 2 * unit)
+    assert close(db, leaves[2].grad, 2 ** -18)
+    assert close(acc_g - 1, dg.double(), 2 ** -14) and close(acc_b - 1, db.double(), 2 ** -14)
+
+
 def test_layernorm_dropout_mask_consistent(C):
     rows, cols, p = 512, 768, 0.1
     x = torch.ones(rows, cols, device="cuda", dtype=torch.bfloat16)
