@@ -76,7 +76,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (threadIdx.x == 0) {
     mbar_init(in_full, 1);
     mbar_init(s_full, 1);
-    mbar_init(p_ready, 128);
+    mbar_init(p_ready, 4);
     mbar_init(o_full, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -197,7 +197,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_before_sync();
       fence_proxy_async_smem();
       if (t == 0) FB_ATTN_TS(4);
-      mbar_arrive(p_ready);
+      arrive_warp(p_ready, lane);
       ok = __all_sync(0xffffffffu, mbar_wait(o_full, 0, abort_flag, p.status, kStatusWaitAccum));   // warp-uniform: the staged stores below use __syncwarp
       if (ok) {
         tc_fence_after_sync();
@@ -280,7 +280,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(kv_full, 1);
     mbar_init(q_full, 1);
     mbar_init(sdp_full, 1);
-    mbar_init(pds_ready, 128);
+    mbar_init(pds_ready, 4);
     mbar_init(grads_full, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -411,7 +411,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_before_sync();
       fence_proxy_async_smem();
       if (t == 0) FB_ATTN_TS(11);
-      mbar_arrive(pds_ready);
+      arrive_warp(pds_ready, lane);
       ok = __all_sync(0xffffffffu, mbar_wait(grads_full, 0, abort_flag, p.status, kStatusWaitAccum));   // warp-uniform: staged stores below
     }
     if (ok) {

@@ -53,6 +53,13 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const void* tmap, ui
       : "memory");
 }
 
+// One arrival for a warp whose lanes are all done. (An arrival is an atomic on the barrier's word; the tensor cores read their
+// operands through the same shared-memory pipe.)
+__device__ __forceinline__ void arrive_warp(uint64_t* bar, int lane) {
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bar);
+}
+
 // Address of the 16-byte chunk holding columns [8*chunk, 8*chunk+8) of `row` in a [128][64] bf16
 // tile stored with the 128-byte swizzle (tile base 1024-byte aligned).
 __device__ __forceinline__ uint32_t swz_chunk(uint32_t tile_base, int row, int chunk) {

@@ -2,15 +2,19 @@
 // key block are in flash_attn.cu.
 //
 // Backward: one CTA per (key block of 128 rows, head, batch) walks the query blocks that see it. K, V and the dK / dV
-// accumulators stay put; Q and dO stream through a three-stage TMA ring. Roles: 8 softmax warps (thread = one query row x
-// 64 keys), 4 warps that drain dQ, one MMA issuer, one TMA producer. S and dP of the next query block are issued as soon
+// accumulators stay put; Q and dO stream through a three-stage TMA ring. Roles: 16 softmax warps (thread = one query row x
+// 32 keys), 4 warps that drain dQ, one MMA issuer, one TMA producer. S and dP of the next query block are issued as soon
 // as the softmax warps have loaded this block's into registers, so the tensor cores work under the exponentials.
-// A query block's dQ is a sum over key blocks, i.e. over CTAs: it is added into an fp32 scratch with 16-byte vector
-// reductions. The scratch is not row-major: within the 32 rows a warp owns, 16-byte chunk c of row r sits at
-// (c * rows + r) * 16, so the 32 lanes of a reduction (one row each) hit 512 contiguous bytes. A pass before zeroes the
-// scratch and leaves D = rowsum(dO * O) in the first word of each dQ row; a pass after turns the scratch into bf16 rows.
-// What bounds it: shared-memory bandwidth (P and dS are written once and read by three products) about level with the
-// exponentials. One CTA per (head, batch) walking all key blocks in turn, which this replaces, left most of the chip idle.
+// A query block's dQ is a sum over key blocks, i.e. over CTAs: it is added into an fp32 scratch with bulk reductions. The
+// scratch is not row-major: within the 32 rows a warp owns, 16-byte chunk c of row r sits at (c * rows + r) * 16, so that
+// the 32 lanes (one row each) write the staging area, which is copied as it is, without bank conflicts. A pass before zeroes
+// the scratch and leaves D = rowsum(dO * O) in the first word of each dQ row; a pass after turns the scratch into bf16 rows.
+// What bounds it: the chain scores -> exponentials -> P and dS in shared memory -> products of one tile, with the shared-memory
+// pipe (P and dS are written once and read by three products) as its slowest part.
+// Forward + backward, bf16, us: B 2 x H 12 x S 4096 causal 96 + 253 (118 + 338 with eight softmax warps, reductions from registers and
+// persistent CTAs), B 4 x H 8 x S 1024 causal 19 + 38 (24 + 47), B 6 x H 12 x S 509 causal 13 + 39 (15 + 43), B 32 x H 8 x S 256 causal
+// 14 + 48 (16 + 49), B 64 x H 12 x S 384 75 + 264 (89 + 257: with three tiles to a CTA its start and end show, which the persistent
+// form hid; longer rows gain more than these lose).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -25,24 +29,24 @@ namespace fb {
 namespace {
 
 constexpr int kSMs = 148;
-constexpr int kBwdSoftmaxWarps = 8;
+constexpr int kBwdStages = 3;
+constexpr int kBwdSoftmaxWarps = 16;
 constexpr int kBwdThreads = 32 * (kBwdSoftmaxWarps + 4 + 2);
 
-// Every byte of it is needed (226.75 KB), so there is no slack for alignment: the kernel relies on the 1024-byte alignment of the
-// dynamic shared-memory window and reports instead of computing if that does not hold.
 struct BwdLong {
-  static constexpr int Q = 0;                                   // 2 x 16 KB
-  static constexpr int DO = Q + 2 * 16384;                      // 2 x 16 KB
-  static constexpr int K = DO + 2 * 16384;
+  static constexpr int Q = 0;                                   // kBwdStages x 16 KB
+  static constexpr int DO = Q + kBwdStages * 16384;             // kBwdStages x 16 KB
+  static constexpr int K = DO + kBwdStages * 16384;
   static constexpr int V = K + 16384;
-  static constexpr int P = V + 16384;                           // 2 x (2 panels of 16 KB)
-  static constexpr int DS = P + 2 * 32768;                      // 2 x (2 panels of 16 KB)
-  static constexpr int STATS = DS + 2 * 32768;                  // 2 x 128 x {lse, D}
+  static constexpr int P = V + 16384;                           // 2 panels of 16 KB
+  static constexpr int DS = P + 2 * 16384;                      // 2 panels of 16 KB
+  static constexpr int DQ = DS + 2 * 16384;                     // 4 warps x 4 KB: dQ on its way out
+  static constexpr int STATS = DQ + 4 * 4096;                   // 2 x 128 x {lse, D}
   static constexpr int MASK = STATS + 2 * 128 * 8;              // 128 floats
   static constexpr int BARS = MASK + 512;
-  static constexpr int TOTAL = BARS + 192;
+  static constexpr int TOTAL = BARS + 256;
 };
-static_assert(BwdLong::TOTAL <= 227 * 1024, "shared memory budget");
+static_assert(BwdLong::TOTAL + 1024 <= 227 * 1024, "shared memory budget");
 
 // CTA index -> (block, head, batch). Causal: every block of equal length before the next shorter one (the longest first, so
 // the last wave is short). Otherwise all blocks of a head together, which keeps its K / V (or Q / dO) in L2.
@@ -59,31 +63,11 @@ __device__ __forceinline__ void decode_block(int lin, int nblk, int H, int B, bo
   h = hb - b * H;
 }
 
-// The (key block, query block) tiles of one CTA of the backward kernel, in order. Work items (key blocks) are dealt out in rounds of
-// gridDim.x, every other round backwards: with the longest items first, that evens out the sums.
-struct BwdTiles {
-  const AttnParams& p;
-  int nblk, round = 0, it = 0;      // `it` counts the query blocks of the current item
-  int j = 0, h = 0, b = 0, i0 = 0, n = 0;
-  bool valid = true;
-  __device__ explicit BwdTiles(const AttnParams& p_) : p(p_), nblk((p_.S + kBlk - 1) / kBlk) { item(); }
-  __device__ void item() {
-    const long long lin = static_cast<long long>(round) * gridDim.x + ((round & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
-    valid = lin < static_cast<long long>(nblk) * p.H * p.B;
-    if (!valid) return;
-    decode_block(static_cast<int>(lin), nblk, p.H, p.B, p.causal != 0, j, h, b);
-    i0 = p.causal ? j : 0;
-    n = nblk - i0;
-  }
-  __device__ void next() {
-    if (++it == n) {
-      it = 0;
-      ++round;
-      item();
-    }
-  }
-  __device__ bool last() const { return it == n - 1; }
-};
+// Adds `bytes` of fp32 values to global memory (both sides 16-byte aligned), as a bulk copy: beside the LSU pipe, which the softmax
+// warps' shared-memory traffic goes through.
+__device__ __forceinline__ void bulk_add(float* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
 
 // Per query row: D = dot(dO, O) into the first word of the row's dQ slot (overwritten by attn_dq_kernel at the end), and the
 // row's share of the dQ scratch zeroed. Eight lanes per row, rows of one (batch, head) consecutive.
@@ -137,38 +121,41 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                      const __grid_constant__ CUtensorMap tmDO, const float* __restrict__ lse, const __nv_bfloat16* __restrict__ dq,
                      __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, float* __restrict__ dq_accum, const AttnParams p) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  if ((smem_u32(smem) & 1023u) != 0) {
-    if (threadIdx.x == 0) set_status(p.status, kStatusBadArg);
-    return;
-  }
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   using L = BwdLong;
-  // Tile g of the CTA (counted over all its items) uses buffer g & 1 of everything that has two: Q / dO, P / dS, dQ, statistics.
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BARS);
-  uint64_t* kv_full = bars;            // K and V of an item have landed
-  uint64_t* acc_free = bars + 1;       // dK and dV of an item have been read out of TMEM
-  uint64_t* sdp_full = bars + 2;       // S and dP are in TMEM
-  uint64_t* sdp_free = bars + 3;       // ... and in the softmax warps' registers
-  uint64_t* pds_ready = bars + 4;      // P and dS are in shared memory
-  uint64_t* q_full = bars + 5;         // [2] Q and dO have landed
-  uint64_t* grads = bars + 7;          // [2] dV, dK, dQ of the tile have retired: its Q / dO, P / dS may be overwritten, its dQ read
-  uint64_t* dq_free = bars + 9;        // [2] dQ has been read
-  uint64_t* stat_full = bars + 11;     // [2] lse and D are in shared memory
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+  uint64_t* kv_full = bars;
+  uint64_t* q_full = bars + 1;                    // [kBwdStages] Q and dO of a query block have landed
+  uint64_t* q_empty = q_full + kBwdStages;        // [kBwdStages] ... and every product that reads them has retired
+  uint64_t* sdp_full = q_empty + kBwdStages;      // S and dP are in TMEM
+  uint64_t* sdp_free = sdp_full + 1;              // ... and in the softmax warps' registers
+  uint64_t* pds_ready = sdp_free + 1;             // P and dS are in shared memory
+  uint64_t* grads_full = pds_ready + 1;           // dV, dK, dQ of the block have retired (P, dS may be overwritten)
+  uint64_t* dq_full = grads_full + 1;             // [2] the same event, per dQ buffer, for the draining warps
+  uint64_t* dq_free = dq_full + 2;                // [2] the buffer has been read
+  uint64_t* stat_full = dq_free + 2;              // [2] lse and D of a query block are in shared memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stat_full + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* mask_s = reinterpret_cast<float*>(smem + L::MASK);
   float2* stats = reinterpret_cast<float2*>(smem + L::STATS);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nblk = (p.S + kBlk - 1) / kBlk;
+  int j, h, b;
+  decode_block(blockIdx.x, nblk, p.H, p.B, p.causal != 0, j, h, b);
+  const int kv0 = j * kBlk, i0 = p.causal ? j : 0, n = nblk - i0;
+  const long long bh = static_cast<long long>(b) * p.H + h;
   const unsigned long long seed = p.seed + (p.seed_dev ? *p.seed_dev : 0ull);
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
-    mbar_init(acc_free, 32 * kBwdSoftmaxWarps);
+    for (int s = 0; s < kBwdStages; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
     mbar_init(sdp_full, 1);
-    mbar_init(sdp_free, 32 * kBwdSoftmaxWarps);
-    mbar_init(pds_ready, 32 * kBwdSoftmaxWarps);
-    for (int s = 0; s < 2; ++s) { mbar_init(&q_full[s], 1); mbar_init(&grads[s], 1); mbar_init(&dq_free[s], 4); mbar_init(&stat_full[s], 128); }
+    mbar_init(sdp_free, kBwdSoftmaxWarps);
+    mbar_init(pds_ready, kBwdSoftmaxWarps);
+    mbar_init(grads_full, 1);
+    for (int s = 0; s < 2; ++s) { mbar_init(&dq_full[s], 1); mbar_init(&dq_free[s], 4); mbar_init(&stat_full[s], 4); }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -183,22 +170,18 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const uint32_t tS = tmem_base, tDP = tmem_base + 128, tDV = tmem_base + 256, tDK = tmem_base + 320, tDQ = tmem_base + 384;
   pdl_entry();
 
-  BwdTiles w(p);
   if (warp == kBwdSoftmaxWarps + 5) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      for (int g = 0; w.valid; ++g, w.next()) {
-        const int buf = g & 1;
-        if (!mbar_wait(&grads[buf], ((g >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEmpty)) break;        // tile g - 2
-        mbar_expect_tx(&q_full[buf], 32768);
-        tma_load_4d(smem + L::Q + buf * 16384, &tmQ, &q_full[buf], 0, (w.i0 + w.it) * kBlk, w.h, w.b);
-        tma_load_4d(smem + L::DO + buf * 16384, &tmDO, &q_full[buf], 0, (w.i0 + w.it) * kBlk, w.h, w.b);
-        if (w.it == 0) {
-          if (g > 0 && !mbar_wait(&grads[buf ^ 1], ((g - 1) >> 1) & 1, abort_flag, p.status, kStatusWaitEmpty)) break;     // the last tile of the item before
-          mbar_expect_tx(kv_full, 32768);
-          tma_load_4d(smem + L::K, &tmK, kv_full, 0, w.j * kBlk, w.h, w.b);
-          tma_load_4d(smem + L::V, &tmV, kv_full, 0, w.j * kBlk, w.h, w.b);
-        }
+      mbar_expect_tx(kv_full, 32768);
+      tma_load_4d(smem + L::K, &tmK, kv_full, 0, kv0, h, b);
+      tma_load_4d(smem + L::V, &tmV, kv_full, 0, kv0, h, b);
+      for (int it = 0; it < n; ++it) {
+        const int st = it % kBwdStages;
+        if (!mbar_wait(&q_empty[st], ((it / kBwdStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitEmpty)) break;
+        mbar_expect_tx(&q_full[st], 32768);
+        tma_load_4d(smem + L::Q + st * 16384, &tmQ, &q_full[st], 0, (i0 + it) * kBlk, h, b);
+        tma_load_4d(smem + L::DO + st * 16384, &tmDO, &q_full[st], 0, (i0 + it) * kBlk, h, b);
       }
     }
   } else if (warp == kBwdSoftmaxWarps + 4) {
@@ -208,9 +191,11 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const uint32_t idesc_mn = make_idesc_bf16(128, kHD, 1, 1);      // dV, dK: A^T (MN-major) x MN-major
       const uint32_t idesc_kn = make_idesc_bf16(128, kHD, 0, 1);      // dQ: K-major x MN-major
       const uint32_t sK = smem_u32(smem + L::K), sV = smem_u32(smem + L::V);
-      auto scores = [&](int g) {
-        const uint32_t sQ = smem_u32(smem + L::Q + (g & 1) * 16384), sDO = smem_u32(smem + L::DO + (g & 1) * 16384);
-        if (!mbar_wait(&q_full[g & 1], (g >> 1) & 1, abort_flag, p.status, kStatusWaitFull)) return false;
+      const uint32_t sP = smem_u32(smem + L::P), sDS = smem_u32(smem + L::DS);
+      auto scores = [&](int it) {
+        const int st = it % kBwdStages;
+        const uint32_t sQ = smem_u32(smem + L::Q + st * 16384), sDO = smem_u32(smem + L::DO + st * 16384);
+        if (!mbar_wait(&q_full[st], (it / kBwdStages) & 1, abort_flag, p.status, kStatusWaitFull)) return false;
         tc_fence_after_sync();
 #pragma unroll
         for (int k4 = 0; k4 < kHD / 16; ++k4)
@@ -221,193 +206,183 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         umma_commit(sdp_full);
         return true;
       };
-      bool ok = true;
-      for (int g = 0; w.valid; ++g, w.next()) {
-        if (w.it == 0) {       // an item's first S overwrites the last S of the item before, whose readers have arrived
-          ok = mbar_wait(kv_full, w.round & 1, abort_flag, p.status, kStatusWaitFull) &&
-               (g == 0 || mbar_wait(sdp_free, (g - 1) & 1, abort_flag, p.status, kStatusWaitEpi)) && scores(g);
+      bool ok = mbar_wait(kv_full, 0, abort_flag, p.status, kStatusWaitFull) && scores(0);
+      for (int it = 0; it < n && ok; ++it) {
+        if (it + 1 < n) {
+          ok = mbar_wait(sdp_free, it & 1, abort_flag, p.status, kStatusWaitEpi) && scores(it + 1);
           if (!ok) break;
         }
-        if (!w.last()) {
-          ok = mbar_wait(sdp_free, g & 1, abort_flag, p.status, kStatusWaitEpi) && scores(g + 1);
-          if (!ok) break;
-        }
-        const int buf = g & 1;
-        const uint32_t sQ = smem_u32(smem + L::Q + buf * 16384), sDO = smem_u32(smem + L::DO + buf * 16384);
-        const uint32_t sP = smem_u32(smem + L::P + buf * 32768), sDS = smem_u32(smem + L::DS + buf * 32768);
-        ok = mbar_wait(pds_ready, g & 1, abort_flag, p.status, kStatusWaitEpi) && mbar_wait(&dq_free[buf], ((g >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi) &&
-             (w.it > 0 || mbar_wait(acc_free, (w.round & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi));
+        const int st = it % kBwdStages, qb = it & 1;
+        const uint32_t sQ = smem_u32(smem + L::Q + st * 16384), sDO = smem_u32(smem + L::DO + st * 16384);
+        ok = mbar_wait(pds_ready, it & 1, abort_flag, p.status, kStatusWaitEpi) &&
+             mbar_wait(&dq_free[qb], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi);
         if (!ok) break;
         tc_fence_after_sync();
         // dV += P^T dO ; dK += dS^T Q   (M = key index, K = query index: 8 steps of 16 rows)
 #pragma unroll
         for (int k8 = 0; k8 < kBlk / 16; ++k8)
-          umma_bf16<1>(tDV, make_smem_desc(sP + k8 * 2048, 16384, 1024), make_smem_desc(sDO + k8 * 2048, 8192, 1024), idesc_mn, w.it > 0 || k8 > 0);
+          umma_bf16<1>(tDV, make_smem_desc(sP + k8 * 2048, 16384, 1024), make_smem_desc(sDO + k8 * 2048, 8192, 1024), idesc_mn, it > 0 || k8 > 0);
 #pragma unroll
         for (int k8 = 0; k8 < kBlk / 16; ++k8)
-          umma_bf16<1>(tDK, make_smem_desc(sDS + k8 * 2048, 16384, 1024), make_smem_desc(sQ + k8 * 2048, 8192, 1024), idesc_mn, w.it > 0 || k8 > 0);
+          umma_bf16<1>(tDK, make_smem_desc(sDS + k8 * 2048, 16384, 1024), make_smem_desc(sQ + k8 * 2048, 8192, 1024), idesc_mn, it > 0 || k8 > 0);
         // dQ_tile = dS K   (M = query, K = key index)
 #pragma unroll
         for (int k8 = 0; k8 < kBlk / 16; ++k8)
-          umma_bf16<1>(tDQ + buf * 64, make_smem_desc(sDS + (k8 >> 2) * 16384 + (k8 & 3) * 32, 16, 1024), make_smem_desc(sK + k8 * 2048, 8192, 1024),
+          umma_bf16<1>(tDQ + qb * 64, make_smem_desc(sDS + (k8 >> 2) * 16384 + (k8 & 3) * 32, 16, 1024), make_smem_desc(sK + k8 * 2048, 8192, 1024),
                        idesc_kn, k8 > 0);
-        umma_commit(&grads[buf]);
+        umma_commit(grads_full);
+        umma_commit(&dq_full[qb]);
+        umma_commit(&q_empty[st]);
       }
     }
   } else if (warp >= kBwdSoftmaxWarps) {
     // ------------------------------------------------------------------ row statistics in, dQ out
     const int quarter = warp & 3, t = quarter * 32 + lane;
-    BwdTiles ahead = w;        // the tile whose statistics are fetched: two in front
-    auto load_stats = [&]() {
-      const int q = (ahead.i0 + ahead.it) * kBlk + t;
+    auto load_stats = [&](int it) {
+      const int q = (i0 + it) * kBlk + t;
       // a row beyond S, or one that no key takes part in, gets +inf: every probability of it is then 2^-inf = 0
       float l = INFINITY, D = 0.f;
       if (q < p.S) {
-        l = __ldg(lse + (static_cast<long long>(ahead.b) * p.H + ahead.h) * p.S + q);
+        l = __ldg(lse + bh * p.S + q);
         l = l == -INFINITY ? INFINITY : l * kLog2e;
-        D = *reinterpret_cast<const float*>(dq + ahead.b * p.gsb + ahead.h * p.gsh + q * p.gss);
+        D = *reinterpret_cast<const float*>(dq + b * p.gsb + h * p.gsh + q * p.gss);
       }
       return make_float2(l, D);
     };
-    auto put_stats = [&](int buf, float2 ld) {
-      stats[buf * 128 + t] = ld;
-      mbar_arrive(&stat_full[buf]);
-      ahead.next();
+    auto put_stats = [&](int it, float2 ld) {
+      stats[(it & 1) * 128 + t] = ld;
+      arrive_warp(&stat_full[it & 1], lane);
     };
-    for (int g = 0; g < 2 && ahead.valid; ++g) put_stats(g, load_stats());
-    for (int g = 0; w.valid; ++g, w.next()) {
-      const int buf = g & 1;
-      const float2 stat = ahead.valid ? load_stats() : make_float2(0.f, 0.f);
-      if (!__all_sync(0xffffffffu, mbar_wait(&grads[buf], (g >> 1) & 1, abort_flag, p.status, kStatusWaitAccum))) break;
+    put_stats(0, load_stats(0));
+    if (n > 1) put_stats(1, load_stats(1));
+    const uint32_t stage = smem_u32(smem + L::DQ) + quarter * 4096;
+    for (int it = 0; it < n; ++it) {
+      const int qb = it & 1;
+      const float2 ahead = it + 2 < n ? load_stats(it + 2) : make_float2(0.f, 0.f);
+      if (!__all_sync(0xffffffffu, mbar_wait(&dq_full[qb], (it >> 1) & 1, abort_flag, p.status, kStatusWaitAccum))) break;
       tc_fence_after_sync();
-      uint32_t v0[32], v1[32];
-      tmem_ld32(tDQ + buf * 64 + (static_cast<uint32_t>(quarter * 32) << 16), v0);
-      tmem_ld32(tDQ + buf * 64 + 32 + (static_cast<uint32_t>(quarter * 32) << 16), v1);
-      tmem_ld_wait();
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&dq_free[buf]);
-      if (ahead.valid) put_stats(buf, stat);      // every softmax thread has read this buffer: its P and dS went into the products
-      const int row0 = (w.i0 + w.it) * kBlk + quarter * 32, nr = min(32, p.S - row0);
-      if (lane < nr) {
-        float* dst = dq_accum + ((static_cast<long long>(w.b) * p.H + w.h) * p.S + row0) * kHD + lane * 4;
+      // 32 columns at a time: 16-byte chunk c of this warp's row r at (c * rows + r) * 16, as in the scratch
+      const int row0 = (i0 + it) * kBlk + quarter * 32, nr = min(32, p.S - row0);
+      float* dst = dq_accum + (bh * p.S + row0) * kHD;
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        uint32_t v[32];
+        tmem_ld32(tDQ + qb * 64 + half * 32 + (static_cast<uint32_t>(quarter * 32) << 16), v);
+        tmem_ld_wait();
+        if (half == 1) {
+          tc_fence_before_sync();
+          arrive_warp(&dq_free[qb], lane);
+        }
+        if (lane == 0) tma_store_wait_read();       // the bulk copy before has read the staging area
+        __syncwarp();
+        if (lane < nr) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          red_add_v4(dst + static_cast<long long>(c) * nr * 4, __uint_as_float(v0[4 * c]), __uint_as_float(v0[4 * c + 1]), __uint_as_float(v0[4 * c + 2]),
-                     __uint_as_float(v0[4 * c + 3]));
-          red_add_v4(dst + static_cast<long long>(c + 8) * nr * 4, __uint_as_float(v1[4 * c]), __uint_as_float(v1[4 * c + 1]), __uint_as_float(v1[4 * c + 2]),
-                     __uint_as_float(v1[4 * c + 3]));
+          for (int c = 0; c < 8; ++c) st_shared_v4(stage + (c * nr + lane) * 16, make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]));
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && nr > 0) {
+          bulk_add(dst + half * 32 * nr, stage, 128 * nr);
+          tma_store_commit();
         }
       }
+      if (it + 2 < n) put_stats(it + 2, ahead);   // every softmax thread has read buffer it & 1: its P and dS went into these products
     }
+    if (lane == 0) tma_store_wait_read();      // the shared memory outlives what reads it; the additions end with the grid
   } else {
-    // ------------------------------------------------------------------ softmax: thread = query row t x 64 keys
-    const int quarter = warp & 3, half = warp >> 2, t = quarter * 32 + lane;
+    // ------------------------------------------------------------------ softmax: thread = query row t x 32 keys
+    const int quarter = warp & 3, part = warp >> 2, t = quarter * 32 + lane, c = part * 32;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
     const float sc = p.scale * kLog2e;
     const float inv_keep = p.p_drop > 0.f ? 1.f / (1.f - p.p_drop) : 1.f;
+    if (threadIdx.x < kBlk) {      // the additive mask (mask * log2e; -inf beyond S)
+      const int kv = kv0 + threadIdx.x;
+      mask_s[threadIdx.x] = kv < p.S ? (p.mask ? __ldg(p.mask + static_cast<long long>(b) * p.S + kv) * kLog2e : 0.f) : -INFINITY;
+    }
+    asm volatile("bar.sync 1, 512;" ::: "memory");
+    const bool masked = p.mask != nullptr || kv0 + kBlk > p.S;
+    const uint32_t pp = smem_u32(smem + L::P) + (part >> 1) * 16384, dp = smem_u32(smem + L::DS) + (part >> 1) * 16384;
     bool ok = true;
-    for (int g = 0; w.valid; ++g, w.next()) {
-      const int buf = g & 1, kv0 = w.j * kBlk;
-      const bool masked = p.mask != nullptr || kv0 + kBlk > p.S;
-      if (w.it == 0 && masked) {      // the item's additive mask (mask * log2e; -inf beyond S)
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (threadIdx.x < kBlk) {
-          const int kv = kv0 + threadIdx.x;
-          mask_s[threadIdx.x] = kv < p.S ? (p.mask ? __ldg(p.mask + static_cast<long long>(w.b) * p.S + kv) * kLog2e : 0.f) : -INFINITY;
-        }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-      }
-      const int q = (w.i0 + w.it) * kBlk + t;
-      const bool diagonal = p.causal && w.i0 + w.it == w.j;
-      const uint32_t pp = smem_u32(smem + L::P + buf * 32768) + half * 16384, dp = smem_u32(smem + L::DS + buf * 32768) + half * 16384;
-      ok = ok && mbar_wait(&stat_full[buf], (g >> 1) & 1, abort_flag, p.status, kStatusWaitFull);
-      const float2 ld = stats[buf * 128 + t];
-      ok = ok && mbar_wait(&grads[buf], ((g >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitAccum);       // tile g - 2 has been read out of P and dS
-      ok = __all_sync(0xffffffffu, ok && mbar_wait(sdp_full, g & 1, abort_flag, p.status, kStatusWaitAccum));
-      if (!ok) continue;        // after a wait that gave up the loop runs out without work, so that no warp is missed at the barrier above
+    for (int it = 0; it < n; ++it) {
+      const int q = (i0 + it) * kBlk + t;
+      const bool diagonal = p.causal && i0 + it == j;
+      ok = mbar_wait(&stat_full[it & 1], (it >> 1) & 1, abort_flag, p.status, kStatusWaitFull);
+      const float2 ld = stats[(it & 1) * 128 + t];
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(sdp_full, it & 1, abort_flag, p.status, kStatusWaitAccum));
+      if (!ok) break;
       tc_fence_after_sync();
+      uint32_t sv[32], dpv[32];
+      tmem_ld32(tS + lane_base + c, sv);
+      tmem_ld32(tDP + lane_base + c, dpv);
+      tmem_ld_wait();
+      tc_fence_before_sync();
+      arrive_warp(sdp_free, lane);
+      // P into sv, dS into dpv
+      if (masked) {
 #pragma unroll
-      for (int cc = 0; cc < 64; cc += 32) {
-        const int c = half * 64 + cc;
-        uint32_t sv[32], dpv[32];
-        tmem_ld32(tS + lane_base + c, sv);
-        tmem_ld32(tDP + lane_base + c, dpv);
-        tmem_ld_wait();
-        if (cc == 32) {
-          tc_fence_before_sync();
-          mbar_arrive(sdp_free);
+        for (int e4 = 0; e4 < 32; e4 += 4) {
+          const float4 mk = *reinterpret_cast<const float4*>(mask_s + c + e4);
+          const float mk4[4] = {mk.x - ld.x, mk.y - ld.x, mk.z - ld.x, mk.w - ld.x};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) sv[e4 + k] = __float_as_uint(ex2_approx(__uint_as_float(sv[e4 + k]) * sc + mk4[k]));
         }
-        // P into sv
-        if (masked) {
+      } else {
 #pragma unroll
-          for (int e4 = 0; e4 < 32; e4 += 4) {
-            const float4 mk = *reinterpret_cast<const float4*>(mask_s + c + e4);
-            const float mk4[4] = {mk.x - ld.x, mk.y - ld.x, mk.z - ld.x, mk.w - ld.x};
+        for (int e = 0; e < 32; ++e) sv[e] = __float_as_uint(ex2_approx(__uint_as_float(sv[e]) * sc - ld.x));
+      }
+      if (diagonal) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) sv[e4 + k] = __float_as_uint(ex2_approx(__uint_as_float(sv[e4 + k]) * sc + mk4[k]));
+        for (int e = 0; e < 32; ++e)
+          if (kv0 + c + e > q) sv[e] = 0u;
+      }
+      if (p.p_drop > 0.f) {
+        const unsigned long long base = (static_cast<unsigned long long>(bh) * p.S + q) * p.S + kv0 + c;
+#pragma unroll
+        for (int e = 0; e < 32; e += 4) {
+          float z[4];
+          dropout_scale4(seed, base + e, p.p_drop, inv_keep, z);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float pe = __uint_as_float(sv[e + k]);
+            dpv[e + k] = __float_as_uint(pe * (__uint_as_float(dpv[e + k]) * z[k] - ld.y) * p.scale);
+            sv[e + k] = __float_as_uint(pe * z[k]);
           }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) sv[e] = __float_as_uint(ex2_approx(__uint_as_float(sv[e]) * sc - ld.x));
         }
-        if (diagonal) {
+      } else {
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (kv0 + c + e > q) sv[e] = 0u;
-        }
-        float ds[32];
-        if (p.p_drop > 0.f) {
-          const unsigned long long base = ((static_cast<unsigned long long>(w.b) * p.H + w.h) * p.S + q) * p.S + kv0 + c;
+        for (int e = 0; e < 32; ++e) dpv[e] = __float_as_uint(__uint_as_float(sv[e]) * (__uint_as_float(dpv[e]) - ld.y) * p.scale);
+      }
+      if (it > 0) {        // the previous block's products have read P and dS
+        ok = __all_sync(0xffffffffu, mbar_wait(grads_full, (it - 1) & 1, abort_flag, p.status, kStatusWaitAccum));
+        if (!ok) break;
+      }
 #pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            float z[4];
-            dropout_scale4(seed, base + e, p.p_drop, inv_keep, z);
+      for (int g8 = 0; g8 < 4; ++g8) {
+        float pr[8], ds[8];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float pe = __uint_as_float(sv[e + k]);
-              ds[e + k] = pe * (__uint_as_float(dpv[e + k]) * z[k] - ld.y) * p.scale;
-              sv[e + k] = __float_as_uint(pe * z[k]);
-            }
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) ds[e] = __uint_as_float(sv[e]) * (__uint_as_float(dpv[e]) - ld.y) * p.scale;
-        }
-#pragma unroll
-        for (int g8 = 0; g8 < 4; ++g8) {
-          float pr[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) pr[e] = __uint_as_float(sv[8 * g8 + e]);
-          st_shared_v4(swz_chunk(pp, t, (cc >> 3) + g8), pack8(pr));
-          st_shared_v4(swz_chunk(dp, t, (cc >> 3) + g8), pack8(ds + 8 * g8));
-        }
+        for (int e = 0; e < 8; ++e) { pr[e] = __uint_as_float(sv[8 * g8 + e]); ds[e] = __uint_as_float(dpv[8 * g8 + e]); }
+        st_shared_v4(swz_chunk(pp, t, (part & 1) * 4 + g8), pack8(pr));
+        st_shared_v4(swz_chunk(dp, t, (part & 1) * 4 + g8), pack8(ds));
       }
       fence_proxy_async_smem();
-      mbar_arrive(pds_ready);
-      if (w.last()) {
-        // dK (warps 0..3) and dV (warps 4..7) out. Every product of the item has then retired, so the rows of P's first buffer that
-        // this warp alone writes serve as its staging area.
-        ok = __all_sync(0xffffffffu, mbar_wait(&grads[buf], (g >> 1) & 1, abort_flag, p.status, kStatusWaitAccum));
-        if (!ok) continue;
-        tc_fence_after_sync();
-        const uint32_t stage = smem_u32(smem + L::P) + warp * 4096;
+      arrive_warp(pds_ready, lane);
+    }
+    // dK (warps 0..3) and dV (warps 4..7) out, through the warp's 4 KB of the P panels, which every product has read
+    ok = __all_sync(0xffffffffu, ok && part < 2 && mbar_wait(grads_full, (n - 1) & 1, abort_flag, p.status, kStatusWaitAccum));
+    if (ok) {
+      tc_fence_after_sync();
+      const uint32_t stage = smem_u32(smem + L::P) + warp * 4096;
 #pragma unroll
-        for (int c = 0; c < kHD; c += 32) {
-          uint32_t v[32];
-          tmem_ld32((half == 0 ? tDK : tDV) + lane_base + c, v);
-          tmem_ld_wait();
-          if (c == 32) {
-            tc_fence_before_sync();
-            mbar_arrive(acc_free);
-          }
-          float f[32];
+      for (int c2 = 0; c2 < kHD; c2 += 32) {
+        uint32_t v[32];
+        tmem_ld32((part == 0 ? tDK : tDV) + lane_base + c2, v);
+        tmem_ld_wait();
+        float f[32];
 #pragma unroll
-          for (int e = 0; e < 32; ++e) f[e] = __uint_as_float(v[e]);
-          stage_half(stage, lane, c, f);
-        }
-        flush_rows(stage, lane, (half == 0 ? dk : dv) + w.b * p.gsb + w.h * p.gsh, p.gss, kv0 + quarter * 32, p.S);
+        for (int e = 0; e < 32; ++e) f[e] = __uint_as_float(v[e]);
+        stage_half(stage, lane, c2, f);
       }
+      flush_rows(stage, lane, (part == 0 ? dk : dv) + b * p.gsb + h * p.gsh, p.gss, kv0 + quarter * 32, p.S);
     }
   }
   tc_fence_before_sync();
@@ -424,7 +399,7 @@ int attn_bwd_long(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
                   const float* lse, void* dq, void* dk, void* dv, float* dq_accum, const AttnParams& p, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(attn_bwd_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdLong::TOTAL);
+    const cudaError_t e = cudaFuncSetAttribute(attn_bwd_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdLong::TOTAL + 1024);
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
@@ -434,7 +409,7 @@ int attn_bwd_long(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
   const int row_grid = static_cast<int>(rows / 32 + 1 < kSMs * 16 ? rows / 32 + 1 : kSMs * 16);
   auto* dq16 = static_cast<__nv_bfloat16*>(dq);
   launch_pdl(attn_bwd_pre_kernel, dim3(row_grid), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), dq16, dq_accum, p);
-  launch_pdl(attn_bwd_long_kernel, dim3(static_cast<unsigned>(items < kSMs ? items : kSMs)), dim3(kBwdThreads), static_cast<size_t>(BwdLong::TOTAL), stream, tq, tk, tv, tdo, lse,
+  launch_pdl(attn_bwd_long_kernel, dim3(static_cast<unsigned>(items)), dim3(kBwdThreads), static_cast<size_t>(BwdLong::TOTAL + 1024), stream, tq, tk, tv, tdo, lse,
              static_cast<const __nv_bfloat16*>(dq16), static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), dq_accum, p);
   launch_pdl(attn_dq_kernel, dim3(row_grid), dim3(256), 0, stream, static_cast<const float*>(dq_accum), dq16, p);
   return static_cast<int>(cudaGetLastError());
@@ -443,7 +418,8 @@ int attn_bwd_long(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
 // ===================================================================================== forward
 namespace {
 
-constexpr int kFwdThreads = 32 * 6;
+constexpr int kFwdSoftmaxWarps = 8;
+constexpr int kFwdThreads = 32 * (kFwdSoftmaxWarps + 2);
 constexpr float kRescaleAt = 8.f;      // log2 of the factor by which a row maximum may grow before its accumulator is rescaled
 
 struct FwdLong {
@@ -451,7 +427,8 @@ struct FwdLong {
   static constexpr int K = 16384;                    // 2 x 16 KB
   static constexpr int V = K + 2 * 16384;            // 2 x 16 KB
   static constexpr int MASK = V + 2 * 16384;         // 2 x 128 floats
-  static constexpr int BARS = MASK + 1024;
+  static constexpr int XCHG = MASK + 1024;           // 2 x 2 x 128 floats: the half rows' maxima, and at the end their sums
+  static constexpr int BARS = XCHG + 2048;
   static constexpr int TOTAL = BARS + 256;
 };
 
@@ -489,13 +466,13 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
     mbar_init(s_full, 1);
-    mbar_init(s_free, 128);
-    mbar_init(p_ready, 128);
+    mbar_init(s_free, kFwdSoftmaxWarps);
+    mbar_init(p_ready, kFwdSoftmaxWarps);
     mbar_init(pv_done, 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 4) {
+  if (warp == kFwdSoftmaxWarps) {
     tmem_alloc<1>(tmem_slot, 256);
     tmem_relinquish<1>();
   }
@@ -506,7 +483,7 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const uint32_t tS = tmem_base, tP = tmem_base + 128, tO = tmem_base + 192;
   pdl_entry();
 
-  if (warp == 5) {
+  if (warp == kFwdSoftmaxWarps + 1) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       mbar_expect_tx(q_full, 16384);
@@ -522,7 +499,7 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tma_load_4d(smem + L::V + st * 16384, &tmV, &v_full[st], 0, j * kBlk, h, b);
       }
     }
-  } else if (warp == 4) {
+  } else if (warp == kFwdSoftmaxWarps) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
       const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
@@ -559,70 +536,84 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
     }
   } else {
-    // ------------------------------------------------------------------ softmax: thread = query row
-    const int t = threadIdx.x, q = q0 + t;
-    const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
+    // ------------------------------------------------------------------ softmax: thread = query row t x 64 keys
+    // (two warps share 32 rows: four warps a scheduler with two CTAs, which is what hides the TMEM loads and the exponentials' latency)
+    const int quarter = warp & 3, half = warp >> 2, t = quarter * 32 + lane, q = q0 + t;
+    const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
     const float sc = p.scale * kLog2e;
     const float inv_keep = kDrop ? 1.f / (1.f - p.p_drop) : 1.f;
-    float m_ref = -INFINITY, l_run = 0.f;       // the maximum the accumulator is relative to, and the row sum
+    float* xchg = reinterpret_cast<float*>(smem + L::XCHG);
+    // the other half row's value; the two warps of a quarter meet, one of the two slots being free for the next exchange
+    auto exchange = [&](int slot, float mine) {
+      xchg[(slot * 2 + half) * kBlk + t] = mine;
+      asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
+      return xchg[(slot * 2 + (half ^ 1)) * kBlk + t];
+    };
+    float m_ref = -INFINITY, l_run = 0.f;       // the maximum the accumulator is relative to, and this half row's sum
     bool ok = true;
+    // After a wait that gave up the loop runs out without work, so that no warp is missed at the barriers.
     for (int j = 0; j < n; ++j) {
-      const int kv0 = j * kBlk;
+      const int kv0 = j * kBlk, c0 = half * 64;
       const bool masked = p.mask != nullptr || kv0 + kBlk > p.S;
       const bool diagonal = p.causal && j == qb;
-      const float* mk_s = mask_s + (j & 1) * kBlk;
+      const float* mk_s = mask_s + (j & 1) * kBlk + c0;
       if (masked) {       // additive mask of this key block (mask * log2e; -inf beyond S); the other buffer may still be in use
-        const int kv = kv0 + t;
-        mask_s[(j & 1) * kBlk + t] = kv < p.S ? (p.mask ? __ldg(p.mask + static_cast<long long>(b) * p.S + kv) * kLog2e : 0.f) : -INFINITY;
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (half == 0) {
+          const int kv = kv0 + t;
+          mask_s[(j & 1) * kBlk + t] = kv < p.S ? (p.mask ? __ldg(p.mask + static_cast<long long>(b) * p.S + kv) * kLog2e : 0.f) : -INFINITY;
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
       }
       ok = __all_sync(0xffffffffu, ok && mbar_wait(s_full, j & 1, abort_flag, p.status, kStatusWaitAccum));
-      if (!ok) continue;        // after a wait that gave up the loop runs out without work, so that no warp is missed at the barrier above
-      tc_fence_after_sync();
-      uint32_t sv[4][32];
+      uint32_t sv[2][32];
+      float m_half = -INFINITY, mul = sc;
+      if (ok) {
+        tc_fence_after_sync();
+        tmem_ld32(tS + lane_base + c0, sv[0]);
+        tmem_ld32(tS + lane_base + c0 + 32, sv[1]);
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        arrive_warp(s_free, lane);
+        // row maximum; with a mask, on the diagonal or for a negative scale the scores are scaled here, otherwise in the exponent below
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        if (masked || diagonal || sc < 0.f) {
+          mul = 1.f;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(tS + lane_base + 32 * c, sv[c]);
-      tmem_ld_wait();
-      tc_fence_before_sync();
-      mbar_arrive(s_free);
-      // row maximum; with a mask, on the diagonal or for a negative scale the scores are scaled here, otherwise in the exponent below
-      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-      float mul = sc;
-      if (masked || diagonal || sc < 0.f) {
-        mul = 1.f;
+          for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+            for (int i4 = 0; i4 < 32; i4 += 4) {
+              const float4 mk = masked ? *reinterpret_cast<const float4*>(mk_s + 32 * c + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
+              const float mk4[4] = {mk.x, mk.y, mk.z, mk.w};
 #pragma unroll
-          for (int i4 = 0; i4 < 32; i4 += 4) {
-            const float4 mk = masked ? *reinterpret_cast<const float4*>(mk_s + 32 * c + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float mk4[4] = {mk.x, mk.y, mk.z, mk.w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              float s = __uint_as_float(sv[c][i4 + k]) * sc + mk4[k];
-              if (diagonal && kv0 + 32 * c + i4 + k > q) s = -INFINITY;
-              sv[c][i4 + k] = __float_as_uint(s);
-              m4[k] = fmaxf(m4[k], s);
+              for (int k = 0; k < 4; ++k) {
+                float s = __uint_as_float(sv[c][i4 + k]) * sc + mk4[k];
+                if (diagonal && kv0 + c0 + 32 * c + i4 + k > q) s = -INFINITY;
+                sv[c][i4 + k] = __float_as_uint(s);
+                m4[k] = fmaxf(m4[k], s);
+              }
             }
-          }
-      } else {
+        } else {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+          for (int c = 0; c < 2; ++c)
 #pragma unroll
-          for (int i = 0; i < 32; ++i) m4[i & 3] = fmaxf(m4[i & 3], __uint_as_float(sv[c][i]));
+            for (int i = 0; i < 32; ++i) m4[i & 3] = fmaxf(m4[i & 3], __uint_as_float(sv[c][i]));
+        }
+        m_half = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * mul;
       }
-      const float m_new = fmaxf(m_ref, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * mul);
+      const float m_new = fmaxf(m_ref, fmaxf(m_half, exchange(j & 1, m_half)));
+      if (!ok) continue;
       if (j == 0) {
         m_ref = m_new;
       } else {
         ok = __all_sync(0xffffffffu, mbar_wait(pv_done, (j - 1) & 1, abort_flag, p.status, kStatusWaitAccum));     // P may be overwritten, O touched
         if (!ok) continue;
         tc_fence_after_sync();
-        if (__any_sync(0xffffffffu, m_new > m_ref + kRescaleAt)) {
+        if (__any_sync(0xffffffffu, m_new > m_ref + kRescaleAt)) {       // the same for both warps of a row; each rescales half of O's columns
           const float alpha = m_new == -INFINITY ? 1.f : ex2_approx(m_ref - m_new);
           m_ref = m_new;
           l_run *= alpha;
 #pragma unroll 1
-          for (int c = 0; c < kHD; c += 16) {
+          for (int c = half * 32; c < half * 32 + 32; c += 16) {
             uint32_t v[16];
             tmem_ld16(tO + lane_base + c, v);
             tmem_ld_wait();
@@ -635,7 +626,7 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref;
       float l4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < 2; ++c) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const float pe = ex2_approx(fmaf(__uint_as_float(sv[c][i]), mul, neg_m));
@@ -643,7 +634,7 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           sv[c][i] = __float_as_uint(pe);
         }
         if constexpr (kDrop) {
-          const unsigned long long base = ((static_cast<unsigned long long>(b) * p.H + h) * p.S + q) * p.S + kv0 + 32 * c;
+          const unsigned long long base = ((static_cast<unsigned long long>(b) * p.H + h) * p.S + q) * p.S + kv0 + c0 + 32 * c;
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             float s4[4];
@@ -658,36 +649,44 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           const __nv_bfloat162 two = __floats2bfloat162_rn(__uint_as_float(sv[c][2 * i]), __uint_as_float(sv[c][2 * i + 1]));
           pk[i] = *reinterpret_cast<const uint32_t*>(&two);
         }
-        tmem_st16(tP + lane_base + 16 * c, pk);
+        tmem_st16(tP + lane_base + half * 32 + 16 * c, pk);
       }
       l_run += (l4[0] + l4[1]) + (l4[2] + l4[3]);
       tmem_st_wait();
       tc_fence_before_sync();
-      mbar_arrive(p_ready);
+      arrive_warp(p_ready, lane);
     }
+    l_run += exchange(n & 1, l_run);
     ok = ok && mbar_wait(pv_done, (n - 1) & 1, abort_flag, p.status, kStatusWaitAccum);
-    if (__all_sync(0xffffffffu, ok)) {
+    ok = __all_sync(0xffffffffu, ok);
+    const uint32_t stage = smem_u32(smem + L::Q) + quarter * 4096;        // every product that reads Q has retired
+    if (ok) {
       tc_fence_after_sync();
       const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
-      const uint32_t stage = smem_u32(smem + L::Q) + warp * 4096;        // every product that reads Q has retired
+      uint32_t v[32];
+      tmem_ld32(tO + lane_base + half * 32, v);
+      tmem_ld_wait();
+      float f[32];
 #pragma unroll
-      for (int c = 0; c < kHD; c += 32) {
-        uint32_t v[32];
-        tmem_ld32(tO + lane_base + c, v);
-        tmem_ld_wait();
-        float f[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]) * inv_l;
-        stage_half(stage, lane, c, f);
-      }
-      flush_rows(stage, lane, o + static_cast<long long>(b) * p.osb + static_cast<long long>(h) * p.osh, p.oss, q0 + warp * 32, p.S);
+      for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]) * inv_l;
+      stage_half(stage, lane, half * 32, f);
       // natural-log LSE of the scaled, masked scores
-      if (q < p.S) lse[(static_cast<long long>(b) * p.H + h) * p.S + q] = (l_run > 0.f) ? (m_ref + log2f(l_run)) / kLog2e : -INFINITY;
+      if (half == 0 && q < p.S) lse[(static_cast<long long>(b) * p.H + h) * p.S + q] = (l_run > 0.f) ? (m_ref + log2f(l_run)) / kLog2e : -INFINITY;
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
+    if (ok) {         // both halves of the quarter's 32 rows are staged: each warp writes 16 of them, eight lanes per row
+      __nv_bfloat16* base = o + static_cast<long long>(b) * p.osb + static_cast<long long>(h) * p.osh;
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int r = half * 16 + it * 4 + (lane >> 3), ch = lane & 7, row = q0 + quarter * 32 + r;
+        const uint4 val = ld_shared_v4(stage + r * 128 + ((ch ^ (r & 7)) << 4));
+        if (row < p.S) *reinterpret_cast<uint4*>(base + static_cast<long long>(row) * p.oss + ch * 8) = val;
+      }
     }
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 4) {
+  if (warp == kFwdSoftmaxWarps) {
     tc_fence_after_sync();
     tmem_dealloc<1>(tmem_base, 256);
   }
