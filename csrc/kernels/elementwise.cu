@@ -268,6 +268,24 @@ scatter_rows_kernel(const T* __restrict__ dxc, long long ldc, const int* __restr
   }
 }
 
+// four columns as they are in memory
+template <typename T>
+struct Vec4;
+template <>
+struct Vec4<float> {
+  using Raw = float4;
+  static __device__ __forceinline__ void unpack(const Raw& q, float (&v)[4]) { v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w; }
+};
+template <>
+struct Vec4<__nv_bfloat16> {
+  using Raw = uint2;
+  static __device__ __forceinline__ void unpack(const Raw& q, float (&v)[4]) {
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.y));
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  }
+};
+constexpr int kEmbRows = 8;       // tokens whose rows a thread has in flight
+
 // dW[ids[t]][:] += dy[t][:] for an embedding table (fp32 accumulation, rows equal to padding_idx skipped).
 template <typename T>
 __global__ void embedding_bwd_kernel(const T* __restrict__ dy, const long long* __restrict__ ids, float* __restrict__ dw,
@@ -281,6 +299,52 @@ __global__ void embedding_bwd_kernel(const T* __restrict__ dy, const long long* 
   const T* src = dy + t * dim;
   float* dst = dw + id * dim;
   for (int c = threadIdx.x & 31; c < dim; c += 32) atomicAdd(dst + c, VecIO<T>::get(src + c));
+}
+
+// The same four columns to a thread and a run of consecutive tokens to a block: neighbours with the same id (segment ids: all of
+// them) are summed in registers first, and what is added goes out as 16-byte reductions. One reduction per token, column and four
+// bytes, which the kernel above makes, is bound by the atomics of one row when many tokens share it. Needs dim and both base
+// addresses in whole vectors of four.
+// us, bf16, 768 columns, against one reduction per token and value: 4096 tokens of one id 6.9 (53), of two ids in any order 12 (26), all
+// different 5.6 (6.4); 32768 tokens of one id 21 (290), of random ids of 30522 26 (23; fp32 35 (36)).
+template <typename T>
+__global__ void __launch_bounds__(256)
+embedding_bwd_vec_kernel(const T* __restrict__ dy, const long long* __restrict__ ids, float* __restrict__ dw, long long tokens, int dim,
+                         long long vocab, long long padding_idx, int per_block) {
+  pdl_entry();
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  if (c >= dim) return;
+  const long long t0 = static_cast<long long>(blockIdx.x) * per_block, t1 = min(tokens, t0 + per_block);
+  long long cur = -1;       // whose row `acc` belongs to
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  auto flush = [&]() {
+    if (cur >= 0) red_add_v4(dw + cur * dim + c, acc[0], acc[1], acc[2], acc[3]);
+  };
+  for (long long t = t0; t < t1; t += kEmbRows) {
+    long long id[kEmbRows];
+    typename Vec4<T>::Raw raw[kEmbRows];
+#pragma unroll
+    for (int u = 0; u < kEmbRows; ++u) id[u] = t + u < t1 ? ids[t + u] : padding_idx;
+#pragma unroll
+    for (int u = 0; u < kEmbRows; ++u)
+      if (t + u < t1) raw[u] = *reinterpret_cast<const typename Vec4<T>::Raw*>(dy + (t + u) * dim + c);
+#pragma unroll
+    for (int u = 0; u < kEmbRows; ++u) {
+      if (t + u >= t1 || id[u] == padding_idx || !FB_INDEX_OK(id[u], vocab, 101) || id[u] < 0 || id[u] >= vocab) continue;
+      float v[4];
+      Vec4<T>::unpack(raw[u], v);
+      if (id[u] != cur) {
+        flush();
+        cur = id[u];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] = v[j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] += v[j];
+      }
+    }
+  }
+  flush();
 }
 
 template <typename TI, typename TO>
@@ -384,6 +448,22 @@ extern "C" int fb_embedding_bwd(const void* dy, const long long* ids, float* dw,
                                 long long padding_idx, int is_bf16, void* stream) {
   if (tokens <= 0 || dim <= 0) return 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const size_t four = is_bf16 ? 8 : 16;
+  if (dim % 4 == 0 && reinterpret_cast<uintptr_t>(dy) % four == 0 && reinterpret_cast<uintptr_t>(dw) % 16 == 0) {
+    // Enough blocks for two or three per SM; long runs spare reductions where neighbours are equal, short ones keep more rows in
+    // flight where they are not.
+    long long per = tokens / 400 / fb::kEmbRows * fb::kEmbRows;
+    per = per < fb::kEmbRows ? fb::kEmbRows : per > 16 ? 16 : per;
+    const int threads = dim / 4 < 256 ? (dim / 4 + 31) / 32 * 32 : 256;
+    const dim3 grid(static_cast<unsigned>((tokens + per - 1) / per), (dim / 4 + threads - 1) / threads);
+    if (is_bf16)
+      fb::launch_pdl(fb::embedding_bwd_vec_kernel<__nv_bfloat16>, grid, dim3(threads), 0, st, static_cast<const __nv_bfloat16*>(dy), ids, dw, tokens, dim, vocab,
+                     padding_idx, static_cast<int>(per));
+    else
+      fb::launch_pdl(fb::embedding_bwd_vec_kernel<float>, grid, dim3(threads), 0, st, static_cast<const float*>(dy), ids, dw, tokens, dim, vocab, padding_idx,
+                     static_cast<int>(per));
+    return static_cast<int>(cudaGetLastError());
+  }
   const int warps = 8;
   const long long grid = (tokens + warps - 1) / warps;
   if (is_bf16)

@@ -187,6 +187,20 @@ def test_layernorm_rows_per_warp(C, dtype, rows, cols):
     assert close(acc_g - 1, dg.double(), 2 ** -14) and close(acc_b - 1, db.double(), 2 ** -14)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens,dim,ids", [(1, 8, "random"), (4099, 768, "equal"), (777, 1028, "runs"), (5000, 64, "random"), (33, 30, "runs")])
+def test_embedding_bwd_runs(C, dtype, tokens, dim, ids):
+    """Equal neighbours are summed in registers first; padding and a table row that nothing touches. Sums of 32 bits in any order."""
+    torch.manual_seed(17)
+    vocab = 50
+    t = {"random": torch.randint(0, vocab - 1, (tokens,)), "equal": torch.full((tokens,), 7), "runs": (torch.arange(tokens) // 5) % (vocab - 1)}[ids].cuda()
+    dy = torch.randn(tokens, dim, device="cuda").to(dtype)
+    dw = torch.ones(vocab, dim, device="cuda")
+    C.embedding_bwd(dy, t, dw, 3)
+    ref = torch.ones(vocab, dim, device="cuda", dtype=torch.double).index_add_(0, t[t != 3], dy.double()[t != 3])
+    assert ((dw.double() - ref).norm() / ref.norm()).item() < 2 ** -18 and torch.all(dw[vocab - 1] == 1)
+
+
 def test_layernorm_dropout_mask_consistent(C):
     rows, cols, p = 512, 768, 0.1
     x = torch.ones(rows, cols, device="cuda", dtype=torch.bfloat16)
