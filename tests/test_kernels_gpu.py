@@ -502,6 +502,26 @@ def test_batchnorm_channels_last_many_blocks_accumulates(C):
     assert (db_acc - 1 - br.grad).abs().max().item() < 0.02 * br.grad.abs().max().item() + 0.5
 
 
+@pytest.mark.parametrize("dtype,Ch", [(torch.float32, 4), (torch.bfloat16, 8), (torch.bfloat16, 24), (torch.bfloat16, 64), (torch.float32, 132), (torch.bfloat16, 136),
+                                      (torch.float32, 256)])
+@pytest.mark.parametrize("pixels", [37, 40000])
+def test_batchnorm_channels_last_sums(C, dtype, Ch, pixels):
+    """From one block to a full wave of them, channel counts that do and do not divide the block: the statistics and the parameter gradients
+    are 32-bit sums over the stored values, whose error grows with the number of terms a thread adds (under a hundred here): 2^-17 in norm."""
+    torch.manual_seed(16)
+    x, dy = (torch.randn(1, Ch, pixels, 2, device="cuda").to(dtype).contiguous(memory_format=torch.channels_last) for _ in range(2))
+    g, b = torch.rand(Ch, device="cuda") + 0.5, torch.randn(Ch, device="cuda")
+    rm, rv = torch.zeros(Ch, device="cuda"), torch.ones(Ch, device="cuda")
+    y, mean, rstd = C.bn_fwd(x, None, g, b, rm, rv, 1e-5, 0.1, False, True)
+    xd, dyd = x.double(), dy.double()
+    sd = (xd.var((0, 2, 3), unbiased=False) + 1e-5).rsqrt()
+    close = lambda got, want: ((got.double() - want).norm() / want.norm()).item() < 2 ** -17
+    assert (mean.double() - xd.mean((0, 2, 3))).abs().max().item() < 2 ** -17 and close(rstd, sd)
+    _, _, dg, db = C.bn_bwd(dy, x, y, g, mean, rstd, False, False, None, None)
+    xh = (xd - mean.double().view(-1, 1, 1)) * rstd.double().view(-1, 1, 1)
+    assert close(dg, (dyd * xh).sum((0, 2, 3))) and close(db, dyd.sum((0, 2, 3)))
+
+
 @pytest.mark.parametrize("N,Ci,Co,HW,k,stride", [(8, 16, 16, 32, 3, 1), (4, 16, 32, 32, 3, 2), (4, 32, 32, 16, 3, 1), (4, 32, 64, 16, 3, 2),
                                                  (6, 64, 64, 8, 3, 1), (4, 16, 32, 32, 1, 2), (2, 32, 8, 16, 3, 1), (150, 16, 16, 32, 3, 1), (2, 64, 16, 64, 3, 1), (3, 16, 32, 28, 3, 1), (2, 32, 64, 7, 3, 1), (300, 32, 32, 16, 3, 1)])
 def test_conv_wgrad_tensor_core(C, N, Ci, Co, HW, k, stride):
