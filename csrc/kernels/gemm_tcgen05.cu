@@ -695,6 +695,195 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------------------------
+// 256x256 pair tiles with the reduction split over two pairs
+// ---------------------------------------------------------------------------------------------
+// For a bf16 result of so few 256x256 tiles that half the SMs would idle (4096 x 512, 2048 x 1024), and a reduction long enough to be
+// worth halving. What bounds such a product is the rate at which an SM takes operands from L2, and a pair tile takes half of what
+// 128x128 tiles on every SM do for the same arithmetic. A cluster of four CTAs works on one tile: CTAs 0, 1 sum the first half of K,
+// CTAs 2, 3 the second. Each CTA hands its partner (two ranks on) the 128 columns that the partner finishes, through the partner's
+// shared memory, adds what it was handed to its own and runs the epilogue.
+// Back to back in one graph, us, against the best of the persistent kernel's tiles: 4096 x 512 x 2048 12.7 (14.4), x 4096 18.6 (24.4);
+// 2048 x 768 x 3072 14.8 (19.0); 2048 x 1024 x 4096 17.6 (23.8); 1024 x 768 x 2048 11.3 (13.7).
+struct SplitCfg {
+  static constexpr int STAGES = 4, STAGE_BYTES = 2 * BM * BK * 2;
+  static constexpr int XCHG_BYTES = BM * 128 * 4;       // 16-byte chunk c of row r at (c * 128 + r) * 16: lanes (rows) side by side
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + XCHG_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+  static_assert(2 * kEpiWarps * 4096 <= STAGES * STAGE_BYTES, "the epilogue stages its stores where the operands were");
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
+};
+// Below this the hand-over costs more than half the reduction: 4096 x 512, K = 1024 10.2 against 9.8 us, 1280 10.9 both, 1536 11.5 against 12.2.
+constexpr int kSplitMinK = 1280;
+
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared::cluster.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+// grid = (4, row tiles, column tiles), cluster (4, 1, 1)
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
+                  const __grid_constant__ CUtensorMap tmAux, const __grid_constant__ GemmParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  using Cfg = SplitCfg;
+  uint8_t* xchg = smem + Cfg::STAGES * Cfg::STAGE_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(xchg + Cfg::XCHG_BYTES);
+  uint64_t* empty_bar = full_bar + Cfg::STAGES;
+  uint64_t* done_bar = empty_bar + Cfg::STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(cluster_ctarank()), side = rank & 1, part = rank >> 1;
+  const int m0 = blockIdx.y * 2 * BM + side * BM, n0 = blockIdx.z * 256;
+  const int num_kb = (p.K + BK - 1) / BK, kb_half = (num_kb + 1) / 2;      // num_kb >= 2
+  const int kb0 = part * kb_half, kb1 = part ? num_kb : kb_half;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < Cfg::STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    mbar_init(done_bar, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+    tma_prefetch_desc(&tmC);
+    if (p.aux_tma) tma_prefetch_desc(&tmAux);
+  }
+  if (warp == 1) {
+    tmem_alloc<2>(tmem_slot, 256);
+    tmem_relinquish<2>();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  pdl_wait();
+  pdl_launch_dependents();
+
+  // what this CTA finishes: columns [part * 128, part * 128 + 128) of the tile
+  const int q = warp & 3, half = (warp - 2) >> 2, row0 = m0 + q * 32;
+  const uint32_t lane_base = tmem + (static_cast<uint32_t>(q * 32) << 16);
+  bool ok = true;
+  if (warp == 0) {
+    if (lane == 0) {
+      int s = 0;
+      uint32_t ph = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty)) break;
+        uint8_t* sa = smem + s * Cfg::STAGE_BYTES;
+        uint8_t* sb = sa + BM * BK * 2;
+        if (side == 0) mbar_expect_tx(&full_bar[s], 2 * Cfg::STAGE_BYTES);
+        tma_load_2d_pair(sa, &tmA, &full_bar[s], kb * BK, m0);
+        if (!p.b_mn) {
+          tma_load_2d_pair(sb, &tmB, &full_bar[s], kb * BK, n0 + side * 128);
+        } else {
+          tma_load_2d_pair(sb, &tmB, &full_bar[s], n0 + side * 128, kb * BK);
+          tma_load_2d_pair(sb + 8192, &tmB, &full_bar[s], n0 + side * 128 + 64, kb * BK);
+        }
+        if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    if (side == 0 && lane == 0) {
+      const uint32_t idesc = make_idesc_bf16(2 * BM, 256, 0, p.b_mn);
+      const uint32_t b_lbo = p.b_mn ? 8192u : 16u, b_kstep = p.b_mn ? 2048u : 32u;
+      const uint16_t pair = static_cast<uint16_t>(3 << (rank & 2));
+      int s = 0;
+      uint32_t ph = 0;
+      for (int kb = kb0; kb < kb1 && ok; ++kb) {
+        ok = mbar_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint32_t sa = smem_u32(smem + s * Cfg::STAGE_BYTES), sb = sa + BM * BK * 2;
+#pragma unroll
+        for (int k4 = 0; k4 < BK / 16; ++k4)
+          umma_bf16<2>(tmem, make_smem_desc(sa + k4 * 32, 16, 1024), make_smem_desc(sb + k4 * b_kstep, b_lbo, 1024), idesc, (kb > kb0 || k4 > 0) ? 1u : 0u);
+        umma_commit_pair(&empty_bar[s], pair);
+        if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
+      }
+      if (ok) umma_commit_pair(done_bar, pair);
+    }
+  } else {
+    ok = __all_sync(0xffffffffu, mbar_wait(done_bar, 0, abort_flag, p.status, kStatusWaitAccum));
+    if (ok) {       // the partner's columns into the partner's shared memory
+      tc_fence_after_sync();
+      uint32_t there;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(smem_u32(xchg)), "r"(rank ^ 2));
+#pragma unroll 1
+      for (int c = half * 64; c < half * 64 + 64; c += 32) {
+        uint32_t v[32];
+        tmem_ld32(lane_base + (part ^ 1) * 128 + c, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          st_cluster_v4(there + ((c / 4 + j) * 128 + q * 32 + lane) * 16, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      }
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();      // every thread gets here, also after a wait that gave up
+  if (warp >= 2) {
+    const int col0 = n0 + part * 128 + half * 64;
+    if (ok && !*abort_flag && row0 < p.M && col0 < p.N) {
+      uint8_t* stage = smem + (warp - 2) * 4096;           // every product that reads the operands has retired
+      uint8_t* stage_x = smem + (kEpiWarps + warp - 2) * 4096;
+      const uint32_t sc = smem_u32(stage), sx = smem_u32(stage_x), mine = smem_u32(xchg);
+      const float none[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        const int c = half * 64 + 32 * hh;
+        uint32_t acc[32];
+        tmem_ld32(lane_base + part * 128 + c, acc);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 t = ld_shared_f4(mine + ((c / 4 + j) * 128 + q * 32 + lane) * 16);
+          acc[4 * j] = __float_as_uint(__uint_as_float(acc[4 * j]) + t.x);
+          acc[4 * j + 1] = __float_as_uint(__uint_as_float(acc[4 * j + 1]) + t.y);
+          acc[4 * j + 2] = __float_as_uint(__uint_as_float(acc[4 * j + 2]) + t.z);
+          acc[4 * j + 3] = __float_as_uint(__uint_as_float(acc[4 * j + 3]) + t.w);
+        }
+        float v0[32], p0[32];
+        epilogue_compute32(p, acc, row0 + lane, col0 + 32 * hh, true, v0, p0, none, -1);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          st_shared_v4(stage_addr(sc, lane, 4 * hh + j), pack_bf16x2(v0[8 * j], v0[8 * j + 1]), pack_bf16x2(v0[8 * j + 2], v0[8 * j + 3]),
+                       pack_bf16x2(v0[8 * j + 4], v0[8 * j + 5]), pack_bf16x2(v0[8 * j + 6], v0[8 * j + 7]));
+        if (p.aux_tma) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            st_shared_v4(stage_addr(sx, lane, 4 * hh + j), pack_bf16x2(p0[8 * j], p0[8 * j + 1]), pack_bf16x2(p0[8 * j + 2], p0[8 * j + 3]),
+                         pack_bf16x2(p0[8 * j + 4], p0[8 * j + 5]), pack_bf16x2(p0[8 * j + 6], p0[8 * j + 7]));
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(&tmC, stage, col0, row0);
+        if (p.aux_tma) tma_store_2d(&tmAux, stage_x, col0, row0);
+        tma_store_commit();
+        tma_store_wait_read();       // before the shared memory goes away
+      }
+      __syncwarp();
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();        // the pair frees its TMEM together
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc<2>(tmem, 256);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -804,6 +993,56 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   return static_cast<int>(e);
 }
 
+static cudaLaunchConfig_t split_config(int M, int N, cudaLaunchAttribute* attr, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(4, (M + 2 * BM - 1) / (2 * BM), (N + 255) / 256);
+  cfg.blockDim = dim3(kGemmThreads, 1, 1);
+  cfg.dynamicSmemBytes = SplitCfg::SMEM_BYTES;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 4;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// How many clusters of gemm_split_kernel the device holds at once (0: none, or it cannot be told).
+static int split_clusters() {
+  static const int n = [] {
+    if (cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg::SMEM_BYTES) != cudaSuccess) return 0;
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = split_config(2 * BM, 256, attr, nullptr);
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, gemm_split_kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return clusters;
+  }();
+  return n;
+}
+
+// Long reductions (kSplitMinK) with no more tiles than the device holds clusters at once: one more and the last tile would run
+// alone, when the persistent kernel does not need the pairs' full number. Mostly padding (less than 0.8 useful) is left to narrower tiles.
+// Products of fewer than 75 tiles of 128 x 64 went to gemm_small.cu before this is asked.
+static bool split_applies(int M, int N, int K) {
+  const long long tiles = static_cast<long long>((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
+  return K >= kSplitMinK && tiles <= split_clusters() && static_cast<long long>(M) * N * 10 >= tiles * 256 * 256 * 8;
+}
+
+static int launch_split(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tx, const GemmParams& p, cudaStream_t stream) {
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = split_config(p.M, p.N, attr, stream);
+  if (pdl_enabled()) {
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
+  }
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_split_kernel, ta, tb, tc, tx, p));
+}
+
 }  // namespace fb
 
 extern "C" int fb_gemm_bf16_ts(const void*, const void*, void*, int, int, int, long long, long long, long long, int, int, int, const void*, int,
@@ -870,12 +1109,17 @@ extern "C" int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, in
   if (split_k < 1) split_k = 1;
   if (split_k > 1 && !c_fp32) return -2;
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
+  bool over_pairs = false;       // the reduction split over two pairs of a cluster
   if (config < 0) {
     // few output tiles, plain bf16 result: the cluster split (gemm_small.cu)
     if (!c_fp32 && !a_mn && !accumulate && split_k == 1 && !m_dyn && !k_dyn && !ts && gemm_small_aligned(N, C, ldc, aux, ldaux))
       if (const int split = gemm_small_split(M, N, K))
         return gemm_small(A, &B, C, M, N, 1, K, lda, ldb, ldc, b_mn, &bias, bias_fp32, epi, aux, ldaux, alpha, split, status, stream);
-    config = fb_gemm_pick_config(M, N, K, split_k);
+    const bool act = epi == FB_EPI_GELU_ERF || epi == FB_EPI_GELU_TANH;
+    if (!c_fp32 && !a_mn && !accumulate && split_k == 1 && !m_dyn && !k_dyn && !ts && ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 &&
+        (!act || !aux || (ldaux % 8 == 0 && (reinterpret_cast<uintptr_t>(aux) & 15) == 0)) && split_applies(M, N, K))
+      over_pairs = true;
+    config = over_pairs ? 0 : fb_gemm_pick_config(M, N, K, split_k);
     if (config == 5 && b_mn) config = 0;          // 256x192 pair tiles need a K-major B
   }
   if (config == 5 && b_mn) return -5;
@@ -919,6 +1163,7 @@ extern "C" int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, in
   p.bias = bias; p.bias_fp32 = bias_fp32; p.epi = epi; p.aux = aux; p.ldaux = ldaux; p.alpha = alpha;
   p.accumulate = accumulate; p.split_k = split_k; p.status = status; p.ts = ts;
   p.m_dyn = m_dyn; p.k_dyn = k_dyn;
+  if (over_pairs) return launch_split(ta, tb, tc, tx, p, stream);
   switch (config) {
     case 0: return launch_gemm<2, 256>(ta, tb, tc, tx, p, stream);
     case 1: return launch_gemm<1, 256>(ta, tb, tc, tx, p, stream);

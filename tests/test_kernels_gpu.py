@@ -106,7 +106,7 @@ def test_gemm_fp32_out_accumulate_splitk_alpha(C):
 
 @pytest.mark.parametrize("M,N,K,b_mn,epi", [(1, 768, 768, False, 0), (77, 768, 3072, False, 0), (77, 3072, 768, False, 1), (128, 64, 64, True, 0), (129, 68, 72, False, 3),
                                             (300, 128, 520, True, 2), (512, 512, 128, True, 4), (130, 60, 4096, False, 0)])
-def test_gemm_few_tiles(C, M, N, K, b_mn, epi):
+def test_gemm_few_tiles(C, M, N, K, b_mn, epi, pad=4):
     """Products of few output tiles, which the dispatch gives to the kernel that splits K over a cluster: edges of tiles and of the split, both
     layouts of B, every epilogue, strided output. Against 64 bits: the output carries one rounding to bf16 (2^-8 at most), GELU' is taken of a
     stored, rounded value, the fast GELU adds 6e-5 absolute; in norm all of it stays below one such rounding."""
@@ -115,7 +115,7 @@ def test_gemm_few_tiles(C, M, N, K, b_mn, epi):
     b = (torch.randn(N, K, device="cuda") / math.sqrt(K)).bfloat16()
     bm = b.t().contiguous() if b_mn else b
     bias = torch.randn(N, device="cuda") if epi in (0, 1, 3) else None
-    out = torch.zeros(M, N + 4, device="cuda").bfloat16()
+    out = torch.zeros(M, N + pad, device="cuda").bfloat16()
     aux = torch.randn(M, N, device="cuda").bfloat16()
     alpha = torch.tensor([0.5], device="cuda") if epi == 0 else None
     C.clear_status(0)
@@ -134,6 +134,15 @@ def test_gemm_few_tiles(C, M, N, K, b_mn, epi):
         ref = x.grad
     assert ((out[:, :N].double() - ref).norm() / ref.norm()).item() < 2 ** -8
     assert torch.all(out[:, N:] == 0)
+
+
+@pytest.mark.parametrize("M,N,K", [(1800, 1000, 1352), (1300, 504, 1544), (4096, 512, 2048)])
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("epi", [0, 1, 2, 3, 4])
+def test_gemm_two_pairs(C, M, N, K, b_mn, epi):
+    """Products of 12 to 32 tiles of 256 x 256 and a long reduction, which the dispatch splits over two pairs of a cluster where the device holds
+    that many clusters: whole and ragged tiles, an odd number of reduction steps. Bounds as for the products of few tiles."""
+    test_gemm_few_tiles(C, M, N, K, b_mn, epi, pad=8)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
