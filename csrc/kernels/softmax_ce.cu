@@ -207,7 +207,11 @@ extern "C" int fb_softmax_ce_dyn(const void* logits, long long ld, const long lo
   // Short rows: a warp each, eight to a block (a block-wide reduction would cost more than the row); the line is where a
   // block's 512 threads get a vector each. Long rows: a block each, as many as stay resident.
   const bool warp_row = V <= (is_bf16 ? 4096 : 2048);
-  const dim3 grid(warp_row ? static_cast<unsigned>((rows + 7) / 8) : static_cast<unsigned>(rows < 3 * 148 ? rows : 3 * 148)), block(warp_row ? 256 : 512);
+  // (Rows of up to 64 KB take half the threads and twice the blocks: a row's barrier and its exponentials then hide behind others'
+  // loads. us, bf16: 2000 x 5000 19.3 -> 14.5, 8192 x 8000 102 -> 82, 8192 x 32000 258 -> 243. Longer ones would leave L2 before their second read.)
+  const bool half_block = static_cast<long long>(V) * (is_bf16 ? 2 : 4) <= 65536;
+  const int resident = 148 * (half_block ? 6 : 3);
+  const dim3 grid(static_cast<unsigned>(warp_row ? (rows + 7) / 8 : rows < resident ? rows : resident)), block(warp_row || half_block ? 256 : 512);
   auto go = [&](auto kern, auto* x, auto* dx) {
     fb::launch_pdl(kern, grid, block, 0, st, x, ld, targets, rows, V, ignore_index, dx, ldd, count_inv, row_loss, counts);
   };

@@ -196,6 +196,23 @@ def test_layernorm_rows_per_warp(C, dtype, rows, cols):
     assert close(acc_g - 1, dg.double(), 2 ** -14) and close(acc_b - 1, db.double(), 2 ** -14)
 
 
+@pytest.mark.parametrize("dtype,V", [(torch.bfloat16, 4104), (torch.bfloat16, 32768), (torch.bfloat16, 32776), (torch.float32, 16384), (torch.float32, 16388)])
+def test_softmax_ce_block_sizes(C, dtype, V):
+    """Either side of the row length at which a block's size changes, with more rows than resident blocks. The gradient carries one rounding to its
+    type; the loss is a mean of 32-bit values near 10, each within two units in the last place."""
+    torch.manual_seed(18)
+    rows = 900
+    x = torch.randn(rows, V, device="cuda").to(dtype)
+    t = torch.randint(0, V, (rows,), device="cuda")
+    loss, dl, _ = C.softmax_ce(x, t, -100, True, False)
+    xd = x.double()
+    p = torch.softmax(xd, 1)
+    p[torch.arange(rows, device="cuda"), t] -= 1
+    ref = torch.nn.functional.cross_entropy(xd, t)
+    assert abs(loss.double().item() - ref.item()) < 2 ** -21 * abs(ref.item())
+    assert ((dl.double() - p / rows).norm() / (p / rows).norm()).item() < (2 ** -8 if dtype == torch.bfloat16 else 2 ** -18)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("tokens,dim,ids", [(1, 8, "random"), (4099, 768, "equal"), (777, 1028, "runs"), (5000, 64, "random"), (33, 30, "runs")])
 def test_embedding_bwd_runs(C, dtype, tokens, dim, ids):
