@@ -420,7 +420,6 @@ namespace {
 
 constexpr int kFwdSoftmaxWarps = 8;
 constexpr int kFwdThreads = 32 * (kFwdSoftmaxWarps + 2);
-constexpr float kRescaleAt = 8.f;      // log2 of the factor by which a row maximum may grow before its accumulator is rescaled
 
 struct FwdLong {
   static constexpr int Q = 0;
@@ -608,7 +607,10 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         ok = __all_sync(0xffffffffu, mbar_wait(pv_done, (j - 1) & 1, abort_flag, p.status, kStatusWaitAccum));     // P may be overwritten, O touched
         if (!ok) continue;
         tc_fence_after_sync();
-        if (__any_sync(0xffffffffu, m_new > m_ref + kRescaleAt)) {       // the same for both warps of a row; each rescales half of O's columns
+        // At every growth, however small: relative to the true maximum a row's largest probability is exactly 1 and takes no rounding to bf16,
+        // relative to an older one it is rounded like the rest (up to a fifth more error where few keys carry a row).
+        // B 2 x H 12 x S 4096 causal: 101 us; 95 with rescaling at growths of 2^8 only.
+        if (__any_sync(0xffffffffu, m_new > m_ref)) {       // the same for both warps of a row; each rescales half of O's columns
           const float alpha = m_new == -INFINITY ? 1.f : ex2_approx(m_ref - m_new);
           m_ref = m_new;
           l_run *= alpha;

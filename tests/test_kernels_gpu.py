@@ -445,6 +445,24 @@ def test_attention_several_key_blocks(C, B, H, S, causal, use_mask):
         assert ((dqkv[:, :, i].double() - t.grad).norm() / t.grad.norm()).item() < 2 ** -7, i     # through P and dS both
 
 
+def test_attention_running_maximum(C):
+    """A key of a later block outweighs the first block's by a factor of 2^1 to 2^8, and it alone has a value: the output is that value over the
+    row's 32-bit sum. Relative to the row's true maximum its probability is 1, so that only the output's own rounding to bf16 is left: 2^-8 of each
+    value at most, and 2^-6 of that for the 32-bit sums and exponentials."""
+    S, D = 384, 64
+    torch.manual_seed(19)
+    qkv = torch.zeros(1, S, 3, 1, D, device="cuda").bfloat16()
+    q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
+    q[0, :, 0, 0] = torch.linspace(0.7, 5.5, S, device="cuda").bfloat16()       # the key's score above the others', in natural units
+    k[0, 200, 0, 0] = 8.0
+    v[0, 200, 0] = torch.randn(D, device="cuda").bfloat16()
+    o, lse = C.attn_fwd(q, k, v, None, 0.125, False)
+    ref = _attn_ref(q.double(), k.double(), v.double(), None, 0.125, False)
+    assert ((o.double() - ref).abs() / ref.abs()).max().item() < 2 ** -8 * (1 + 2 ** -6)
+    x = q[0, :, 0, 0].double()
+    assert (lse[0, 0].double() - torch.log(x.exp() + S - 1)).abs().max().item() < 2 ** -18
+
+
 def test_attention_several_key_blocks_dropout(C):
     """O is linear in V for fixed probabilities, so <dO, O> = <dV, V> exactly if and only if backward drops what forward dropped."""
     torch.manual_seed(12)
