@@ -11,9 +11,9 @@
 // the scratch and leaves D = rowsum(dO * O) in the first word of each dQ row; a pass after turns the scratch into bf16 rows.
 // What bounds it: the chain scores -> exponentials -> P and dS in shared memory -> products of one tile, with the shared-memory
 // pipe (P and dS are written once and read by three products) as its slowest part.
-// Forward + backward, bf16, us: B 2 x H 12 x S 4096 causal 96 + 253 (118 + 338 with eight softmax warps, reductions from registers and
-// persistent CTAs), B 4 x H 8 x S 1024 causal 19 + 38 (24 + 47), B 6 x H 12 x S 509 causal 13 + 39 (15 + 43), B 32 x H 8 x S 256 causal
-// 14 + 48 (16 + 49), B 64 x H 12 x S 384 75 + 264 (89 + 257: with three tiles to a CTA its start and end show, which the persistent
+// Forward + backward, bf16, us: B 2 x H 12 x S 4096 causal 100 + 253 (118 + 338 with eight softmax warps, reductions from registers and
+// persistent CTAs), B 4 x H 8 x S 1024 causal 20 + 38 (24 + 47), B 6 x H 12 x S 509 causal 13 + 39 (15 + 43), B 32 x H 8 x S 256 causal
+// 14 + 48 (16 + 49), B 64 x H 12 x S 384 78 + 264 (89 + 257: with three tiles to a CTA its start and end show, which the persistent
 // form hid; longer rows gain more than these lose).
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -431,7 +431,10 @@ struct FwdLong {
   static constexpr int TOTAL = BARS + 256;
 };
 
-template <bool kDrop>
+// kMask: whether there is an additive mask. The last, ragged key block without one is cut off like the diagonal. Instances of their own, because
+// the mask is needed twice, for the maximum and for the exponent: both forms in one kernel spilled (B 64 x H 12 x S 384 with a mask 118 us against
+// 102, B 2 x H 12 x S 4096 causal without 120 against 100).
+template <bool kDrop, bool kMask>
 __global__ void __launch_bounds__(kFwdThreads, 2)
 attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                      __nv_bfloat16* __restrict__ o, float* __restrict__ lse, const AttnParams p) {
@@ -539,8 +542,9 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // (two warps share 32 rows: four warps a scheduler with two CTAs, which is what hides the TMEM loads and the exponentials' latency)
     const int quarter = warp & 3, half = warp >> 2, t = quarter * 32 + lane, q = q0 + t;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-    const float sc = p.scale * kLog2e;
+    const float sc = p.scale == 0.f ? 1e-37f : p.scale * kLog2e;       // never 0: a score of -inf has to stay one
     const float inv_keep = kDrop ? 1.f / (1.f - p.p_drop) : 1.f;
+    const float hidden = sc < 0.f ? INFINITY : -INFINITY;               // the score of a key that the row does not see
     float* xchg = reinterpret_cast<float*>(smem + L::XCHG);
     // the other half row's value; the two warps of a quarter meet, one of the two slots being free for the next exchange
     auto exchange = [&](int slot, float mine) {
@@ -553,19 +557,18 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // After a wait that gave up the loop runs out without work, so that no warp is missed at the barriers.
     for (int j = 0; j < n; ++j) {
       const int kv0 = j * kBlk, c0 = half * 64;
-      const bool masked = p.mask != nullptr || kv0 + kBlk > p.S;
       const bool diagonal = p.causal && j == qb;
       const float* mk_s = mask_s + (j & 1) * kBlk + c0;
-      if (masked) {       // additive mask of this key block (mask * log2e; -inf beyond S); the other buffer may still be in use
+      if constexpr (kMask) {       // additive mask of this key block (mask * log2e; -inf beyond S); the other buffer may still be in use
         if (half == 0) {
           const int kv = kv0 + t;
-          mask_s[(j & 1) * kBlk + t] = kv < p.S ? (p.mask ? __ldg(p.mask + static_cast<long long>(b) * p.S + kv) * kLog2e : 0.f) : -INFINITY;
+          mask_s[(j & 1) * kBlk + t] = kv < p.S ? __ldg(p.mask + static_cast<long long>(b) * p.S + kv) * kLog2e : -INFINITY;
         }
         asm volatile("bar.sync 1, 256;" ::: "memory");
       }
       ok = __all_sync(0xffffffffu, ok && mbar_wait(s_full, j & 1, abort_flag, p.status, kStatusWaitAccum));
       uint32_t sv[2][32];
-      float m_half = -INFINITY, mul = sc;
+      float m_half = -INFINITY;
       if (ok) {
         tc_fence_after_sync();
         tmem_ld32(tS + lane_base + c0, sv[0]);
@@ -573,31 +576,40 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tmem_ld_wait();
         tc_fence_before_sync();
         arrive_warp(s_free, lane);
-        // row maximum; with a mask, on the diagonal or for a negative scale the scores are scaled here, otherwise in the exponent below
+        // row maximum of score * scale (+ mask); the scores stay as they came for the exponent below
+        if (kMask ? diagonal : diagonal || kv0 + kBlk > p.S) {
+          const int seen = (p.causal ? min(q, p.S - 1) : p.S - 1) - kv0 - c0;
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (32 * c + i > seen) sv[c][i] = __float_as_uint(hidden);
+        }
         float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-        if (masked || diagonal || sc < 0.f) {
-          mul = 1.f;
+        if constexpr (kMask) {
 #pragma unroll
           for (int c = 0; c < 2; ++c)
 #pragma unroll
             for (int i4 = 0; i4 < 32; i4 += 4) {
-              const float4 mk = masked ? *reinterpret_cast<const float4*>(mk_s + 32 * c + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
+              const float4 mk = *reinterpret_cast<const float4*>(mk_s + 32 * c + i4);
               const float mk4[4] = {mk.x, mk.y, mk.z, mk.w};
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                float s = __uint_as_float(sv[c][i4 + k]) * sc + mk4[k];
-                if (diagonal && kv0 + c0 + 32 * c + i4 + k > q) s = -INFINITY;
-                sv[c][i4 + k] = __float_as_uint(s);
-                m4[k] = fmaxf(m4[k], s);
-              }
+              for (int k = 0; k < 4; ++k) m4[k] = fmaxf(m4[k], fmaf(__uint_as_float(sv[c][i4 + k]), sc, mk4[k]));
             }
+          m_half = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+        } else if (sc < 0.f) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int i = 0; i < 32; ++i) m4[i & 3] = fmaxf(m4[i & 3], -__uint_as_float(sv[c][i]));
+          m_half = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * -sc;
         } else {
 #pragma unroll
           for (int c = 0; c < 2; ++c)
 #pragma unroll
             for (int i = 0; i < 32; ++i) m4[i & 3] = fmaxf(m4[i & 3], __uint_as_float(sv[c][i]));
+          m_half = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * sc;
         }
-        m_half = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * mul;
       }
       const float m_new = fmaxf(m_ref, fmaxf(m_half, exchange(j & 1, m_half)));
       if (!ok) continue;
@@ -609,7 +621,7 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tc_fence_after_sync();
         // At every growth, however small: relative to the true maximum a row's largest probability is exactly 1 and takes no rounding to bf16,
         // relative to an older one it is rounded like the rest (up to a fifth more error where few keys carry a row).
-        // B 2 x H 12 x S 4096 causal: 101 us; 95 with rescaling at growths of 2^8 only.
+        // B 2 x H 12 x S 4096 causal: 100 us; 95 with rescaling at growths of 2^8 only.
         if (__any_sync(0xffffffffu, m_new > m_ref)) {       // the same for both warps of a row; each rescales half of O's columns
           const float alpha = m_new == -INFINITY ? 1.f : ex2_approx(m_ref - m_new);
           m_ref = m_new;
@@ -630,10 +642,18 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float pe = ex2_approx(fmaf(__uint_as_float(sv[c][i]), mul, neg_m));
-          l4[i & 3] += pe;
-          sv[c][i] = __float_as_uint(pe);
+        for (int i4 = 0; i4 < 32; i4 += 4) {
+          float off[4] = {neg_m, neg_m, neg_m, neg_m};
+          if constexpr (kMask) {       // mask - maximum first, then one FMA: a large mask common to the row's keys costs the scores no bits
+            const float4 mk = *reinterpret_cast<const float4*>(mk_s + 32 * c + i4);
+            off[0] += mk.x; off[1] += mk.y; off[2] += mk.z; off[3] += mk.w;
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float pe = ex2_approx(fmaf(__uint_as_float(sv[c][i4 + k]), sc, off[k]));
+            l4[k] += pe;
+            sv[c][i4 + k] = __float_as_uint(pe);
+          }
         }
         if constexpr (kDrop) {
           const unsigned long long base = ((static_cast<unsigned long long>(b) * p.H + h) * p.S + q) * p.S + kv0 + c0 + 32 * c;
@@ -697,10 +717,11 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 }  // namespace
 
 int attn_fwd_long(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* o, float* lse, const AttnParams& p, cudaStream_t stream) {
-  const auto kern = p.p_drop > 0.f ? attn_fwd_long_kernel<true> : attn_fwd_long_kernel<false>;
+  const auto kern = p.p_drop > 0.f ? (p.mask ? attn_fwd_long_kernel<true, true> : attn_fwd_long_kernel<true, false>)
+                                   : (p.mask ? attn_fwd_long_kernel<false, true> : attn_fwd_long_kernel<false, false>);
   static bool configured = false;
   if (!configured) {
-    for (auto k : {attn_fwd_long_kernel<true>, attn_fwd_long_kernel<false>}) {
+    for (auto k : {attn_fwd_long_kernel<true, true>, attn_fwd_long_kernel<true, false>, attn_fwd_long_kernel<false, true>, attn_fwd_long_kernel<false, false>}) {
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdLong::TOTAL + 1024);
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       if (e != cudaSuccess) return static_cast<int>(e);

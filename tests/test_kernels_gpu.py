@@ -463,6 +463,20 @@ def test_attention_running_maximum(C):
     assert (lse[0, 0].double() - torch.log(x.exp() + S - 1)).abs().max().item() < 2 ** -18
 
 
+def test_attention_mask_common_to_all_keys(C):
+    """A mask value that all keys of a text share does not change the softmax. The score plus -1e6 keeps three bits after the point in
+    32 bits; the kernel has to take the maximum off the mask before it adds the score. Bound as for the cases above: 2^-8 in norm."""
+    torch.manual_seed(20)
+    for S, causal in ((300, False), (300, True), (640, False)):
+        q, k, v = torch.randn(2, S, 3, 2, 64, device="cuda").bfloat16().unbind(2)
+        mask = torch.zeros(2, S, device="cuda")
+        mask[1] = -1e6
+        o, _ = C.attn_fwd(q, k, v, mask, 0.125, causal)
+        ref = _attn_ref(q.double(), k.double(), v.double(), None, 0.125, causal)
+        for b in range(2):
+            assert ((o[b].double() - ref[b]).norm() / ref[b].norm()).item() < 2 ** -8, (S, causal, b)
+
+
 def test_attention_several_key_blocks_dropout(C):
     """O is linear in V for fixed probabilities, so <dO, O> = <dV, V> exactly if and only if backward drops what forward dropped."""
     torch.manual_seed(12)
