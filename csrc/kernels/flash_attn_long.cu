@@ -3,18 +3,19 @@
 //
 // Backward: one CTA per (key block of 128 rows, head, batch) walks the query blocks that see it. K, V and the dK / dV
 // accumulators stay put; Q and dO stream through a three-stage TMA ring. Roles: 16 softmax warps (thread = one query row x
-// 32 keys), 4 warps that drain dQ, one MMA issuer, one TMA producer. S and dP of the next query block are issued as soon
-// as the softmax warps have loaded this block's into registers, so the tensor cores work under the exponentials.
-// A query block's dQ is a sum over key blocks, i.e. over CTAs: it is added into an fp32 scratch with bulk reductions. The
-// scratch is not row-major: within the 32 rows a warp owns, 16-byte chunk c of row r sits at (c * rows + r) * 16, so that
-// the 32 lanes (one row each) write the staging area, which is copied as it is, without bank conflicts. A pass before zeroes
-// the scratch and leaves D = rowsum(dO * O) in the first word of each dQ row; a pass after turns the scratch into bf16 rows.
+// 32 keys), 4 warps that drain dQ, one that adds it to the scratch, one MMA issuer, one TMA producer. S and dP of the next query
+// block are issued as soon as the softmax warps have loaded this block's into registers, so the tensor cores work under the exponentials.
+// A query block's dQ is a sum over key blocks, i.e. over CTAs: it is added into an fp32 scratch with bulk reductions, in the order of
+// the key blocks, so that two calls give the same bits. The scratch is not row-major: within the 32 rows a warp owns, 16-byte chunk c of
+// row r sits at (c * rows + r) * 16, so that the 32 lanes (one row each) write the staging area, which is copied as it is, without bank
+// conflicts. A pass before zeroes the scratch and leaves D = rowsum(dO * O) in the first word of each dQ row; a pass after turns the
+// scratch into bf16 rows.
 // What bounds it: the chain scores -> exponentials -> P and dS in shared memory -> products of one tile, with the shared-memory
-// pipe (P and dS are written once and read by three products) as its slowest part.
-// Forward + backward, bf16, us: B 2 x H 12 x S 4096 causal 100 + 253 (118 + 338 with eight softmax warps, reductions from registers and
-// persistent CTAs), B 4 x H 8 x S 1024 causal 20 + 38 (24 + 47), B 6 x H 12 x S 509 causal 13 + 39 (15 + 43), B 32 x H 8 x S 256 causal
-// 14 + 48 (16 + 49), B 64 x H 12 x S 384 78 + 264 (89 + 257: with three tiles to a CTA its start and end show, which the persistent
-// form hid; longer rows gain more than these lose).
+// pipe (P and dS are written once and read by three products) as its slowest part. The fixed order costs a causal head's first CTAs, which start
+// together, about 4 us for each block between them (from the end of one's additions to the start of the next one's).
+// Forward + backward, bf16, us; in brackets the backward with additions in order of arrival: B 2 x H 12 x S 4096 causal 99 + 275 (252), full
+// 204 + 490 (496), B 4 x H 8 x S 1024 causal 20 + 45 (37), B 6 x H 12 x S 509 causal 13 + 33 (31), B 32 x H 8 x S 256 causal 14 + 46 (47),
+// B 64 x H 12 x S 384 78 + 275 (262). Eight softmax warps, reductions from registers and persistent CTAs took 338 at 4096 causal.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -31,7 +32,7 @@ namespace {
 constexpr int kSMs = 148;
 constexpr int kBwdStages = 3;
 constexpr int kBwdSoftmaxWarps = 16;
-constexpr int kBwdThreads = 32 * (kBwdSoftmaxWarps + 4 + 2);
+constexpr int kBwdThreads = 32 * (kBwdSoftmaxWarps + 4 + 3);
 
 struct BwdLong {
   static constexpr int Q = 0;                                   // kBwdStages x 16 KB
@@ -40,25 +41,24 @@ struct BwdLong {
   static constexpr int V = K + 16384;
   static constexpr int P = V + 16384;                           // 2 panels of 16 KB
   static constexpr int DS = P + 2 * 16384;                      // 2 panels of 16 KB
-  static constexpr int DQ = DS + 2 * 16384;                     // 4 warps x 4 KB: dQ on its way out
-  static constexpr int STATS = DQ + 4 * 4096;                   // 2 x 128 x {lse, D}
+  static constexpr int DQ = DS + 2 * 16384;                     // 4 warps x 8 KB: dQ on its way out
+  static constexpr int STATS = DQ + 4 * 8192;                   // 2 x 128 x {lse, D}
   static constexpr int MASK = STATS + 2 * 128 * 8;              // 128 floats
   static constexpr int BARS = MASK + 512;
   static constexpr int TOTAL = BARS + 256;
 };
-static_assert(BwdLong::TOTAL + 1024 <= 227 * 1024, "shared memory budget");
+static_assert(BwdLong::TOTAL <= 227 * 1024, "shared memory budget");
 
-// CTA index -> (block, head, batch). Causal: every block of equal length before the next shorter one (the longest first, so
-// the last wave is short). Otherwise all blocks of a head together, which keeps its K / V (or Q / dO) in L2.
-__device__ __forceinline__ void decode_block(int lin, int nblk, int H, int B, bool causal, int& blk, int& h, int& b) {
-  int hb;
-  if (causal) {
-    blk = lin / (H * B);
-    hb = lin - blk * (H * B);
-  } else {
-    hb = lin / nblk;
-    blk = lin - hb * nblk;
-  }
+// Work item -> (block, head, batch). Causal: every block of equal length before the next shorter one (the longest first, so the last wave is
+// short). Otherwise all blocks of a head together, which keeps its K / V (or Q / dO) in L2 (a group of 1), or one block of each of
+// `group` heads after the other, so that blocks of one head, which add to dQ in turn, seldom run side by side (B 2 x H 12 x S 4096, all heads
+// in one group 490 us, groups of 1 635).
+__device__ __forceinline__ void decode_block(int lin, int nblk, int H, int B, bool causal, int group, int& blk, int& h, int& b) {
+  const int heads = H * B;
+  if (causal) group = heads;
+  const int first = lin / (group * nblk) * group, size = min(group, heads - first), rest = lin - first * nblk;
+  blk = rest / size;
+  const int hb = first + rest - blk * size;
   b = hb / H;
   h = hb - b * H;
 }
@@ -69,8 +69,33 @@ __device__ __forceinline__ void bulk_add(float* dst, uint32_t src, uint32_t byte
   asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
 }
 
-// Per query row: D = dot(dO, O) into the first word of the row's dQ slot (overwritten by attn_dq_kernel at the end), and the
-// row's share of the dQ scratch zeroed. Eight lanes per row, rows of one (batch, head) consecutive.
+// What the first words of a dQ row hold until the row itself is written.
+struct DqSlot {
+  float D;
+  unsigned int added;        // of a query block's first row: how many key blocks have been added to the block's scratch
+  unsigned int ticket;       // of the very first row: work items handed out
+  unsigned int unused;
+};
+
+// Waits until `want` key blocks have been added. Bounded like mbar_wait; a block that gave up never adds, which its status tells the others.
+__device__ __forceinline__ bool wait_added(const unsigned int* added, unsigned int want, volatile int* abort_flag, int* status) {
+  for (uint32_t it = 0; it < (1u << 20); ++it) {
+    unsigned int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(added) : "memory");
+    if (v >= want) {
+      fence_proxy_async_global();
+      return true;
+    }
+    if (*abort_flag || ((it & 4095) == 4095 && status && *reinterpret_cast<volatile int*>(status) != kStatusOk)) break;
+    if (it > 16) __nanosleep(40);
+  }
+  *abort_flag = 1;
+  set_status(status, kStatusWaitAccum);
+  return false;
+}
+
+// Per query row: the first words of the row's dQ slot (overwritten by attn_dq_kernel at the end) take D = dot(dO, O) and two zeroed
+// counters (DqSlot), and the row's share of the dQ scratch is zeroed. Eight lanes per row, rows of one (batch, head) consecutive.
 __global__ void __launch_bounds__(256) attn_bwd_pre_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                                                            __nv_bfloat16* __restrict__ dq, float* __restrict__ dq_accum, const AttnParams p) {
   pdl_entry();
@@ -94,7 +119,7 @@ __global__ void __launch_bounds__(256) attn_bwd_pre_kernel(const __nv_bfloat16* 
     d += __shfl_xor_sync(m, d, 1);
     d += __shfl_xor_sync(m, d, 2);
     d += __shfl_xor_sync(m, d, 4);
-    if (ch == 0) *reinterpret_cast<float*>(dq + b * p.gsb + h * p.gsh + s * p.gss) = d;
+    if (ch == 0) *reinterpret_cast<uint4*>(dq + b * p.gsb + h * p.gsh + s * p.gss) = make_uint4(__float_as_uint(d), 0u, 0u, 0u);
     float4* z = reinterpret_cast<float4*>(dq_accum + r * kHD + ch * 8);
     z[0] = z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -119,10 +144,16 @@ __global__ void __launch_bounds__(256) attn_dq_kernel(const float* __restrict__ 
 
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                     const __grid_constant__ CUtensorMap tmDO, const float* __restrict__ lse, const __nv_bfloat16* __restrict__ dq,
+                     const __grid_constant__ CUtensorMap tmDO, const float* __restrict__ lse, __nv_bfloat16* dq,
                      __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, float* __restrict__ dq_accum, const AttnParams p) {
+  // No room for alignment slack: the kernel relies on the 1024-byte alignment of the dynamic shared-memory window and reports instead of
+  // computing if that does not hold.
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw;
+  if ((smem_u32(smem_raw) & 1023u) != 0) {
+    if (threadIdx.x == 0) set_status(p.status, kStatusBadArg);
+    return;
+  }
   using L = BwdLong;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BARS);
   uint64_t* kv_full = bars;
@@ -135,19 +166,26 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint64_t* dq_full = grads_full + 1;             // [2] the same event, per dQ buffer, for the draining warps
   uint64_t* dq_free = dq_full + 2;                // [2] the buffer has been read
   uint64_t* stat_full = dq_free + 2;              // [2] lse and D of a query block are in shared memory
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stat_full + 2);
+  uint64_t* staged = stat_full + 2;               // dQ of a query block is in shared memory
+  uint64_t* stage_free = staged + 1;              // ... and has been read from there
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stage_free + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* item = abort_flag + 1;            // key block, head, batch: reloaded where needed, the softmax warps have no registers to spare
   float* mask_s = reinterpret_cast<float*>(smem + L::MASK);
   float2* stats = reinterpret_cast<float2*>(smem + L::STATS);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nblk = (p.S + kBlk - 1) / kBlk;
-  int j, h, b;
-  decode_block(blockIdx.x, nblk, p.H, p.B, p.causal != 0, j, h, b);
-  const int kv0 = j * kBlk, i0 = p.causal ? j : 0, n = nblk - i0;
-  const long long bh = static_cast<long long>(b) * p.H + h;
-  const unsigned long long seed = p.seed + (p.seed_dev ? *p.seed_dev : 0ull);
-
+  // The key blocks of a head add to dQ in order (below), so a block may only wait for blocks that run already: the work is handed out by a
+  // counter, in an order in which a head's earlier key blocks come first.
+  const bool ordered = nblk > 2;
+  if (ordered) pdl_entry();       // the counter is the previous kernel's
+  if (warp == kBwdSoftmaxWarps + 5 && lane == 0) {
+    const int lin = ordered ? static_cast<int>(atomicAdd(&reinterpret_cast<DqSlot*>(dq)->ticket, 1u)) : blockIdx.x;
+    int j, h, b;
+    decode_block(lin, nblk, p.H, p.B, p.causal != 0, ordered ? kSMs : 1, j, h, b);
+    item[0] = j; item[1] = h; item[2] = b;
+  }
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     for (int s = 0; s < kBwdStages; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
@@ -156,6 +194,8 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     mbar_init(pds_ready, kBwdSoftmaxWarps);
     mbar_init(grads_full, 1);
     for (int s = 0; s < 2; ++s) { mbar_init(&dq_full[s], 1); mbar_init(&dq_free[s], 4); mbar_init(&stat_full[s], 4); }
+    mbar_init(staged, 4);
+    mbar_init(stage_free, 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -168,20 +208,25 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tS = tmem_base, tDP = tmem_base + 128, tDV = tmem_base + 256, tDK = tmem_base + 320, tDQ = tmem_base + 384;
-  pdl_entry();
+  if (!ordered) pdl_entry();
+  // Query blocks from the last to the first that sees the keys: key blocks of a causal head that start together meet at their first query
+  // block and then stay one hand-over apart; from the first to the last they would meet anew, one block later, at every step.
+  const int n = p.causal ? nblk - item[0] : nblk;
+  const auto query_block = [&](int it) { return nblk - 1 - it; };
 
   if (warp == kBwdSoftmaxWarps + 5) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
+      const int j = item[0], h = item[1], b = item[2];
       mbar_expect_tx(kv_full, 32768);
-      tma_load_4d(smem + L::K, &tmK, kv_full, 0, kv0, h, b);
-      tma_load_4d(smem + L::V, &tmV, kv_full, 0, kv0, h, b);
+      tma_load_4d(smem + L::K, &tmK, kv_full, 0, j * kBlk, h, b);
+      tma_load_4d(smem + L::V, &tmV, kv_full, 0, j * kBlk, h, b);
       for (int it = 0; it < n; ++it) {
         const int st = it % kBwdStages;
         if (!mbar_wait(&q_empty[st], ((it / kBwdStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitEmpty)) break;
         mbar_expect_tx(&q_full[st], 32768);
-        tma_load_4d(smem + L::Q + st * 16384, &tmQ, &q_full[st], 0, (i0 + it) * kBlk, h, b);
-        tma_load_4d(smem + L::DO + st * 16384, &tmDO, &q_full[st], 0, (i0 + it) * kBlk, h, b);
+        tma_load_4d(smem + L::Q + st * 16384, &tmQ, &q_full[st], 0, query_block(it) * kBlk, h, b);
+        tma_load_4d(smem + L::DO + st * 16384, &tmDO, &q_full[st], 0, query_block(it) * kBlk, h, b);
       }
     }
   } else if (warp == kBwdSoftmaxWarps + 4) {
@@ -235,17 +280,41 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         umma_commit(&q_empty[st]);
       }
     }
+  } else if (warp == kBwdSoftmaxWarps + 6) {
+    // ------------------------------------------------------------------ dQ into the scratch
+    // One thread adds a query block's 128 rows at once. A sum of three or more depends on its order, so the third and later key blocks wait
+    // for the ones before them; the first two may come either way round, 0 + a + b being 0 + b + a.
+    if (lane == 0) {
+      const int j = item[0], h = item[1], b = item[2];
+      const uint32_t src = smem_u32(smem + L::DQ);
+      for (int it = 0; it < n; ++it) {
+        const int qblk = query_block(it), row0 = qblk * kBlk, adders = p.causal ? qblk + 1 : nblk;
+        unsigned int* added = &reinterpret_cast<DqSlot*>(dq + b * p.gsb + h * p.gsh + row0 * p.gss)->added;
+        if (!mbar_wait(staged, it & 1, abort_flag, p.status, kStatusWaitAccum)) break;
+        if (j >= 2 && !wait_added(added, static_cast<unsigned int>(j), abort_flag, p.status)) break;
+        bulk_add(dq_accum + ((static_cast<long long>(b) * p.H + h) * p.S + row0) * kHD, src, min(kBlk, p.S - row0) * kHD * 4);
+        tma_store_commit();
+        tma_store_wait_read();
+        mbar_arrive(stage_free);
+        if (adders > 2 && j + 1 < adders) {
+          tma_store_wait_all();        // the additions are done, not only read
+          fence_proxy_async_global();
+          asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(added) : "memory");
+        }
+      }
+    }
   } else if (warp >= kBwdSoftmaxWarps) {
     // ------------------------------------------------------------------ row statistics in, dQ out
-    const int quarter = warp & 3, t = quarter * 32 + lane;
+    const int quarter = warp & 3, t = quarter * 32 + lane, h = item[1], b = item[2];
+    const long long bh = static_cast<long long>(b) * p.H + h;
     auto load_stats = [&](int it) {
-      const int q = (i0 + it) * kBlk + t;
+      const int q = query_block(it) * kBlk + t;
       // a row beyond S, or one that no key takes part in, gets +inf: every probability of it is then 2^-inf = 0
       float l = INFINITY, D = 0.f;
       if (q < p.S) {
         l = __ldg(lse + bh * p.S + q);
         l = l == -INFINITY ? INFINITY : l * kLog2e;
-        D = *reinterpret_cast<const float*>(dq + b * p.gsb + h * p.gsh + q * p.gss);
+        D = __ldcg(&reinterpret_cast<const DqSlot*>(dq + b * p.gsb + h * p.gsh + q * p.gss)->D);
       }
       return make_float2(l, D);
     };
@@ -255,57 +324,49 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     };
     put_stats(0, load_stats(0));
     if (n > 1) put_stats(1, load_stats(1));
-    const uint32_t stage = smem_u32(smem + L::DQ) + quarter * 4096;
+    const uint32_t stage = smem_u32(smem + L::DQ) + quarter * 8192;
     for (int it = 0; it < n; ++it) {
       const int qb = it & 1;
       const float2 ahead = it + 2 < n ? load_stats(it + 2) : make_float2(0.f, 0.f);
-      if (!__all_sync(0xffffffffu, mbar_wait(&dq_full[qb], (it >> 1) & 1, abort_flag, p.status, kStatusWaitAccum))) break;
+      bool ok = mbar_wait(&dq_full[qb], (it >> 1) & 1, abort_flag, p.status, kStatusWaitAccum);
+      ok = ok && (it == 0 || mbar_wait(stage_free, (it - 1) & 1, abort_flag, p.status, kStatusWaitEpi));
+      if (!__all_sync(0xffffffffu, ok)) break;
       tc_fence_after_sync();
-      // 32 columns at a time: 16-byte chunk c of this warp's row r at (c * rows + r) * 16, as in the scratch
-      const int row0 = (i0 + it) * kBlk + quarter * 32, nr = min(32, p.S - row0);
-      float* dst = dq_accum + (bh * p.S + row0) * kHD;
+      // 16-byte chunk c of this warp's row r at (c * rows + r) * 16, as in the scratch
+      const int nr = min(32, p.S - query_block(it) * kBlk - quarter * 32);
 #pragma unroll 1
       for (int half = 0; half < 2; ++half) {
         uint32_t v[32];
         tmem_ld32(tDQ + qb * 64 + half * 32 + (static_cast<uint32_t>(quarter * 32) << 16), v);
         tmem_ld_wait();
-        if (half == 1) {
-          tc_fence_before_sync();
-          arrive_warp(&dq_free[qb], lane);
-        }
-        if (lane == 0) tma_store_wait_read();       // the bulk copy before has read the staging area
-        __syncwarp();
         if (lane < nr) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c) st_shared_v4(stage + (c * nr + lane) * 16, make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]));
-        }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0 && nr > 0) {
-          bulk_add(dst + half * 32 * nr, stage, 128 * nr);
-          tma_store_commit();
+          for (int c = 0; c < 8; ++c) st_shared_v4(stage + ((half * 8 + c) * nr + lane) * 16, make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]));
         }
       }
+      tc_fence_before_sync();
+      arrive_warp(&dq_free[qb], lane);
+      fence_proxy_async_smem();
+      arrive_warp(staged, lane);
       if (it + 2 < n) put_stats(it + 2, ahead);   // every softmax thread has read buffer it & 1: its P and dS went into these products
     }
-    if (lane == 0) tma_store_wait_read();      // the shared memory outlives what reads it; the additions end with the grid
   } else {
     // ------------------------------------------------------------------ softmax: thread = query row t x 32 keys
     const int quarter = warp & 3, part = warp >> 2, t = quarter * 32 + lane, c = part * 32;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
     const float sc = p.scale * kLog2e;
     const float inv_keep = p.p_drop > 0.f ? 1.f / (1.f - p.p_drop) : 1.f;
+    const int kv0 = item[0] * kBlk;
     if (threadIdx.x < kBlk) {      // the additive mask (mask * log2e; -inf beyond S)
       const int kv = kv0 + threadIdx.x;
-      mask_s[threadIdx.x] = kv < p.S ? (p.mask ? __ldg(p.mask + static_cast<long long>(b) * p.S + kv) * kLog2e : 0.f) : -INFINITY;
+      mask_s[threadIdx.x] = kv < p.S ? (p.mask ? __ldg(p.mask + static_cast<long long>(item[2]) * p.S + kv) * kLog2e : 0.f) : -INFINITY;
     }
     asm volatile("bar.sync 1, 512;" ::: "memory");
     const bool masked = p.mask != nullptr || kv0 + kBlk > p.S;
     const uint32_t pp = smem_u32(smem + L::P) + (part >> 1) * 16384, dp = smem_u32(smem + L::DS) + (part >> 1) * 16384;
     bool ok = true;
     for (int it = 0; it < n; ++it) {
-      const int q = (i0 + it) * kBlk + t;
-      const bool diagonal = p.causal && i0 + it == j;
+      const bool diagonal = p.causal && it == n - 1;
       ok = mbar_wait(&stat_full[it & 1], (it >> 1) & 1, abort_flag, p.status, kStatusWaitFull);
       const float2 ld = stats[(it & 1) * 128 + t];
       ok = __all_sync(0xffffffffu, ok && mbar_wait(sdp_full, it & 1, abort_flag, p.status, kStatusWaitAccum));
@@ -333,10 +394,12 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (diagonal) {
 #pragma unroll
         for (int e = 0; e < 32; ++e)
-          if (kv0 + c + e > q) sv[e] = 0u;
+          if (c + e > t) sv[e] = 0u;
       }
       if (p.p_drop > 0.f) {
-        const unsigned long long base = (static_cast<unsigned long long>(bh) * p.S + q) * p.S + kv0 + c;
+        const unsigned long long base =
+            ((static_cast<unsigned long long>(item[2]) * p.H + item[1]) * p.S + query_block(it) * kBlk + t) * p.S + item[0] * kBlk + c;
+        const unsigned long long seed = p.seed + (p.seed_dev ? *p.seed_dev : 0ull);
 #pragma unroll
         for (int e = 0; e < 32; e += 4) {
           float z[4];
@@ -382,7 +445,7 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int e = 0; e < 32; ++e) f[e] = __uint_as_float(v[e]);
         stage_half(stage, lane, c2, f);
       }
-      flush_rows(stage, lane, (part == 0 ? dk : dv) + b * p.gsb + h * p.gsh, p.gss, kv0 + quarter * 32, p.S);
+      flush_rows(stage, lane, (part == 0 ? dk : dv) + item[2] * p.gsb + item[1] * p.gsh, p.gss, item[0] * kBlk + quarter * 32, p.S);
     }
   }
   tc_fence_before_sync();
@@ -399,7 +462,7 @@ int attn_bwd_long(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
                   const float* lse, void* dq, void* dk, void* dv, float* dq_accum, const AttnParams& p, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(attn_bwd_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdLong::TOTAL + 1024);
+    const cudaError_t e = cudaFuncSetAttribute(attn_bwd_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdLong::TOTAL);
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
@@ -409,8 +472,8 @@ int attn_bwd_long(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
   const int row_grid = static_cast<int>(rows / 32 + 1 < kSMs * 16 ? rows / 32 + 1 : kSMs * 16);
   auto* dq16 = static_cast<__nv_bfloat16*>(dq);
   launch_pdl(attn_bwd_pre_kernel, dim3(row_grid), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), dq16, dq_accum, p);
-  launch_pdl(attn_bwd_long_kernel, dim3(static_cast<unsigned>(items)), dim3(kBwdThreads), static_cast<size_t>(BwdLong::TOTAL + 1024), stream, tq, tk, tv, tdo, lse,
-             static_cast<const __nv_bfloat16*>(dq16), static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), dq_accum, p);
+  launch_pdl(attn_bwd_long_kernel, dim3(static_cast<unsigned>(items)), dim3(kBwdThreads), static_cast<size_t>(BwdLong::TOTAL), stream, tq, tk, tv, tdo, lse,
+             dq16, static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), dq_accum, p);
   launch_pdl(attn_dq_kernel, dim3(row_grid), dim3(256), 0, stream, static_cast<const float*>(dq_accum), dq16, p);
   return static_cast<int>(cudaGetLastError());
 }
@@ -458,7 +521,7 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nblk = (p.S + kBlk - 1) / kBlk;
   int qb, h, b;
-  decode_block(blockIdx.x, nblk, p.H, p.B, p.causal != 0, qb, h, b);
+  decode_block(blockIdx.x, nblk, p.H, p.B, p.causal != 0, 1, qb, h, b);
   if (p.causal) qb = nblk - 1 - qb;          // the last query block sees the most keys
   const int q0 = qb * kBlk;
   const int n = p.causal ? qb + 1 : nblk;

@@ -170,6 +170,10 @@ __device__ __forceinline__ void tma_store_wait_read() {
 __device__ __forceinline__ void tma_store_wait_read_but_one() {
   asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
 }
+// Orders bulk copies to and from global memory with plain accesses to it.
+__device__ __forceinline__ void fence_proxy_async_global() {
+  asm volatile("fence.proxy.async.global;" ::: "memory");
+}
 // Make generic-proxy smem writes visible to the async proxy (TMA store / tcgen05.mma reads).
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -477,6 +477,20 @@ def test_attention_mask_common_to_all_keys(C):
             assert ((o[b].double() - ref[b]).norm() / ref[b].norm()).item() < 2 ** -8, (S, causal, b)
 
 
+@pytest.mark.parametrize("B,H,S,causal", [(4, 12, 384, False), (2, 5, 385, False), (3, 7, 1000, False), (8, 12, 1024, True), (1, 30, 1333, True)])
+def test_attention_backward_repeats_itself(C, B, H, S, causal):
+    """dQ is a sum over the CTAs of a head, added in a fixed order: the same bits from every call."""
+    torch.manual_seed(21)
+    q, k, v = torch.randn(B, S, 3, H, 64, device="cuda").bfloat16().unbind(2)
+    o, lse = C.attn_fwd(q, k, v, None, 0.125, causal)
+    do = torch.randn_like(o)
+    C.clear_status(0)
+    first = C.attn_bwd(q, k, v, o, do, lse, None, 0.125, causal)
+    for _ in range(5):
+        assert torch.equal(C.attn_bwd(q, k, v, o, do, lse, None, 0.125, causal), first)
+    assert C.read_status(0) == 0
+
+
 def test_attention_several_key_blocks_dropout(C):
     """O is linear in V for fixed probabilities, so <dO, O> = <dV, V> exactly if and only if backward drops what forward dropped."""
     torch.manual_seed(12)
