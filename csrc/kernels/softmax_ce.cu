@@ -55,7 +55,8 @@ struct OnlineSum {
     for (int j = 0; j < N; ++j) s += __expf(v[j] - base);
   }
 };
-__device__ __forceinline__ float sum_rebased(float s, float m, float to) { return m == -INFINITY ? 0.f : s * __expf(m - to); }
+// A sum without a maximum is 0, or NaN if all its values were NaN, and stays what it is.
+__device__ __forceinline__ float sum_rebased(float s, float m, float to) { return m == -INFINITY ? s : s * __expf(m - to); }
 
 // One row per block (or, for short rows, per warp), blocks striding over the rows. The row is read twice, for the statistics
 // and for the gradient, and written once; few enough rows are in flight (three 512-thread blocks on each SM) that the second read finds the

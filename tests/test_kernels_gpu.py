@@ -308,6 +308,23 @@ def test_softmax_ce_row_alignments(C, dtype, rows, V, offset):
     assert abs(loss2.item() - ref.item()) < 1e-5 * max(1.0, abs(ref.item()))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V", [1, 10, 4097])
+def test_softmax_ce_nan_logit(C, dtype, V):
+    """One NaN among a row's logits, wherever it is and also where a thread sees nothing else: the loss and that row's gradient are NaN, the other
+    rows' gradients are not."""
+    torch.manual_seed(22)
+    rows = 9
+    tgt = torch.randint(0, V, (rows,), device="cuda")
+    for at in sorted({0, 1 % V, V // 2, V - 1}):
+        x = torch.randn(rows, V, device="cuda").to(dtype)
+        x[4, at] = float("nan")
+        loss, dl, _ = C.softmax_ce(x, tgt, -100, True, False)
+        assert torch.isnan(loss).item(), at
+        nan = torch.isnan(dl.float())
+        assert torch.all(nan[4]) and not torch.any(nan[:4]) and not torch.any(nan[5:]), at
+
+
 def test_adam_matches_reference(C):
     n = 100003
     torch.manual_seed(4)
