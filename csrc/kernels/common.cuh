@@ -2,6 +2,7 @@
 // packing, warp/block reductions and a counter-based RNG (Philox-4x32-10) for dropout masks that
 // the backward pass regenerates instead of storing.
 #pragma once
+#include <atomic>
 #include <cstdlib>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -217,6 +218,50 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 __device__ __forceinline__ void pdl_entry() {
   pdl_wait();
   pdl_launch_dependents();
+}
+
+// A number per device of the process, made on first use there. A device's properties and a kernel's attributes are its own: worker threads with a
+// device each share these functions. `make` returns a positive number; anything else (a failed call) is not kept.
+class PerDevice {
+ public:
+  template <typename Make>
+  int get(Make make) {
+    int dev = 0;
+    const bool known = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMost;
+    if (known)
+      if (const int v = values_[dev].load(std::memory_order_acquire)) return v;
+    const int v = make();
+    if (known && v > 0) values_[dev].store(v, std::memory_order_release);
+    return v;
+  }
+
+ private:
+  static constexpr int kMost = 64;
+  std::atomic<int> values_[kMost] = {};
+};
+
+// SMs of the current device.
+inline int sm_count() {
+  static PerDevice sms;
+  const int n = sms.get([] {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) v = 0;
+    return v;
+  });
+  return n > 0 ? n : 148;
+}
+
+// Lets kKernel be launched with up to `bytes` of dynamic shared memory on the current device; `whole`: with as much of the SM's memory as there is.
+template <auto kKernel>
+cudaError_t allow_smem(int bytes, bool whole = false) {
+  static PerDevice allowed;
+  cudaError_t e = cudaSuccess;
+  allowed.get([&] {
+    e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && whole) e = cudaFuncSetAttribute(kKernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return e == cudaSuccess ? 1 : 0;
+  });
+  return e;
 }
 
 // Host switch: FLODL_B200_PDL=0 turns the launch attribute off everywhere.

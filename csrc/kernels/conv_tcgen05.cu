@@ -1103,12 +1103,7 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, in
   p.status = status;
   const int smem = p.bars_off + 512 + 1024;
   if (smem > 220 * 1024) return -4;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(conv3x3_wgrad_halo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  if (const cudaError_t e = allow_smem<conv3x3_wgrad_halo_kernel>(220 * 1024)) return static_cast<int>(e);
   int grid = p.chunks / 2;       // at least two chunks per CTA amortise the epilogue's reduce-add
   if (grid > 148) grid = 148;
   if (grid < 1) grid = 1;
@@ -1195,12 +1190,7 @@ extern "C" int fb_conv_wgrad(const void* x, const void* dy, float* dw, int N, in
   if ((r = make_tmap_nhwc(&tdy, dy, N, p.Ho, p.Wo, Co, 64, p.wbox, p.hbox, 1))) return r;
   if ((r = make_tmap_nhwc(&tx, x, N, H, W, Ci, cb, p.wbox, p.hbox, stride))) return r;
   const int smem = p.bars_off + 512 + 1024;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(conv_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  if (const cudaError_t e = allow_smem<conv_wgrad_kernel>(200 * 1024)) return static_cast<int>(e);
   if (smem > 200 * 1024) return -4;
   // one CTA per 64-pixel patch up to the machine size: the copy engine's row rate bounds a CTA, so more
   // CTAs win even though each adds its own reduce-add of the whole filter (ResNet-20 step, measured:
@@ -1294,12 +1284,7 @@ int launch_conv_fwd(const void* in, const void* w, void* out, float* stats, int 
   if ((r = make_tmap_filter(&tw, w, Co, p.taps, Ci))) return r;
   const int smem = p.bars_off + 512 + 4 * 2 * p.Nout * 4 + 1024;
   if (smem > 220 * 1024) return -4;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(conv_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  if (const cudaError_t e = allow_smem<conv_fwd_kernel>(220 * 1024)) return static_cast<int>(e);
   int grid = p.tiles < 148 ? p.tiles : 148;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
@@ -1362,12 +1347,7 @@ int launch_conv_halo(const void* in, const void* w, void* out, float* stats, int
   if ((r = make_tmap_filter(&tw, w, Co, 9, Ci))) return r;
   const int smem = p.bars_off + 512 + 4 * 2 * p.Nout * 4 + 1024;
   if (smem > 220 * 1024) return -4;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(conv3x3_halo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  if (const cudaError_t e = allow_smem<conv3x3_halo_kernel>(220 * 1024)) return static_cast<int>(e);
   const int grid = p.tiles < 148 ? p.tiles : 148;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);

@@ -471,13 +471,7 @@ extern "C" int fb_attn_fwd(const void* q, const void* k, const void* v, void* o,
   if ((r = make_tmap_bshd(&tv, v, B, H, S, sb, ss, sh))) return r;
   const AttnParams p = make_params(B, H, S, qkv_strides, o_strides, o_strides, mask, scale, causal, p_drop, seed, seed_dev, status);
   if (S > kBlk) return attn_fwd_long(tq, tk, tv, o, lse, p, static_cast<cudaStream_t>(stream));
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem::TOTAL + 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  if (const cudaError_t e = allow_smem<attn_fwd_kernel>(FwdSmem::TOTAL + 1024, true)) return static_cast<int>(e);
   const cudaError_t le = launch_pdl(attn_fwd_kernel, dim3(H, B), dim3(kAttnThreads), static_cast<size_t>(FwdSmem::TOTAL + 1024), static_cast<cudaStream_t>(stream), tq, tk, tv,
                                     static_cast<__nv_bfloat16*>(o), lse, p);
   return static_cast<int>(le != cudaSuccess ? le : cudaGetLastError());
@@ -507,13 +501,7 @@ extern "C" int fb_attn_bwd(const void* q, const void* k, const void* v, const vo
   if ((r = make_tmap_bshd(&tdo, d_o, B, H, S, o_strides[0], o_strides[1], o_strides[2]))) return r;
   const AttnParams p = make_params(B, H, S, qkv_strides, o_strides, g_strides, mask, scale, causal, p_drop, seed, seed_dev, status);
   if (S > kBlk) return attn_bwd_long(tq, tk, tv, tdo, o, d_o, lse, dq, dk, dv, dq_accum, p, static_cast<cudaStream_t>(stream));
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::TOTAL);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  if (const cudaError_t e = allow_smem<attn_bwd_kernel>(BwdSmem::TOTAL, true)) return static_cast<int>(e);
   const cudaError_t le = launch_pdl(attn_bwd_kernel, dim3(H, B), dim3(kAttnThreads), static_cast<size_t>(BwdSmem::TOTAL), static_cast<cudaStream_t>(stream),
                                     tq, tk, tv, tdo, static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), lse,
                                     static_cast<__nv_bfloat16*>(dq), static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), p);

@@ -460,12 +460,7 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
 int attn_bwd_long(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const void* o, const void* d_o,
                   const float* lse, void* dq, void* dk, void* dv, float* dq_accum, const AttnParams& p, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(attn_bwd_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdLong::TOTAL);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  if (const cudaError_t e = allow_smem<attn_bwd_long_kernel>(BwdLong::TOTAL)) return static_cast<int>(e);
   const long long items = static_cast<long long>((p.S + kBlk - 1) / kBlk) * p.H * p.B;
   const long long rows = static_cast<long long>(p.B) * p.H * p.S;
   if (items > 0x7fffffffll) return -4;
@@ -782,18 +777,13 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 int attn_fwd_long(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* o, float* lse, const AttnParams& p, cudaStream_t stream) {
   const auto kern = p.p_drop > 0.f ? (p.mask ? attn_fwd_long_kernel<true, true> : attn_fwd_long_kernel<true, false>)
                                    : (p.mask ? attn_fwd_long_kernel<false, true> : attn_fwd_long_kernel<false, false>);
-  static bool configured = false;
-  if (!configured) {
-    for (auto k : {attn_fwd_long_kernel<true, true>, attn_fwd_long_kernel<true, false>, attn_fwd_long_kernel<false, true>, attn_fwd_long_kernel<false, false>}) {
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdLong::TOTAL + 1024);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-      if (e != cudaSuccess) return static_cast<int>(e);
-    }
-    configured = true;
-  }
+  constexpr int smem = FwdLong::TOTAL + 1024;
+  for (const cudaError_t e : {allow_smem<attn_fwd_long_kernel<true, true>>(smem, true), allow_smem<attn_fwd_long_kernel<true, false>>(smem, true),
+                              allow_smem<attn_fwd_long_kernel<false, true>>(smem, true), allow_smem<attn_fwd_long_kernel<false, false>>(smem, true)})
+    if (e != cudaSuccess) return static_cast<int>(e);
   const long long ctas = static_cast<long long>((p.S + kBlk - 1) / kBlk) * p.H * p.B;
   if (ctas > 0x7fffffffll) return -4;
-  const cudaError_t e = launch_pdl(kern, dim3(static_cast<unsigned>(ctas)), dim3(kFwdThreads), static_cast<size_t>(FwdLong::TOTAL + 1024), stream, tq, tk,
+  const cudaError_t e = launch_pdl(kern, dim3(static_cast<unsigned>(ctas)), dim3(kFwdThreads), static_cast<size_t>(smem), stream, tq, tk,
                                    tv, static_cast<__nv_bfloat16*>(o), lse, p);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }

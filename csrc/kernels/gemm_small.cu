@@ -256,13 +256,7 @@ int gemm_small(const void* A, const void* const* B, void* C, int M, int group, i
     r = b_mn ? make_tmap_bf16_2d(&tb.b[g], b, group, K, ldb, 64, kTK) : make_tmap_bf16_2d(&tb.b[g], b, K, group, ldb, kTK, kTN);
   }
   if (r) return r;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_small_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  if (const cudaError_t e = allow_smem<gemm_small_kernel>(kSmem, true)) return static_cast<int>(e);
   const int num_kb = (K + kTK - 1) / kTK;
   SmallGemm p{M, N, K, b_mn, (num_kb + split - 1) / split, group, {nullptr, nullptr, nullptr}, static_cast<__nv_bfloat16*>(C), ldc, bias_fp32, epi,
               static_cast<__nv_bfloat16*>(aux), ldaux, alpha, status};

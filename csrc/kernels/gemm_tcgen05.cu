@@ -946,27 +946,12 @@ static int make_tmap_out(CUtensorMap* out, const void* base, uint64_t cols, uint
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
-static int sm_count() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  }
-  return n;
-}
-
 template <int kCG, int kBN>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tx, const GemmParams& p,
                        cudaStream_t stream) {
   using Cfg = GemmCfg<kCG, kBN>;
-  static bool configured = false;
   auto kern = gemm_bf16_kernel<kCG, kBN>;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  if (const cudaError_t e = allow_smem<gemm_bf16_kernel<kCG, kBN>>(Cfg::SMEM_BYTES)) return static_cast<int>(e);
   const int num_m = (p.M + BM * kCG - 1) / (BM * kCG);
   const int num_n = (p.N + kBN - 1) / kBN;
   const int units = num_m * num_n * p.split_k;
@@ -1010,8 +995,9 @@ static cudaLaunchConfig_t split_config(int M, int N, cudaLaunchAttribute* attr, 
 
 // How many clusters of gemm_split_kernel the device holds at once (0: none, or it cannot be told).
 static int split_clusters() {
-  static const int n = [] {
-    if (cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg::SMEM_BYTES) != cudaSuccess) return 0;
+  static PerDevice held;
+  return held.get([] {
+    if (allow_smem<gemm_split_kernel>(SplitCfg::SMEM_BYTES) != cudaSuccess) return 0;
     cudaLaunchAttribute attr[2];
     const cudaLaunchConfig_t cfg = split_config(2 * BM, 256, attr, nullptr);
     int clusters = 0;
@@ -1020,8 +1006,7 @@ static int split_clusters() {
       return 0;
     }
     return clusters;
-  }();
-  return n;
+  });
 }
 
 // Long reductions (kSplitMinK) with no more tiles than the device holds clusters at once: one more and the last tile would run

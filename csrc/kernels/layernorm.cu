@@ -345,21 +345,12 @@ ln_bwd_finalize_kernel(const float* __restrict__ partial, float* __restrict__ dg
   }
 }
 
-static int ln_sms() {
-  static const int n = [] {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms > 0 ? sms : 148;
-  }();
-  return n;
-}
-
 template <typename T, int VPL, typename P>
 static int ln_fwd_launch(const void* x, const void* res, const P* gamma, const P* beta, void* y,
                          void* pre, float* mean, float* rstd, int rows, int cols, float eps, float p,
                          uint64_t seed, const unsigned long long* seed_dev, cudaStream_t st) {
   // fp32 rows are twice the registers: there a block per four rows measured better (32768 x 768: 62 against 72 us)
-  const int need = (rows + kLnWarps - 1) / kLnWarps, wave = ln_sms() * ln_fwd_blocks(VPL * VecIO<T>::kVec);
+  const int need = (rows + kLnWarps - 1) / kLnWarps, wave = sm_count() * ln_fwd_blocks(VPL * VecIO<T>::kVec);
   launch_pdl(ln_fwd_kernel<T, VPL, P>, dim3(need < wave || sizeof(T) == 4 ? need : wave), dim3(kLnWarps * 32), 0, st, static_cast<const T*>(x), static_cast<const T*>(res), gamma, beta, static_cast<T*>(y),
       static_cast<T*>(pre), mean, rstd, rows, cols, eps, p, seed, seed_dev);
   return static_cast<int>(cudaGetLastError());
@@ -370,7 +361,7 @@ template <typename T, int VPL>
 static int ln_bwd_launch(const void* dy, const void* pre, const float* mean, const float* rstd,
                          const float* gamma, void* dpre, void* dxd, float* partial, float* dgamma, float* dbeta, int accumulate, int most,
                          int rows, int cols, float p, uint64_t seed, const unsigned long long* seed_dev, cudaStream_t st) {
-  const int wave = ln_sms() * ln_bwd_blocks(VPL * VecIO<T>::kVec);
+  const int wave = sm_count() * ln_bwd_blocks(VPL * VecIO<T>::kVec);
   const int grid = most < wave ? most : wave;
   const bool fold = partial && !accumulate && (dgamma || dbeta);      // through the partial rows
   const bool add = partial && accumulate;
@@ -437,7 +428,7 @@ extern "C" int fb_layernorm_fwd_p16(const void* x, const void* residual, const v
 
 // The most blocks the backward kernel uses: one resident wave (its dgamma / dbeta sums stay in registers).
 extern "C" int fb_layernorm_bwd_grid(int rows) {
-  const int cap = 4 * fb::ln_sms(), g = (rows + fb::kLnWarps - 1) / fb::kLnWarps;
+  const int cap = 4 * fb::sm_count(), g = (rows + fb::kLnWarps - 1) / fb::kLnWarps;
   return g < cap ? g : cap;
 }
 
