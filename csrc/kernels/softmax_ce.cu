@@ -5,6 +5,8 @@
 // bf16 or fp32; all math is fp32. The gradient (softmax - onehot) / n_valid is produced in the
 // forward launch (it may overwrite the logits), so the backward pass is a scalar multiply that the
 // consumer GEMMs take as their `alpha`.
+#include <type_traits>
+
 #include "../include/flodl_b200.h"
 #include "common.cuh"
 
@@ -58,107 +60,104 @@ struct OnlineSum {
 // A sum without a maximum is 0, or NaN if all its values were NaN, and stays what it is.
 __device__ __forceinline__ float sum_rebased(float s, float m, float to) { return m == -INFINITY ? s : s * __expf(m - to); }
 
-// One row per block (or, for short rows, per warp), blocks striding over the rows. The row is read twice, for the statistics
-// and for the gradient, and written once; few enough rows are in flight (three 512-thread blocks on each SM) that the second read finds the
-// row in L2, so HBM sees one read and one write, which is what bounds the kernel.
-// fp32 [4096, 30522], rows 8-byte aligned, with the backward scaling by one: 704 us when unaligned rows were read value by value,
-// eight 256-thread blocks per SM spilled the rows out of L2 and the factor of one was multiplied through; now 233 us (4.3 TB/s).
-template <typename T, bool kWarpRow>
-__global__ void __launch_bounds__(512, 3)
+// One row per block or, for short rows, per warp. The row is read twice, for the statistics and for the gradient, and written once. What bounds it is
+// HBM where the second read finds the row in L2, so that a row's threads times the resident blocks' rows decide: few threads to a row keep the
+// barrier and the exponentials of one row behind the loads of others, but put more rows in flight; long rows then leave L2 between their reads.
+// us for a mean loss with its gradient; in brackets a 256-thread block per row that takes rows off a 16-byte boundary value by value, and
+// 512-thread (up to 64 KB 256-thread) blocks striding over the rows:
+//   bf16 4843 x 392 9.9 (13.3, 10.4), 4000 x 3000 18.9 (19.8, 19.0), 8192 x 8000 73.5 (72.7, 88.5), 8192 x 32000 238 (266, 255), 4096 x 50304 in place
+//   199 (214, 206), 2048 x 128000 256 (294, 266); fp32 8192 x 4000 55.5 (64.0, 75.8), 2094 x 23544 79 (107, 88), 4096 x 30522 187 (396, 220).
+// kUnroll vectors in flight per thread, kBlocks blocks of kThreads on an SM.
+template <typename T, bool kWarpRow, int kThreads, int kBlocks, int kUnroll>
+__global__ void __launch_bounds__(kThreads, kBlocks)
 ce_fwd_kernel(const T* __restrict__ logits, long long ld, const long long* __restrict__ targets, int rows,
               int V, long long ignore_index, T* __restrict__ dlogits, long long ldd,
               const float* __restrict__ count_inv, float* __restrict__ row_loss, const int* __restrict__ counts) {
   pdl_entry();
   constexpr int VEC = VecIO<T>::kVec;
-  constexpr int kUnroll = 16 / VEC;       // 16 values in flight per thread: what three blocks' registers hold
-  __shared__ float red_m[2][16], red_s[2][16];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  const int me = kWarpRow ? lane : threadIdx.x, step = kWarpRow ? 32 : blockDim.x;
-  const int first = kWarpRow ? blockIdx.x * warps + warp : blockIdx.x, stride = kWarpRow ? gridDim.x * warps : gridDim.x;
-  const float inv_n = count_inv ? count_inv[1] : 1.f;
-  const int live_rows = counts ? counts[1] : rows;
+  constexpr int kWarps = kThreads / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int me = kWarpRow ? lane : threadIdx.x, row = kWarpRow ? blockIdx.x * kWarps + warp : blockIdx.x;
+  constexpr int step = kWarpRow ? 32 : kThreads;
+  if (kWarpRow && row >= rows) return;
   if (counts) (void)FB_INDEX_OK(counts[0], static_cast<long long>(rows) + 1, 202);
-  int turn = 0;
-  for (int row = first; row < rows; row += stride) {
-    if (row >= live_rows) {      // compacted input: nothing lives past the padded count
-      if (row_loss && me == 0) row_loss[row] = 0.f;
-      continue;
-    }
-    const long long t = targets[row];
-    const T* lr = logits + static_cast<long long>(row) * ld;
-    T* dr = dlogits ? dlogits + static_cast<long long>(row) * ldd : nullptr;
-    const RowSplit<T> sp(lr, dr, V);
-    if (t != ignore_index) (void)FB_INDEX_OK(t, V, 201);        // a label outside the vocabulary is recorded (and treated as ignored)
-    if (t == ignore_index || t < 0 || t >= V) {
-      if (row_loss && me == 0) row_loss[row] = 0.f;
-      if (dr) {
-        float z[VEC];
+  if (counts && row >= counts[1]) {      // compacted input: nothing lives past the padded count
+    if (row_loss && me == 0) row_loss[row] = 0.f;
+    return;
+  }
+  const long long t = targets[row];
+  const T* lr = logits + static_cast<long long>(row) * ld;
+  T* dr = dlogits ? dlogits + static_cast<long long>(row) * ldd : nullptr;
+  const RowSplit<T> sp(lr, dr, V);
+  if (t != ignore_index) (void)FB_INDEX_OK(t, V, 201);        // a label outside the vocabulary is recorded (and treated as ignored)
+  if (t == ignore_index || t < 0 || t >= V) {
+    if (row_loss && me == 0) row_loss[row] = 0.f;
+    if (dr) {
+      float z[VEC];
 #pragma unroll
-        for (int j = 0; j < VEC; ++j) z[j] = 0.f;
-        for (int k = me; k < sp.head; k += step) VecIO<T>::put(dr + k, 0.f);
-        for (int i = me; i < sp.nvec; i += step) VecIO<T>::store(dr + sp.head + i * VEC, z);
-        for (int k = sp.tail + me; k < V; k += step) VecIO<T>::put(dr + k, 0.f);
-      }
-      continue;
+      for (int j = 0; j < VEC; ++j) z[j] = 0.f;
+      for (int k = me; k < sp.head; k += step) VecIO<T>::put(dr + k, 0.f);
+      for (int i = me; i < sp.nvec; i += step) VecIO<T>::store(dr + sp.head + i * VEC, z);
+      for (int k = sp.tail + me; k < V; k += step) VecIO<T>::put(dr + k, 0.f);
     }
-    const float x_t = me == 0 && row_loss ? VecIO<T>::get(lr + t) : 0.f;      // before the gradient may overwrite it
-    if constexpr (kWarpRow) __syncwarp();
+    return;
+  }
+  const float x_t = me == 0 && row_loss ? VecIO<T>::get(lr + t) : 0.f;      // before the gradient may overwrite it
+  if constexpr (kWarpRow) __syncwarp();
 
-    OnlineSum acc;
-    for (int k = me; k < sp.head; k += step) { const float v[1] = {VecIO<T>::get(lr + k)}; acc.add(v); }
-    for (int k = sp.tail + me; k < V; k += step) { const float v[1] = {VecIO<T>::get(lr + k)}; acc.add(v); }
-    const T* body = lr + sp.head;
-    int i = me;
-    for (; i + (kUnroll - 1) * step < sp.nvec; i += kUnroll * step) {
-      float v[kUnroll][VEC];
+  OnlineSum acc;
+  for (int k = me; k < sp.head; k += step) { const float v[1] = {VecIO<T>::get(lr + k)}; acc.add(v); }
+  for (int k = sp.tail + me; k < V; k += step) { const float v[1] = {VecIO<T>::get(lr + k)}; acc.add(v); }
+  const T* body = lr + sp.head;
+  int i = me;
+  for (; i + (kUnroll - 1) * step < sp.nvec; i += kUnroll * step) {
+    float v[kUnroll][VEC];
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) VecIO<T>::load(body + static_cast<long long>(i + u * step) * VEC, v[u]);
+    for (int u = 0; u < kUnroll; ++u) VecIO<T>::load(body + static_cast<long long>(i + u * step) * VEC, v[u]);
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) acc.add(v[u]);
-    }
-    for (; i < sp.nvec; i += step) {
-      float v[VEC];
-      VecIO<T>::load(body + static_cast<long long>(i) * VEC, v);
-      acc.add(v);
-    }
-    float gmax = warp_max(acc.m);
-    float gsum = warp_sum(sum_rebased(acc.s, acc.m, gmax));
-    if constexpr (!kWarpRow) {
-      // two sets of slots in turn: a warp can be at most one row ahead of another, because of the barrier
-      if (lane == 0) { red_m[turn][warp] = gmax; red_s[turn][warp] = gsum; }
-      __syncthreads();
-      const float wm = lane < warps ? red_m[turn][lane] : -INFINITY, ws = lane < warps ? red_s[turn][lane] : 0.f;
-      gmax = warp_max(wm);
-      gsum = warp_sum(sum_rebased(ws, wm, gmax));
-      turn ^= 1;
-    }
-    if (row_loss && me == 0) row_loss[row] = __logf(gsum) + gmax - x_t;
-    if (!dr) continue;
+    for (int u = 0; u < kUnroll; ++u) acc.add(v[u]);
+  }
+  for (; i < sp.nvec; i += step) {
+    float v[VEC];
+    VecIO<T>::load(body + static_cast<long long>(i) * VEC, v);
+    acc.add(v);
+  }
+  float gmax = warp_max(acc.m);
+  float gsum = warp_sum(sum_rebased(acc.s, acc.m, gmax));
+  if constexpr (!kWarpRow) {
+    __shared__ float red_m[kWarps], red_s[kWarps];
+    if (lane == 0) { red_m[warp] = gmax; red_s[warp] = gsum; }
+    __syncthreads();
+    const float wm = lane < kWarps ? red_m[lane] : -INFINITY, ws = lane < kWarps ? red_s[lane] : 0.f;
+    gmax = warp_max(wm);
+    gsum = warp_sum(sum_rebased(ws, wm, gmax));
+  }
+  if (row_loss && me == 0) row_loss[row] = __logf(gsum) + gmax - x_t;
+  if (!dr) return;
 
-    const float inv_sum = 1.f / gsum;
-    T* dbody = dr + sp.head;
-    auto grad = [&](float x, int k) { return (__expf(x - gmax) * inv_sum - (k == t ? 1.f : 0.f)) * inv_n; };
-    for (int k = me; k < sp.head; k += step) VecIO<T>::put(dr + k, grad(VecIO<T>::get(lr + k), k));
-    for (int k = sp.tail + me; k < V; k += step) VecIO<T>::put(dr + k, grad(VecIO<T>::get(lr + k), k));
-    i = me;
-    for (; i + (kUnroll - 1) * step < sp.nvec; i += kUnroll * step) {
-      float v[kUnroll][VEC];
+  const float inv_n = count_inv ? count_inv[1] : 1.f, inv_sum = 1.f / gsum;
+  T* dbody = dr + sp.head;
+  auto grad = [&](float x, int k) { return (__expf(x - gmax) * inv_sum - (k == t ? 1.f : 0.f)) * inv_n; };
+  for (int k = me; k < sp.head; k += step) VecIO<T>::put(dr + k, grad(VecIO<T>::get(lr + k), k));
+  for (int k = sp.tail + me; k < V; k += step) VecIO<T>::put(dr + k, grad(VecIO<T>::get(lr + k), k));
+  i = me;
+  for (; i + (kUnroll - 1) * step < sp.nvec; i += kUnroll * step) {
+    float v[kUnroll][VEC];
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) VecIO<T>::load(body + static_cast<long long>(i + u * step) * VEC, v[u]);
+    for (int u = 0; u < kUnroll; ++u) VecIO<T>::load(body + static_cast<long long>(i + u * step) * VEC, v[u]);
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < kUnroll; ++u) {
 #pragma unroll
-        for (int j = 0; j < VEC; ++j) v[u][j] = grad(v[u][j], sp.head + (i + u * step) * VEC + j);
-        VecIO<T>::store(dbody + static_cast<long long>(i + u * step) * VEC, v[u]);
-      }
+      for (int j = 0; j < VEC; ++j) v[u][j] = grad(v[u][j], sp.head + (i + u * step) * VEC + j);
+      VecIO<T>::store(dbody + static_cast<long long>(i + u * step) * VEC, v[u]);
     }
-    for (; i < sp.nvec; i += step) {
-      float v[VEC];
-      VecIO<T>::load(body + static_cast<long long>(i) * VEC, v);
+  }
+  for (; i < sp.nvec; i += step) {
+    float v[VEC];
+    VecIO<T>::load(body + static_cast<long long>(i) * VEC, v);
 #pragma unroll
-      for (int j = 0; j < VEC; ++j) v[j] = grad(v[j], sp.head + i * VEC + j);
-      VecIO<T>::store(dbody + static_cast<long long>(i) * VEC, v);
-    }
+    for (int j = 0; j < VEC; ++j) v[j] = grad(v[j], sp.head + i * VEC + j);
+    VecIO<T>::store(dbody + static_cast<long long>(i) * VEC, v);
   }
 }
 
@@ -205,26 +204,33 @@ extern "C" int fb_softmax_ce_dyn(const void* logits, long long ld, const long lo
   if (rows <= 0) return 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   fb::launch_pdl(fb::ce_count_kernel, dim3(1), dim3(1024), 0, st, targets, rows, ignore_index, count_inv);
-  // Short rows: a warp each, eight to a block (a block-wide reduction would cost more than the row); the line is where a
-  // block's 512 threads get a vector each. Long rows: a block each, as many as stay resident.
-  const bool warp_row = V <= (is_bf16 ? 4096 : 2048);
-  // (Rows of up to 64 KB take half the threads and twice the blocks: a row's barrier and its exponentials then hide behind others'
-  // loads. us, bf16: 2000 x 5000 19.3 -> 14.5, 8192 x 8000 102 -> 82, 8192 x 32000 258 -> 243. Longer ones would leave L2 before their second read.)
-  const bool half_block = static_cast<long long>(V) * (is_bf16 ? 2 : 4) <= 65536;
-  const int resident = 148 * (half_block ? 6 : 3);
-  const dim3 grid(static_cast<unsigned>(warp_row ? (rows + 7) / 8 : rows < resident ? rows : resident)), block(warp_row || half_block ? 256 : 512);
-  auto go = [&](auto kern, auto* x, auto* dx) {
-    fb::launch_pdl(kern, grid, block, 0, st, x, ld, targets, rows, V, ignore_index, dx, ldd, count_inv, row_loss, counts);
+  // By the row's bytes and by how many rows there are to an SM; the lines lie where the measured curves cross. Up to 1 KB, or 2 KB of many rows, a
+  // warp. Few rows are a latency: 256 threads each. Otherwise as few threads as fill the loads: 128 up to 32 KB in bf16, 20 KB in fp32; beyond, rows
+  // have to find themselves in L2 again, so 256 threads of more values each in bf16, 512 from 96 KB on; in fp32 256 up to 32 KB,
+  // 512 up to 96 KB and then 1024.
+  const long long bytes = static_cast<long long>(V) * (is_bf16 ? 2 : 4);
+  const int per_sm = rows / fb::sm_count();
+  auto go = [&](auto kern, int threads, int rows_per_block, auto* x, auto* dx) {
+    fb::launch_pdl(kern, dim3((rows + rows_per_block - 1) / rows_per_block), dim3(threads), 0, st, x, ld, targets, rows, V, ignore_index, dx, ldd, count_inv, row_loss, counts);
   };
-  if (is_bf16) {
-    const auto* x = static_cast<const __nv_bfloat16*>(logits);
-    auto* dx = static_cast<__nv_bfloat16*>(dlogits);
-    warp_row ? go(fb::ce_fwd_kernel<__nv_bfloat16, true>, x, dx) : go(fb::ce_fwd_kernel<__nv_bfloat16, false>, x, dx);
-  } else {
-    const auto* x = static_cast<const float*>(logits);
-    auto* dx = static_cast<float*>(dlogits);
-    warp_row ? go(fb::ce_fwd_kernel<float, true>, x, dx) : go(fb::ce_fwd_kernel<float, false>, x, dx);
-  }
+  auto pick = [&](auto* x, auto* dx) {
+    using T = std::remove_pointer_t<decltype(dx)>;
+    constexpr int one = sizeof(T) == 2 ? 1 : 2;      // vectors that make eight values
+    if (bytes <= 1024 || (bytes <= 2048 && per_sm >= 16)) return go(fb::ce_fwd_kernel<T, true, 128, 16, one>, 128, 4, x, dx);
+    if constexpr (sizeof(T) == 2) {
+      if (per_sm < 4) go(fb::ce_fwd_kernel<T, false, 256, 4, 2 * one>, 256, 1, x, dx);
+      else if (bytes <= 32768) go(fb::ce_fwd_kernel<T, false, 128, 12, 2 * one>, 128, 1, x, dx);
+      else if (bytes <= 98304) go(fb::ce_fwd_kernel<T, false, 256, 6, 2 * one>, 256, 1, x, dx);
+      else go(fb::ce_fwd_kernel<T, false, 512, 3, 2 * one>, 512, 1, x, dx);
+    } else {
+      if (bytes <= 20480 && per_sm >= 4) go(fb::ce_fwd_kernel<T, false, 128, 16, one>, 128, 1, x, dx);
+      else if (bytes <= 32768) go(fb::ce_fwd_kernel<T, false, 256, 8, one>, 256, 1, x, dx);
+      else if (bytes <= 98304) go(fb::ce_fwd_kernel<T, false, 512, 4, one>, 512, 1, x, dx);
+      else go(fb::ce_fwd_kernel<T, false, 1024, 2, one>, 1024, 1, x, dx);
+    }
+  };
+  if (is_bf16) pick(static_cast<const __nv_bfloat16*>(logits), static_cast<__nv_bfloat16*>(dlogits));
+  else pick(static_cast<const float*>(logits), static_cast<float*>(dlogits));
   if (loss) fb::launch_pdl(fb::ce_finalize_kernel, dim3(1), dim3(1024), 0, st, row_loss, rows, count_inv, loss);
   return static_cast<int>(cudaGetLastError());
 }

@@ -308,6 +308,27 @@ def test_softmax_ce_row_alignments(C, dtype, rows, V, offset):
     assert abs(loss2.item() - ref.item()) < 1e-5 * max(1.0, abs(ref.item()))
 
 
+@pytest.mark.parametrize("dtype,V", [(torch.bfloat16, v) for v in (512, 513, 1024, 1025, 10240, 10241, 16384, 16385)] +
+                         [(torch.float32, v) for v in (256, 257, 512, 513, 5120, 5121, 8192, 8193, 24576, 24577)])
+@pytest.mark.parametrize("rows", [7, 601])
+def test_softmax_ce_either_side_of_each_block_size(C, dtype, V, rows):
+    """Row lengths at which the threads of a row change, of few rows and of many; bounds as above."""
+    torch.manual_seed(23)
+    x = torch.randn(rows, V, device="cuda").to(dtype)
+    t = torch.randint(0, V, (rows,), device="cuda")
+    t[::6] = -100
+    n = int((t != -100).sum())
+    xd = x.double()
+    ref = torch.nn.functional.cross_entropy(xd, t, ignore_index=-100)
+    p = torch.softmax(xd, 1)
+    p[torch.arange(rows, device="cuda"), t.clamp_min(0)] -= 1
+    p[t == -100] = 0
+    for inplace in (False, True):
+        loss, dl, _ = C.softmax_ce(x, t, -100, True, inplace)
+        assert abs(loss.double().item() - ref.item()) < 2 ** -21 * abs(ref.item())
+        assert ((dl.double() - p / n).norm() / (p / n).norm()).item() < (2 ** -8 if dtype == torch.bfloat16 else 2 ** -18)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("V", [1, 10, 4097])
 def test_softmax_ce_nan_logit(C, dtype, V):
