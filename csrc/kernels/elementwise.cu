@@ -284,7 +284,6 @@ struct Vec4<__nv_bfloat16> {
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
   }
 };
-constexpr int kEmbRows = 8;       // tokens whose rows a thread has in flight
 
 // dW[ids[t]][:] += dy[t][:] for an embedding table (fp32 accumulation, rows equal to padding_idx skipped).
 template <typename T>
@@ -305,9 +304,10 @@ __global__ void embedding_bwd_kernel(const T* __restrict__ dy, const long long* 
 // them) are summed in registers first, and what is added goes out as 16-byte reductions. One reduction per token, column and four
 // bytes, which the kernel above makes, is bound by the atomics of one row when many tokens share it. Needs dim and both base
 // addresses in whole vectors of four.
-// us, bf16, 768 columns, against one reduction per token and value: 4096 tokens of one id 6.9 (53), of two ids in any order 12 (26), all
-// different 5.6 (6.4); 32768 tokens of one id 21 (290), of random ids of 30522 26 (23; fp32 35 (36)).
-template <typename T>
+// kEmbRows tokens' rows are in flight per thread.
+// us, 768 columns, in brackets one reduction per token and value: bf16 4096 tokens of one id 6.1 (51), of two ids in any order 11 (26), random ids of 30522
+// 4.2 (4.3); 32768 tokens of one id 21 (288), of random ids 22 (22); fp32 35 (35).
+template <typename T, int kEmbRows>
 __global__ void __launch_bounds__(256)
 embedding_bwd_vec_kernel(const T* __restrict__ dy, const long long* __restrict__ ids, float* __restrict__ dw, long long tokens, int dim,
                          long long vocab, long long padding_idx, int per_block) {
@@ -450,18 +450,16 @@ extern "C" int fb_embedding_bwd(const void* dy, const long long* ids, float* dw,
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t four = is_bf16 ? 8 : 16;
   if (dim % 4 == 0 && reinterpret_cast<uintptr_t>(dy) % four == 0 && reinterpret_cast<uintptr_t>(dw) % 16 == 0) {
-    // Enough blocks for two or three per SM; long runs spare reductions where neighbours are equal, short ones keep more rows in
-    // flight where they are not.
-    long long per = tokens / 400 / fb::kEmbRows * fb::kEmbRows;
-    per = per < fb::kEmbRows ? fb::kEmbRows : per > 16 ? 16 : per;
+    // Long runs spare reductions where neighbours are equal, short ones make more blocks: two tokens to a block while there are not enough for the chip,
+    // sixteen once that makes a wave or two. Four rows in flight leave room for more blocks than eight (32768 random bf16 tokens 22 us against 25); only
+    // many fp32 rows want eight (32768 tokens 35 against 36.5).
+    const int per = tokens < 1024 ? 2 : tokens < 8192 ? 8 : 16;
     const int threads = dim / 4 < 256 ? (dim / 4 + 31) / 32 * 32 : 256;
     const dim3 grid(static_cast<unsigned>((tokens + per - 1) / per), (dim / 4 + threads - 1) / threads);
-    if (is_bf16)
-      fb::launch_pdl(fb::embedding_bwd_vec_kernel<__nv_bfloat16>, grid, dim3(threads), 0, st, static_cast<const __nv_bfloat16*>(dy), ids, dw, tokens, dim, vocab,
-                     padding_idx, static_cast<int>(per));
-    else
-      fb::launch_pdl(fb::embedding_bwd_vec_kernel<float>, grid, dim3(threads), 0, st, static_cast<const float*>(dy), ids, dw, tokens, dim, vocab, padding_idx,
-                     static_cast<int>(per));
+    auto go = [&](auto kern, const auto* rows) { fb::launch_pdl(kern, grid, dim3(threads), 0, st, rows, ids, dw, tokens, dim, vocab, padding_idx, per); };
+    if (is_bf16) go(fb::embedding_bwd_vec_kernel<__nv_bfloat16, 4>, static_cast<const __nv_bfloat16*>(dy));
+    else if (tokens >= 16384) go(fb::embedding_bwd_vec_kernel<float, 8>, static_cast<const float*>(dy));
+    else go(fb::embedding_bwd_vec_kernel<float, 4>, static_cast<const float*>(dy));
     return static_cast<int>(cudaGetLastError());
   }
   const int warps = 8;

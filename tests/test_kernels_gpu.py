@@ -227,6 +227,20 @@ def test_embedding_bwd_runs(C, dtype, tokens, dim, ids):
     assert ((dw.double() - ref).norm() / ref.norm()).item() < 2 ** -18 and torch.all(dw[vocab - 1] == 1)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens", [1023, 1025, 8191, 8193, 16383, 16387])
+def test_embedding_bwd_run_lengths(C, dtype, tokens):
+    """Either side of the token counts at which a block's run of tokens and the rows in flight change; ids that repeat after 1 to 40 tokens."""
+    torch.manual_seed(24)
+    vocab, dim = 300, 36
+    t = torch.repeat_interleave(torch.randint(0, vocab, (tokens,)), torch.randint(1, 41, (tokens,)))[:tokens].cuda()
+    dy = torch.randn(tokens, dim, device="cuda").to(dtype)
+    dw = torch.zeros(vocab, dim, device="cuda")
+    C.embedding_bwd(dy, t, dw, 5)
+    ref = torch.zeros(vocab, dim, device="cuda", dtype=torch.double).index_add_(0, t[t != 5], dy.double()[t != 5])
+    assert ((dw.double() - ref).norm() / ref.norm()).item() < 2 ** -18 and torch.all(dw[5] == 0)
+
+
 def test_layernorm_dropout_mask_consistent(C):
     rows, cols, p = 512, 768, 0.1
     x = torch.ones(rows, cols, device="cuda", dtype=torch.bfloat16)
