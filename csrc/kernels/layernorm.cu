@@ -60,17 +60,18 @@ __device__ __forceinline__ void load_f32_vec(const __nv_bfloat16* __restrict__ p
   }
 }
 
-// Blocks per SM: what the registers of `values` columns per lane, two rows in flight, leave room for.
-constexpr int ln_fwd_blocks(int values) { return values <= 24 ? 5 : 3; }
+// Blocks per SM: of one row of `size`-byte values in the forward pass (one more for fp32 makes a whole wave of 4096 rows: 1024 wide 6.2 us, with six 9.0),
+// and in the backward pass what `values` columns per lane and two rows in flight leave registers for.
+constexpr int ln_fwd_blocks(int size) { return size == 4 ? 7 : 6; }
 constexpr int ln_bwd_blocks(int values) { return values <= 16 ? 4 : values <= 24 ? 3 : 2; }
 
-// One resident wave of blocks walks the rows, and each warp has the next row's 16-byte loads in flight while it reduces and writes
-// this one: a row's two warp-wide sums are a serial chain of shuffles that would otherwise leave the memory idle. HBM bounds both.
-// bf16, 65536 x 768 (residual, pre kept): 67 us, 6.0 TB/s; without the rows ahead, a block per four rows, 81 us. 4096 x 768: 10.4
-// against 11.0. The backward below, parameter gradients accumulated: 65536 x 768 55 us (5.5 TB/s) against 104, 4096 x 768 8.6 against
-// 13.1; 65536 x 1024, where two blocks fit an SM, 133 against 245; fp32 32768 x 768 62 against 97.
+// A warp per row, all its loads issued before anything is done with them, six or seven blocks on an SM: a row's two warp-wide sums are a serial chain of
+// shuffles, which other warps' loads cover. HBM bounds it (65536 x 768 bf16, residual, pre kept: 61 us, 6.5 TB/s), below some 16 MB L2.
+// us, plain / with residual, in brackets a load where it is used, and one wave of warps that walk the rows with the next row's loads in flight:
+// bf16 65536 x 768 49 / 61 (60 / 81, 50 / 65), 4096 x 768 5.0 / 5.6 (5.6 / 6.0, 6.2 / 6.5), 65536 x 256 20 / 25 (21 / 30, 31 / 36), 4096 x 1024 6.2 / 6.9
+// (6.4 / 6.8, 7.8 / 8.4), fp32 4096 x 1024 6.2 / 8.7 (7.3 / 9.3, 10.9 / 11.2), 65536 x 1024 95 / 166 (110 / 165, 119 / 156).
 template <typename T, int VPL, typename P>
-__global__ void __launch_bounds__(kLnWarps * 32, ln_fwd_blocks(VPL * VecIO<T>::kVec))
+__global__ void __launch_bounds__(kLnWarps * 32, ln_fwd_blocks(sizeof(T)))
 ln_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const P* __restrict__ gamma,
               const P* __restrict__ beta, T* __restrict__ y, T* __restrict__ pre_out,
               float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols, float eps,
@@ -82,89 +83,88 @@ ln_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const P* 
   const int nvec = cols / V;
   const float inv_keep = p_drop > 0.f ? 1.f / (1.f - p_drop) : 1.f;
 
+  const int row = blockIdx.x * kLnWarps + warp;
+  if (row >= rows) return;
+  // all loads of the row before anything is done with them
   uint4 nx[VPL], nr[VPL];
-  auto fetch = [&](int row) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<long long>(row) * cols);
-    const uint4* rr = reinterpret_cast<const uint4*>(residual + static_cast<long long>(row) * cols);
+  const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<long long>(row) * cols);
+  const uint4* rr = reinterpret_cast<const uint4*>(residual + static_cast<long long>(row) * cols);
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int vi = lane + i * 32;
-      if (vi < nvec) {
-        nx[i] = xr[vi];
-        if (residual) nr[i] = rr[vi];
-      }
+  for (int i = 0; i < VPL; ++i) {
+    const int vi = lane + i * 32;
+    if (vi < nvec) {
+      nx[i] = xr[vi];
+      if (residual) nr[i] = rr[vi];
     }
-  };
-  int row = blockIdx.x * kLnWarps + warp;
-  if (row < rows) fetch(row);
-  for (; row < rows; row += gridDim.x * kLnWarps) {
-    float v[VPL][V];
-    float sum = 0.f;
+  }
+  float v[VPL][V];
+  float sum = 0.f;
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int vi = lane + i * 32;
-      if (vi < nvec) {
-        VecIO<T>::unpack(nx[i], v[i]);
-        if (p_drop > 0.f) {
-          const uint64_t base = static_cast<uint64_t>(row) * cols + static_cast<uint64_t>(vi) * V;
+  for (int i = 0; i < VPL; ++i) {
+    const int vi = lane + i * 32;
+    if (vi < nvec) {
+      VecIO<T>::unpack(nx[i], v[i]);
+      if (p_drop > 0.f) {
+        const uint64_t base = static_cast<uint64_t>(row) * cols + static_cast<uint64_t>(vi) * V;
 #pragma unroll
-          for (int j = 0; j < V; j += 4) {
-            float s[4];
-            dropout_scale4(seed, base + j, p_drop, inv_keep, s);
+        for (int j = 0; j < V; j += 4) {
+          float s[4];
+          dropout_scale4(seed, base + j, p_drop, inv_keep, s);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) v[i][j + k] *= s[k];
-          }
-        }
-        if (residual) {
-          float r[V];
-          VecIO<T>::unpack(nr[i], r);
-#pragma unroll
-          for (int j = 0; j < V; ++j) v[i][j] += r[j];
-        }
-        if (pre_out) {
-          // keep what the backward pass will see: the value rounded to the storage type
-          VecIO<T>::store(pre_out + static_cast<long long>(row) * cols + vi * V, v[i]);
-        }
-#pragma unroll
-        for (int j = 0; j < V; ++j) sum += v[i][j];
-      } else {
-#pragma unroll
-        for (int j = 0; j < V; ++j) v[i][j] = 0.f;
-      }
-    }
-    if (row + gridDim.x * kLnWarps < rows) fetch(row + gridDim.x * kLnWarps);
-    const float mean = warp_sum(sum) / cols;
-    float sq = 0.f;
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      if (lane + i * 32 < nvec) {
-#pragma unroll
-        for (int j = 0; j < V; ++j) {
-          const float d = v[i][j] - mean;
-          sq += d * d;
+          for (int k = 0; k < 4; ++k) v[i][j + k] *= s[k];
         }
       }
-    }
-    const float rstd = rsqrtf(warp_sum(sq) / cols + eps);
-    if (lane == 0) {
-      if (mean_out) mean_out[row] = mean;
-      if (rstd_out) rstd_out[row] = rstd;
-    }
+      if (residual) {
+        float r[V];
+        VecIO<T>::unpack(nr[i], r);
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int vi = lane + i * 32;
-      if (vi < nvec) {
-        float o[V], g[V], b[V];
-        load_f32_vec<V>(gamma, vi * V, 1.f, g);
-        load_f32_vec<V>(beta, vi * V, 0.f, b);
-#pragma unroll
-        for (int j = 0; j < V; ++j) o[j] = fmaf((v[i][j] - mean) * rstd, g[j], b[j]);
-        VecIO<T>::store(y + static_cast<long long>(row) * cols + vi * V, o);
+        for (int j = 0; j < V; ++j) v[i][j] += r[j];
       }
+      if (pre_out) {
+        // keep what the backward pass will see: the value rounded to the storage type
+        VecIO<T>::store(pre_out + static_cast<long long>(row) * cols + vi * V, v[i]);
+      }
+#pragma unroll
+      for (int j = 0; j < V; ++j) sum += v[i][j];
+    } else {
+#pragma unroll
+      for (int j = 0; j < V; ++j) v[i][j] = 0.f;
+    }
+  }
+  const float mean = warp_sum(sum) / cols;
+  float sq = 0.f;
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    if (lane + i * 32 < nvec) {
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        const float d = v[i][j] - mean;
+        sq += d * d;
+      }
+    }
+  }
+  const float rstd = rsqrtf(warp_sum(sq) / cols + eps);
+  if (lane == 0) {
+    if (mean_out) mean_out[row] = mean;
+    if (rstd_out) rstd_out[row] = rstd;
+  }
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    const int vi = lane + i * 32;
+    if (vi < nvec) {
+      float o[V], g[V], b[V];
+      load_f32_vec<V>(gamma, vi * V, 1.f, g);
+      load_f32_vec<V>(beta, vi * V, 0.f, b);
+#pragma unroll
+      for (int j = 0; j < V; ++j) o[j] = fmaf((v[i][j] - mean) * rstd, g[j], b[j]);
+      VecIO<T>::store(y + static_cast<long long>(row) * cols + vi * V, o);
     }
   }
 }
 
+// One resident wave of blocks walks the rows, because each keeps sums for the parameter gradients, and each warp has the next row's 16-byte loads
+// in flight while it reduces and writes this one. HBM bounds it. bf16, parameter gradients accumulated, against a block per four rows: 65536 x 768
+// 54 us (5.5 TB/s) against 104, 65536 x 1024, where two blocks fit an SM, 133 against 245; fp32 32768 x 768 60 against 97.
 template <typename T, int VPL>
 __global__ void __launch_bounds__(kLnWarps * 32, ln_bwd_blocks(VPL * VecIO<T>::kVec))
 ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ pre, const float* __restrict__ mean,
@@ -349,9 +349,7 @@ template <typename T, int VPL, typename P>
 static int ln_fwd_launch(const void* x, const void* res, const P* gamma, const P* beta, void* y,
                          void* pre, float* mean, float* rstd, int rows, int cols, float eps, float p,
                          uint64_t seed, const unsigned long long* seed_dev, cudaStream_t st) {
-  // fp32 rows are twice the registers: there a block per four rows measured better (32768 x 768: 62 against 72 us)
-  const int need = (rows + kLnWarps - 1) / kLnWarps, wave = sm_count() * ln_fwd_blocks(VPL * VecIO<T>::kVec);
-  launch_pdl(ln_fwd_kernel<T, VPL, P>, dim3(need < wave || sizeof(T) == 4 ? need : wave), dim3(kLnWarps * 32), 0, st, static_cast<const T*>(x), static_cast<const T*>(res), gamma, beta, static_cast<T*>(y),
+  launch_pdl(ln_fwd_kernel<T, VPL, P>, dim3((rows + kLnWarps - 1) / kLnWarps), dim3(kLnWarps * 32), 0, st, static_cast<const T*>(x), static_cast<const T*>(res), gamma, beta, static_cast<T*>(y),
       static_cast<T*>(pre), mean, rstd, rows, cols, eps, p, seed, seed_dev);
   return static_cast<int>(cudaGetLastError());
 }
