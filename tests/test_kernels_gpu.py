@@ -196,6 +196,13 @@ def test_layernorm_rows_per_warp(C, dtype, rows, cols):
     assert close(acc_g - 1, dg.double(), 2 ** -14) and close(acc_b - 1, db.double(), 2 ** -14)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,cols", [(1183, 128), (1185, 64), (2371, 256), (9473, 128), (3555, 768)])
+def test_layernorm_backward_grids(C, dtype, rows, cols):
+    """Row counts around those at which the backward pass takes fewer blocks than a wave; bounds as above."""
+    test_layernorm_rows_per_warp(C, dtype, rows, cols)
+
+
 @pytest.mark.parametrize("dtype,V", [(torch.bfloat16, 4104), (torch.bfloat16, 32768), (torch.bfloat16, 32776), (torch.float32, 16384), (torch.float32, 16388)])
 def test_softmax_ce_block_sizes(C, dtype, V):
     """Either side of the row length at which a block's size changes, with more rows than resident blocks. The gradient carries one rounding to its
