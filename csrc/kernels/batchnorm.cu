@@ -255,7 +255,7 @@ bn_bwd_apply_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* 
 // block. The last block to finish (device counter) folds the partial rows, so each pass is still
 // one launch: statistics pass -> mean / rstd / running stats, backward reduction -> dgamma, dbeta
 // and the two means the dx pass needs.
-constexpr int kBnMaxBlocks = 592;     // 4 per SM on a 148-SM part
+constexpr int kBnMaxBlocks = 592;     // partial rows that the scratch holds; the passes take at most this many blocks
 
 template <typename T>
 struct NhwcMap {
@@ -357,14 +357,16 @@ __device__ __forceinline__ void nhwc_fold(const float* __restrict__ partial, int
   __syncthreads();
 }
 
-// The channels-last passes below read up to three tensors and write up to two, once each: HBM (or, at CIFAR batches, L2) bounds
-// them if enough loads are in flight, so a thread fetches kBnBatch pixels of every tensor before it works on the first. ResNet-20
-// steps with one pixel at a time and four blocks per SM against this: batch 128 1199 -> 1173 us, batch 1000 3829 -> 3699 us.
-constexpr int kBnBatch = 2;
-constexpr int kBnPerSm = 3;      // resident blocks per SM that the registers of such a batch allow; the grid is one wave of them
+// The channels-last passes below read up to three tensors and write up to two, once each: HBM (or, at CIFAR batches, L2) bounds them if enough
+// loads are in flight. A thread fetches four pixels of every tensor before it works on the first, on as many blocks per SM as the registers of that
+// allow, in one wave; the statistics pass, one tensor and two sums, does better with more blocks and a loop that the compiler unrolls.
+// us back to back, bf16, [pixels, channels] of 128 x 32 x 32 x 16 / 1000 x 32 x 32 x 64, in brackets all passes with two pixels and three blocks: statistics
+// 5.7 / 31 (6.4 / 55), apply 3.2 / 43 (3.4 / 51), with residual 3.5 / 64 (3.8 / 63), backward sums 6.7 / 65 (7.7 / 67), backward apply 3.6 / 79 (5.7 / 97).
+constexpr int kBnBatch = 4;
+constexpr int kBnStatsPerSm = 4, kBnApplyPerSm = 3, kBnBwdPerSm = 2;
 
 template <typename T>
-__global__ void __launch_bounds__(kBnThreads, kBnPerSm)
+__global__ void __launch_bounds__(kBnThreads, kBnStatsPerSm)
 bn_nhwc_stats_kernel(const T* __restrict__ x, float* __restrict__ partial, unsigned int* __restrict__ counter,
                      float* __restrict__ running_mean, float* __restrict__ running_var, float* __restrict__ save_mean,
                      float* __restrict__ save_rstd, long long P, int C, float eps, float momentum) {
@@ -376,20 +378,11 @@ bn_nhwc_stats_kernel(const T* __restrict__ x, float* __restrict__ partial, unsig
 #pragma unroll
   for (int j = 0; j < V; ++j) a[j] = b[j] = 0.f;
   if (m.active()) {
-    const long long step = static_cast<long long>(gridDim.x) * m.lanes;
-    for (long long p0 = static_cast<long long>(blockIdx.x) * m.lanes + m.lane(); p0 < P; p0 += kBnBatch * step) {
-      uint4 xr[kBnBatch];
+    for (long long p = static_cast<long long>(blockIdx.x) * m.lanes + m.lane(); p < P; p += static_cast<long long>(gridDim.x) * m.lanes) {
+      float v[V];
+      VecIO<T>::load(x + p * C + m.col(), v);
 #pragma unroll
-      for (int u = 0; u < kBnBatch; ++u)
-        if (p0 + u * step < P) xr[u] = *reinterpret_cast<const uint4*>(x + (p0 + u * step) * C + m.col());
-#pragma unroll
-      for (int u = 0; u < kBnBatch; ++u) {
-        if (p0 + u * step >= P) break;
-        float v[V];
-        VecIO<T>::unpack(xr[u], v);
-#pragma unroll
-        for (int j = 0; j < V; ++j) { a[j] += v[j]; b[j] += v[j] * v[j]; }
-      }
+      for (int j = 0; j < V; ++j) { a[j] += v[j]; b[j] += v[j] * v[j]; }
     }
   }
   if (!nhwc_publish<T>(m, C, a, b, partial, counter, sm)) return;
@@ -412,7 +405,7 @@ bn_nhwc_stats_kernel(const T* __restrict__ x, float* __restrict__ partial, unsig
 // also records them for the backward pass and updates the running statistics. One launch, no
 // statistics pass over x.
 template <typename T, bool kFromSums>
-__global__ void __launch_bounds__(kBnThreads, kBnPerSm)
+__global__ void __launch_bounds__(kBnThreads, kBnApplyPerSm)
 bn_nhwc_apply_kernel(const T* __restrict__ x, const T* __restrict__ residual, const float* __restrict__ gamma,
                      const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ rstd,
                      T* __restrict__ y, long long P, int C, int relu, const float* __restrict__ sums, float* __restrict__ save_mean,
@@ -476,7 +469,7 @@ bn_nhwc_apply_kernel(const T* __restrict__ x, const T* __restrict__ residual, co
 
 // fold[0..C) = mean of dy', fold[C..2C) = mean of dy' * xhat
 template <typename T>
-__global__ void __launch_bounds__(kBnThreads, kBnPerSm)
+__global__ void __launch_bounds__(kBnThreads, kBnBwdPerSm)
 bn_nhwc_bwd_reduce_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ y, const float* __restrict__ mean,
                           const float* __restrict__ rstd, float* __restrict__ partial, unsigned int* __restrict__ counter,
                           float* __restrict__ fold, float* __restrict__ dgamma, float* __restrict__ dbeta, int accumulate,
@@ -534,7 +527,7 @@ bn_nhwc_bwd_reduce_kernel(const T* __restrict__ dy, const T* __restrict__ x, con
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kBnThreads, kBnPerSm)
+__global__ void __launch_bounds__(kBnThreads, kBnBwdPerSm)
 bn_nhwc_bwd_apply_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ y, const float* __restrict__ gamma,
                          const float* __restrict__ mean, const float* __restrict__ rstd, const float* __restrict__ fold,
                          T* __restrict__ dx, T* __restrict__ dres, long long P, int C, int relu) {
@@ -592,12 +585,13 @@ static int nhwc_iters() {
   }
   return it;
 }
-static int nhwc_grid(long long P, int C, int V) {
+static int nhwc_grid(long long P, int C, int V, int per_sm) {
   const int lanes = kBnThreads / (C / V);
   const long long per = static_cast<long long>(lanes) * nhwc_iters();
   long long want = (P + per - 1) / per;
   if (want < 1) want = 1;
-  const int wave = 148 * kBnPerSm;
+  int wave = sm_count() * per_sm;
+  if (wave > kBnMaxBlocks) wave = kBnMaxBlocks;
   return static_cast<int>(want < wave ? want : wave);
 }
 
@@ -616,14 +610,14 @@ extern "C" int fb_bn_nhwc_fwd(const void* x, const void* residual, const float* 
   const int V = is_bf16 ? 8 : 4;
   if (C % V || C > kBnThreads) return -4;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int grid = nhwc_grid(P, C, V);
+  const int grid_stats = nhwc_grid(P, C, V, kBnStatsPerSm), grid = nhwc_grid(P, C, V, kBnApplyPerSm);
   const int lanes = kBnThreads / (C / V);
   const size_t smem = sizeof(float) * 2 * lanes * C;
   const float* mean = training ? save_mean : running_mean;
   if (is_bf16) {
     using T = __nv_bfloat16;
     if (training)
-      launch_pdl(bn_nhwc_stats_kernel<T>, dim3(grid), dim3(kBnThreads), smem, st, static_cast<const T*>(x), scratch, counter, running_mean, running_var,
+      launch_pdl(bn_nhwc_stats_kernel<T>, dim3(grid_stats), dim3(kBnThreads), smem, st, static_cast<const T*>(x), scratch, counter, running_mean, running_var,
                                                              save_mean, save_rstd, P, C, eps, momentum);
     else return -6;   // evaluation mode goes through the framework's generic path
     launch_pdl(bn_nhwc_apply_kernel<T, false>, dim3(grid), dim3(kBnThreads), 0, st, static_cast<const T*>(x), static_cast<const T*>(residual), gamma, beta, mean,
@@ -632,7 +626,7 @@ extern "C" int fb_bn_nhwc_fwd(const void* x, const void* residual, const float* 
   } else {
     using T = float;
     if (training)
-      launch_pdl(bn_nhwc_stats_kernel<T>, dim3(grid), dim3(kBnThreads), smem, st, static_cast<const T*>(x), scratch, counter, running_mean, running_var,
+      launch_pdl(bn_nhwc_stats_kernel<T>, dim3(grid_stats), dim3(kBnThreads), smem, st, static_cast<const T*>(x), scratch, counter, running_mean, running_var,
                                                              save_mean, save_rstd, P, C, eps, momentum);
     else return -6;
     launch_pdl(bn_nhwc_apply_kernel<T, false>, dim3(grid), dim3(kBnThreads), 0, st, static_cast<const T*>(x), static_cast<const T*>(residual), gamma, beta, mean,
@@ -652,7 +646,7 @@ extern "C" int fb_bn_nhwc_fwd_sums(const void* x, const void* residual, const fl
   const int V = is_bf16 ? 8 : 4;
   if (C % V || C > kBnThreads || !sums) return -4;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int grid = nhwc_grid(P, C, V);
+  const int grid = nhwc_grid(P, C, V, kBnApplyPerSm);
   if (is_bf16) {
     using T = __nv_bfloat16;
     launch_pdl(bn_nhwc_apply_kernel<T, true>, dim3(grid), dim3(kBnThreads), 0, st, static_cast<const T*>(x), static_cast<const T*>(residual), gamma, beta, nullptr,
@@ -675,7 +669,7 @@ extern "C" int fb_bn_nhwc_bwd(const void* dy, const void* x, const void* y, cons
   const int V = is_bf16 ? 8 : 4;
   if (C % V || C > kBnThreads) return -4;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int grid = nhwc_grid(P, C, V);
+  const int grid = nhwc_grid(P, C, V, kBnBwdPerSm);
   const int lanes = kBnThreads / (C / V);
   const size_t smem = sizeof(float) * 2 * lanes * C;
   float* fold = scratch + static_cast<long long>(kBnMaxBlocks) * 2 * C;
