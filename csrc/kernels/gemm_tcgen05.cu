@@ -1011,7 +1011,7 @@ static int split_clusters() {
 
 // Long reductions (kSplitMinK) with no more tiles than the device holds clusters at once: one more and the last tile would run
 // alone, when the persistent kernel does not need the pairs' full number. Mostly padding (less than 0.8 useful) is left to narrower tiles.
-// Products of fewer than 75 tiles of 128 x 64 went to gemm_small.cu before this is asked.
+// Products of so few tiles of 128 x 64 that gemm_small.cu applies went there before this is asked.
 static bool split_applies(int M, int N, int K) {
   const long long tiles = static_cast<long long>((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
   return K >= kSplitMinK && tiles <= split_clusters() && static_cast<long long>(M) * N * 10 >= tiles * 256 * 256 * 8;

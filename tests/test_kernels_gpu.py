@@ -136,6 +136,36 @@ def test_gemm_few_tiles(C, M, N, K, b_mn, epi, pad=4):
     assert torch.all(out[:, N:] == 0)
 
 
+def _launched(call):
+    """Names of the kernels that a call launches."""
+    from torch.profiler import ProfilerActivity, profile
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as seen:
+        call()
+        torch.cuda.synchronize()
+    return " ".join(e.name for e in seen.events() if e.device_type == torch.autograd.DeviceType.CUDA)
+
+
+@pytest.mark.parametrize("M,N,K,kernel", [(96, 128, 64, "small"), (97, 128, 448, "bf16"), (97, 128, 512, "small"), (128, 37 * 64, 512, "small"), (128, 38 * 64, 512, "bf16"),
+                                          (128, 74 * 64, 768, "small"), (128, 75 * 64, 768, "bf16"), (130, 64, 4096, "small"), (1, 768, 768, "small"),
+                                          (2048, 1024, 1280, "split"), (2048, 1024, 1272, "bf16"), (1300, 504, 1544, "split"), (1800, 1000, 1352, "split"), (4096, 512, 2048, "split"),
+                                          (4096, 3072, 2048, "bf16")])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_gemm_goes_to_the_kernel_that_the_dispatch_means(C, M, N, K, kernel, b_mn):
+    """Both sides of each line of the dispatch, as it lies on 148 SMs, most shapes of the two tests around this one among them."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines are proportional to the number of SMs")
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    b = torch.randn(*((K, N) if b_mn else (N, K)), device="cuda").bfloat16()
+    out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    names = _launched(lambda: C.gemm(a, b, out, False, b_mn))
+    assert f"gemm_{kernel}_kernel" in names, names
+    A, B = a.double(), (b.t() if b_mn else b).double()
+    ref = A @ B.t()
+    assert ((out.double() - ref).norm() / ref.norm()).item() < 2 ** -8
+
+
 @pytest.mark.parametrize("M,N,K", [(1800, 1000, 1352), (1300, 504, 1544), (4096, 512, 2048)])
 @pytest.mark.parametrize("b_mn", [False, True])
 @pytest.mark.parametrize("epi", [0, 1, 2, 3, 4])
