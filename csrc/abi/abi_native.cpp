@@ -8,6 +8,7 @@
 // is bf16 already, or autocast is on for CUDA with bf16 (`flodl_autocast_*`). Everything else, and every
 // shape the kernels do not cover, returns false and the caller forwards to ATen. FLODL_B200_NATIVE=0
 // turns the native paths off (for A/B timing).
+#include "device_word.h"
 #include "abi_common.hpp"
 
 #include <ATen/autocast_mode.h>
@@ -64,11 +65,15 @@ void check(int rc, const char* what) {
 // One status word per device for the kernels with bounded waits (GEMM, attention).
 int* status_word(int device) {
   static std::mutex mu;
-  static std::vector<Tensor> words(64);
+  static std::vector<int*> words(64, nullptr);
   std::lock_guard<std::mutex> lock(mu);
   TORCH_CHECK(device >= 0 && device < 64);
-  if (!words[device].defined()) words[device] = torch::zeros({1}, torch::dtype(torch::kInt32).device(torch::kCUDA, device));
-  return words[device].data_ptr<int>();
+  if (!words[device]) {
+    c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+    const cudaError_t e = fb::zeroed_device_word(&words[device]);
+    TORCH_CHECK(e == cudaSuccess, "device word: ", cudaGetErrorString(e));
+  }
+  return words[device];
 }
 int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 // [rows, cols] tensor whose row stride is a multiple of 8 elements (what a TMA descriptor can address)

@@ -6,9 +6,11 @@
 #include <torch/extension.h>
 
 #include <array>
+#include <mutex>
 #include <optional>
 #include <vector>
 
+#include "device_word.h"
 #include "flodl_b200.h"
 
 namespace {
@@ -44,13 +46,28 @@ const unsigned long long* seed_ptr(const OptTensor& t) {
   return reinterpret_cast<const unsigned long long*>(t->data_ptr());
 }
 
-// one status word per device, shared by every kernel that has bounded waits
+// One zeroed word per device and kind, for good.
+struct DeviceWords {
+  std::mutex mu;
+  std::vector<Tensor> words{64};
+  Tensor& get(int device) {
+    TORCH_CHECK(device >= 0 && device < 64);
+    std::lock_guard<std::mutex> lock(mu);
+    if (!words[device].defined()) {
+      c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+      int* word = nullptr;
+      const cudaError_t e = fb::zeroed_device_word(&word);
+      TORCH_CHECK(e == cudaSuccess, "device word: ", cudaGetErrorString(e));
+      words[device] = torch::from_blob(word, {1}, torch::dtype(torch::kInt32).device(torch::kCUDA, device));
+    }
+    return words[device];
+  }
+};
+
+// the status word, shared by every kernel that has bounded waits
 Tensor& status_word(int device) {
-  static std::vector<Tensor> words(64);
-  TORCH_CHECK(device >= 0 && device < 64);
-  if (!words[device].defined())
-    words[device] = torch::zeros({1}, torch::dtype(torch::kInt32).device(torch::kCUDA, device));
-  return words[device];
+  static DeviceWords words;
+  return words.get(device);
 }
 
 // ------------------------------------------------------------------------------------------ GEMM
@@ -398,11 +415,8 @@ Tensor grad_norm(const Tensor& g, double max_norm, double extra_scale) {
 // ------------------------------------------------------------------------------------ batch norm
 // one zeroed word per device for the channels-last BatchNorm "last block folds" counter
 Tensor& bn_counter(int device) {
-  static std::vector<Tensor> words(64);
-  TORCH_CHECK(device >= 0 && device < 64);
-  if (!words[device].defined())
-    words[device] = torch::zeros({1}, torch::dtype(torch::kInt32).device(torch::kCUDA, device));
-  return words[device];
+  static DeviceWords words;
+  return words.get(device);
 }
 bool is_channels_last_4d(const Tensor& t) {
   return t.dim() == 4 && t.is_contiguous(at::MemoryFormat::ChannelsLast) && !t.is_contiguous();

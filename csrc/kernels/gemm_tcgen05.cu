@@ -905,11 +905,15 @@ static EncodeTiledFn get_encode_fn() {
 }
 
 // The tensor-map encoder is a driver-API call and wants a context current on the calling thread;
-// autograd's backward threads only have the runtime's lazy binding, so bind once per thread.
+// autograd's backward threads only have the runtime's lazy binding, so bind once per thread. The call that does it is refused while a stream is
+// captured, and a thread's first product may be under capture, so it is made in the relaxed mode.
 void ensure_thread_context() {
   static thread_local bool ready = false;
   if (!ready) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     cudaFree(nullptr);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     ready = true;
   }
 }

@@ -944,3 +944,37 @@ def test_packed_linear_without_gradients(C, rows, N, K, bias, dtype, order):
     assert close(got, want, 2 ** -8) and close(norm, ref, 2 ** -7)
     act = torch.nn.functional.gelu(want[:, 0].detach().double())
     assert close(ffn, act, 2 ** -7)
+
+
+def test_first_calls_of_a_process_under_capture():
+    """An eager step of small tensors runs no native kernel, so that a process may meet its first one while it captures: the calls that set a thread
+    or a device up have to be legal there, and the status word must not be part of the graph."""
+    code = """
+import torch
+from flodl_b200 import _ext
+C = _ext.require()
+a, b = torch.randn(200, 128, device="cuda").bfloat16(), torch.randn(64, 128, device="cuda").bfloat16()
+q, k, v = torch.randn(1, 300, 3, 2, 64, device="cuda").bfloat16().unbind(2)
+out = torch.zeros(200, 64, device="cuda", dtype=torch.bfloat16)
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g, capture_error_mode="thread_local"):
+    C.gemm(a, b, out)
+    o, lse = C.attn_fwd(q, k, v, None, 0.125, False)
+assert C.read_status(0) == 0
+g.replay()
+torch.cuda.synchronize()
+assert C.read_status(0) == 0
+ref = a.double() @ b.double().t()
+assert ((out.double() - ref).norm() / ref.norm()).item() < 2 ** -8
+s = torch.softmax(torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) * 0.125, -1)
+ref = torch.einsum("bhqk,bkhd->bqhd", s, v.double())
+assert ((o.double() - ref).norm() / ref.norm()).item() < 2 ** -8
+print("CAPTURE_OK")
+"""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    res = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=root)
+    assert res.returncode == 0 and "CAPTURE_OK" in res.stdout, res.stdout[-2000:] + res.stderr[-3000:]
