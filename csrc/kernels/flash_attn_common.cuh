@@ -156,6 +156,7 @@ struct AttnParams {
   unsigned long long seed;
   const unsigned long long* seed_dev;
   int* status;
+  int group;                 // heads whose key blocks are handed out together in the backward pass: one for each SM
 };
 
 inline AttnParams make_params(int B, int H, int S, const long long* qs, const long long* os, const long long* gs, const float* mask,
@@ -166,6 +167,7 @@ inline AttnParams make_params(int B, int H, int S, const long long* qs, const lo
   p.osb = os[0]; p.oss = os[1]; p.osh = os[2];
   p.gsb = gs[0]; p.gss = gs[1]; p.gsh = gs[2]; p.scale = scale; p.causal = causal;
   p.p_drop = p_drop; p.seed = seed; p.seed_dev = seed_dev; p.status = status;
+  p.group = sm_count();
   return p;
 }
 

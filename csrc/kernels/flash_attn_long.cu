@@ -29,7 +29,6 @@ namespace fb {
 // ==================================================================================== backward
 namespace {
 
-constexpr int kSMs = 148;
 constexpr int kBwdStages = 3;
 constexpr int kBwdSoftmaxWarps = 16;
 constexpr int kBwdThreads = 32 * (kBwdSoftmaxWarps + 4 + 3);
@@ -183,7 +182,7 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (warp == kBwdSoftmaxWarps + 5 && lane == 0) {
     const int lin = ordered ? static_cast<int>(atomicAdd(&reinterpret_cast<DqSlot*>(dq)->ticket, 1u)) : blockIdx.x;
     int j, h, b;
-    decode_block(lin, nblk, p.H, p.B, p.causal != 0, ordered ? kSMs : 1, j, h, b);
+    decode_block(lin, nblk, p.H, p.B, p.causal != 0, ordered ? p.group : 1, j, h, b);
     item[0] = j; item[1] = h; item[2] = b;
   }
   if (threadIdx.x == 0) {
@@ -464,7 +463,7 @@ int attn_bwd_long(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
   const long long items = static_cast<long long>((p.S + kBlk - 1) / kBlk) * p.H * p.B;
   const long long rows = static_cast<long long>(p.B) * p.H * p.S;
   if (items > 0x7fffffffll) return -4;
-  const int row_grid = static_cast<int>(rows / 32 + 1 < kSMs * 16 ? rows / 32 + 1 : kSMs * 16);
+  const int row_grid = static_cast<int>(rows / 32 + 1 < p.group * 16 ? rows / 32 + 1 : p.group * 16);
   auto* dq16 = static_cast<__nv_bfloat16*>(dq);
   launch_pdl(attn_bwd_pre_kernel, dim3(row_grid), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), dq16, dq_accum, p);
   launch_pdl(attn_bwd_long_kernel, dim3(static_cast<unsigned>(items)), dim3(kBwdThreads), static_cast<size_t>(BwdLong::TOTAL), stream, tq, tk, tv, tdo, lse,
