@@ -592,6 +592,99 @@ def test_attention_several_key_blocks_dropout(C):
     assert abs(a - b) < 2 ** -7 * abs(a), (a, b)
 
 
+def _attn_restated(q, k, v, do, mask, scale, causal, z=None):
+    """Output and gradients of attention in 64 bits, exact, and again with what the kernels round to bf16 rounded: O before it is used in D, the
+    probabilities and dS before their products. A row without a live key has an output and gradients of zero."""
+    q, k, v, do = (t.double().permute(0, 2, 1, 3) for t in (q, k, v, do))
+    s = q @ k.transpose(-1, -2) * scale
+    if mask is not None:
+        s = s + mask.double()[:, None, None, :]
+    if causal:
+        s = s.masked_fill(torch.ones(s.shape[-2:], dtype=torch.bool, device=s.device).triu(1), float("-inf"))
+    p = torch.softmax(s, -1).nan_to_num(0.0)
+    z = torch.ones_like(p) if z is None else z
+
+    def results(r):
+        o = (r(p * z) @ v)
+        ds = r(p * (do @ v.transpose(-1, -2) * z - (do * r(o)).sum(-1, keepdim=True)) * scale)
+        return [t.permute(0, 2, 1, 3) for t in (o, ds @ k, ds.transpose(-1, -2) @ q, r(p * z).transpose(-1, -2) @ do)]
+
+    return results(lambda t: t), results(lambda t: t.bfloat16().double())
+
+
+def _attn_check(C, q, k, v, mask, scale, causal, p_drop=0.0, seed=0, z=None):
+    """Forward and backward against 64 bits: in norm at most twice as far off as the restatement that rounds where the kernels have to, and the
+    rounding of the results themselves (2^-9)."""
+    do = torch.randn_like(q).contiguous()
+    C.clear_status(0)
+    o, lse = C.attn_fwd(q, k, v, mask, scale, causal, p_drop, seed)
+    dqkv = C.attn_bwd(q, k, v, o, do, lse, mask, scale, causal, p_drop, seed)
+    assert C.read_status(0) == 0
+    exact, rounded = _attn_restated(q, k, v, do, mask, scale, causal, z)
+    for name, got, want, near in zip(("o", "dq", "dk", "dv"), (o, dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]), exact, rounded):
+        assert torch.isfinite(got.float()).all(), name
+        err, norm = (got.double() - want).norm().item(), want.norm().item()
+        assert err <= 2 * (near - want).norm().item() + 2 ** -9 * norm + 1e-30, (name, err / norm, ((near - want).norm() / norm).item())
+    return o, lse, dqkv
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("scale", [0.125, -0.125])
+@pytest.mark.parametrize("S", [257, 641])
+def test_attention_growing_maxima(C, S, scale, causal):
+    """Row maxima that grow by ten and more in log2 from block to block in every other row, and hardly in the rows between, so that the accumulator is
+    rescaled in some rows of a warp; scores of either sign of the scale."""
+    torch.manual_seed(25)
+    q, k, v = (t.clone() for t in torch.randn(2, S, 3, 2, 64, device="cuda").bfloat16().unbind(2))       # three tensors, not slices of one
+    q[:, 1::2] *= 0.05
+    k *= (1 + 3 * (torch.arange(S, device="cuda") // 128))[None, :, None, None]
+    _attn_check(C, q, k, v, None, scale, causal)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("value", [-1e4, float("-inf")])
+def test_attention_first_block_and_whole_texts_masked(C, value, causal):
+    """Padding on the left that covers the first key block and more (the maximum starts at -inf, or far below), a text of which every key is masked, and
+    one of which none is. Where -inf leaves a row no key at all, output and gradients are zero."""
+    torch.manual_seed(26)
+    B, S = 3, 400
+    q, k, v = torch.randn(B, S, 3, 2, 64, device="cuda").bfloat16().unbind(2)
+    mask = torch.zeros(B, S, device="cuda")
+    mask[0, :150] = value
+    mask[1] = value
+    o, lse, dqkv = _attn_check(C, q, k, v, mask, 0.125, causal)
+    if value == float("-inf"):
+        dead = torch.zeros(B, S, dtype=torch.bool, device="cuda")
+        dead[1] = True
+        if causal:
+            dead[0, :150] = True
+        assert torch.all(o[dead] == 0) and torch.all(dqkv[:, :, 0][dead] == 0) and torch.all(lse.permute(0, 2, 1)[dead] == float("-inf"))
+        assert torch.all(dqkv[1] == 0)
+
+
+@pytest.mark.parametrize("causal,use_mask", [(False, False), (True, False), (False, True), (True, True)])
+def test_attention_several_key_blocks_dropout_gradients(C, causal, use_mask):
+    """All three gradients under dropout. The factors are read off the forward pass: with equal scores an output is the mean over the keys of factor times
+    value, and values that are unit vectors for 64 keys at a time pick the factors out."""
+    torch.manual_seed(27)
+    B, S, H, p_drop, seed = 2, 300, 2, 0.25, 77
+    zero = torch.zeros(B, S, H, 64, device="cuda").bfloat16()
+    z = torch.empty(B, H, S, S, device="cuda", dtype=torch.double)
+    for k0 in range(0, S, 64):
+        n = min(64, S - k0)
+        unit = zero.clone()
+        unit[:, k0:k0 + n] = torch.eye(64, device="cuda")[:n, None].bfloat16()
+        o, _ = C.attn_fwd(zero, zero, unit, None, 0.125, False, p_drop, seed)
+        z[..., k0:k0 + n] = (o.double().permute(0, 2, 1, 3)[..., :n] > 0).double() / (1 - p_drop)
+    assert abs((z > 0).double().mean().item() - (1 - p_drop)) < 0.01
+    q, k, v = torch.randn(B, S, 3, H, 64, device="cuda").bfloat16().unbind(2)
+    mask = None
+    if use_mask:
+        mask = torch.zeros(B, S, device="cuda")
+        mask[0, 200:] = -1e4
+    _attn_check(C, q, k, v, mask, 0.125, causal, p_drop, seed, z)
+
+
 def test_attention_dropout_statistics(C):
     torch.manual_seed(6)
     B, H, S, D = 2, 2, 128, 64
