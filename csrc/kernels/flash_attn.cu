@@ -6,9 +6,8 @@
 // (flodl/src/nn/attention.rs:108-151): additive key mask [B,S], causal masking, attention-prob
 // dropout, O(S) memory (only the log-sum-exp per row is saved).
 //
-// Work split: one CTA per (query block of 128 rows, head, batch) in the forward pass; in the backward pass one CTA
-// per (head, batch) for a single key block (S <= 128), see flash_attn_long.cu for more. 4 warps (one TMEM lane = one query row per thread) do the
-// softmax arithmetic; a fifth warp issues every TMA load and every `tcgen05.mma` from one thread.
+// This file: a single key block (S <= 128), one CTA per (head, batch) in either pass; flash_attn_long.cu has more. 4 warps (one TMEM lane = one
+// query row per thread) do the softmax arithmetic; a fifth warp issues every TMA load and every `tcgen05.mma` from one thread.
 // Q, K, V, dO tiles arrive by TMA with 128-byte swizzle in their natural [row][64] layout; the
 // same tile serves as a K-major operand (QK^T, dO V^T) or an MN-major operand (P V, P^T dO,
 // dS^T Q, dS K) by flipping the major bit of the instruction descriptor, so nothing is transposed.
@@ -350,8 +349,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const float inv_keep = p.p_drop > 0.f ? 1.f / (1.f - p.p_drop) : 1.f;
     const int q = t;
     const bool q_ok = q < p.S;
-    // the mask and the row statistics are in flight together: the LSE of a query row and D = rowsum(dO * O) (eight lanes
-    // per row, coalesced)
+    // The mask and the row statistics are in flight together: the LSE of a query row and D = rowsum(dO * O) (eight lanes per row, coalesced). The four
+    // warps start them at once, behind the tensor loads: 256 x 12 heads x 128 tokens 111 us, without the barrier 132.
+    asm volatile("bar.sync 1, 128;");
     const float mraw = (t < p.S && p.mask) ? __ldg(p.mask + static_cast<long long>(b) * p.S + t) : 0.f;
     const float lse_q = q_ok ? __ldg(lse + (static_cast<long long>(b) * p.H + h) * p.S + q) * kLog2e : 0.f;
     const float Dq = row_dot64(o + static_cast<long long>(b) * p.osb + static_cast<long long>(h) * p.osh,
