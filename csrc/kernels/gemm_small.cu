@@ -227,13 +227,14 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // CTAs per tile, or 0 where this kernel does not apply. It is taken up to half as many tiles of 128 x 64 as SMs; with more the split has no SMs to spread
 // over. The reduction has to be long enough for the split to pay for its hand-over, unless the tile is mostly padding, of which this kernel writes less:
 // us against the persistent kernel, 1024 x 256 x 256 5.3 (4.6), 4096 x 128 x 512 6.3 (5.9), 512 x 512 x 512 5.0 (5.8), 512 x 768 x 768 6.4 (7.3), 32 x 128 x 128
-// 2.9 (3.4), 128 x 128 x 128 4.0 (3.9). The reduction is split until every SM has a CTA or a CTA is down to two 64-wide steps: a step's products are over
+// 2.9 (3.4), 128 x 128 x 128 4.0 (3.9). `several` products in one launch save launches as well and are taken with any reduction: six encoder layers of width
+// 256 over 4 x 128 tokens 206 us, with Q, K and V one after the other 258. The reduction is split until every SM has a CTA or a CTA is down to two 64-wide steps: a step's products are over
 // long before its loads are.
-int gemm_small_split(int M, int N, int K) {
+int gemm_small_split(int M, int N, int K, bool several) {
   const long long tiles = static_cast<long long>((M + kTM - 1) / kTM) * ((N + kTN - 1) / kTN);
   const int num_kb = (K + kTK - 1) / kTK, sms = sm_count();
   if (tiles > sms / 2) return 0;
-  if (M > 96 && K < 768 && (K < 512 || tiles > sms / 4)) return 0;
+  if (!several && M > 96 && K < 768 && (K < 512 || tiles > sms / 4)) return 0;
   int split = static_cast<int>(sms / tiles);
   if (split > 8) split = 8;
   if (split > num_kb / 2) split = num_kb / 2;

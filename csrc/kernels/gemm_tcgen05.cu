@@ -47,7 +47,7 @@
 namespace fb {
 
 // gemm_small.cu
-int gemm_small_split(int M, int N, int K);
+int gemm_small_split(int M, int N, int K, bool several = false);
 bool gemm_small_aligned(int N, const void* C, long long ldc, const void* aux, long long ldaux);
 int gemm_small(const void* A, const void* const* B, void* C, int M, int group, int groups, int K, long long lda, long long ldb, long long ldc, int b_mn,
                const void* const* bias, int bias_fp32, int epi, void* aux, long long ldaux, const float* alpha, int split, int* status, cudaStream_t stream);
@@ -1174,7 +1174,7 @@ extern "C" int fb_gemm_bf16_grouped(const void* A, const void* const* B, void* C
   if (!bias) bias = none;
   bool aligned = lda % 8 == 0 && ldb % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && N % 64 == 0 && gemm_small_aligned(N, C, ldc, nullptr, 0);
   for (int g = 0; g < groups; ++g) aligned = aligned && (reinterpret_cast<uintptr_t>(B[g]) & 15) == 0;
-  const int split = aligned ? gemm_small_split(M, N * groups, K) : 0;
+  const int split = aligned ? gemm_small_split(M, N * groups, K, groups > 1) : 0;
   if (split)
     return gemm_small(A, B, C, M, N, groups, K, lda, ldb, ldc, 0, bias, bias_fp32, FB_EPI_NONE, nullptr, 0, nullptr, split, status, static_cast<cudaStream_t>(stream_));
   for (int g = 0; g < groups; ++g) {

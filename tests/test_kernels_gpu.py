@@ -166,6 +166,21 @@ def test_gemm_goes_to_the_kernel_that_the_dispatch_means(C, M, N, K, kernel, b_m
     assert ((out.double() - ref).norm() / ref.norm()).item() < 2 ** -8
 
 
+@pytest.mark.parametrize("M,N,K,launches", [(512, 256, 256, 1), (200, 512, 512, 1), (128, 1536, 64, 1), (128, 1600, 64, 3)])
+def test_grouped_gemm_is_one_launch_where_it_is_small(C, M, N, K, launches):
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the line is proportional to the number of SMs")
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    ws = [(torch.randn(N, K, device="cuda") / math.sqrt(K)).bfloat16() for _ in range(3)]
+    bs = [torch.randn(N, device="cuda") for _ in range(3)]
+    out = torch.empty(M, 3 * N, device="cuda", dtype=torch.bfloat16)
+    names = _launched(lambda: C.gemm_grouped(a, ws, out, bs))
+    assert names.count("gemm_") == launches and (launches == 3 or "gemm_small_kernel" in names), names
+    for g in range(3):
+        ref = a.double() @ ws[g].double().t() + bs[g].double()
+        assert ((out[:, g * N:(g + 1) * N].double() - ref).norm() / ref.norm()).item() < 2 ** -8
+
+
 @pytest.mark.parametrize("M,N,K", [(1800, 1000, 1352), (1300, 504, 1544), (4096, 512, 2048)])
 @pytest.mark.parametrize("b_mn", [False, True])
 @pytest.mark.parametrize("epi", [0, 1, 2, 3, 4])
