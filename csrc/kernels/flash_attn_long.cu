@@ -20,6 +20,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "../include/flodl_b200.h"
 #include "flash_attn_common.cuh"
@@ -774,17 +775,19 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 }  // namespace
 
 int attn_fwd_long(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* o, float* lse, const AttnParams& p, cudaStream_t stream) {
-  const auto kern = p.p_drop > 0.f ? (p.mask ? attn_fwd_long_kernel<true, true> : attn_fwd_long_kernel<true, false>)
-                                   : (p.mask ? attn_fwd_long_kernel<false, true> : attn_fwd_long_kernel<false, false>);
-  constexpr int smem = FwdLong::TOTAL + 1024;
-  for (const cudaError_t e : {allow_smem<attn_fwd_long_kernel<true, true>>(smem, true), allow_smem<attn_fwd_long_kernel<true, false>>(smem, true),
-                              allow_smem<attn_fwd_long_kernel<false, true>>(smem, true), allow_smem<attn_fwd_long_kernel<false, false>>(smem, true)})
-    if (e != cudaSuccess) return static_cast<int>(e);
   const long long ctas = static_cast<long long>((p.S + kBlk - 1) / kBlk) * p.H * p.B;
   if (ctas > 0x7fffffffll) return -4;
-  const cudaError_t e = launch_pdl(kern, dim3(static_cast<unsigned>(ctas)), dim3(kFwdThreads), static_cast<size_t>(smem), stream, tq, tk,
-                                   tv, static_cast<__nv_bfloat16*>(o), lse, p);
-  return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+  const auto go = [&](auto drop, auto mask) {
+    constexpr auto kern = attn_fwd_long_kernel<decltype(drop)::value, decltype(mask)::value>;
+    constexpr int smem = FwdLong::TOTAL + 1024;
+    if (const cudaError_t e = allow_smem<kern>(smem, true)) return static_cast<int>(e);
+    const cudaError_t e = launch_pdl(kern, dim3(static_cast<unsigned>(ctas)), dim3(kFwdThreads), static_cast<size_t>(smem), stream, tq, tk, tv,
+                                     static_cast<__nv_bfloat16*>(o), lse, p);
+    return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+  };
+  constexpr std::true_type yes;
+  constexpr std::false_type no;
+  return p.p_drop > 0.f ? (p.mask ? go(yes, yes) : go(yes, no)) : (p.mask ? go(no, yes) : go(no, no));
 }
 
 }  // namespace fb
