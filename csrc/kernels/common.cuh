@@ -171,6 +171,69 @@ __device__ __forceinline__ float dgelu_tanh_fast(float x) {
   return fmaf(0.5f * x * (1.0f - t * t), du, fmaf(0.5f, t, 0.5f));
 }
 
+// ---- two fp32 values per instruction ------------------------------------------------------------------
+// The .f32x2 forms take one issue slot for two values, each rounded as the scalar instruction rounds it.
+struct F2 {
+  uint64_t v;
+};
+__device__ __forceinline__ F2 f2_make(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f2_get(F2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v)); }
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_splat(float x) { return f2_make(x, x); }
+__device__ __forceinline__ F2 f2_tanh(F2 a) {
+  float lo, hi;
+  f2_get(a, lo, hi);
+  return f2_make(tanh_approx(lo), tanh_approx(hi));
+}
+// tanh argument of the erf form. The polynomial's own argument is held at 64 instead of clamping x: beyond |x| = 8 the result is 1.86 x,
+// where tanh has long saturated.
+__device__ __forceinline__ F2 f2_erf_tanh_arg(F2 x, F2 x2) {
+  float lo, hi;
+  f2_get(x2, lo, hi);
+  const F2 u2 = f2_make(fminf(lo, 64.f), fminf(hi, 64.f));
+  return f2_mul(x, f2_fma(u2, f2_fma(u2, f2_splat(-0.00031580707f), f2_splat(0.03679825612f)), f2_splat(0.7977178338f)));
+}
+__device__ __forceinline__ F2 f2_gelu_erf(F2 x) {
+  const F2 hx = f2_mul(x, f2_splat(0.5f));
+  return f2_fma(hx, f2_tanh(f2_erf_tanh_arg(x, f2_mul(x, x))), hx);
+}
+__device__ __forceinline__ F2 f2_gelu_tanh(F2 x) {
+  const F2 hx = f2_mul(x, f2_splat(0.5f));
+  return f2_fma(hx, f2_tanh(f2_mul(x, f2_fma(f2_mul(x, x), f2_splat(0.0356774081f), f2_splat(0.7978845608f)))), hx);
+}
+__device__ __forceinline__ F2 f2_dgelu_erf(F2 x) {
+  const F2 x2 = f2_mul(x, x), half = f2_splat(0.5f);
+  const F2 cdf = f2_fma(half, f2_tanh(f2_erf_tanh_arg(x, x2)), half);
+  float lo, hi;
+  f2_get(f2_mul(x2, f2_splat(-0.7213475204f)), lo, hi);
+  return f2_fma(x, f2_mul(f2_make(ex2_approx(lo), ex2_approx(hi)), f2_splat(0.3989422804f)), cdf);
+}
+__device__ __forceinline__ F2 f2_dgelu_tanh(F2 x) {
+  const F2 x2 = f2_mul(x, x), half = f2_splat(0.5f);
+  const F2 t = f2_tanh(f2_mul(x, f2_fma(x2, f2_splat(0.0356774081f), f2_splat(0.7978845608f))));
+  const F2 du = f2_fma(x2, f2_splat(0.1070322243f), f2_splat(0.7978845608f));
+  const F2 s = f2_fma(f2_mul(t, f2_splat(-1.f)), t, f2_splat(1.f));
+  return f2_fma(f2_mul(f2_mul(half, x), s), du, f2_fma(half, t, half));
+}
+
 
 // ---- bounds-checked debug build -------------------------------------------------------------------
 // With -DFLODL_BOUNDS_CHECK=1 (FLODL_B200_BOUNDS_CHECK=1 at build time) every index that a kernel

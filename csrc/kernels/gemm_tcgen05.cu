@@ -26,6 +26,7 @@
 #include <stdint.h>
 
 #include <cstring>
+#include <type_traits>
 #include <mutex>
 #include <unordered_map>
 
@@ -72,7 +73,8 @@ struct GemmParams {
   int accumulate;
   int split_k;
   int c_mode;      // 0 = per-thread global stores, 1 = staged TMA store, 2 = staged TMA reduce-add (fp32)
-  int aux_tma;     // the GELU pre-activation goes out through its own staged TMA store
+  int kind;        // EpiKind: what the epilogue does
+  int aux_tma;     // 1: the GELU pre-activation goes out through its own staged TMA store; 2: GELU' takes it in through TMA loads
   int* status;
   long long* ts;   // optional per-CTA timeline (8 slots each), for tuning
   // Optional device-side problem sizes (produced by an earlier kernel of the stream): the kernel
@@ -96,9 +98,10 @@ struct GemmCfg {
   static constexpr int EPI_SPLIT = (kBN == 192) ? 128 : kBN / 2;
   // epilogue staging: 4 KB (32 rows x 128 B, swizzled) per epilogue warp for C, the same again for aux
   static constexpr int EPI_BYTES = 2 * kEpiWarps * 4096;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align slack*/ + 512 /*barriers*/;
+  static constexpr int BAR_BYTES = 512, BIAS_BYTES = 2 * 256 * 4;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + BAR_BYTES + BIAS_BYTES;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
-  static_assert((2 * STAGES + 4) * 8 + 8 <= 512, "barrier block");
+  static_assert((2 * STAGES + 5 + 2 * kEpiWarps) * 8 + 8 <= BAR_BYTES, "barrier block");
   static_assert(TMEM_COLS <= 512, "accumulators do not fit TMEM");
 };
 
@@ -169,16 +172,6 @@ __device__ __forceinline__ void add_bias32(const GemmParams& p, int col0, int nv
   }
 }
 
-// The bias of the up to 128 columns an epilogue warp owns lives in registers, four consecutive
-// columns per lane (fetched while the tensor cores were still working on the tile, so the
-// global-memory latency is off the critical path). v[0..32) += bias of columns [cc, cc+32) of the
-// warp's range: the owner lane of column cc+i is (cc+i)/4.
-__device__ __forceinline__ void add_bias32_regs(const float (&breg)[4], int cc, float (&v)[32]) {
-  const int lane0 = cc >> 2;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] += __shfl_sync(0xffffffffu, breg[i & 3], lane0 + (i >> 2));
-}
-
 // Epilogue for 32 consecutive columns of one output row. Every loop over the 32 values is fully
 // unrolled with compile-time indices (tails are handled by predicates), so the values stay in
 // registers: a dynamically indexed copy would be demoted to local memory and every access to it
@@ -187,7 +180,7 @@ __device__ __forceinline__ void add_bias32_regs(const float (&breg)[4], int cc, 
 // pre-activation (only meaningful for the GELU epilogues). Rows/cols outside the problem yield
 // harmless values; the caller's store clips them.
 __device__ __forceinline__ void epilogue_compute32(const GemmParams& p, const uint32_t (&acc)[32], int row, int col0,
-                                                   bool add_bias, float (&v)[32], float (&pre)[32], const float (&breg)[4], int bias_cc) {
+                                                   bool add_bias, float (&v)[32], float (&pre)[32]) {
   if (p.alpha) {
     const float alpha = __ldg(p.alpha);
 #pragma unroll
@@ -197,10 +190,7 @@ __device__ __forceinline__ void epilogue_compute32(const GemmParams& p, const ui
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(acc[i]);
   }
   const int nvalid = (col0 + 32 <= p.N) ? 32 : (p.N > col0 ? p.N - col0 : 0);
-  if (p.bias && add_bias) {
-    if (bias_cc >= 0) add_bias32_regs(breg, bias_cc, v);
-    else add_bias32(p, col0, nvalid, v);
-  }
+  if (p.bias && add_bias) add_bias32(p, col0, nvalid, v);
   if (p.epi == FB_EPI_GELU_ERF) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) { pre[i] = v[i]; v[i] = gelu_erf_f(v[i]); }
@@ -246,6 +236,182 @@ __device__ __forceinline__ void tma_reduce_add_2d(const void* tmap, const void* 
   asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(tmap),
                "r"(smem_u32(smem_src)), "r"(x), "r"(y)
                : "memory");
+}
+
+__device__ __forceinline__ uint32_t f2_pack_bf16(F2 a) {
+  float lo, hi;
+  f2_get(a, lo, hi);
+  return pack_bf16x2(lo, hi);
+}
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+  uint4 q;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w) : "r"(addr) : "memory");
+  return q;
+}
+
+// What a staged epilogue does. One of these per launch: testing the kernel's parameters for every 64 columns took 350 cycles of them.
+enum EpiKind { kEpiDirect, kEpiPlain, kEpiGelu, kEpiGeluAux, kEpiDgelu, kEpiDgeluTanh, kEpiF32 };
+
+// An epilogue warp's 32 rows: the two staging tiles, which take turns, and the stores issued so far.
+struct EpiWarp {
+  uint8_t* stage[2];
+  uint64_t* aux_bar;       // pre-activations landed in stage[0], stage[1]
+  uint32_t staged;
+  int lane;
+};
+
+// This lane's row of a 32 x 64 bf16 staging tile.
+__device__ __forceinline__ void stage_row64(uint32_t tile, int lane, const F2 (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    st_shared_v4(stage_addr(tile, lane, j), f2_pack_bf16(v[4 * j]), f2_pack_bf16(v[4 * j + 1]), f2_pack_bf16(v[4 * j + 2]), f2_pack_bf16(v[4 * j + 3]));
+}
+// This lane's row of a staging tile that holds pre-activations: each 16-byte piece is replaced by v times the activation's derivative there.
+template <bool kTanh>
+__device__ __forceinline__ void dgelu_row64(uint32_t tile, int lane, const F2 (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t addr = stage_addr(tile, lane, j);
+    const uint4 q = ld_shared_v4(addr);
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float lo, hi;
+      unpack_bf16x2(w[i], lo, hi);
+      const F2 x = f2_make(lo, hi);
+      o[i] = f2_pack_bf16(f2_mul(v[4 * j + i], kTanh ? f2_dgelu_tanh(x) : f2_dgelu_erf(x)));
+    }
+    st_shared_v4(addr, o[0], o[1], o[2], o[3]);
+  }
+}
+
+// fp32 results: 32 columns (128 bytes of a row) per staged store or reduction.
+template <typename HandBack>
+__device__ __forceinline__ void epilogue_tile_f32(const GemmParams& p, const CUtensorMap& tmC, EpiWarp& w, uint32_t taddr, int col0, int row0, int cols, uint32_t bias,
+                                                  const HandBack& hand_back) {
+#pragma unroll 1
+  for (int c = 0; c < cols; c += 32) {
+    uint32_t acc[32];
+    tmem_ld32_sync(taddr + c, acc);
+    if (c + 32 >= cols) hand_back();
+    if (p.alpha) {
+      const float alpha = __ldg(p.alpha);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) * alpha);
+    }
+    if (bias) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint4 q = ld_shared_v4(bias + c * 4 + j * 16);
+        acc[4 * j] = __float_as_uint(__uint_as_float(acc[4 * j]) + __uint_as_float(q.x));
+        acc[4 * j + 1] = __float_as_uint(__uint_as_float(acc[4 * j + 1]) + __uint_as_float(q.y));
+        acc[4 * j + 2] = __float_as_uint(__uint_as_float(acc[4 * j + 2]) + __uint_as_float(q.z));
+        acc[4 * j + 3] = __float_as_uint(__uint_as_float(acc[4 * j + 3]) + __uint_as_float(q.w));
+      }
+    }
+    uint8_t* tile = w.stage[w.staged++ & 1];
+    if (w.lane == 0) tma_store_wait_read_but_one();
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) st_shared_v4(stage_addr(smem_u32(tile), w.lane, j), acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (w.lane == 0) {
+      if (p.c_mode == 2) tma_reduce_add_2d(&tmC, tile, col0 + c, row0);
+      else tma_store_2d(&tmC, tile, col0 + c, row0);
+      tma_store_commit();
+    }
+  }
+}
+
+// `chunks` times 64 columns from `col0` of rows [row0, row0 + 32), out of TMEM columns from `taddr` on. `bias`: shared memory, one fp32 per column
+// (0: none). `hand_back` runs when the accumulator has been read, `next_aux` (lane 0) issues the next load of pre-activations. False: a wait gave up.
+// Unrolled over 64 columns: rolled over 16 or 32, with the next ones on their way from TMEM, GELU at 4096 x 3072 x 768 took 25.5 us instead of 24.0.
+template <int kKind, typename HandBack, typename NextAux>
+__device__ __forceinline__ bool epilogue_tile(const GemmParams& p, const CUtensorMap& tmC, const CUtensorMap& tmAux, EpiWarp& w, uint32_t taddr, int col0, int row0,
+                                              int chunks, uint32_t bias, volatile int* abort_flag, const HandBack& hand_back, const NextAux& next_aux) {
+#pragma unroll 1
+  for (int ch = 0; ch < chunks; ++ch) {
+    const int col = col0 + ch * 64;
+    F2 v[32];
+    {
+      uint32_t a[32], b[32];
+      tmem_ld64_sync(taddr + ch * 64, a, b);
+      if (ch == chunks - 1) hand_back();
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        v[i] = f2_make(__uint_as_float(a[2 * i]), __uint_as_float(a[2 * i + 1]));
+        v[16 + i] = f2_make(__uint_as_float(b[2 * i]), __uint_as_float(b[2 * i + 1]));
+      }
+    }
+    if (p.alpha) {
+      const F2 alpha = f2_splat(__ldg(p.alpha));
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = f2_mul(v[i], alpha);
+    }
+    if (bias) {          // every lane reads the same 16 bytes: a load serves four columns of 32 rows
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const uint4 q = ld_shared_v4(bias + ch * 256 + j * 16);
+        v[2 * j] = f2_add(v[2 * j], f2_make(__uint_as_float(q.x), __uint_as_float(q.y)));
+        v[2 * j + 1] = f2_add(v[2 * j + 1], f2_make(__uint_as_float(q.z), __uint_as_float(q.w)));
+      }
+    }
+    if constexpr (kKind == kEpiDgelu || kKind == kEpiDgeluTanh) {
+      const uint32_t b = w.staged & 1;
+      const bool ok = mbar_wait(&w.aux_bar[b], (w.staged >> 1) & 1, abort_flag, p.status, kStatusWaitFull);
+      if (!__all_sync(0xffffffffu, ok)) return false;
+      dgelu_row64<kKind == kEpiDgeluTanh>(smem_u32(w.stage[b]), w.lane, v);
+      ++w.staged;
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (w.lane == 0) {
+        tma_store_2d(&tmC, w.stage[b], col, row0);
+        tma_store_commit();
+        if (ch == chunks - 1) {         // the next tile's loads, each once its staging tile has been read
+          if (chunks == 2) {
+            tma_store_wait_read_but_one();
+            next_aux();
+          }
+          tma_store_wait_read();
+          next_aux();
+        }
+      }
+    } else {
+      const auto take_turn = [&]() -> uint8_t* {      // the staging tile whose store two turns ago has been read
+        if (w.lane == 0) tma_store_wait_read_but_one();
+        __syncwarp();
+        return w.stage[w.staged++ & 1];
+      };
+      const auto send = [&](const CUtensorMap* map, const uint8_t* tile, int x) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (w.lane == 0) {
+          tma_store_2d(map, tile, x, row0);
+          tma_store_commit();
+        }
+      };
+      if constexpr (kKind == kEpiGeluAux) {
+        uint8_t* tile = take_turn();
+        stage_row64(smem_u32(tile), w.lane, v);
+        send(&tmAux, tile, col);
+      }
+      if constexpr (kKind == kEpiGelu || kKind == kEpiGeluAux) {
+        if (p.epi == FB_EPI_GELU_ERF) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = f2_gelu_erf(v[i]);
+        } else if (p.epi == FB_EPI_GELU_TANH) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = f2_gelu_tanh(v[i]);
+        }
+      }
+      uint8_t* tile = take_turn();
+      stage_row64(smem_u32(tile), w.lane, v);
+      send(&tmC, tile, col);
+    }
+  }
+  return true;
 }
 
 __device__ __forceinline__ void epilogue_store32(const GemmParams& p, const uint32_t (&acc)[32],
@@ -372,22 +538,36 @@ __device__ __forceinline__ void epilogue_store32(const GemmParams& p, const uint
   }
 }
 
+// Tile t of the list: row tiles fastest.
+__device__ __forceinline__ void tile_of(int t, int num_m, int& tm, int& tn) {
+  tn = t / num_m;
+  tm = t - tn * num_m;
+}
+
 template <int kCG, int kBN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAux, const GemmParams p) {
   using Cfg = GemmCfg<kCG, kBN>;
-  extern __shared__ uint8_t smem_raw[];
-  // 1024-byte alignment: the 128-byte swizzle pattern is a function of address bits [4,10).
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  // 1024-byte alignment: the 128-byte swizzle pattern is a function of address bits [4,10). Dynamic shared memory starts so where a kernel has no
+  // other; there is no room to round up.
+  uint8_t* smem = smem_raw;
+  if (smem_u32(smem) & 1023) {
+    set_status(p.status, kStatusBadArg);
+    return;
+  }
   uint8_t* stage_base = smem;
   uint8_t* epi_smem = smem + Cfg::STAGES * Cfg::STAGE_BYTES;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_smem + Cfg::EPI_BYTES);
   uint64_t* empty_bar = full_bar + Cfg::STAGES;
   uint64_t* tfull_bar = empty_bar + Cfg::STAGES;
   uint64_t* tempty_bar = tfull_bar + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
+  uint64_t* aux_bar = tempty_bar + 2;          // two per epilogue warp
+  uint64_t* peer_bar = aux_bar + 2 * kEpiWarps;      // the pair's other CTA holds its TMEM
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(peer_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* bias_smem = reinterpret_cast<float*>(epi_smem + Cfg::EPI_BYTES + Cfg::BAR_BYTES);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -403,33 +583,51 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     p.ts[blockIdx.x * 8 + 1] = clock64();
   }
 #endif
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < Cfg::STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+  // The loads wait for the barriers alone (of both CTAs), not for the TMEM allocation, which the other warps hear of through barrier 1.
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int s = 0; s < Cfg::STAGES; ++s) {
+        mbar_init(&full_bar[s], 1);
+        mbar_init(&empty_bar[s], 1);
+      }
+      for (int a = 0; a < 2; ++a) {
+        mbar_init(&tfull_bar[a], 1);
+        mbar_init(&tempty_bar[a], kEpiWarps * kCG);
+      }
+      if (p.aux_tma == 2)
+        for (int w = 0; w < 2 * kEpiWarps; ++w) mbar_init(&aux_bar[w], 1);
+      if (kCG == 2) mbar_init(peer_bar, 1);
+      *abort_flag = 0;
+      mbar_fence_init();
     }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], kEpiWarps * kCG);
+    __syncwarp();
+  }
+  if constexpr (kCG == 2) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (warp == 0) {
+    asm volatile("bar.arrive 1, %0;" ::"n"(kGemmThreads) : "memory");
+    if (lane == 0) {
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmB);
     }
-    *abort_flag = 0;
-    mbar_fence_init();
+    __syncwarp();
+  } else {
+    if (warp == 2 && lane == 0) {
+      if (p.c_mode) tma_prefetch_desc(&tmC);
+      if (p.aux_tma) tma_prefetch_desc(&tmAux);
+    }
+    if (warp == 1) {
+      tmem_alloc<kCG>(tmem_slot, Cfg::TMEM_COLS);
+      tmem_relinquish<kCG>();
+    }
+    tc_fence_before_sync();
+    asm volatile("bar.sync 1, %0;" ::"n"(kGemmThreads) : "memory");
+    tc_fence_after_sync();
   }
-  if (warp == 0 && lane == 0) {
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
-    if (p.c_mode) tma_prefetch_desc(&tmC);
-    if (p.aux_tma) tma_prefetch_desc(&tmAux);
-  }
-  if (warp == 1) {
-    tmem_alloc<kCG>(tmem_slot, Cfg::TMEM_COLS);
-    tmem_relinquish<kCG>();
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  if constexpr (kCG == 2) cluster_sync_all();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  if constexpr (kCG == 2) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if constexpr (kCG == 1) __syncthreads();        // one CTA: nothing to gain by starting its loads earlier
+  const uint32_t tmem_base = warp == 0 ? 0 : *tmem_slot;
+  if constexpr (kCG == 2)
+    if (warp == 1 && lane == 0 && rank == 1) mbar_arrive_cluster(peer_bar, 0);
   // Programmatic dependent launch: everything above (barriers, descriptor prefetch, TMEM) touched
   // no global data and may run while the previous kernel of the stream drains; from here on this
   // kernel reads what that kernel wrote.
@@ -454,9 +652,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       bool ok = true;
       for (int u = group; u < num_units && ok; u += num_groups) {
         const int ks = u % p.split_k;
-        const int t = u / p.split_k;
-        const int m0 = (t % num_m) * BM * kCG + static_cast<int>(rank) * BM;
-        const int n0 = (t / num_m) * kBN + static_cast<int>(rank) * Cfg::BN_CTA;
+        int tm, tn;
+        tile_of(u / p.split_k, num_m, tm, tn);
+        const int m0 = tm * BM * kCG + static_cast<int>(rank) * BM;
+        const int n0 = tn * kBN + static_cast<int>(rank) * Cfg::BN_CTA;
         const int kb0 = ks * kb_per;
         const int kb1 = min(num_kb, kb0 + kb_per);
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -510,6 +709,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t ph = 0;
       int it = 0;
       bool ok = true;
+      if constexpr (kCG == 2) ok = mbar_wait(peer_bar, 0, abort_flag, p.status, kStatusWaitEpi);
       for (int u = group; u < num_units && ok; u += num_groups, ++it) {
         const int ks = u % p.split_k;
         const int kb0 = ks * kb_per;
@@ -544,136 +744,118 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else {
     // ------------------------------------------------------------------ epilogue warps
+    // What bounds a tile of a short reduction (K = 768: 6.1k cycles of products) is this part, so it is kept below that: 64 columns come out
+    // of TMEM per wait, two values share an instruction, the accumulator is handed back before the last columns are worked on, the bias waits in
+    // shared memory, and GELU' finds the pre-activations in the staging tile, where a TMA load of the previous tile's time has put them, and
+    // leaves its result in their place. Cycles per tile of a launch's first tiles, before and now: plain 3.7k and 2.0k, bias 4.7k and 2.6k, GELU
+    // with its pre-activation 9.2k and 7.2k, GELU' 21k (its loads of 64 bytes per row were not coalesced) and 9k. At 4096 x 3072 x 768: 21.6 -> 20.0,
+    // 29.0 -> 24.3 and 44.8 -> 26.8 us. Sixteen epilogue warps instead of eight shorten a tile further but start 0.3 us later: 20.0 us again.
     const int q = warp & 3;                 // TMEM lane quarter this warp may touch
     const int half = (warp - 2) >> 2;       // which half of the tile's columns
     constexpr int kSplit = Cfg::EPI_SPLIT;
-    int it = 0;
-    uint32_t chunk_ix = 0;     // staged stores issued by this warp so far: picks the staging tile in turn
-    bool ok = true;
-    for (int u = group; u < num_units && ok; u += num_groups, ++it) {
-      const int ks = u % p.split_k;
-      const int t = u / p.split_k;
-      const int m0 = (t % num_m) * BM * kCG + static_cast<int>(rank) * BM;
-      const int n0 = (t / num_m) * kBN;
-      const int acc = it & 1;
-      // This warp's slice of the bias is fetched now, while the tensor cores are still working on the
-      // tile: by the time the accumulator is ready the global-memory latency has been paid.
-      const bool stage_bias = p.bias != nullptr && ks == 0 && p.c_mode != 0;
-      float breg[4] = {0.f, 0.f, 0.f, 0.f};
-      if (stage_bias) {
-        const int wcols = half ? kBN - Cfg::EPI_SPLIT : Cfg::EPI_SPLIT;
-        const int cbase = n0 + half * Cfg::EPI_SPLIT + lane * 4;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int col = cbase + j;
-          if (lane * 4 + j < wcols && col < p.N)
-            breg[j] = p.bias_fp32 ? __ldg(static_cast<const float*>(p.bias) + col) : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col]);
-        }
+    const int cols = half ? kBN - kSplit : kSplit;
+    constexpr bool kStaged = kBN >= 128;    // a warp of a 64-wide tile has less than a staged store's 64 columns
+    EpiWarp w;
+    w.stage[0] = epi_smem + (warp - 2) * 4096;
+    w.stage[1] = epi_smem + (kEpiWarps + warp - 2) * 4096;
+    w.aux_bar = aux_bar + 2 * (warp - 2);
+    w.staged = 0;
+    w.lane = lane;
+    int aux_u = group, aux_c = 0;           // where the next load of pre-activations starts (lane 0)
+    uint32_t aux_issued = 0;
+    const auto load_aux = [&] {             // the next 64 columns of this warp's rows, into the staging tile whose turn it is
+      for (; aux_u < num_units; aux_u += num_groups, aux_c = 0) {
+        int tm, tn;
+        tile_of(aux_u, num_m, tm, tn);
+        const int col = tn * kBN + half * kSplit + aux_c;
+        if (aux_c >= cols || col >= p.N) continue;
+        const uint32_t b = aux_issued++ & 1;
+        mbar_expect_tx(&w.aux_bar[b], 4096);
+        tma_load_2d(w.stage[b], &tmAux, &w.aux_bar[b], col, tm * BM * kCG + static_cast<int>(rank) * BM + q * 32);
+        aux_c += 64;
+        return;
       }
-      ok = mbar_wait(&tfull_bar[acc], (it >> 1) & 1, abort_flag, p.status, kStatusWaitAccum);
-      if (!ok) break;
+    };
+    if (kStaged && p.aux_tma == 2 && lane == 0) {
+      load_aux();
+      load_aux();
+    }
+    // Thread i of the four warps of a half keeps column i's bias of the tile to come.
+    const bool staged_bias = kStaged && p.bias != nullptr && p.kind != kEpiDirect;
+    const auto bias_of = [&](int u) -> float {
+      int tm, tn;
+      tile_of(u / p.split_k, num_m, tm, tn);
+      const int c = q * 32 + lane, col = tn * kBN + half * kSplit + c;
+      if (u >= num_units || c >= cols || col >= p.N) return 0.f;
+      return p.bias_fp32 ? __ldg(static_cast<const float*>(p.bias) + col) : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col]);
+    };
+    float next_bias = staged_bias ? bias_of(group) : 0.f;
+    int it = 0;
+    bool ok = true;
+    for (int u = group; u < num_units; u += num_groups, ++it) {
+      const int ks = u % p.split_k;
+      int tm, tn;
+      tile_of(u / p.split_k, num_m, tm, tn);
+      const int row0 = tm * BM * kCG + static_cast<int>(rank) * BM + q * 32;
+      const int ncol0 = tn * kBN + half * kSplit;
+      const int acc = it & 1;
+      uint32_t bias = 0;
+      if (staged_bias) {
+        // Two slices in turn: this one was last read a tile before the previous barrier. A warp whose wait gave up still comes here for every
+        // tile, so the barrier never lacks one.
+        float* slice = bias_smem + acc * 256 + half * 128;
+        slice[q * 32 + lane] = next_bias;
+        if (half) asm volatile("bar.sync 3, 128;" ::: "memory");
+        else asm volatile("bar.sync 2, 128;" ::: "memory");
+        next_bias = bias_of(u + num_groups);
+        if (ks == 0) bias = smem_u32(slice);
+      }
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&tfull_bar[acc], (it >> 1) & 1, abort_flag, p.status, kStatusWaitAccum));
+      if (!ok) continue;
       tc_fence_after_sync();
       FB_TIMELINE_ONLY(if (p.ts && it == 0 && warp == 2 && lane == 0) p.ts[blockIdx.x * 8 + 4] = clock64();)
-      const int row = m0 + q * 32 + lane;
-      const int row0 = m0 + q * 32;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * kBN + half * kSplit;
-      const int ncol0 = n0 + half * kSplit;
-      const int COLS_PER_WARP = half ? kBN - kSplit : kSplit;
-      if (p.c_mode == 0) {
-#pragma unroll 1
-        for (int c = 0; c < COLS_PER_WARP; c += 32) {
-          uint32_t v[32];
-          tmem_ld32(taddr + c, v);
-          tmem_ld_wait();
-          epilogue_store32(p, v, row, ncol0 + c, ks == 0);
+      const auto hand_back = [&] {          // this warp has read all it needs of the accumulator
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          if (kCG == 1 || rank == 0) mbar_arrive(&tempty_bar[acc]);
+          else mbar_arrive_cluster_tmem(&tempty_bar[acc], 0);
         }
-      } else {
-        const uint32_t sc = smem_u32(epi_smem + (warp - 2) * 4096);
-        const uint32_t sx = smem_u32(epi_smem + (kEpiWarps + warp - 2) * 4096);
-        if (!p.c_fp32) {
-          // bf16 output: 64 columns (128 bytes per row) per staged store
-          // Without an aux store the second staging tile is free: the two take turns, so a chunk only
-          // waits for the store issued two chunks ago.
-          const bool pingpong = !p.aux_tma;
-#pragma unroll 1
-          for (int c = 0; c < COLS_PER_WARP; c += 64) {
-            if (ncol0 + c >= p.N) break;
-            const bool odd = pingpong && (chunk_ix & 1);
-            ++chunk_ix;
-            const uint32_t sc_cur = odd ? sx : sc;
-            uint8_t* sc_ptr = epi_smem + ((odd ? kEpiWarps : 0) + warp - 2) * 4096;
-            if (lane == 0) {
-              if (pingpong) tma_store_wait_read_but_one();
-              else tma_store_wait_read();           // the previous chunk's store has read the staging tile
-            }
-            __syncwarp();
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {          // two 32-column halves, one at a time (register pressure)
-              uint32_t r0[32];
-              tmem_ld32(taddr + c + 32 * hh, r0);
-              tmem_ld_wait();
-              float v0[32], p0[32];
-              epilogue_compute32(p, r0, row, ncol0 + c + 32 * hh, ks == 0, v0, p0, breg, stage_bias ? c + 32 * hh : -1);
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                st_shared_v4(stage_addr(sc_cur, lane, 4 * hh + j), pack_bf16x2(v0[8 * j], v0[8 * j + 1]), pack_bf16x2(v0[8 * j + 2], v0[8 * j + 3]),
-                             pack_bf16x2(v0[8 * j + 4], v0[8 * j + 5]), pack_bf16x2(v0[8 * j + 6], v0[8 * j + 7]));
-              if (p.aux_tma) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                  st_shared_v4(stage_addr(sx, lane, 4 * hh + j), pack_bf16x2(p0[8 * j], p0[8 * j + 1]), pack_bf16x2(p0[8 * j + 2], p0[8 * j + 3]),
-                               pack_bf16x2(p0[8 * j + 4], p0[8 * j + 5]), pack_bf16x2(p0[8 * j + 6], p0[8 * j + 7]));
-              }
-            }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&tmC, sc_ptr, ncol0 + c, row0);
-              if (p.aux_tma) tma_store_2d(&tmAux, epi_smem + (kEpiWarps + warp - 2) * 4096, ncol0 + c, row0);
-              tma_store_commit();
-            }
-          }
-        } else {
-          // fp32 output: 32 columns (128 bytes per row) per staged store or reduce-add
-#pragma unroll 1
-          for (int c = 0; c < COLS_PER_WARP; c += 32) {
-            if (ncol0 + c >= p.N) break;
-            uint32_t r0[32];
-            tmem_ld32(taddr + c, r0);
-            tmem_ld_wait();
-            float v0[32], p0[32];
-            epilogue_compute32(p, r0, row, ncol0 + c, ks == 0, v0, p0, breg, stage_bias ? c : -1);
-            const bool odd = chunk_ix & 1;           // the two staging tiles take turns
-            ++chunk_ix;
-            const uint32_t sc_cur = odd ? sx : sc;
-            uint8_t* sc_ptr = epi_smem + ((odd ? kEpiWarps : 0) + warp - 2) * 4096;
-            if (lane == 0) tma_store_wait_read_but_one();
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              st_shared_v4(stage_addr(sc_cur, lane, j), __float_as_uint(v0[4 * j]), __float_as_uint(v0[4 * j + 1]),
-                           __float_as_uint(v0[4 * j + 2]), __float_as_uint(v0[4 * j + 3]));
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              if (p.c_mode == 2) tma_reduce_add_2d(&tmC, sc_ptr, ncol0 + c, row0);
-              else tma_store_2d(&tmC, sc_ptr, ncol0 + c, row0);
-              tma_store_commit();
-            }
-          }
+      };
+      if constexpr (kStaged) {
+        const int chunks = ncol0 >= p.N ? 0 : (min(cols, p.N - ncol0) + 63) / 64;
+        const auto run = [&](auto kind) {
+          ok = epilogue_tile<decltype(kind)::value>(p, tmC, tmAux, w, taddr, ncol0, row0, chunks, bias, abort_flag, hand_back, load_aux);
+        };
+        if (p.kind != kEpiDirect) {
+          if (chunks == 0) hand_back();
+          else if (p.kind == kEpiPlain) run(std::integral_constant<int, kEpiPlain>());
+          else if (p.kind == kEpiF32) epilogue_tile_f32(p, tmC, w, taddr, ncol0, row0, min(cols, p.N - ncol0), bias, hand_back);
+          else if (p.kind == kEpiGelu) run(std::integral_constant<int, kEpiGelu>());
+          else if (p.kind == kEpiGeluAux) run(std::integral_constant<int, kEpiGeluAux>());
+          else if (p.kind == kEpiDgelu) run(std::integral_constant<int, kEpiDgelu>());
+          else run(std::integral_constant<int, kEpiDgeluTanh>());
+          continue;
         }
       }
-      tc_fence_before_sync();
-      __syncwarp();
+#pragma unroll 1
+      for (int c = 0; c < cols; c += 32) {
+        uint32_t v[32];
+        tmem_ld32(taddr + c, v);
+        tmem_ld_wait();
+        epilogue_store32(p, v, row0 + lane, ncol0 + c, ks == 0);
+      }
+      hand_back();
       FB_TIMELINE_ONLY(if (p.ts && it == 0 && warp == 2 && lane == 0) p.ts[blockIdx.x * 8 + 5] = clock64();)
-      if (lane == 0) {
-        if (kCG == 1 || rank == 0) mbar_arrive(&tempty_bar[acc]);
-        else mbar_arrive_cluster(&tempty_bar[acc], 0);
-      }
     }
-    // The staging tiles must have been read before the CTA (and its shared memory) goes away; the
+    // The staging tiles must have been read, and loads into them must have landed, before the CTA (and its shared memory) goes away; the
     // writes themselves complete with the grid, as every other global store does.
-    if (p.c_mode && lane == 0) tma_store_wait_read();
+    if (kStaged && p.kind != kEpiDirect && lane == 0) {
+      tma_store_wait_read();
+      for (uint32_t n = w.staged; n < aux_issued; ++n)      // none, unless a wait gave up
+        for (uint32_t polls = 0; polls < (1u << 20) && !mbar_test(&w.aux_bar[n & 1], (n >> 1) & 1); ++polls) __nanosleep(40);
+    }
   }
 
   // ------------------------------------------------------------------ teardown
@@ -727,7 +909,7 @@ __device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
                   const __grid_constant__ CUtensorMap tmAux, const __grid_constant__ GemmParams p) {
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   using Cfg = SplitCfg;
   uint8_t* xchg = smem + Cfg::STAGES * Cfg::STAGE_BYTES;
@@ -753,7 +935,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
     tma_prefetch_desc(&tmC);
-    if (p.aux_tma) tma_prefetch_desc(&tmAux);
+    if (p.aux_tma == 1) tma_prefetch_desc(&tmAux);
   }
   if (warp == 1) {
     tmem_alloc<2>(tmem_slot, 256);
@@ -835,7 +1017,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       uint8_t* stage = smem + (warp - 2) * 4096;           // every product that reads the operands has retired
       uint8_t* stage_x = smem + (kEpiWarps + warp - 2) * 4096;
       const uint32_t sc = smem_u32(stage), sx = smem_u32(stage_x), mine = smem_u32(xchg);
-      const float none[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         const int c = half * 64 + 32 * hh;
@@ -851,12 +1032,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           acc[4 * j + 3] = __float_as_uint(__uint_as_float(acc[4 * j + 3]) + t.w);
         }
         float v0[32], p0[32];
-        epilogue_compute32(p, acc, row0 + lane, col0 + 32 * hh, true, v0, p0, none, -1);
+        epilogue_compute32(p, acc, row0 + lane, col0 + 32 * hh, true, v0, p0);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           st_shared_v4(stage_addr(sc, lane, 4 * hh + j), pack_bf16x2(v0[8 * j], v0[8 * j + 1]), pack_bf16x2(v0[8 * j + 2], v0[8 * j + 3]),
                        pack_bf16x2(v0[8 * j + 4], v0[8 * j + 5]), pack_bf16x2(v0[8 * j + 6], v0[8 * j + 7]));
-        if (p.aux_tma) {
+        if (p.aux_tma == 1) {
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             st_shared_v4(stage_addr(sx, lane, 4 * hh + j), pack_bf16x2(p0[8 * j], p0[8 * j + 1]), pack_bf16x2(p0[8 * j + 2], p0[8 * j + 3]),
@@ -867,7 +1048,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       __syncwarp();
       if (lane == 0) {
         tma_store_2d(&tmC, stage, col0, row0);
-        if (p.aux_tma) tma_store_2d(&tmAux, stage_x, col0, row0);
+        if (p.aux_tma == 1) tma_store_2d(&tmAux, stage_x, col0, row0);
         tma_store_commit();
         tma_store_wait_read();       // before the shared memory goes away
       }
@@ -1133,11 +1314,16 @@ extern "C" int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, in
     if (c_fp32) c_mode = (accumulate || split_k > 1) ? 2 : 1;
     else if (!accumulate) c_mode = 1;
   }
-  if (bn < 128) c_mode = 0;   // 32 columns per epilogue warp: narrower than one staged bf16 box
   const bool gelu_fwd = (epi == FB_EPI_GELU_ERF || epi == FB_EPI_GELU_TANH);
+  if (c_fp32 && gelu_fwd) c_mode = 0;
+  if (bn < 128) c_mode = 0;   // 32 columns per epilogue warp: narrower than one staged bf16 box
   int aux_tma = 0;
   if (gelu_fwd && aux) {
     if (c_mode == 1 && !c_fp32 && (reinterpret_cast<uintptr_t>(aux) & 15) == 0 && (ldaux * 2) % 16 == 0) aux_tma = 1;
+    else c_mode = 0;
+  }
+  if (epi == FB_EPI_DGELU_ERF || epi == FB_EPI_DGELU_TANH) {
+    if (c_mode == 1 && !c_fp32 && (reinterpret_cast<uintptr_t>(aux) & 15) == 0 && (ldaux * 2) % 16 == 0) aux_tma = 2;
     else c_mode = 0;
   }
   CUtensorMap tc, tx;
@@ -1148,6 +1334,7 @@ extern "C" int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, in
 
   GemmParams p;
   p.c_mode = c_mode; p.aux_tma = aux_tma;
+  p.kind = c_mode == 0 ? kEpiDirect : c_fp32 ? kEpiF32 : aux_tma == 2 ? (epi == FB_EPI_DGELU_ERF ? kEpiDgelu : kEpiDgeluTanh) : aux_tma == 1 ? kEpiGeluAux : gelu_fwd ? kEpiGelu : kEpiPlain;
   p.M = M; p.N = N; p.K = K; p.a_mn = a_mn; p.b_mn = b_mn; p.C = C; p.ldc = ldc; p.c_fp32 = c_fp32;
   p.bias = bias; p.bias_fp32 = bias_fp32; p.epi = epi; p.aux = aux; p.ldaux = ldaux; p.alpha = alpha;
   p.accumulate = accumulate; p.split_k = split_k; p.status = status; p.ts = ts;

@@ -71,6 +71,13 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t cta)
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote)
                : "memory");
 }
+// As above where the arrival publishes no memory, only the end of this warp's TMEM reads (fenced by tcgen05.fence::before_thread_sync): at
+// cluster scope the release would wait for every store of the thread still on its way.
+__device__ __forceinline__ void mbar_arrive_cluster_tmem(uint64_t* bar, uint32_t cta) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(bar)), "r"(cta));
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
+}
 // One non-blocking probe of the barrier's phase.
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -109,7 +116,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   set_status(status, code);
   return false;
 }
-
 // ---------------------------------------------------------------------------------------------
 // TMA
 // ---------------------------------------------------------------------------------------------
@@ -301,6 +307,22 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
         "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
       : "r"(taddr)
       : "memory");
+}
+
+// 64 consecutive columns, read together and waited for: the values are not touched before they have arrived.
+__device__ __forceinline__ void tmem_ld64_sync(uint32_t taddr, uint32_t (&a)[32], uint32_t (&b)[32]) {
+  tmem_ld32(taddr, a);
+  tmem_ld32(taddr + 32, b);
+  tmem_ld_wait();
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(a[i]), "+r"(b[i]));
+}
+
+__device__ __forceinline__ void tmem_ld32_sync(uint32_t taddr, uint32_t (&v)[32]) {
+  tmem_ld32(taddr, v);
+  tmem_ld_wait();
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(v[i]));
 }
 
 // The way back: thread t of the warp writes row (lane base + t), 16 or 32 consecutive columns.

@@ -82,6 +82,47 @@ def test_gemm_bias_gelu_aux(C, config):
     assert (dpre.float() - x.grad).abs().max().item() < 0.06
 
 
+@pytest.mark.parametrize("config", [0, 1, 2, 3, 4, 5])
+@pytest.mark.parametrize("M,N,K,pad,bias", [(300, 328, 64, 0, "fp32"), (513, 1160, 72, 8, "bf16"), (2500, 2824, 128, 0, "offset"), (129, 72, 200, 4, "none")])
+def test_gemm_staged_epilogues(C, config, M, N, K, pad, bias):
+    """Scale, bias, GELU with its pre-activation and GELU' where tiles are ragged, a CTA has several of them, rows of `aux` are not 16-byte aligned, the bias
+    is of either type and starts anywhere. Bounds: one rounding to bf16 (2^-8 of the value) plus 3e-4 of the factor's scale for the hardware's tanh."""
+    torch.manual_seed(M + config)
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    b = (torch.randn(N, K, device="cuda") / math.sqrt(K)).bfloat16()
+    v = {"fp32": torch.randn(N, device="cuda"), "bf16": torch.randn(N, device="cuda").bfloat16(), "offset": torch.randn(N + 1, device="cuda")[1:], "none": None}[bias]
+    lin = a.double() @ b.double().t()
+    pre = lin + (0 if v is None else v.double())
+
+    def close(got, want, scale=1.0, tail=3e-4):
+        assert C.read_status(0) == 0
+        assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + tail * scale + 1e-4).all()
+    C.clear_status(0)
+    out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    C.gemm(a, b, out, bias=v, config=config)
+    close(out, pre)
+    alpha = torch.tensor([-0.5], device="cuda")
+    out32 = torch.ones(M, N, device="cuda")
+    C.gemm(a, b, out32, bias=v, config=config, alpha=alpha, accumulate=True)
+    close(out32, 1 - 0.5 * lin + (0 if v is None else v.double()))
+    for tanh in (False, True):
+        aux = torch.full((M, N + pad), 9.0, device="cuda", dtype=torch.bfloat16)
+        C.gemm(a, b, out, bias=v, epi=3 if tanh else 1, aux=aux[:, :N], config=config)
+        close(aux[:, :N], pre)
+        assert (aux[:, N:] == 9).all()
+        close(out, F.gelu(pre, approximate="tanh" if tanh else "none"), pre.abs() + 1)
+        C.gemm(a, b, out, bias=v, epi=3 if tanh else 1, config=config)
+        close(out, F.gelu(pre, approximate="tanh" if tanh else "none"), pre.abs() + 1)
+        aux[0, 0], aux[M - 1, N - 1], aux[M - 1, 0] = float("nan"), 40.0, -40.0
+        x = aux[:, :N].double().requires_grad_()
+        F.gelu(x, approximate="tanh" if tanh else "none").sum().backward()
+        dpre = torch.empty_like(out)
+        C.gemm(a, b, dpre, epi=4 if tanh else 2, aux=aux[:, :N], config=config)
+        assert dpre[0, 0].isnan()
+        dpre[0, 0] = x.grad[0, 0] = 0
+        close(dpre, lin * x.grad, lin.abs() + 1)
+
+
 def test_gemm_fp32_out_accumulate_splitk_alpha(C):
     M, N, K = 256, 384, 1024
     torch.manual_seed(1)
