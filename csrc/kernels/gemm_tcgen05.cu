@@ -569,7 +569,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* bias_smem = reinterpret_cast<float*>(epi_smem + Cfg::EPI_BYTES + Cfg::BAR_BYTES);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // the same in a whole warp, for the compiler too
   const int lane = threadIdx.x & 31;
   const uint32_t rank = (kCG == 2) ? cluster_ctarank() : 0u;
   const int group = blockIdx.x / kCG;          // CTA (pair) index
@@ -646,7 +646,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    // The whole warp walks the loop and one lane issues: addresses, coordinates and descriptors then stay in uniform registers, where the
+    // instructions want them.
+    {
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -659,47 +661,37 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int kb0 = ks * kb_per;
         const int kb1 = min(num_kb, kb0 + kb_per);
         for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty);
+          ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty));
           if (!ok) break;
           uint8_t* sa = stage_base + s * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + Cfg::A_BYTES;
-          if (kCG == 1 || rank == 0) mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES * kCG);
-          if constexpr (kCG == 1) {
+          if (elect_one()) {
+            if (kCG == 1 || rank == 0) mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES * kCG);
+            const auto load = [&](uint8_t* to, const CUtensorMap* map, int x, int y) {
+              if constexpr (kCG == 1) tma_load_2d(to, map, &full_bar[s], x, y);
+              else tma_load_2d_pair(to, map, &full_bar[s], x, y);
+            };
             if (!p.a_mn) {
-              tma_load_2d(sa, &tmA, &full_bar[s], kb * BK, m0);
+              load(sa, &tmA, kb * BK, m0);
             } else {
-              tma_load_2d(sa, &tmA, &full_bar[s], m0, kb * BK);
-              tma_load_2d(sa + 8192, &tmA, &full_bar[s], m0 + 64, kb * BK);
+              load(sa, &tmA, m0, kb * BK);
+              load(sa + 8192, &tmA, m0 + 64, kb * BK);
             }
             if (!p.b_mn) {
-              tma_load_2d(sb, &tmB, &full_bar[s], kb * BK, n0);
+              load(sb, &tmB, kb * BK, n0);
             } else {
 #pragma unroll
-              for (int q = 0; q < Cfg::BN_CTA / 64; ++q)
-                tma_load_2d(sb + q * 8192, &tmB, &full_bar[s], n0 + q * 64, kb * BK);
-            }
-          } else {
-            if (!p.a_mn) {
-              tma_load_2d_pair(sa, &tmA, &full_bar[s], kb * BK, m0);
-            } else {
-              tma_load_2d_pair(sa, &tmA, &full_bar[s], m0, kb * BK);
-              tma_load_2d_pair(sa + 8192, &tmA, &full_bar[s], m0 + 64, kb * BK);
-            }
-            if (!p.b_mn) {
-              tma_load_2d_pair(sb, &tmB, &full_bar[s], kb * BK, n0);
-            } else {
-#pragma unroll
-              for (int q = 0; q < Cfg::BN_CTA / 64; ++q)
-                tma_load_2d_pair(sb + q * 8192, &tmB, &full_bar[s], n0 + q * 64, kb * BK);
+              for (int q = 0; q < Cfg::BN_CTA / 64; ++q) load(sb + q * 8192, &tmB, n0 + q * 64, kb * BK);
             }
           }
+          __syncwarp();
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (rank == 0 && lane == 0) {
+    if (rank == 0) {
       const uint32_t idesc = make_idesc_bf16(BM * kCG, kBN, p.a_mn, p.b_mn);
       const uint32_t a_lbo = p.a_mn ? 8192u : 16u;
       const uint32_t b_lbo = p.b_mn ? 8192u : 16u;
@@ -709,36 +701,42 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t ph = 0;
       int it = 0;
       bool ok = true;
-      if constexpr (kCG == 2) ok = mbar_wait(peer_bar, 0, abort_flag, p.status, kStatusWaitEpi);
+      if constexpr (kCG == 2) ok = __all_sync(0xffffffffu, mbar_wait(peer_bar, 0, abort_flag, p.status, kStatusWaitEpi));
       for (int u = group; u < num_units && ok; u += num_groups, ++it) {
         const int ks = u % p.split_k;
         const int kb0 = ks * kb_per;
         const int kb1 = min(num_kb, kb0 + kb_per);
         const int acc = it & 1;
-        ok = mbar_wait(&tempty_bar[acc], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi);
+        ok = __all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi));
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * kBN;
         for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
+          ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull));
           if (!ok) break;
           tc_fence_after_sync();
           FB_TIMELINE_ONLY(if (p.ts && it == 0 && kb == kb0) p.ts[blockIdx.x * 8 + 2] = clock64();)
           const uint32_t sa = smem_u32(stage_base + s * Cfg::STAGE_BYTES);
           const uint32_t sb = sa + Cfg::A_BYTES;
+          if (elect_one()) {
 #pragma unroll
-          for (int k4 = 0; k4 < BK / 16; ++k4) {
-            const uint64_t da = make_smem_desc(sa + k4 * a_kstep, a_lbo, 1024);
-            const uint64_t db = make_smem_desc(sb + k4 * b_kstep, b_lbo, 1024);
-            umma_bf16<kCG>(d_tmem, da, db, idesc, (kb > kb0 || k4 > 0) ? 1u : 0u);
+            for (int k4 = 0; k4 < BK / 16; ++k4) {
+              const uint64_t da = make_smem_desc(sa + k4 * a_kstep, a_lbo, 1024);
+              const uint64_t db = make_smem_desc(sb + k4 * b_kstep, b_lbo, 1024);
+              umma_bf16<kCG>(d_tmem, da, db, idesc, (kb > kb0 || k4 > 0) ? 1u : 0u);
+            }
+            if constexpr (kCG == 1) umma_commit(&empty_bar[s]);
+            else umma_commit_pair(&empty_bar[s], 3);
           }
-          if constexpr (kCG == 1) umma_commit(&empty_bar[s]);
-          else umma_commit_pair(&empty_bar[s], 3);
+          __syncwarp();
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
         }
         if (!ok) break;
-        if constexpr (kCG == 1) umma_commit(&tfull_bar[acc]);
-        else umma_commit_pair(&tfull_bar[acc], 3);
+        if (elect_one()) {
+          if constexpr (kCG == 1) umma_commit(&tfull_bar[acc]);
+          else umma_commit_pair(&tfull_bar[acc], 3);
+        }
+        __syncwarp();
         FB_TIMELINE_ONLY(if (p.ts && it == 0) p.ts[blockIdx.x * 8 + 3] = clock64();)
       }
     }
