@@ -174,7 +174,7 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   float* mask_s = reinterpret_cast<float*>(smem + L::MASK);
   float2* stats = reinterpret_cast<float2*>(smem + L::STATS);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int nblk = (p.S + kBlk - 1) / kBlk;
   // The key blocks of a head add to dQ in order (below), so a block may only wait for blocks that run already: the work is handed out by a
   // counter, in an order in which a head's earlier key blocks come first.
@@ -215,33 +215,37 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const auto query_block = [&](int it) { return nblk - 1 - it; };
 
   if (warp == kBwdSoftmaxWarps + 5) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      const int j = item[0], h = item[1], b = item[2];
+    // ------------------------------------------------------------------ TMA producer (this loop and the next one: the whole warp, one lane issues)
+    const int j = item[0], h = item[1], b = item[2];
+    if (elect_one()) {
       mbar_expect_tx(kv_full, 32768);
       tma_load_4d(smem + L::K, &tmK, kv_full, 0, j * kBlk, h, b);
       tma_load_4d(smem + L::V, &tmV, kv_full, 0, j * kBlk, h, b);
-      for (int it = 0; it < n; ++it) {
-        const int st = it % kBwdStages;
-        if (!mbar_wait(&q_empty[st], ((it / kBwdStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitEmpty)) break;
+    }
+    __syncwarp();
+    for (int it = 0; it < n; ++it) {
+      const int st = it % kBwdStages;
+      if (!warp_wait(&q_empty[st], ((it / kBwdStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitEmpty)) break;
+      if (elect_one()) {
         mbar_expect_tx(&q_full[st], 32768);
         tma_load_4d(smem + L::Q + st * 16384, &tmQ, &q_full[st], 0, query_block(it) * kBlk, h, b);
         tma_load_4d(smem + L::DO + st * 16384, &tmDO, &q_full[st], 0, query_block(it) * kBlk, h, b);
       }
+      __syncwarp();
     }
   } else if (warp == kBwdSoftmaxWarps + 4) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc_kk = make_idesc_bf16(128, 128, 0, 0);      // S, dP: both operands K-major
-      const uint32_t idesc_mn = make_idesc_bf16(128, kHD, 1, 1);      // dV, dK: A^T (MN-major) x MN-major
-      const uint32_t idesc_kn = make_idesc_bf16(128, kHD, 0, 1);      // dQ: K-major x MN-major
-      const uint32_t sK = smem_u32(smem + L::K), sV = smem_u32(smem + L::V);
-      const uint32_t sP = smem_u32(smem + L::P), sDS = smem_u32(smem + L::DS);
-      auto scores = [&](int it) {
-        const int st = it % kBwdStages;
-        const uint32_t sQ = smem_u32(smem + L::Q + st * 16384), sDO = smem_u32(smem + L::DO + st * 16384);
-        if (!mbar_wait(&q_full[st], (it / kBwdStages) & 1, abort_flag, p.status, kStatusWaitFull)) return false;
-        tc_fence_after_sync();
+    const uint32_t idesc_kk = make_idesc_bf16(128, 128, 0, 0);      // S, dP: both operands K-major
+    const uint32_t idesc_mn = make_idesc_bf16(128, kHD, 1, 1);      // dV, dK: A^T (MN-major) x MN-major
+    const uint32_t idesc_kn = make_idesc_bf16(128, kHD, 0, 1);      // dQ: K-major x MN-major
+    const uint32_t sK = smem_u32(smem + L::K), sV = smem_u32(smem + L::V);
+    const uint32_t sP = smem_u32(smem + L::P), sDS = smem_u32(smem + L::DS);
+    auto scores = [&](int it) {
+      const int st = it % kBwdStages;
+      const uint32_t sQ = smem_u32(smem + L::Q + st * 16384), sDO = smem_u32(smem + L::DO + st * 16384);
+      if (!warp_wait(&q_full[st], (it / kBwdStages) & 1, abort_flag, p.status, kStatusWaitFull)) return false;
+      tc_fence_after_sync();
+      if (elect_one()) {
 #pragma unroll
         for (int k4 = 0; k4 < kHD / 16; ++k4)
           umma_bf16<1>(tS, make_smem_desc(sQ + k4 * 32, 16, 1024), make_smem_desc(sK + k4 * 32, 16, 1024), idesc_kk, k4 > 0);
@@ -249,20 +253,23 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int k4 = 0; k4 < kHD / 16; ++k4)
           umma_bf16<1>(tDP, make_smem_desc(sDO + k4 * 32, 16, 1024), make_smem_desc(sV + k4 * 32, 16, 1024), idesc_kk, k4 > 0);
         umma_commit(sdp_full);
-        return true;
-      };
-      bool ok = mbar_wait(kv_full, 0, abort_flag, p.status, kStatusWaitFull) && scores(0);
-      for (int it = 0; it < n && ok; ++it) {
-        if (it + 1 < n) {
-          ok = mbar_wait(sdp_free, it & 1, abort_flag, p.status, kStatusWaitEpi) && scores(it + 1);
-          if (!ok) break;
-        }
-        const int st = it % kBwdStages, qb = it & 1;
-        const uint32_t sQ = smem_u32(smem + L::Q + st * 16384), sDO = smem_u32(smem + L::DO + st * 16384);
-        ok = mbar_wait(pds_ready, it & 1, abort_flag, p.status, kStatusWaitEpi) &&
-             mbar_wait(&dq_free[qb], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi);
+      }
+      __syncwarp();
+      return true;
+    };
+    bool ok = warp_wait(kv_full, 0, abort_flag, p.status, kStatusWaitFull) && scores(0);
+    for (int it = 0; it < n && ok; ++it) {
+      if (it + 1 < n) {
+        ok = warp_wait(sdp_free, it & 1, abort_flag, p.status, kStatusWaitEpi) && scores(it + 1);
         if (!ok) break;
-        tc_fence_after_sync();
+      }
+      const int st = it % kBwdStages, qb = it & 1;
+      const uint32_t sQ = smem_u32(smem + L::Q + st * 16384), sDO = smem_u32(smem + L::DO + st * 16384);
+      ok = warp_wait(pds_ready, it & 1, abort_flag, p.status, kStatusWaitEpi) &&
+           warp_wait(&dq_free[qb], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi);
+      if (!ok) break;
+      tc_fence_after_sync();
+      if (elect_one()) {
         // dV += P^T dO ; dK += dS^T Q   (M = key index, K = query index: 8 steps of 16 rows)
 #pragma unroll
         for (int k8 = 0; k8 < kBlk / 16; ++k8)
@@ -279,6 +286,7 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         umma_commit(&dq_full[qb]);
         umma_commit(&q_empty[st]);
       }
+      __syncwarp();
     }
   } else if (warp == kBwdSoftmaxWarps + 6) {
     // ------------------------------------------------------------------ dQ into the scratch
@@ -513,7 +521,7 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* mask_s = reinterpret_cast<float*>(smem + L::MASK);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int nblk = (p.S + kBlk - 1) / kBlk;
   int qb, h, b;
   decode_block(blockIdx.x, nblk, p.H, p.B, p.causal != 0, 1, qb, h, b);
@@ -545,55 +553,66 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   if (warp == kFwdSoftmaxWarps + 1) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, 16384);
       tma_load_4d(smem + L::Q, &tmQ, q_full, 0, q0, h, b);
-      for (int j = 0; j < n; ++j) {
-        const int st = j & 1;
-        const uint32_t ph = ((j >> 1) & 1) ^ 1;
-        if (!mbar_wait(&k_empty[st], ph, abort_flag, p.status, kStatusWaitEmpty)) break;
+    }
+    __syncwarp();
+    for (int j = 0; j < n; ++j) {
+      const int st = j & 1;
+      const uint32_t ph = ((j >> 1) & 1) ^ 1;
+      if (!warp_wait(&k_empty[st], ph, abort_flag, p.status, kStatusWaitEmpty)) break;
+      if (elect_one()) {
         mbar_expect_tx(&k_full[st], 16384);
         tma_load_4d(smem + L::K + st * 16384, &tmK, &k_full[st], 0, j * kBlk, h, b);
-        if (!mbar_wait(&v_empty[st], ph, abort_flag, p.status, kStatusWaitEmpty)) break;
+      }
+      __syncwarp();
+      if (!warp_wait(&v_empty[st], ph, abort_flag, p.status, kStatusWaitEmpty)) break;
+      if (elect_one()) {
         mbar_expect_tx(&v_full[st], 16384);
         tma_load_4d(smem + L::V + st * 16384, &tmV, &v_full[st], 0, j * kBlk, h, b);
       }
+      __syncwarp();
     }
   } else if (warp == kFwdSoftmaxWarps) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
-      const uint32_t idesc_o = make_idesc_bf16(128, kHD, 0, 1);
-      const uint32_t sQ = smem_u32(smem + L::Q);
-      auto scores = [&](int j) {
-        const int st = j & 1;
-        const uint32_t sK = smem_u32(smem + L::K + st * 16384);
-        if (!mbar_wait(&k_full[st], (j >> 1) & 1, abort_flag, p.status, kStatusWaitFull)) return false;
-        tc_fence_after_sync();
+    const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
+    const uint32_t idesc_o = make_idesc_bf16(128, kHD, 0, 1);
+    const uint32_t sQ = smem_u32(smem + L::Q);
+    auto scores = [&](int j) {
+      const int st = j & 1;
+      const uint32_t sK = smem_u32(smem + L::K + st * 16384);
+      if (!warp_wait(&k_full[st], (j >> 1) & 1, abort_flag, p.status, kStatusWaitFull)) return false;
+      tc_fence_after_sync();
+      if (elect_one()) {
 #pragma unroll
         for (int k4 = 0; k4 < kHD / 16; ++k4)
           umma_bf16<1>(tS, make_smem_desc(sQ + k4 * 32, 16, 1024), make_smem_desc(sK + k4 * 32, 16, 1024), idesc_s, k4 > 0);
         umma_commit(s_full);
         umma_commit(&k_empty[st]);
-        return true;
-      };
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.status, kStatusWaitFull) && scores(0);
-      for (int j = 0; j < n && ok; ++j) {
-        if (j + 1 < n) {
-          ok = mbar_wait(s_free, j & 1, abort_flag, p.status, kStatusWaitEpi) && scores(j + 1);
-          if (!ok) break;
-        }
-        const int st = j & 1;
-        const uint32_t sV = smem_u32(smem + L::V + st * 16384);
-        ok = mbar_wait(p_ready, j & 1, abort_flag, p.status, kStatusWaitEpi) && mbar_wait(&v_full[st], (j >> 1) & 1, abort_flag, p.status, kStatusWaitFull);
+      }
+      __syncwarp();
+      return true;
+    };
+    bool ok = warp_wait(q_full, 0, abort_flag, p.status, kStatusWaitFull) && scores(0);
+    for (int j = 0; j < n && ok; ++j) {
+      if (j + 1 < n) {
+        ok = warp_wait(s_free, j & 1, abort_flag, p.status, kStatusWaitEpi) && scores(j + 1);
         if (!ok) break;
-        tc_fence_after_sync();
+      }
+      const int st = j & 1;
+      const uint32_t sV = smem_u32(smem + L::V + st * 16384);
+      ok = warp_wait(p_ready, j & 1, abort_flag, p.status, kStatusWaitEpi) && warp_wait(&v_full[st], (j >> 1) & 1, abort_flag, p.status, kStatusWaitFull);
+      if (!ok) break;
+      tc_fence_after_sync();
+      if (elect_one()) {
 #pragma unroll
         for (int k8 = 0; k8 < kBlk / 16; ++k8)
           umma_bf16_ts(tO, tP + k8 * 8, make_smem_desc(sV + k8 * 2048, 8192, 1024), idesc_o, j > 0 || k8 > 0);
         umma_commit(pv_done);
         umma_commit(&v_empty[st]);
       }
+      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------------ softmax: thread = query row t x 64 keys

@@ -569,7 +569,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* bias_smem = reinterpret_cast<float*>(epi_smem + Cfg::EPI_BYTES + Cfg::BAR_BYTES);
 
-  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // the same in a whole warp, for the compiler too
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = (kCG == 2) ? cluster_ctarank() : 0u;
   const int group = blockIdx.x / kCG;          // CTA (pair) index
@@ -646,8 +646,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    // The whole warp walks the loop and one lane issues: addresses, coordinates and descriptors then stay in uniform registers, where the
-    // instructions want them.
     {
       int s = 0;
       uint32_t ph = 0;
@@ -661,7 +659,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int kb0 = ks * kb_per;
         const int kb1 = min(num_kb, kb0 + kb_per);
         for (int kb = kb0; kb < kb1; ++kb) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty));
+          ok = warp_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty);
           if (!ok) break;
           uint8_t* sa = stage_base + s * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + Cfg::A_BYTES;
@@ -701,18 +699,18 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t ph = 0;
       int it = 0;
       bool ok = true;
-      if constexpr (kCG == 2) ok = __all_sync(0xffffffffu, mbar_wait(peer_bar, 0, abort_flag, p.status, kStatusWaitEpi));
+      if constexpr (kCG == 2) ok = warp_wait(peer_bar, 0, abort_flag, p.status, kStatusWaitEpi);
       for (int u = group; u < num_units && ok; u += num_groups, ++it) {
         const int ks = u % p.split_k;
         const int kb0 = ks * kb_per;
         const int kb1 = min(num_kb, kb0 + kb_per);
         const int acc = it & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi));
+        ok = warp_wait(&tempty_bar[acc], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi);
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * kBN;
         for (int kb = kb0; kb < kb1; ++kb) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull));
+          ok = warp_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
           if (!ok) break;
           tc_fence_after_sync();
           FB_TIMELINE_ONLY(if (p.ts && it == 0 && kb == kb0) p.ts[blockIdx.x * 8 + 2] = clock64();)
@@ -808,7 +806,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         next_bias = bias_of(u + num_groups);
         if (ks == 0) bias = smem_u32(slice);
       }
-      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&tfull_bar[acc], (it >> 1) & 1, abort_flag, p.status, kStatusWaitAccum));
+      if (ok) ok = warp_wait(&tfull_bar[acc], (it >> 1) & 1, abort_flag, p.status, kStatusWaitAccum);
       if (!ok) continue;
       tc_fence_after_sync();
       FB_TIMELINE_ONLY(if (p.ts && it == 0 && warp == 2 && lane == 0) p.ts[blockIdx.x * 8 + 4] = clock64();)
@@ -917,7 +915,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_ctarank()), side = rank & 1, part = rank >> 1;
   const int m0 = blockIdx.y * 2 * BM + side * BM, n0 = blockIdx.z * 256;
   const int num_kb = (p.K + BK - 1) / BK, kb_half = (num_kb + 1) / 2;      // num_kb >= 2
@@ -952,13 +950,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const uint32_t lane_base = tmem + (static_cast<uint32_t>(q * 32) << 16);
   bool ok = true;
   if (warp == 0) {
-    if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 0;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty)) break;
-        uint8_t* sa = smem + s * Cfg::STAGE_BYTES;
-        uint8_t* sb = sa + BM * BK * 2;
+    int s = 0;
+    uint32_t ph = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!warp_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty)) break;
+      uint8_t* sa = smem + s * Cfg::STAGE_BYTES;
+      uint8_t* sb = sa + BM * BK * 2;
+      if (elect_one()) {
         if (side == 0) mbar_expect_tx(&full_bar[s], 2 * Cfg::STAGE_BYTES);
         tma_load_2d_pair(sa, &tmA, &full_bar[s], kb * BK, m0);
         if (!p.b_mn) {
@@ -967,31 +965,36 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           tma_load_2d_pair(sb, &tmB, &full_bar[s], n0 + side * 128, kb * BK);
           tma_load_2d_pair(sb + 8192, &tmB, &full_bar[s], n0 + side * 128 + 64, kb * BK);
         }
-        if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
       }
+      __syncwarp();
+      if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
-    if (side == 0 && lane == 0) {
+    if (side == 0) {
       const uint32_t idesc = make_idesc_bf16(2 * BM, 256, 0, p.b_mn);
       const uint32_t b_lbo = p.b_mn ? 8192u : 16u, b_kstep = p.b_mn ? 2048u : 32u;
       const uint16_t pair = static_cast<uint16_t>(3 << (rank & 2));
       int s = 0;
       uint32_t ph = 0;
       for (int kb = kb0; kb < kb1 && ok; ++kb) {
-        ok = mbar_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
+        ok = warp_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t sa = smem_u32(smem + s * Cfg::STAGE_BYTES), sb = sa + BM * BK * 2;
+        if (elect_one()) {
 #pragma unroll
-        for (int k4 = 0; k4 < BK / 16; ++k4)
-          umma_bf16<2>(tmem, make_smem_desc(sa + k4 * 32, 16, 1024), make_smem_desc(sb + k4 * b_kstep, b_lbo, 1024), idesc, (kb > kb0 || k4 > 0) ? 1u : 0u);
-        umma_commit_pair(&empty_bar[s], pair);
+          for (int k4 = 0; k4 < BK / 16; ++k4)
+            umma_bf16<2>(tmem, make_smem_desc(sa + k4 * 32, 16, 1024), make_smem_desc(sb + k4 * b_kstep, b_lbo, 1024), idesc, (kb > kb0 || k4 > 0) ? 1u : 0u);
+          umma_commit_pair(&empty_bar[s], pair);
+        }
+        __syncwarp();
         if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
       }
-      if (ok) umma_commit_pair(done_bar, pair);
+      if (ok && elect_one()) umma_commit_pair(done_bar, pair);
+      __syncwarp();
     }
   } else {
-    ok = __all_sync(0xffffffffu, mbar_wait(done_bar, 0, abort_flag, p.status, kStatusWaitAccum));
+    ok = warp_wait(done_bar, 0, abort_flag, p.status, kStatusWaitAccum);
     if (ok) {       // the partner's columns into the partner's shared memory
       tc_fence_after_sync();
       uint32_t there;
