@@ -140,7 +140,7 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int taps = p.kh * p.kw;
 
   if (threadIdx.x == 0) {
@@ -180,7 +180,7 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constan
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
+    {
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -188,28 +188,31 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constan
         const int t0 = pass * p.taps_per_pass;
         const int nt = min(p.taps_per_pass, taps - t0);
         if (pass > 0) {   // the epilogue stages its results in the pipeline buffers: wait until it is done with them
-          ok = mbar_wait(drained_bar, (pass - 1) & 1, abort_flag, p.status, kStatusWaitEpi);
+          ok = warp_wait(drained_bar, (pass - 1) & 1, abort_flag, p.status, kStatusWaitEpi);
           if (!ok) break;
         }
         for (int c = blockIdx.x; c < p.chunks && ok; c += gridDim.x) {
-          ok = mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty);
+          ok = warp_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty);
           if (!ok) break;
           const int n = c / per_img, r = c - n * per_img;
           const int ho0 = (r / per_row) * p.hbox, wo0 = (r % per_row) * p.wbox;
           uint8_t* sa = smem + s * stage_bytes;
-          mbar_expect_tx(&full_bar[s], kPanel + nt * p.b_bytes);
-          tma4(sa, &tmDy, &full_bar[s], 0, wo0, ho0, n);
-          for (int t = 0; t < nt; ++t) {
-            const int tap = t0 + t, dy = tap / p.kw, dx = tap - dy * p.kw;
-            tma4(sa + kPanel + t * p.b_bytes, &tmX, &full_bar[s], 0, wo0 * p.stride + dx - p.pad, ho0 * p.stride + dy - p.pad, n);
+          if (elect_one()) {
+            mbar_expect_tx(&full_bar[s], kPanel + nt * p.b_bytes);
+            tma4(sa, &tmDy, &full_bar[s], 0, wo0, ho0, n);
+            for (int t = 0; t < nt; ++t) {
+              const int tap = t0 + t, dy = tap / p.kw, dx = tap - dy * p.kw;
+              tma4(sa + kPanel + t * p.b_bytes, &tmX, &full_bar[s], 0, wo0 * p.stride + dx - p.pad, ho0 * p.stride + dy - p.pad, n);
+            }
           }
+          __syncwarp();
           if (++s == kConvStages) { s = 0; ph ^= 1; }
         }
       }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
       const uint32_t idesc = make_idesc_bf16(128, p.Ci, 1, 1);
       int s = 0;
       uint32_t ph = 0;
@@ -218,31 +221,35 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constan
         const int t0 = pass * p.taps_per_pass;
         const int nt = min(p.taps_per_pass, taps - t0);
         if (pass > 0) {   // the epilogue must have emptied the accumulators of the previous pass
-          ok = mbar_wait(drained_bar, (pass - 1) & 1, abort_flag, p.status, kStatusWaitEpi);
+          ok = warp_wait(drained_bar, (pass - 1) & 1, abort_flag, p.status, kStatusWaitEpi);
           if (!ok) break;
           tc_fence_after_sync();
         }
         bool first = true;
         for (int c = blockIdx.x; c < p.chunks && ok; c += gridDim.x) {
-          ok = mbar_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
+          ok = warp_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
           if (!ok) break;
           tc_fence_after_sync();
           const uint32_t sa = smem_u32(smem + s * stage_bytes);
           const uint32_t a_lbo = smem_u32(smem + p.zero_off) - sa;      // panel 0 -> the shared zero panel
-          for (int t = 0; t < nt; ++t) {
-            const uint32_t sb = sa + kPanel + t * p.b_bytes;
+          if (elect_one()) {
+            for (int t = 0; t < nt; ++t) {
+              const uint32_t sb = sa + kPanel + t * p.b_bytes;
 #pragma unroll
-            for (int k4 = 0; k4 < kPix / 16; ++k4) {
-              const uint64_t da = conv_desc(sa + k4 * 2048, a_lbo, 1024, 2);
-              const uint64_t db = conv_desc(sb + k4 * p.b_kstep, p.b_bytes, p.b_sbo, p.b_layout);
-              umma_bf16<1>(tmem_base + t * p.Ci, da, db, idesc, (first && k4 == 0) ? 0u : 1u);
+              for (int k4 = 0; k4 < kPix / 16; ++k4) {
+                const uint64_t da = conv_desc(sa + k4 * 2048, a_lbo, 1024, 2);
+                const uint64_t db = conv_desc(sb + k4 * p.b_kstep, p.b_bytes, p.b_sbo, p.b_layout);
+                umma_bf16<1>(tmem_base + t * p.Ci, da, db, idesc, (first && k4 == 0) ? 0u : 1u);
+              }
             }
+            umma_commit(&empty_bar[s]);
           }
+          __syncwarp();
           first = false;
-          umma_commit(&empty_bar[s]);
           if (++s == kConvStages) { s = 0; ph ^= 1; }
         }
-        if (ok) umma_commit(acc_bar);
+        if (ok && elect_one()) umma_commit(acc_bar);
+        __syncwarp();
       }
     }
   } else {
@@ -340,7 +347,7 @@ conv_fwd_kernel(const __grid_constant__ CUtensorMap tmIn, const __grid_constant_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* stat_smem = reinterpret_cast<float*>(smem + p.bars_off + 512);   // [4 warps][2][Nout]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int acc_cols = p.Nout <= 32 ? 32 : p.Nout <= 64 ? 64 : p.Nout <= 128 ? 128 : 256;   // columns of one buffer
 
   if (threadIdx.x == 0) {
@@ -373,59 +380,69 @@ conv_fwd_kernel(const __grid_constant__ CUtensorMap tmIn, const __grid_constant_
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      mbar_expect_tx(w_bar, p.taps * p.w_bytes);
-      for (int t = 0; t < p.taps; ++t) tma_load_2d(smem + t * p.w_bytes, &tmW, w_bar, t * p.Ci, 0);
+    {
+      if (elect_one()) {
+        mbar_expect_tx(w_bar, p.taps * p.w_bytes);
+        for (int t = 0; t < p.taps; ++t) tma_load_2d(smem + t * p.w_bytes, &tmW, w_bar, t * p.Ci, 0);
+      }
+      __syncwarp();
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
       const int box_bytes = p.a_bytes / p.nbox;
       for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
         for (int t = 0; t < p.taps && ok; ++t) {
-          ok = mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty);
+          ok = warp_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty);
           if (!ok) break;
           const int dy = t / p.kw, dx = t - dy * p.kw;
           uint8_t* sa = ring + s * p.a_bytes;
-          mbar_expect_tx(&full_bar[s], p.a_bytes);
-          for (int b = 0; b < p.nbox; ++b) {
-            const int c = tile * p.nbox + b;
-            const int n = c / p.per_img, r = c - n * p.per_img;      // n may reach `images`: the box is then all zero fill
-            const int ho0 = r * p.hbox;
-            tma4(sa + b * box_bytes, &tmIn, &full_bar[s], 0, p.sign * (dx - p.pad), ho0 * p.stride + p.sign * (dy - p.pad), n);
+          if (elect_one()) {
+            mbar_expect_tx(&full_bar[s], p.a_bytes);
+            for (int b = 0; b < p.nbox; ++b) {
+              const int c = tile * p.nbox + b;
+              const int n = c / p.per_img, r = c - n * p.per_img;      // n may reach `images`: the box is then all zero fill
+              const int ho0 = r * p.hbox;
+              tma4(sa + b * box_bytes, &tmIn, &full_bar[s], 0, p.sign * (dx - p.pad), ho0 * p.stride + p.sign * (dy - p.pad), n);
+            }
           }
+          __syncwarp();
           if (++s == p.stages) { s = 0; ph ^= 1; }
         }
       }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
       const uint32_t idesc = make_idesc_bf16(128, p.Nout, 0, p.b_mn);
-      bool ok = mbar_wait(w_bar, 0, abort_flag, p.status, kStatusWaitFull);
+      bool ok = warp_wait(w_bar, 0, abort_flag, p.status, kStatusWaitFull);
       int s = 0, it = 0;
       uint32_t ph = 0;
       const uint32_t w0 = smem_u32(smem);
       for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x, ++it) {
         const int buf = it & 1;
-        ok = mbar_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi);
+        ok = warp_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi);
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t d = tmem_base + buf * acc_cols;
         for (int t = 0; t < p.taps && ok; ++t) {
-          ok = mbar_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
+          ok = warp_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
           if (!ok) break;
           tc_fence_after_sync();
           const uint32_t sa = smem_u32(ring + s * p.a_bytes);
           const uint32_t sw = w0 + t * p.w_bytes;
-          for (int k = 0; k < p.Kc / 16; ++k) {
-            const uint64_t da = conv_desc(sa + k * 32, 16, p.a_sbo, p.a_layout);
-            const uint64_t db = conv_desc(sw + k * p.w_kstep, 16, p.w_sbo, p.w_layout);
-            umma_bf16<1>(d, da, db, idesc, (t == 0 && k == 0) ? 0u : 1u);
+          if (elect_one()) {
+            for (int k = 0; k < p.Kc / 16; ++k) {
+              const uint64_t da = conv_desc(sa + k * 32, 16, p.a_sbo, p.a_layout);
+              const uint64_t db = conv_desc(sw + k * p.w_kstep, 16, p.w_sbo, p.w_layout);
+              umma_bf16<1>(d, da, db, idesc, (t == 0 && k == 0) ? 0u : 1u);
+            }
+            umma_commit(&empty_bar[s]);
           }
-          umma_commit(&empty_bar[s]);
+          __syncwarp();
           if (++s == p.stages) { s = 0; ph ^= 1; }
         }
-        if (ok) umma_commit(&acc_full[buf]);
+        if (ok && elect_one()) umma_commit(&acc_full[buf]);
+        __syncwarp();
       }
     }
   } else {
