@@ -694,14 +694,15 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmW, const HaloParams p)
       int s = 0, it = 0;
       uint32_t ph = 0;
       const uint64_t db0 = conv_desc(smem_u32(smem), 16, p.w_sbo, p.w_layout);
+      const uint32_t b_lo0 = static_cast<uint32_t>(db0), b_hi = static_cast<uint32_t>(db0 >> 32);
       const int ksteps = p.Kc / 16, a_kstep16 = (2 * p.plane_bytes) >> 4, w_kstep16 = p.w_kstep >> 4;
       // per-tap constants: start-address offsets of both operands (16-byte units) and the accumulator group
-      uint64_t a_off[9], b_off[9];
+      uint32_t a_off[9], b_off[9];
       uint32_t dcol[9];
 #pragma unroll
       for (int tp = 0; tp < 9; ++tp) {
-        a_off[tp] = static_cast<uint64_t>(static_cast<int64_t>(p.sign * ((tp / 3 - 1) * p.pitch + (tp % 3 - 1))));
-        b_off[tp] = static_cast<uint64_t>((tp * p.w_bytes) >> 4);
+        a_off[tp] = static_cast<uint32_t>(p.sign * ((tp / 3 - 1) * p.pitch + (tp % 3 - 1)));
+        b_off[tp] = b_lo0 + static_cast<uint32_t>((tp * p.w_bytes) >> 4);
         dcol[tp] = static_cast<uint32_t>((tp % p.groups) * p.Nout);
       }
       for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x, ++it) {
@@ -716,10 +717,11 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmW, const HaloParams p)
         // descriptors differ from one instruction to the next only in their 16-byte-granular start
         // address field (bits 0..13), which never carries out of the field for these offsets
         const uint64_t da0 = conv_desc(smem_u32(ring + s * p.a_bytes) + p.halo * 16, p.plane_bytes, 128, 0);
+        const uint32_t a_lo = static_cast<uint32_t>(da0), a_hi = static_cast<uint32_t>(da0 >> 32);
         for (int k = 0; k < ksteps; ++k) {
 #pragma unroll
           for (int tp = 0; tp < 9; ++tp)
-            umma_bf16<1>(d + dcol[tp], da0 + a_off[tp] + static_cast<uint64_t>(k * a_kstep16), db0 + b_off[tp] + static_cast<uint64_t>(k * w_kstep16), idesc,
+            umma_bf16<1>(d + dcol[tp], desc_of(a_lo + a_off[tp] + k * a_kstep16, a_hi), desc_of(b_off[tp] + k * w_kstep16, b_hi), idesc,
                          (k == 0 && tp < groups) ? 0u : 1u);
         }
         umma_commit(&empty_bar[s]);
@@ -992,13 +994,14 @@ conv3x3_wgrad_halo_kernel(const WgHaloParams p) {
           const uint64_t da0 = conv_desc(a_base, 128, kWgAPlane, 0);
           // index u of a plane is pixel q0 - pitch + u (+ dx - 1): row dy of the filter starts at u = dy * pitch
           const uint64_t db0 = conv_desc(a_base + kWgABytes, 128, p.b_plane_bytes, 0);
+          const uint32_t a_lo = static_cast<uint32_t>(da0), a_hi = static_cast<uint32_t>(da0 >> 32), b_lo = static_cast<uint32_t>(db0), b_hi = static_cast<uint32_t>(db0 >> 32);
           // pixel group outermost, filter row innermost: consecutive instructions go to different accumulators
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks) {
             const uint32_t acc = (first && ks == 0) ? 0u : 1u;
 #pragma unroll
             for (int rr = 0; rr < 3; ++rr)
-              umma_bf16<1>(tmem_base + rr * 3 * p.Ci, da0 + ks * 16, db0 + static_cast<uint64_t>(rr * p.pitch + ks * 16), idesc, acc);
+              umma_bf16<1>(tmem_base + rr * 3 * p.Ci, desc_of(a_lo + ks * 16, a_hi), desc_of(b_lo + rr * p.pitch + ks * 16, b_hi), idesc, acc);
           }
           first = false;
           umma_commit(&empty_bar[s]);

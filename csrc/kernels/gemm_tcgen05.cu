@@ -693,8 +693,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t idesc = make_idesc_bf16(BM * kCG, kBN, p.a_mn, p.b_mn);
       const uint32_t a_lbo = p.a_mn ? 8192u : 16u;
       const uint32_t b_lbo = p.b_mn ? 8192u : 16u;
-      const uint32_t a_kstep = p.a_mn ? 2048u : 32u;
-      const uint32_t b_kstep = p.b_mn ? 2048u : 32u;
+      const uint32_t a_kstep = (p.a_mn ? 2048u : 32u) >> 4;
+      const uint32_t b_kstep = (p.b_mn ? 2048u : 32u) >> 4;
+      const uint32_t a_first = smem_desc_lo(smem_u32(stage_base), a_lbo), b_first = smem_desc_lo(smem_u32(stage_base) + Cfg::A_BYTES, b_lbo);
+      const uint32_t hi = smem_desc_hi(1024);
       int s = 0;
       uint32_t ph = 0;
       int it = 0;
@@ -714,15 +716,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (!ok) break;
           tc_fence_after_sync();
           FB_TIMELINE_ONLY(if (p.ts && it == 0 && kb == kb0) p.ts[blockIdx.x * 8 + 2] = clock64();)
-          const uint32_t sa = smem_u32(stage_base + s * Cfg::STAGE_BYTES);
-          const uint32_t sb = sa + Cfg::A_BYTES;
+          const uint32_t a_lo = a_first + s * (Cfg::STAGE_BYTES >> 4), b_lo = b_first + s * (Cfg::STAGE_BYTES >> 4);
           if (elect_one()) {
 #pragma unroll
-            for (int k4 = 0; k4 < BK / 16; ++k4) {
-              const uint64_t da = make_smem_desc(sa + k4 * a_kstep, a_lbo, 1024);
-              const uint64_t db = make_smem_desc(sb + k4 * b_kstep, b_lbo, 1024);
-              umma_bf16<kCG>(d_tmem, da, db, idesc, (kb > kb0 || k4 > 0) ? 1u : 0u);
-            }
+            for (int k4 = 0; k4 < BK / 16; ++k4)
+              umma_bf16<kCG>(d_tmem, desc_of(a_lo + k4 * a_kstep, hi), desc_of(b_lo + k4 * b_kstep, hi), idesc, (kb > kb0 || k4 > 0) ? 1u : 0u);
             if constexpr (kCG == 1) umma_commit(&empty_bar[s]);
             else umma_commit_pair(&empty_bar[s], 3);
           }

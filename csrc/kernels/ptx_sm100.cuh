@@ -369,6 +369,15 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
   return d;
 }
 
+// The two words of such a descriptor: steps through a tile change the start address alone (16-byte units, no carry below 256 KB), one 32-bit sum.
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) { return (smem_addr >> 4) | (lbo_bytes >> 4) << 16; }
+__device__ __forceinline__ uint32_t smem_desc_hi(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | 1u << 14 | 2u << 29; }
+__device__ __forceinline__ uint64_t desc_of(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+
 // Instruction descriptor for kind::f16 with bf16 A/B and fp32 accumulate.
 //   [4,6) D fmt (1 = f32)  [7,10) A fmt (1 = bf16)  [10,13) B fmt (1 = bf16)
 //   [15] A major (0 = K, 1 = MN)  [16] B major  [17,23) N >> 3  [24,29) M >> 4
