@@ -589,7 +589,7 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmW, const HaloParams p)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* stat_smem = reinterpret_cast<float*>(smem + p.bars_off + 512);   // [4 warps][2][Nout]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   // Consecutive MMAs into one accumulator wait for each other (about 0.1 us each, measured), so the
   // nine taps of a tile are spread round-robin over `groups` accumulators that the epilogue adds up.
   const int groups = p.groups;
@@ -686,11 +686,14 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmW, const HaloParams p)
     }
   } else if (warp == 4) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      mbar_expect_tx(w_bar, 9 * p.w_bytes);
-      for (int tp = 0; tp < 9; ++tp) tma_load_2d(smem + tp * p.w_bytes, &tmW, w_bar, tp * p.Ci, 0);
+    {
+      if (elect_one()) {
+        mbar_expect_tx(w_bar, 9 * p.w_bytes);
+        for (int tp = 0; tp < 9; ++tp) tma_load_2d(smem + tp * p.w_bytes, &tmW, w_bar, tp * p.Ci, 0);
+      }
+      __syncwarp();
       const uint32_t idesc = make_idesc_bf16(128, p.Nout, 0, p.b_mn);
-      bool ok = mbar_wait(w_bar, 0, abort_flag, p.status, kStatusWaitFull);
+      bool ok = warp_wait(w_bar, 0, abort_flag, p.status, kStatusWaitFull);
       int s = 0, it = 0;
       uint32_t ph = 0;
       const uint64_t db0 = conv_desc(smem_u32(smem), 16, p.w_sbo, p.w_layout);
@@ -707,26 +710,29 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmW, const HaloParams p)
       }
       for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x, ++it) {
         const int buf = it & 1;
-        ok = mbar_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi);
+        ok = warp_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi);
         if (!ok) break;
-        ok = mbar_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
+        ok = warp_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
         if (!ok) break;
-        if (it < 10) ts_mark(p.ts, 12 + it);
+        if (lane == 0 && it < 10) ts_mark(p.ts, 12 + it);
         tc_fence_after_sync();
         const uint32_t d = tmem_base + buf * acc_cols;
         // descriptors differ from one instruction to the next only in their 16-byte-granular start
         // address field (bits 0..13), which never carries out of the field for these offsets
         const uint64_t da0 = conv_desc(smem_u32(ring + s * p.a_bytes) + p.halo * 16, p.plane_bytes, 128, 0);
         const uint32_t a_lo = static_cast<uint32_t>(da0), a_hi = static_cast<uint32_t>(da0 >> 32);
-        for (int k = 0; k < ksteps; ++k) {
+        if (elect_one()) {
+          for (int k = 0; k < ksteps; ++k) {
 #pragma unroll
-          for (int tp = 0; tp < 9; ++tp)
-            umma_bf16<1>(d + dcol[tp], desc_of(a_lo + a_off[tp] + k * a_kstep16, a_hi), desc_of(b_off[tp] + k * w_kstep16, b_hi), idesc,
-                         (k == 0 && tp < groups) ? 0u : 1u);
+            for (int tp = 0; tp < 9; ++tp)
+              umma_bf16<1>(d + dcol[tp], desc_of(a_lo + a_off[tp] + k * a_kstep16, a_hi), desc_of(b_off[tp] + k * w_kstep16, b_hi), idesc,
+                           (k == 0 && tp < groups) ? 0u : 1u);
+          }
+          umma_commit(&empty_bar[s]);
+          umma_commit(&acc_full[buf]);
         }
-        umma_commit(&empty_bar[s]);
-        umma_commit(&acc_full[buf]);
-        if (it < 10) ts_mark(p.ts, 22 + it);
+        __syncwarp();
+        if (lane == 0 && it < 10) ts_mark(p.ts, 22 + it);
         if (++s == p.stages) { s = 0; ph ^= 1; }
       }
     }
@@ -880,7 +886,7 @@ conv3x3_wgrad_halo_kernel(const WgHaloParams p) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
@@ -979,7 +985,7 @@ conv3x3_wgrad_halo_kernel(const WgHaloParams p) {
     }
   } else if (warp == 4) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
       const uint32_t idesc = make_idesc_bf16(128, 3 * p.Ci, 1, 1);
       int s = 0;
       uint32_t ph = 0;
@@ -987,7 +993,7 @@ conv3x3_wgrad_halo_kernel(const WgHaloParams p) {
       {
         bool first = true;
         for (int j = 0; j < per_pass && ok; ++j) {
-          ok = mbar_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
+          ok = warp_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
           if (!ok) break;
           tc_fence_after_sync();
           const uint32_t a_base = smem_u32(smem + s * p.stage_bytes);
@@ -996,18 +1002,22 @@ conv3x3_wgrad_halo_kernel(const WgHaloParams p) {
           const uint64_t db0 = conv_desc(a_base + kWgABytes, 128, p.b_plane_bytes, 0);
           const uint32_t a_lo = static_cast<uint32_t>(da0), a_hi = static_cast<uint32_t>(da0 >> 32), b_lo = static_cast<uint32_t>(db0), b_hi = static_cast<uint32_t>(db0 >> 32);
           // pixel group outermost, filter row innermost: consecutive instructions go to different accumulators
+          if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint32_t acc = (first && ks == 0) ? 0u : 1u;
+            for (int ks = 0; ks < 8; ++ks) {
+              const uint32_t acc = (first && ks == 0) ? 0u : 1u;
 #pragma unroll
-            for (int rr = 0; rr < 3; ++rr)
-              umma_bf16<1>(tmem_base + rr * 3 * p.Ci, desc_of(a_lo + ks * 16, a_hi), desc_of(b_lo + rr * p.pitch + ks * 16, b_hi), idesc, acc);
+              for (int rr = 0; rr < 3; ++rr)
+                umma_bf16<1>(tmem_base + rr * 3 * p.Ci, desc_of(a_lo + ks * 16, a_hi), desc_of(b_lo + rr * p.pitch + ks * 16, b_hi), idesc, acc);
+            }
+            umma_commit(&empty_bar[s]);
           }
+          __syncwarp();
           first = false;
-          umma_commit(&empty_bar[s]);
           if (++s == p.stages) { s = 0; ph ^= 1; }
         }
-        if (ok) umma_commit(acc_bar);
+        if (ok && elect_one()) umma_commit(acc_bar);
+        __syncwarp();
       }
     }
   } else {

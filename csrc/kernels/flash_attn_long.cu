@@ -27,6 +27,12 @@
 
 namespace fb {
 
+namespace {
+// Descriptor of the operand at `base` moved on by a constant number of bytes; K-major, or MN-major with `lbo` bytes between its 64-wide panels.
+__device__ __forceinline__ uint64_t k_desc(uint32_t base, int bytes) { return desc_of(smem_desc_lo(base, 16) + (bytes >> 4), smem_desc_hi(1024)); }
+__device__ __forceinline__ uint64_t mn_desc(uint32_t base, int bytes, int lbo) { return desc_of(smem_desc_lo(base, lbo) + (bytes >> 4), smem_desc_hi(1024)); }
+}  // namespace
+
 // ==================================================================================== backward
 namespace {
 
@@ -248,10 +254,10 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (elect_one()) {
 #pragma unroll
         for (int k4 = 0; k4 < kHD / 16; ++k4)
-          umma_bf16<1>(tS, make_smem_desc(sQ + k4 * 32, 16, 1024), make_smem_desc(sK + k4 * 32, 16, 1024), idesc_kk, k4 > 0);
+          umma_bf16<1>(tS, k_desc(sQ, k4 * 32), k_desc(sK, k4 * 32), idesc_kk, k4 > 0);
 #pragma unroll
         for (int k4 = 0; k4 < kHD / 16; ++k4)
-          umma_bf16<1>(tDP, make_smem_desc(sDO + k4 * 32, 16, 1024), make_smem_desc(sV + k4 * 32, 16, 1024), idesc_kk, k4 > 0);
+          umma_bf16<1>(tDP, k_desc(sDO, k4 * 32), k_desc(sV, k4 * 32), idesc_kk, k4 > 0);
         umma_commit(sdp_full);
       }
       __syncwarp();
@@ -273,14 +279,14 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         // dV += P^T dO ; dK += dS^T Q   (M = key index, K = query index: 8 steps of 16 rows)
 #pragma unroll
         for (int k8 = 0; k8 < kBlk / 16; ++k8)
-          umma_bf16<1>(tDV, make_smem_desc(sP + k8 * 2048, 16384, 1024), make_smem_desc(sDO + k8 * 2048, 8192, 1024), idesc_mn, it > 0 || k8 > 0);
+          umma_bf16<1>(tDV, mn_desc(sP, k8 * 2048, 16384), mn_desc(sDO, k8 * 2048, 8192), idesc_mn, it > 0 || k8 > 0);
 #pragma unroll
         for (int k8 = 0; k8 < kBlk / 16; ++k8)
-          umma_bf16<1>(tDK, make_smem_desc(sDS + k8 * 2048, 16384, 1024), make_smem_desc(sQ + k8 * 2048, 8192, 1024), idesc_mn, it > 0 || k8 > 0);
+          umma_bf16<1>(tDK, mn_desc(sDS, k8 * 2048, 16384), mn_desc(sQ, k8 * 2048, 8192), idesc_mn, it > 0 || k8 > 0);
         // dQ_tile = dS K   (M = query, K = key index)
 #pragma unroll
         for (int k8 = 0; k8 < kBlk / 16; ++k8)
-          umma_bf16<1>(tDQ + qb * 64, make_smem_desc(sDS + (k8 >> 2) * 16384 + (k8 & 3) * 32, 16, 1024), make_smem_desc(sK + k8 * 2048, 8192, 1024),
+          umma_bf16<1>(tDQ + qb * 64, k_desc(sDS, (k8 >> 2) * 16384 + (k8 & 3) * 32), mn_desc(sK, k8 * 2048, 8192),
                        idesc_kn, k8 > 0);
         umma_commit(grads_full);
         umma_commit(&dq_full[qb]);
@@ -587,7 +593,7 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (elect_one()) {
 #pragma unroll
         for (int k4 = 0; k4 < kHD / 16; ++k4)
-          umma_bf16<1>(tS, make_smem_desc(sQ + k4 * 32, 16, 1024), make_smem_desc(sK + k4 * 32, 16, 1024), idesc_s, k4 > 0);
+          umma_bf16<1>(tS, k_desc(sQ, k4 * 32), k_desc(sK, k4 * 32), idesc_s, k4 > 0);
         umma_commit(s_full);
         umma_commit(&k_empty[st]);
       }
@@ -608,7 +614,7 @@ attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (elect_one()) {
 #pragma unroll
         for (int k8 = 0; k8 < kBlk / 16; ++k8)
-          umma_bf16_ts(tO, tP + k8 * 8, make_smem_desc(sV + k8 * 2048, 8192, 1024), idesc_o, j > 0 || k8 > 0);
+          umma_bf16_ts(tO, tP + k8 * 8, mn_desc(sV, k8 * 2048, 8192), idesc_o, j > 0 || k8 > 0);
         umma_commit(pv_done);
         umma_commit(&v_empty[st]);
       }
