@@ -129,6 +129,26 @@ void gemm_grouped(const Tensor& a, const std::vector<Tensor>& bs, Tensor& out, c
         "fb_gemm_bf16_grouped");
 }
 
+// dx = dy w (times the activation's derivative at aux), dw += dy^T x, db += column sums of dy, in one launch; false: not taken, nothing done.
+bool gemm_backward(const Tensor& dy, const Tensor& w, const Tensor& x, Tensor& dx, Tensor& dw, const OptTensor& db, int epi, const OptTensor& aux) {
+  want_cuda(dy, "dy");
+  c10::cuda::CUDAGuard guard(dy.device());
+  for (const Tensor* t : {&dy, &w, &x, static_cast<const Tensor*>(&dx)})
+    TORCH_CHECK(t->is_cuda() && is_bf16(*t) && t->dim() == 2 && t->stride(1) == 1, "bf16 [rows, cols] with unit inner stride");
+  const int64_t rows = dy.size(0), n = dy.size(1), k = x.size(1);
+  TORCH_CHECK(w.size(0) == n && w.size(1) == k && x.size(0) == rows && dx.size(0) == rows && dx.size(1) == k, "shapes do not fit together");
+  TORCH_CHECK(dw.is_cuda() && dw.scalar_type() == at::kFloat && dw.dim() == 2 && dw.size(0) == n && dw.size(1) == k && dw.stride(1) == 1, "dw must be fp32 [n, k]");
+  if (db.has_value()) TORCH_CHECK(db->is_cuda() && db->scalar_type() == at::kFloat && db->numel() == n && db->is_contiguous(), "db must be fp32 [n]");
+  if (aux.has_value()) TORCH_CHECK(aux->is_cuda() && is_bf16(*aux) && aux->dim() == 2 && aux->stride(1) == 1 && aux->size(0) == rows && aux->size(1) == k, "aux must be bf16 [rows, k]");
+  const int rc = fb_gemm_backward(dy.data_ptr(), w.data_ptr(), x.data_ptr(), dx.data_ptr(), dw.data_ptr<float>(), db.has_value() ? db->data_ptr<float>() : nullptr,
+                                  (int)rows, (int)n, (int)k, dy.stride(0), w.stride(0), x.stride(0), dx.stride(0), dw.stride(0), epi,
+                                  aux.has_value() ? aux->data_ptr() : nullptr, aux.has_value() ? aux->stride(0) : 0,
+                                  status_word(dy.get_device()).data_ptr<int>(), stream_of(dy));
+  if (rc == -7) return false;
+  check(rc, "fb_gemm_backward");
+  return true;
+}
+
 int gemm_pick_config(int M, int N, int K, int split_k) { return fb_gemm_pick_config(M, N, K, split_k); }
 
 // Bounds-check record of the debug build (FLODL_BOUNDS_CHECK): one host-mapped int[4] = {site, index, limit, 0}.
@@ -676,6 +696,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gelu_fwd", &gelu_fwd);
   m.def("gelu_bwd", &gelu_bwd);
   m.def("dropout", &dropout, py::arg("x"), py::arg("p"), py::arg("seed"), py::arg("seed_dev") = py::none());
+  m.def("gemm_backward", &gemm_backward, py::arg("dy"), py::arg("w"), py::arg("x"), py::arg("dx"), py::arg("dw"), py::arg("db") = py::none(),
+        py::arg("epi") = 0, py::arg("aux") = py::none());
   m.def("colsum", &colsum, py::arg("x"), py::arg("out"), py::arg("rows_dyn") = py::none());
   m.def("compact_targets", &compact_targets);
   m.def("gather_rows", &gather_rows);

@@ -109,6 +109,10 @@ int fb_gelu_fwd(const void* x, void* y, long long n, int tanh_approx, int is_bf1
 int fb_gelu_bwd(const void* dy, const void* x, void* dx, long long n, int tanh_approx, int is_bf16, void* stream);
 int fb_dropout(const void* x, void* y, long long n, float p, unsigned long long seed, const unsigned long long* seed_dev,
                int is_bf16, void* stream);
+/* Gradients of y = x W^T + b in one launch: dX = dY W (times the activation's derivative at `aux` with epi 2 or 4), dW += dY^T x, db += column sums
+ * of dY (db may be null). bf16 operands and dX, fp32 dW and db. -7: not taken (size or alignment), nothing launched. */
+int fb_gemm_backward(const void* dY, const void* W, const void* X, void* dX, float* dW, float* db, int rows, int n, int k, long long ldy, long long ldw,
+                     long long ldx, long long lddx, long long lddw, int epi, const void* aux, long long ldaux, int* status, void* stream);
 /* out[c] += sum over rows of x[r][c] (the caller zeroes `out`, or passes a gradient slot to accumulate into). */
 int fb_colsum(const void* x, float* out, int rows, int cols, long long ld, int is_bf16, void* stream);
 /* As fb_colsum over the first min(rows, *rows_dyn) rows (device-side count). */

@@ -485,24 +485,23 @@ __device__ __forceinline__ void epilogue_store32(const GemmParams& p, const uint
 
   if (p.c_fp32) {
     float* c = static_cast<float*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
-    if (p.split_k > 1) {
+    const bool vec = full && ((reinterpret_cast<uintptr_t>(c) & 15) == 0);
+    if (p.split_k > 1 || p.accumulate) {       // added without being read
+      if (vec) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (i < nvalid) atomicAdd(c + i, v[i]);
-    } else if (full && ((reinterpret_cast<uintptr_t>(c) & 15) == 0)) {
+        for (int j = 0; j < 8; ++j) red_add_v4(c + 4 * j, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      } else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float4 o = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        if (p.accumulate) {
-          const float4 old = *reinterpret_cast<const float4*>(c + 4 * j);
-          o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-        }
-        *reinterpret_cast<float4*>(c + 4 * j) = o;
+        for (int i = 0; i < 32; ++i)
+          if (i < nvalid) atomicAdd(c + i, v[i]);
       }
+    } else if (vec) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(c + 4 * j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     } else {
 #pragma unroll
       for (int i = 0; i < 32; ++i)
-        if (i < nvalid) c[i] = p.accumulate ? c[i] + v[i] : v[i];
+        if (i < nvalid) c[i] = v[i];
     }
   } else {
     __nv_bfloat16* c = static_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
@@ -552,10 +551,122 @@ __device__ __forceinline__ void tile_of(int t, int num_m, int num_n, int band, i
   tn = first + t - tm * width;
 }
 
-template <int kCG, int kBN>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAux, const GemmParams p) {
+// One product, or two in one launch: the data gradient of a linear layer and the weight gradient from the same dY, whose column sums (the bias
+// gradient) two more warps of every CTA take on the side.
+template <int kProblems>
+struct alignas(64) GemmLaunch {
+  CUtensorMap a[kProblems], b[kProblems], c[kProblems], aux;      // aux: the first product's
+  GemmParams p[kProblems];
+  // The second product's K blocks in one line, tile after tile: the pairs that have a tile of the first product more than the others (the first
+  // `ahead` of them) take `share_ahead` of these each, the others `share`, in 1/256 of a block.
+  int ahead, share_ahead, share;
+  const __nv_bfloat16* sum_x;
+  float* sum_out;
+  int sum_rows, sum_cols;
+  long long sum_ld;
+};
+
+// What a pair (or CTA) works on next: K blocks [kb0, kb1) of a tile.
+struct Segment {
+  int prob, tm, tn, kb0, kb1, ks;
+};
+template <int kCG, int kBN, int kProblems>
+struct Worklist {
+  const GemmLaunch<kProblems>& g;
+  int step, num_m, num_n, num_kb, kb_per, units, u;      // the first product: whole tiles, or their K splits
+  int num_m1, num_n1, num_kb1, at, end;                  // the second: a stretch of its K blocks
+
+  __device__ __forceinline__ Worklist(const GemmLaunch<kProblems>& g_, int group, int groups, int m_eff, int k_eff) : g(g_), step(groups), u(group) {
+    const GemmParams& p = g.p[0];
+    num_m = (m_eff + BM * kCG - 1) / (BM * kCG);
+    num_n = (p.N + kBN - 1) / kBN;
+    num_kb = (k_eff + BK - 1) / BK;
+    kb_per = (num_kb + p.split_k - 1) / p.split_k;
+    units = num_kb > 0 ? num_m * num_n * p.split_k : 0;
+    if constexpr (kProblems == 2) {
+      const GemmParams& q = g.p[1];
+      num_m1 = (q.M + BM * kCG - 1) / (BM * kCG);
+      num_n1 = (q.N + kBN - 1) / kBN;
+      num_kb1 = (q.K + BK - 1) / BK;
+      const int total = num_m1 * num_n1 * num_kb1;
+      // stretches begin at every fourth block: a part shorter than that costs more to add to memory than to compute
+      const auto start = [&](int pair) {
+        const int v = pair < g.ahead ? pair * g.share_ahead : g.ahead * g.share_ahead + (pair - g.ahead) * g.share;
+        return min(total, v >> 8 & ~3);
+      };
+      at = start(group);
+      end = group + 1 < groups ? start(group + 1) : total;
+    }
+  }
+  __device__ __forceinline__ bool next(Segment& s) {
+    if (u < units) {
+      int t = u;
+      s.ks = 0;
+      if (kProblems == 1 && g.p[0].split_k > 1) {
+        t = u / g.p[0].split_k;
+        s.ks = u - t * g.p[0].split_k;
+      }
+      tile_of(t, num_m, num_n, g.p[0].band, s.tm, s.tn);
+      s.prob = 0;
+      s.kb0 = s.ks * kb_per;
+      s.kb1 = min(num_kb, s.kb0 + kb_per);
+      u += step;
+      return true;
+    }
+    if (kProblems == 2 && at < end) {
+      const int t = at / num_kb1;
+      s.prob = 1;
+      s.ks = 0;
+      s.kb0 = at - t * num_kb1;
+      s.kb1 = min(num_kb1, s.kb0 + end - at);
+      at += s.kb1 - s.kb0;
+      tile_of(t, num_m1, num_n1, g.p[1].band, s.tm, s.tn);
+      return true;
+    }
+    return false;
+  }
+};
+
+// Column sums of sum_x added to sum_out, by two warps of every CTA: 256 columns by a stretch of rows at a time, eight rows in flight.
+template <int kProblems>
+__device__ __forceinline__ void column_sums(const GemmLaunch<kProblems>& g, int warp, int lane) {
+  const int col_groups = (g.sum_cols + 255) / 256, warps = 2 * static_cast<int>(gridDim.x);
+  const int parts = max(1, min(warps / col_groups, g.sum_rows / 32)), per = (g.sum_rows + parts - 1) / parts;
+  for (int item = 2 * blockIdx.x + warp; item < col_groups * parts; item += warps) {
+    const int part = item / col_groups, col = (item - part * col_groups) * 256 + lane * 8;
+    const int r0 = part * per, r1 = min(g.sum_rows, r0 + per);
+    if (col >= g.sum_cols || r0 >= r1) continue;
+    F2 acc[4] = {f2_splat(0.f), f2_splat(0.f), f2_splat(0.f), f2_splat(0.f)};
+    const __nv_bfloat16* x = g.sum_x + col;
+    for (int r = r0; r < r1; r += 8) {
+      uint4 q[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) q[i] = r + i < r1 ? __ldg(reinterpret_cast<const uint4*>(x + static_cast<long long>(r + i) * g.sum_ld)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t w[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float lo, hi;
+          unpack_bf16x2(w[j], lo, hi);
+          acc[j] = f2_add(acc[j], f2_make(lo, hi));
+        }
+      }
+    }
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) f2_get(acc[j], v[2 * j], v[2 * j + 1]);
+    red_add_v4(g.sum_out + col, v[0], v[1], v[2], v[3]);
+    red_add_v4(g.sum_out + col + 4, v[4], v[5], v[6], v[7]);
+  }
+}
+
+constexpr int gemm_threads(int problems) { return kGemmThreads + (problems == 2 ? 64 : 0); }
+
+template <int kCG, int kBN, int kProblems>
+__global__ void __launch_bounds__(gemm_threads(kProblems), 1)
+gemm_bf16_kernel(const __grid_constant__ GemmLaunch<kProblems> g) {
+  const GemmParams& p = g.p[0];
   using Cfg = GemmCfg<kCG, kBN>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // 1024-byte alignment: the 128-byte swizzle pattern is a function of address bits [4,10). Dynamic shared memory starts so where a kernel has no
@@ -614,14 +725,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (warp == 0) {
     asm volatile("bar.arrive 1, %0;" ::"n"(kGemmThreads) : "memory");
     if (lane == 0) {
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
+      for (int i = 0; i < kProblems; ++i) {
+        tma_prefetch_desc(&g.a[i]);
+        tma_prefetch_desc(&g.b[i]);
+      }
     }
     __syncwarp();
-  } else {
+  } else if (warp < 2 + kEpiWarps) {
     if (warp == 2 && lane == 0) {
-      if (p.c_mode) tma_prefetch_desc(&tmC);
-      if (p.aux_tma) tma_prefetch_desc(&tmAux);
+      for (int i = 0; i < kProblems; ++i)
+        if (g.p[i].c_mode) tma_prefetch_desc(&g.c[i]);
+      if (p.aux_tma) tma_prefetch_desc(&g.aux);
     }
     if (warp == 1) {
       tmem_alloc<kCG>(tmem_slot, Cfg::TMEM_COLS);
@@ -633,7 +747,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
   if constexpr (kCG == 2) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if constexpr (kCG == 1) __syncthreads();        // one CTA: nothing to gain by starting its loads earlier
-  const uint32_t tmem_base = warp == 0 ? 0 : *tmem_slot;
+  const uint32_t tmem_base = warp == 0 || warp >= 2 + kEpiWarps ? 0 : *tmem_slot;
   if constexpr (kCG == 2)
     if (warp == 1 && lane == 0 && rank == 1) mbar_arrive_cluster(peer_bar, 0);
   // Programmatic dependent launch: everything above (barriers, descriptor prefetch, TMEM) touched
@@ -644,13 +758,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   pdl_launch_dependents();
 
   int m_eff = p.M, k_eff = p.K;
-  if (p.m_dyn) m_eff = max(0, min(p.M, *p.m_dyn));
-  if (p.k_dyn) k_eff = max(0, min(p.K, *p.k_dyn));
-  const int num_m = (m_eff + BM * kCG - 1) / (BM * kCG);
-  const int num_n = (p.N + kBN - 1) / kBN;
-  const int num_kb = (k_eff + BK - 1) / BK;
-  const int kb_per = (num_kb + p.split_k - 1) / p.split_k;
-  const int num_units = (num_kb > 0) ? num_m * num_n * p.split_k : 0;
+  if (kProblems == 1 && p.m_dyn) m_eff = max(0, min(p.M, *p.m_dyn));
+  if (kProblems == 1 && p.k_dyn) k_eff = max(0, min(p.K, *p.k_dyn));
+  Worklist<kCG, kBN, kProblems> work(g, group, num_groups, m_eff, k_eff);
+  Segment seg;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -658,15 +769,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      for (int u = group; u < num_units && ok; u += num_groups) {
-        const int ks = u % p.split_k;
-        int tm, tn;
-        tile_of(u / p.split_k, num_m, num_n, p.band, tm, tn);
-        const int m0 = tm * BM * kCG + static_cast<int>(rank) * BM;
-        const int n0 = tn * kBN + static_cast<int>(rank) * Cfg::BN_CTA;
-        const int kb0 = ks * kb_per;
-        const int kb1 = min(num_kb, kb0 + kb_per);
-        for (int kb = kb0; kb < kb1; ++kb) {
+      while (ok && work.next(seg)) {
+        const int prob = kProblems == 1 ? 0 : seg.prob;
+        const CUtensorMap *tmA = &g.a[prob], *tmB = &g.b[prob];
+        const int a_mn = g.p[prob].a_mn, b_mn = g.p[prob].b_mn;
+        const int m0 = seg.tm * BM * kCG + static_cast<int>(rank) * BM;
+        const int n0 = seg.tn * kBN + static_cast<int>(rank) * Cfg::BN_CTA;
+        for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
           ok = warp_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, kStatusWaitEmpty);
           if (!ok) break;
           uint8_t* sa = stage_base + s * Cfg::STAGE_BYTES;
@@ -677,17 +786,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               if constexpr (kCG == 1) tma_load_2d(to, map, &full_bar[s], x, y);
               else tma_load_2d_pair(to, map, &full_bar[s], x, y);
             };
-            if (!p.a_mn) {
-              load(sa, &tmA, kb * BK, m0);
+            if (!a_mn) {
+              load(sa, tmA, kb * BK, m0);
             } else {
-              load(sa, &tmA, m0, kb * BK);
-              load(sa + 8192, &tmA, m0 + 64, kb * BK);
+              load(sa, tmA, m0, kb * BK);
+              load(sa + 8192, tmA, m0 + 64, kb * BK);
             }
-            if (!p.b_mn) {
-              load(sb, &tmB, kb * BK, n0);
+            if (!b_mn) {
+              load(sb, tmB, kb * BK, n0);
             } else {
 #pragma unroll
-              for (int q = 0; q < Cfg::BN_CTA / 64; ++q) load(sb + q * 8192, &tmB, n0 + q * 64, kb * BK);
+              for (int q = 0; q < Cfg::BN_CTA / 64; ++q) load(sb + q * 8192, tmB, n0 + q * 64, kb * BK);
             }
           }
           __syncwarp();
@@ -698,37 +807,32 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (rank == 0) {
-      const uint32_t idesc = make_idesc_bf16(BM * kCG, kBN, p.a_mn, p.b_mn);
-      const uint32_t a_lbo = p.a_mn ? 8192u : 16u;
-      const uint32_t b_lbo = p.b_mn ? 8192u : 16u;
-      const uint32_t a_kstep = (p.a_mn ? 2048u : 32u) >> 4;
-      const uint32_t b_kstep = (p.b_mn ? 2048u : 32u) >> 4;
-      const uint32_t a_first = smem_desc_lo(smem_u32(stage_base), a_lbo), b_first = smem_desc_lo(smem_u32(stage_base) + Cfg::A_BYTES, b_lbo);
       const uint32_t hi = smem_desc_hi(1024);
       int s = 0;
       uint32_t ph = 0;
       int it = 0;
       bool ok = true;
       if constexpr (kCG == 2) ok = warp_wait(peer_bar, 0, abort_flag, p.status, kStatusWaitEpi);
-      for (int u = group; u < num_units && ok; u += num_groups, ++it) {
-        const int ks = u % p.split_k;
-        const int kb0 = ks * kb_per;
-        const int kb1 = min(num_kb, kb0 + kb_per);
+      for (; ok && work.next(seg); ++it) {
+        const int a_mn = g.p[kProblems == 1 ? 0 : seg.prob].a_mn, b_mn = g.p[kProblems == 1 ? 0 : seg.prob].b_mn;
+        const uint32_t idesc = make_idesc_bf16(BM * kCG, kBN, a_mn, b_mn);
+        const uint32_t a_kstep = (a_mn ? 2048u : 32u) >> 4, b_kstep = (b_mn ? 2048u : 32u) >> 4;
+        const uint32_t a_first = smem_desc_lo(smem_u32(stage_base), a_mn ? 8192u : 16u), b_first = smem_desc_lo(smem_u32(stage_base) + Cfg::A_BYTES, b_mn ? 8192u : 16u);
         const int acc = it & 1;
         ok = warp_wait(&tempty_bar[acc], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kStatusWaitEpi);
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * kBN;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
           ok = warp_wait(&full_bar[s], ph, abort_flag, p.status, kStatusWaitFull);
           if (!ok) break;
           tc_fence_after_sync();
-          FB_TIMELINE_ONLY(if (p.ts && it == 0 && kb == kb0) p.ts[blockIdx.x * 8 + 2] = clock64();)
+          FB_TIMELINE_ONLY(if (p.ts && it == 0 && kb == seg.kb0) p.ts[blockIdx.x * 8 + 2] = clock64();)
           const uint32_t a_lo = a_first + s * (Cfg::STAGE_BYTES >> 4), b_lo = b_first + s * (Cfg::STAGE_BYTES >> 4);
           if (elect_one()) {
 #pragma unroll
             for (int k4 = 0; k4 < BK / 16; ++k4)
-              umma_bf16<kCG>(d_tmem, desc_of(a_lo + k4 * a_kstep, hi), desc_of(b_lo + k4 * b_kstep, hi), idesc, (kb > kb0 || k4 > 0) ? 1u : 0u);
+              umma_bf16<kCG>(d_tmem, desc_of(a_lo + k4 * a_kstep, hi), desc_of(b_lo + k4 * b_kstep, hi), idesc, (kb > seg.kb0 || k4 > 0) ? 1u : 0u);
             if constexpr (kCG == 1) umma_commit(&empty_bar[s]);
             else umma_commit_pair(&empty_bar[s], 3);
           }
@@ -744,6 +848,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         FB_TIMELINE_ONLY(if (p.ts && it == 0) p.ts[blockIdx.x * 8 + 3] = clock64();)
       }
     }
+  } else if (kProblems == 2 && warp >= 2 + kEpiWarps) {
+    if (g.sum_out) column_sums(g, warp - 2 - kEpiWarps, lane);
   } else {
     // ------------------------------------------------------------------ epilogue warps
     // What bounds a tile of a short reduction (K = 768: 6.1k cycles of products) is this part, so it is kept below that: 64 columns come out
@@ -766,14 +872,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     int aux_u = group, aux_c = 0;           // where the next load of pre-activations starts (lane 0)
     uint32_t aux_issued = 0;
     const auto load_aux = [&] {             // the next 64 columns of this warp's rows, into the staging tile whose turn it is
-      for (; aux_u < num_units; aux_u += num_groups, aux_c = 0) {
+      for (; aux_u < work.units; aux_u += num_groups, aux_c = 0) {
         int tm, tn;
-        tile_of(aux_u, num_m, num_n, p.band, tm, tn);
+        tile_of(aux_u, work.num_m, work.num_n, p.band, tm, tn);
         const int col = tn * kBN + half * kSplit + aux_c;
         if (aux_c >= cols || col >= p.N) continue;
         const uint32_t b = aux_issued++ & 1;
         mbar_expect_tx(&w.aux_bar[b], 4096);
-        tma_load_2d(w.stage[b], &tmAux, &w.aux_bar[b], col, tm * BM * kCG + static_cast<int>(rank) * BM + q * 32);
+        tma_load_2d(w.stage[b], &g.aux, &w.aux_bar[b], col, tm * BM * kCG + static_cast<int>(rank) * BM + q * 32);
         aux_c += 64;
         return;
       }
@@ -783,23 +889,22 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       load_aux();
     }
     // Thread i of the four warps of a half keeps column i's bias of the tile to come.
-    const bool staged_bias = kStaged && p.bias != nullptr && p.kind != kEpiDirect;
+    const bool staged_bias = kStaged && kProblems == 1 && p.bias != nullptr && p.kind != kEpiDirect;
     const auto bias_of = [&](int u) -> float {
       int tm, tn;
-      tile_of(u / p.split_k, num_m, num_n, p.band, tm, tn);
+      tile_of(u / p.split_k, work.num_m, work.num_n, p.band, tm, tn);
       const int c = q * 32 + lane, col = tn * kBN + half * kSplit + c;
-      if (u >= num_units || c >= cols || col >= p.N) return 0.f;
+      if (u >= work.units || c >= cols || col >= p.N) return 0.f;
       return p.bias_fp32 ? __ldg(static_cast<const float*>(p.bias) + col) : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col]);
     };
     float next_bias = staged_bias ? bias_of(group) : 0.f;
     int it = 0;
     bool ok = true;
-    for (int u = group; u < num_units; u += num_groups, ++it) {
-      const int ks = u % p.split_k;
-      int tm, tn;
-      tile_of(u / p.split_k, num_m, num_n, p.band, tm, tn);
-      const int row0 = tm * BM * kCG + static_cast<int>(rank) * BM + q * 32;
-      const int ncol0 = tn * kBN + half * kSplit;
+    for (; work.next(seg); ++it) {
+      const GemmParams& pp = g.p[kProblems == 1 ? 0 : seg.prob];
+      const CUtensorMap& tmC = g.c[kProblems == 1 ? 0 : seg.prob];
+      const int row0 = seg.tm * BM * kCG + static_cast<int>(rank) * BM + q * 32;
+      const int ncol0 = seg.tn * kBN + half * kSplit;
       const int acc = it & 1;
       uint32_t bias = 0;
       if (staged_bias) {
@@ -809,8 +914,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         slice[q * 32 + lane] = next_bias;
         if (half) asm volatile("bar.sync 3, 128;" ::: "memory");
         else asm volatile("bar.sync 2, 128;" ::: "memory");
-        next_bias = bias_of(u + num_groups);
-        if (ks == 0) bias = smem_u32(slice);
+        next_bias = bias_of(work.u);
+        if (seg.ks == 0) bias = smem_u32(slice);
       }
       if (ok) ok = warp_wait(&tfull_bar[acc], (it >> 1) & 1, abort_flag, p.status, kStatusWaitAccum);
       if (!ok) continue;
@@ -826,17 +931,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       };
       if constexpr (kStaged) {
-        const int chunks = ncol0 >= p.N ? 0 : (min(cols, p.N - ncol0) + 63) / 64;
+        const int chunks = ncol0 >= pp.N ? 0 : (min(cols, pp.N - ncol0) + 63) / 64;
         const auto run = [&](auto kind) {
-          ok = epilogue_tile<decltype(kind)::value>(p, tmC, tmAux, w, taddr, ncol0, row0, chunks, bias, abort_flag, hand_back, load_aux);
+          ok = epilogue_tile<decltype(kind)::value>(pp, tmC, g.aux, w, taddr, ncol0, row0, chunks, bias, abort_flag, hand_back, load_aux);
         };
-        if (p.kind != kEpiDirect) {
+        if (pp.kind != kEpiDirect) {
           if (chunks == 0) hand_back();
-          else if (p.kind == kEpiPlain) run(std::integral_constant<int, kEpiPlain>());
-          else if (p.kind == kEpiF32) epilogue_tile_f32(p, tmC, w, taddr, ncol0, row0, min(cols, p.N - ncol0), bias, hand_back);
-          else if (p.kind == kEpiGelu) run(std::integral_constant<int, kEpiGelu>());
-          else if (p.kind == kEpiGeluAux) run(std::integral_constant<int, kEpiGeluAux>());
-          else if (p.kind == kEpiDgelu) run(std::integral_constant<int, kEpiDgelu>());
+          else if (pp.kind == kEpiPlain) run(std::integral_constant<int, kEpiPlain>());
+          else if (pp.kind == kEpiF32) epilogue_tile_f32(pp, tmC, w, taddr, ncol0, row0, min(cols, pp.N - ncol0), bias, hand_back);
+          else if (pp.kind == kEpiGelu) run(std::integral_constant<int, kEpiGelu>());
+          else if (pp.kind == kEpiGeluAux) run(std::integral_constant<int, kEpiGeluAux>());
+          else if (pp.kind == kEpiDgelu) run(std::integral_constant<int, kEpiDgelu>());
           else run(std::integral_constant<int, kEpiDgeluTanh>());
           continue;
         }
@@ -846,7 +951,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         uint32_t v[32];
         tmem_ld32(taddr + c, v);
         tmem_ld_wait();
-        epilogue_store32(p, v, row0 + lane, ncol0 + c, ks == 0);
+        epilogue_store32(pp, v, row0 + lane, ncol0 + c, seg.ks == 0);
       }
       hand_back();
       FB_TIMELINE_ONLY(if (p.ts && it == 0 && warp == 2 && lane == 0) p.ts[blockIdx.x * 8 + 5] = clock64();)
@@ -1138,20 +1243,14 @@ static int make_tmap_out(CUtensorMap* out, const void* base, uint64_t cols, uint
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
-template <int kCG, int kBN>
-static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tx, const GemmParams& p,
-                       cudaStream_t stream) {
+template <int kCG, int kBN, int kProblems>
+static int launch_gemm(const GemmLaunch<kProblems>& g, int groups, cudaStream_t stream) {
   using Cfg = GemmCfg<kCG, kBN>;
-  auto kern = gemm_bf16_kernel<kCG, kBN>;
-  if (const cudaError_t e = allow_smem<gemm_bf16_kernel<kCG, kBN>>(Cfg::SMEM_BYTES)) return static_cast<int>(e);
-  const int num_m = (p.M + BM * kCG - 1) / (BM * kCG);
-  const int num_n = (p.N + kBN - 1) / kBN;
-  const int units = num_m * num_n * p.split_k;
-  int groups = sm_count() / kCG;
-  if (units < groups) groups = units;
+  auto kern = gemm_bf16_kernel<kCG, kBN, kProblems>;
+  if (const cudaError_t e = allow_smem<gemm_bf16_kernel<kCG, kBN, kProblems>>(Cfg::SMEM_BYTES)) return static_cast<int>(e);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(groups * kCG, 1, 1);
-  cfg.blockDim = dim3(kGemmThreads, 1, 1);
+  cfg.blockDim = dim3(gemm_threads(kProblems), 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -1166,9 +1265,30 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = 2;
   }
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, tx, p);
-  return static_cast<int>(e);
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, g));
 }
+template <int kCG, int kBN>
+static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tx, const GemmParams& p, cudaStream_t stream) {
+  GemmLaunch<1> g;
+  std::memset(&g, 0, sizeof(g));
+  g.a[0] = ta; g.b[0] = tb; g.c[0] = tc; g.aux = tx; g.p[0] = p;
+  const int units = ((p.M + BM * kCG - 1) / (BM * kCG)) * ((p.N + kBN - 1) / kBN) * p.split_k;
+  return launch_gemm<kCG, kBN, 1>(g, units < sm_count() / kCG ? units : sm_count() / kCG, stream);
+}
+
+// Bands of at most 12 column tiles: the pairs at work at one time then share about as many column as row panels of the operands (row tiles fastest,
+// all read one column's), and rows are read from HBM once where they used to be again for every column. 24576 x 768 x 3072 109 -> 95 us, 24576 x 3072 x 768
+// with GELU 129 -> 114, 8192 x 2048 x 512 (dX) 18.7 -> 17.7; bands of 8 or 16 are within 1 % of these.
+static int band_of(int N, int tile) {
+  const int tiles = (N + tile - 1) / tile, bands = (tiles + 11) / 12;
+  return (tiles + bands - 1) / bands;
+}
+
+// Whether dX and dW of a linear layer go out as one launch (fb_gemm_backward). Us against dX, dW and db on two streams, rows x n x k: 4096 x 768 x 768
+// 15.9 (19.5), 4096 x 768 x 3072 with GELU' 39.2 (47.7), 4096 x 3072 x 768 33.3 (39.5), 8192 x 512 x 512 15.6 (20.6), 2048 x 512 x 512 8.5 (11.2), 512 x 128 x 128
+// 6.2 (10.2). Not for few rows, whose dX has few tiles and whose dW has little to sum per tile (77 x 768 x 768 12.7 against 10.9), nor for a dX of few
+// tiles with a long reduction, which others split over a cluster (1024 x 3072 x 768 19.4 against 17.1, 768 x 3072 x 768 19.2 against 21.7).
+static bool backward_in_one(int rows, int n, int tiles0) { return rows >= 256 && (n < 2304 || tiles0 > 12); }
 
 static cudaLaunchConfig_t split_config(int M, int N, cudaLaunchAttribute* attr, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
@@ -1346,19 +1466,15 @@ extern "C" int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, in
   p.bias = bias; p.bias_fp32 = bias_fp32; p.epi = epi; p.aux = aux; p.ldaux = ldaux; p.alpha = alpha;
   p.accumulate = accumulate; p.split_k = split_k; p.status = status; p.ts = ts;
   p.m_dyn = m_dyn; p.k_dyn = k_dyn;
-  // Bands of at most 12 column tiles: the pairs at work at one time then share about as many column as row panels of the operands (row tiles fastest,
-  // all read one column's), and rows are read from HBM once where they used to be again for every column. 24576 x 768 x 3072 109 -> 95 us, 24576 x 3072 x 768
-  // with GELU 129 -> 114, 8192 x 2048 x 512 (dX) 18.7 -> 17.7; bands of 8 or 16 are within 1 % of these.
-  const int col_tiles = (N + bn - 1) / bn, bands = (col_tiles + 11) / 12;
-  p.band = (col_tiles + bands - 1) / bands;
+  p.band = band_of(N, bn);
   if (over_pairs) return launch_split(ta, tb, tc, tx, p, stream);
   switch (config) {
-    case 0: return launch_gemm<2, 256>(ta, tb, tc, tx, p, stream);
-    case 1: return launch_gemm<1, 256>(ta, tb, tc, tx, p, stream);
-    case 2: return launch_gemm<1, 128>(ta, tb, tc, tx, p, stream);
-    case 4: return launch_gemm<1, 192>(ta, tb, tc, tx, p, stream);
-    case 5: return launch_gemm<2, 192>(ta, tb, tc, tx, p, stream);
-    default: return launch_gemm<1, 64>(ta, tb, tc, tx, p, stream);
+    case 0: return launch_one<2, 256>(ta, tb, tc, tx, p, stream);
+    case 1: return launch_one<1, 256>(ta, tb, tc, tx, p, stream);
+    case 2: return launch_one<1, 128>(ta, tb, tc, tx, p, stream);
+    case 4: return launch_one<1, 192>(ta, tb, tc, tx, p, stream);
+    case 5: return launch_one<2, 192>(ta, tb, tc, tx, p, stream);
+    default: return launch_one<1, 64>(ta, tb, tc, tx, p, stream);
   }
 }
 
@@ -1382,4 +1498,54 @@ extern "C" int fb_gemm_bf16_grouped(const void* A, const void* const* B, void* C
     if (r) return r;
   }
   return 0;
+}
+
+// The gradients of y = x W^T + b from dY in one launch: dX = dY W (times the activation's derivative at `aux`, the pre-activation that x came from,
+// with `epi`), dW += dY^T x, db += column sums of dY (db may be null). dY [rows, n], W [n, k], x [rows, k] bf16; dX bf16; dW, db fp32.
+// Returns -7 where two launches serve better or the layout does not fit: nothing has been launched then.
+//
+// dX comes in whole 256 x 256 tiles, one or two to a pair of SMs, which alone leave up to half the pairs idle at the end; dW's reduction can be
+// cut anywhere, for its parts are added to memory, so it fills what dX leaves: each pair's share of dW's K blocks makes its total the same. One launch
+// also has one start-up and one draining end instead of three of each, and leaves the stream's chain of programmatic launches whole.
+extern "C" int fb_gemm_backward(const void* dY, const void* W, const void* X, void* dX, float* dW, float* db, int rows, int n, int k, long long ldy,
+                                long long ldw, long long ldx, long long lddx, long long lddw, int epi, const void* aux, long long ldaux, int* status,
+                                void* stream_) {
+  using namespace fb;
+  const auto aligned = [](const void* q, long long ld, int esz) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && (ld * esz) % 16 == 0; };
+  if (rows <= 0 || n <= 0 || k <= 0) return -7;
+  if (!aligned(dY, ldy, 2) || !aligned(W, ldw, 2) || !aligned(X, ldx, 2) || !aligned(dX, lddx, 2) || !aligned(dW, lddw, 4)) return -7;
+  if (db && ((reinterpret_cast<uintptr_t>(db) & 15) || n % 8)) return -7;
+  const bool dgelu = epi == FB_EPI_DGELU_ERF || epi == FB_EPI_DGELU_TANH;
+  if (dgelu ? !aux || !aligned(aux, ldaux, 2) : epi != FB_EPI_NONE) return -7;
+  int pairs = sm_count() / 2;
+  const int tiles0 = ((rows + 255) / 256) * ((k + 255) / 256), tiles1 = ((n + 255) / 256) * ((k + 255) / 256);
+  const int kb0 = (n + BK - 1) / BK, kb1 = (rows + BK - 1) / BK;
+  if (!backward_in_one(rows, n, tiles0)) return -7;
+  if (tiles1 * static_cast<long long>(kb1) > (1 << 22)) return -7;       // shares are counted in 1/256 of a block
+  if (const int most = tiles0 + tiles1 * kb1 / 4; most < pairs) pairs = most > 0 ? most : 1;
+
+  GemmLaunch<2> g;
+  std::memset(&g, 0, sizeof(g));
+  int r;
+  if ((r = make_tmap_bf16_2d(&g.a[0], dY, n, rows, ldy, BK, BM)) || (r = make_tmap_bf16_2d(&g.b[0], W, k, n, ldw, 64, BK)) ||
+      (r = make_tmap_bf16_2d(&g.a[1], dY, n, rows, ldy, 64, BK)) || (r = make_tmap_bf16_2d(&g.b[1], X, k, rows, ldx, 64, BK)) ||
+      (r = make_tmap_out(&g.c[0], dX, k, rows, lddx, false)) || (r = make_tmap_out(&g.c[1], dW, k, n, lddw, true)))
+    return r;
+  if (dgelu && (r = make_tmap_out(&g.aux, aux, k, rows, ldaux, false))) return r;
+  GemmParams& p = g.p[0];
+  p.M = rows; p.N = k; p.K = n; p.a_mn = 0; p.b_mn = 1; p.C = dX; p.ldc = lddx; p.epi = epi; p.aux = const_cast<void*>(aux); p.ldaux = ldaux;
+  p.split_k = 1; p.c_mode = 1; p.aux_tma = dgelu ? 2 : 0; p.kind = !dgelu ? kEpiPlain : epi == FB_EPI_DGELU_ERF ? kEpiDgelu : kEpiDgeluTanh;
+  p.band = band_of(k, 256); p.status = status;
+  GemmParams& q = g.p[1];
+  q.M = n; q.N = k; q.K = rows; q.a_mn = 1; q.b_mn = 1; q.C = dW; q.ldc = lddw; q.c_fp32 = 1; q.accumulate = 1; q.split_k = 1; q.c_mode = 2;
+  q.kind = kEpiF32; q.band = band_of(k, 256); q.status = status;
+  // Shares in K blocks of 64, which a pair's products take 530 cycles for; a tile of dX costs its epilogue on top, or that alone where it is the longer.
+  const int cost = (dgelu ? (kb0 > 15 ? kb0 : 15) : kb0) + 3;
+  const long long total = static_cast<long long>(tiles1) * kb1;
+  g.ahead = tiles0 % pairs;
+  const long long rest = pairs - g.ahead, level = g.ahead ? cost : 0;
+  g.share_ahead = total > rest * level ? static_cast<int>((total - rest * level) * 256 / pairs) : 0;
+  g.share = static_cast<int>((total * 256 - static_cast<long long>(g.ahead) * g.share_ahead) / rest);
+  g.sum_x = static_cast<const __nv_bfloat16*>(dY); g.sum_out = db; g.sum_rows = rows; g.sum_cols = n; g.sum_ld = ldy;
+  return launch_gemm<2, 256, 2>(g, pairs, static_cast<cudaStream_t>(stream_));
 }

@@ -302,6 +302,22 @@ def _bias_grad(dy2: torch.Tensor, b: torch.Tensor, alpha=None, rows_dyn=None):
     return tmp.to(b.dtype)
 
 
+def _backward_in_one(dy2: torch.Tensor, w16: torch.Tensor, x2: torch.Tensor, dx2: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], epi: int = 0,
+                     aux: Optional[torch.Tensor] = None) -> bool:
+    """dX (times the activation's derivative at `aux`), dW and db of a linear layer as one launch, the latter two into their gradient slots.
+    False where they have none or the kernel does not take the sizes: nothing has been done then."""
+    slot, bslot = _grad_slot(w), _grad_slot(b)
+    if slot is None or (b is not None and bslot is None):
+        return False
+    if not _C().gemm_backward(dy2, w16, x2, dx2, slot.view(dy2.shape[1], x2.shape[1]), None if b is None else bslot.view(-1), epi, aux):
+        return False
+    _launched()
+    _touched(w)
+    if b is not None:
+        _touched(b)
+    return True
+
+
 # ----------------------------------------------------------------------------------------- linear
 class _LinearFn(torch.autograd.Function):
     @staticmethod
@@ -331,6 +347,10 @@ class _LinearFn(torch.autograd.Function):
             _launched()
         dy2 = _as_operand(dy2)
         dx = dw = db = None
+        if ctx.needs_input_grad[0] and ctx.needs_input_grad[1] and (b is None or ctx.needs_input_grad[2]):
+            dx2 = _new_rows(x2.shape[0], x2.shape[1], BF16, dy.device)
+            if _backward_in_one(dy2, w16, x2, dx2, w, b):
+                return dx2.view(ctx.xshape), None, None, None
         fork = _Fork(dy.device, dy2.shape[0] * dy2.shape[1] * x2.shape[1])
         with fork:
             if ctx.needs_input_grad[1]:
@@ -436,6 +456,19 @@ class _FeedForwardFn(torch.autograd.Function):
         dy2 = _as_operand(dy.reshape(-1, N))
         M, F1 = a.shape
         dpre = _new_rows(M, F1, BF16, dy.device)
+        if ctx.needs_input_grad[0] and ctx.needs_input_grad[1] and ctx.needs_input_grad[3] and all(
+                p is None or ctx.needs_input_grad[i] for i, p in ((2, b1), (4, b2))) and _backward_in_one(dy2, w2s, a, dpre, w2, b2, _DEPI[ctx.act], h_pre):
+            dx2 = _new_rows(M, x2.shape[1], BF16, dy.device)
+            if _backward_in_one(dpre, w1s, x2, dx2, w1, b1):
+                return dx2.view(ctx.xshape), None, None, None, None, None
+            fork = _Fork(dy.device, M * F1 * x2.shape[1])
+            with fork:
+                dw1 = _weight_grad(dpre, x2, w1)
+                db1 = _bias_grad(dpre, b1) if b1 is not None else None
+            C.gemm(dpre, w1s, dx2, False, True)
+            _launched()
+            fork.join()
+            return dx2.view(ctx.xshape), dw1, db1, None, None, None
         fork = _Fork(dy.device, M * F1 * N)
         with fork:       # the second layer's parameter gradients need only dy: beside the d(pre-activation) GEMM
             dw2 = _weight_grad(dy2, a, w2) if ctx.needs_input_grad[3] else None

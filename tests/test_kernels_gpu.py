@@ -123,6 +123,42 @@ def test_gemm_staged_epilogues(C, config, M, N, K, pad, bias):
         close(dpre, lin * x.grad, lin.abs() + 1)
 
 
+@pytest.mark.parametrize("rows,n,k,epi,bias", [(4096, 768, 768, 0, True), (3054, 768, 3072, 2, True), (2500, 2304, 768, 0, False), (8192, 520, 1032, 4, True),
+                                               (20000, 264, 256, 0, True), (1030, 2056, 264, 0, True), (3400, 2312, 264, 0, True), (256, 8, 8, 0, True)])
+def test_linear_gradients_in_one_launch(C, rows, n, k, epi, bias):
+    """dX, dW and db from one launch where tiles are ragged and the pairs' shares of dW start anywhere in a tile. dX is rounded to bf16 once (and the
+    activation's derivative takes the hardware's tanh: 3e-4); dW and db are fp32 sums of exact products."""
+    torch.manual_seed(rows + n)
+    dy, w, x = (torch.randn(s, device="cuda").bfloat16() for s in ((rows, n), (n, k), (rows, k)))
+    dy, w = dy * 0.1, w / math.sqrt(n)
+    aux = torch.randn(rows, k, device="cuda").bfloat16() if epi else None
+    dx = torch.empty(rows, k, device="cuda", dtype=torch.bfloat16)
+    dw, db = torch.randn(n, k, device="cuda"), torch.randn(n, device="cuda")
+    want_dw, want_db = dw.double() + dy.double().t() @ x.double(), db.double() + dy.double().sum(0)
+    lin = want = dy.double() @ w.double()
+    if epi:
+        h = aux.double().requires_grad_()
+        F.gelu(h, approximate="none" if epi == 2 else "tanh").sum().backward()
+        want = lin * h.grad
+    C.clear_status(0)
+    assert C.gemm_backward(dy, w, x, dx, dw, db if bias else None, epi, aux)
+    assert C.read_status(0) == 0
+    assert ((dx.double() - want).abs() <= want.abs() * 2.0 ** -8 + (3e-4 if epi else 0) * (lin.abs() + 1) + 1e-5).all()
+    # fp32 sums over `rows` terms: a few ulp of the sum of magnitudes
+    assert ((dw.double() - want_dw).abs() <= 2.0 ** -20 * (dy.double().abs().t() @ x.double().abs() + 8)).all()
+    if bias:
+        assert ((db.double() - want_db).abs() <= 2.0 ** -20 * (dy.double().abs().sum(0) + 8)).all()
+
+
+def test_linear_gradients_in_one_launch_are_refused_where_they_do_not_fit(C):
+    dy, w, x = (torch.randn(s, device="cuda").bfloat16() for s in ((2048, 1024), (1024, 1024), (2048, 1024)))
+    dx, dw, db = torch.zeros_like(x), torch.zeros(1024, 1024, device="cuda"), torch.zeros(1028, device="cuda")
+    assert not C.gemm_backward(dy, w, x, dx, dw, db[1:1025])                                        # sums go out sixteen bytes at a time
+    assert not C.gemm_backward(dy, w, x, torch.zeros(2048, 1028, device="cuda", dtype=torch.bfloat16)[:, 4:], dw)
+    assert not C.gemm_backward(dy[:64], w, x[:64], dx[:64], dw)                                     # too little work
+    assert not dx.any() and not dw.any() and not db.any()
+
+
 def test_gemm_fp32_out_accumulate_splitk_alpha(C):
     M, N, K = 256, 384, 1024
     torch.manual_seed(1)
