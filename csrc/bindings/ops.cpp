@@ -130,7 +130,8 @@ void gemm_grouped(const Tensor& a, const std::vector<Tensor>& bs, Tensor& out, c
 }
 
 // dx = dy w (times the activation's derivative at aux), dw += dy^T x, db += column sums of dy, in one launch; false: not taken, nothing done.
-bool gemm_backward(const Tensor& dy, const Tensor& w, const Tensor& x, Tensor& dx, Tensor& dw, const OptTensor& db, int epi, const OptTensor& aux) {
+bool gemm_backward(const Tensor& dy, const Tensor& w, const Tensor& x, Tensor& dx, Tensor& dw, const OptTensor& db, int epi, const OptTensor& aux,
+                   const OptTensor& alpha) {
   want_cuda(dy, "dy");
   c10::cuda::CUDAGuard guard(dy.device());
   for (const Tensor* t : {&dy, &w, &x, static_cast<const Tensor*>(&dx)})
@@ -140,9 +141,10 @@ bool gemm_backward(const Tensor& dy, const Tensor& w, const Tensor& x, Tensor& d
   TORCH_CHECK(dw.is_cuda() && dw.scalar_type() == at::kFloat && dw.dim() == 2 && dw.size(0) == n && dw.size(1) == k && dw.stride(1) == 1, "dw must be fp32 [n, k]");
   if (db.has_value()) TORCH_CHECK(db->is_cuda() && db->scalar_type() == at::kFloat && db->numel() == n && db->is_contiguous(), "db must be fp32 [n]");
   if (aux.has_value()) TORCH_CHECK(aux->is_cuda() && is_bf16(*aux) && aux->dim() == 2 && aux->stride(1) == 1 && aux->size(0) == rows && aux->size(1) == k, "aux must be bf16 [rows, k]");
+  if (alpha.has_value()) TORCH_CHECK(alpha->is_cuda() && alpha->scalar_type() == at::kFloat && alpha->numel() == 1, "alpha must be one fp32");
   const int rc = fb_gemm_backward(dy.data_ptr(), w.data_ptr(), x.data_ptr(), dx.data_ptr(), dw.data_ptr<float>(), db.has_value() ? db->data_ptr<float>() : nullptr,
                                   (int)rows, (int)n, (int)k, dy.stride(0), w.stride(0), x.stride(0), dx.stride(0), dw.stride(0), epi,
-                                  aux.has_value() ? aux->data_ptr() : nullptr, aux.has_value() ? aux->stride(0) : 0,
+                                  aux.has_value() ? aux->data_ptr() : nullptr, aux.has_value() ? aux->stride(0) : 0, ptr<const float>(alpha),
                                   status_word(dy.get_device()).data_ptr<int>(), stream_of(dy));
   if (rc == -7) return false;
   check(rc, "fb_gemm_backward");
@@ -321,8 +323,15 @@ void gather_rows(const Tensor& x, const Tensor& idx, const Tensor& counts, Tenso
 void scatter_rows(const Tensor& dxc, const Tensor& idx, const Tensor& counts, Tensor& dx) {
   want_float_kind(dxc, "dxc");
   c10::cuda::CUDAGuard guard(dxc.device());
-  TORCH_CHECK(dx.dim() == 2 && dxc.dim() == 2 && dx.stride(1) == 1 && dxc.stride(1) == 1 && dx.sizes() == dxc.sizes() && dx.scalar_type() == dxc.scalar_type());
+  TORCH_CHECK(dx.dim() == 2 && dxc.dim() == 2 && dx.stride(1) == 1 && dxc.stride(1) == 1 && dx.sizes() == dxc.sizes());
+  TORCH_CHECK(dx.scalar_type() == dxc.scalar_type() || (is_bf16(dx) && dxc.scalar_type() == at::kFloat), "scatter_rows: rows of one type, or fp32 to bf16");
   TORCH_CHECK(idx.scalar_type() == at::kInt && idx.numel() == dx.size(0) && counts.scalar_type() == at::kInt && counts.numel() == 2);
+  if (dx.scalar_type() != dxc.scalar_type()) {
+    check(fb_scatter_rows_f32(dxc.data_ptr<float>(), dxc.stride(0), idx.data_ptr<int>(), counts.data_ptr<int>(), dx.data_ptr(), dx.stride(0), (int)dx.size(0),
+                              (int)dx.size(1), stream_of(dx)),
+          "fb_scatter_rows_f32");
+    return;
+  }
   check(fb_scatter_rows(dxc.data_ptr(), dxc.stride(0), idx.data_ptr<int>(), counts.data_ptr<int>(), dx.data_ptr(), dx.stride(0), (int)dx.size(0),
                         (int)dx.size(1), is_bf16(dx), stream_of(dx)),
         "fb_scatter_rows");
@@ -697,7 +706,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gelu_bwd", &gelu_bwd);
   m.def("dropout", &dropout, py::arg("x"), py::arg("p"), py::arg("seed"), py::arg("seed_dev") = py::none());
   m.def("gemm_backward", &gemm_backward, py::arg("dy"), py::arg("w"), py::arg("x"), py::arg("dx"), py::arg("dw"), py::arg("db") = py::none(),
-        py::arg("epi") = 0, py::arg("aux") = py::none());
+        py::arg("epi") = 0, py::arg("aux") = py::none(), py::arg("alpha") = py::none());
   m.def("colsum", &colsum, py::arg("x"), py::arg("out"), py::arg("rows_dyn") = py::none());
   m.def("compact_targets", &compact_targets);
   m.def("gather_rows", &gather_rows);

@@ -110,9 +110,9 @@ int fb_gelu_bwd(const void* dy, const void* x, void* dx, long long n, int tanh_a
 int fb_dropout(const void* x, void* y, long long n, float p, unsigned long long seed, const unsigned long long* seed_dev,
                int is_bf16, void* stream);
 /* Gradients of y = x W^T + b in one launch: dX = dY W (times the activation's derivative at `aux` with epi 2 or 4), dW += dY^T x, db += column sums
- * of dY (db may be null). bf16 operands and dX, fp32 dW and db. -7: not taken (size or alignment), nothing launched. */
+ * of dY (db may be null), all times *alpha (may be null). bf16 operands and dX, fp32 dW and db. -7: not taken (size or alignment), nothing launched. */
 int fb_gemm_backward(const void* dY, const void* W, const void* X, void* dX, float* dW, float* db, int rows, int n, int k, long long ldy, long long ldw,
-                     long long ldx, long long lddx, long long lddw, int epi, const void* aux, long long ldaux, int* status, void* stream);
+                     long long ldx, long long lddx, long long lddw, int epi, const void* aux, long long ldaux, const float* alpha, int* status, void* stream);
 /* out[c] += sum over rows of x[r][c] (the caller zeroes `out`, or passes a gradient slot to accumulate into). */
 int fb_colsum(const void* x, float* out, int rows, int cols, long long ld, int is_bf16, void* stream);
 /* As fb_colsum over the first min(rows, *rows_dyn) rows (device-side count). */
@@ -126,6 +126,8 @@ int fb_compact_targets(const long long* targets, int rows, long long ignore_inde
 int fb_gather_rows(const void* x, long long ld, const int* idx, const int* counts, void* xc, long long ldc, int rows,
                    int cols, int is_bf16, void* stream);
 /* dx[idx[i]] = dxc[i] for i < counts[0]; dx must be zeroed by the caller. */
+int fb_scatter_rows_f32(const float* dxc, long long ldc, const int* idx, const int* counts, void* dx, long long ld, int rows, int cols,
+                        void* stream);   /* fp32 rows to bf16 ones; widths and strides multiples of 8 */
 int fb_scatter_rows(const void* dxc, long long ldc, const int* idx, const int* counts, void* dx, long long ld, int rows,
                     int cols, int is_bf16, void* stream);
 int fb_embedding_bwd(const void* dy, const long long* ids, float* dw, long long tokens, int dim, long long vocab,

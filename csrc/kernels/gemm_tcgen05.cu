@@ -655,7 +655,10 @@ __device__ __forceinline__ void column_sums(const GemmLaunch<kProblems>& g, int 
     }
     float v[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) f2_get(acc[j], v[2 * j], v[2 * j + 1]);
+    for (int j = 0; j < 4; ++j) {
+      if (g.p[0].alpha) acc[j] = f2_mul(acc[j], f2_splat(__ldg(g.p[0].alpha)));
+      f2_get(acc[j], v[2 * j], v[2 * j + 1]);
+    }
     red_add_v4(g.sum_out + col, v[0], v[1], v[2], v[3]);
     red_add_v4(g.sum_out + col + 4, v[4], v[5], v[6], v[7]);
   }
@@ -1288,7 +1291,11 @@ static int band_of(int N, int tile) {
 // 15.9 (19.5), 4096 x 768 x 3072 with GELU' 39.2 (47.7), 4096 x 3072 x 768 33.3 (39.5), 8192 x 512 x 512 15.6 (20.6), 2048 x 512 x 512 8.5 (11.2), 512 x 128 x 128
 // 6.2 (10.2). Not for few rows, whose dX has few tiles and whose dW has little to sum per tile (77 x 768 x 768 12.7 against 10.9), nor for a dX of few
 // tiles with a long reduction, which others split over a cluster (1024 x 3072 x 768 19.4 against 17.1, 768 x 3072 x 768 19.2 against 21.7).
-static bool backward_in_one(int rows, int n, int tiles0) { return rows >= 256 && (n < 2304 || tiles0 > 12); }
+// Nor where a tile of dX alone (`chain` K blocks) takes longer than a pair's share of everything (`share`), when that is long: the caller splits its
+// reduction (2048 x 32000 x 512 187 against 153, 4096 x 32000 x 512 207 against 255).
+static bool backward_in_one(int rows, int n, int tiles0, long long chain, long long share) {
+  return rows >= 256 && (n < 2304 || tiles0 > 12) && (n < 6400 || chain * 4 <= share * 5);
+}
 
 static cudaLaunchConfig_t split_config(int M, int N, cudaLaunchAttribute* attr, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
@@ -1504,12 +1511,14 @@ extern "C" int fb_gemm_bf16_grouped(const void* A, const void* const* B, void* C
 // with `epi`), dW += dY^T x, db += column sums of dY (db may be null). dY [rows, n], W [n, k], x [rows, k] bf16; dX bf16; dW, db fp32.
 // Returns -7 where two launches serve better or the layout does not fit: nothing has been launched then.
 //
+// All three times *alpha (may be null).
+//
 // dX comes in whole 256 x 256 tiles, one or two to a pair of SMs, which alone leave up to half the pairs idle at the end; dW's reduction can be
 // cut anywhere, for its parts are added to memory, so it fills what dX leaves: each pair's share of dW's K blocks makes its total the same. One launch
 // also has one start-up and one draining end instead of three of each, and leaves the stream's chain of programmatic launches whole.
 extern "C" int fb_gemm_backward(const void* dY, const void* W, const void* X, void* dX, float* dW, float* db, int rows, int n, int k, long long ldy,
-                                long long ldw, long long ldx, long long lddx, long long lddw, int epi, const void* aux, long long ldaux, int* status,
-                                void* stream_) {
+                                long long ldw, long long ldx, long long lddx, long long lddw, int epi, const void* aux, long long ldaux,
+                                const float* alpha, int* status, void* stream_) {
   using namespace fb;
   const auto aligned = [](const void* q, long long ld, int esz) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && (ld * esz) % 16 == 0; };
   if (rows <= 0 || n <= 0 || k <= 0) return -7;
@@ -1520,7 +1529,11 @@ extern "C" int fb_gemm_backward(const void* dY, const void* W, const void* X, vo
   int pairs = sm_count() / 2;
   const int tiles0 = ((rows + 255) / 256) * ((k + 255) / 256), tiles1 = ((n + 255) / 256) * ((k + 255) / 256);
   const int kb0 = (n + BK - 1) / BK, kb1 = (rows + BK - 1) / BK;
-  if (!backward_in_one(rows, n, tiles0)) return -7;
+  // Work is counted in K blocks of 64, which a pair's products take 530 cycles for; a tile of dX costs its epilogue on top, or that alone where it is
+  // the longer.
+  const int cost = (dgelu ? (kb0 > 15 ? kb0 : 15) : kb0) + 3;
+  if (!backward_in_one(rows, n, tiles0, static_cast<long long>((tiles0 + pairs - 1) / pairs) * cost, (static_cast<long long>(tiles0) * cost + static_cast<long long>(tiles1) * kb1) / pairs))
+    return -7;
   if (tiles1 * static_cast<long long>(kb1) > (1 << 22)) return -7;       // shares are counted in 1/256 of a block
   if (const int most = tiles0 + tiles1 * kb1 / 4; most < pairs) pairs = most > 0 ? most : 1;
 
@@ -1535,12 +1548,11 @@ extern "C" int fb_gemm_backward(const void* dY, const void* W, const void* X, vo
   GemmParams& p = g.p[0];
   p.M = rows; p.N = k; p.K = n; p.a_mn = 0; p.b_mn = 1; p.C = dX; p.ldc = lddx; p.epi = epi; p.aux = const_cast<void*>(aux); p.ldaux = ldaux;
   p.split_k = 1; p.c_mode = 1; p.aux_tma = dgelu ? 2 : 0; p.kind = !dgelu ? kEpiPlain : epi == FB_EPI_DGELU_ERF ? kEpiDgelu : kEpiDgeluTanh;
-  p.band = band_of(k, 256); p.status = status;
+  p.band = band_of(k, 256); p.status = status; p.alpha = alpha;
   GemmParams& q = g.p[1];
+  q.alpha = alpha;
   q.M = n; q.N = k; q.K = rows; q.a_mn = 1; q.b_mn = 1; q.C = dW; q.ldc = lddw; q.c_fp32 = 1; q.accumulate = 1; q.split_k = 1; q.c_mode = 2;
   q.kind = kEpiF32; q.band = band_of(k, 256); q.status = status;
-  // Shares in K blocks of 64, which a pair's products take 530 cycles for; a tile of dX costs its epilogue on top, or that alone where it is the longer.
-  const int cost = (dgelu ? (kb0 > 15 ? kb0 : 15) : kb0) + 3;
   const long long total = static_cast<long long>(tiles1) * kb1;
   g.ahead = tiles0 % pairs;
   const long long rest = pairs - g.ahead, level = g.ahead ? cost : 0;

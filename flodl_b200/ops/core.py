@@ -303,13 +303,13 @@ def _bias_grad(dy2: torch.Tensor, b: torch.Tensor, alpha=None, rows_dyn=None):
 
 
 def _backward_in_one(dy2: torch.Tensor, w16: torch.Tensor, x2: torch.Tensor, dx2: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], epi: int = 0,
-                     aux: Optional[torch.Tensor] = None) -> bool:
+                     aux: Optional[torch.Tensor] = None, alpha: Optional[torch.Tensor] = None) -> bool:
     """dX (times the activation's derivative at `aux`), dW and db of a linear layer as one launch, the latter two into their gradient slots.
     False where they have none or the kernel does not take the sizes: nothing has been done then."""
     slot, bslot = _grad_slot(w), _grad_slot(b)
     if slot is None or (b is not None and bslot is None):
         return False
-    if not _C().gemm_backward(dy2, w16, x2, dx2, slot.view(dy2.shape[1], x2.shape[1]), None if b is None else bslot.view(-1), epi, aux):
+    if not _C().gemm_backward(dy2, w16, x2, dx2, slot.view(dy2.shape[1], x2.shape[1]), None if b is None else bslot.view(-1), epi, aux, alpha):
         return False
     _launched()
     _touched(w)
@@ -707,6 +707,10 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
         alpha = g.detach().float().reshape(1)
         n_dyn = None if counts is None else counts[0:1]
         dx = dw = db = None
+        if counts is None and ctx.needs_input_grad[0] and ctx.needs_input_grad[1] and (b is None or ctx.needs_input_grad[2]):
+            dx2 = _new_rows(x2.shape[0], x2.shape[1], BF16, dl.device)
+            if _backward_in_one(dl, w16, x2, dx2, w, b, alpha=alpha):
+                return dx2.view(ctx.xshape), None, None, None, None, None
         fork = _Fork(dl.device, dl.shape[0] * dl.shape[1] * x2.shape[1])
         with fork:
             if ctx.needs_input_grad[1]:
@@ -714,14 +718,25 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
             if b is not None and ctx.needs_input_grad[2]:
                 db = _bias_grad(dl, b, alpha=alpha, rows_dyn=n_dyn)
         if ctx.needs_input_grad[0]:
-            dx2 = _new_rows(x2.shape[0], x2.shape[1], BF16, dl.device)
-            C.gemm(dl, w16, dx2, False, True, alpha=alpha, m_dyn=n_dyn)
+            rows, K = x2.shape
+            # Few rows (of a masked-LM batch about a sixth is labelled) make few tiles and the vocabulary a long reduction: that is split until every
+            # pair of SMs has a part, summed in fp32.
+            tiles = math.ceil((rows if counts is None else max(1, rows // 6)) / 256) * math.ceil(K / 256)
+            split = min(74 // tiles, dl.shape[1] // 1024)
+            if split > 1:
+                dx2 = torch.zeros(rows, K, dtype=torch.float32, device=dl.device)
+                C.gemm(dl, w16, dx2, False, True, alpha=alpha, accumulate=True, split_k=split, config=0, m_dyn=n_dyn)
+            else:
+                dx2 = _new_rows(rows, K, BF16, dl.device)
+                C.gemm(dl, w16, dx2, False, True, alpha=alpha, m_dyn=n_dyn)
             _launched()
             if counts is not None:
-                full = torch.zeros_like(dx2)
+                full = torch.zeros(rows, K, dtype=BF16, device=dl.device)
                 C.scatter_rows(dx2, idx, counts, full)
                 _launched(2)
                 dx2 = full
+            elif split > 1:
+                dx2 = dx2.to(BF16)
             dx = dx2.view(ctx.xshape)
         fork.join()
         return dx, dw, db, None, None, None

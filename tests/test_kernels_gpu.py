@@ -150,6 +150,29 @@ def test_linear_gradients_in_one_launch(C, rows, n, k, epi, bias):
         assert ((db.double() - want_db).abs() <= 2.0 ** -20 * (dy.double().abs().sum(0) + 8)).all()
 
 
+@pytest.mark.parametrize("rows,V,K,sparse", [(1024, 4104, 200, True), (4096, 8200, 768, True), (1500, 3000, 264, False), (4096, 8200, 264, False)])
+def test_linear_cross_entropy_gradients_with_few_rows(monkeypatch, rows, V, K, sparse):
+    """The projection's dX, whose reduction over the vocabulary is split where rows make few tiles, and its dW and db. dX is rounded to bf16 once from
+    gradients of the logits that are rounded to bf16 (2^-8 each; their errors add like independent ones over V terms)."""
+    from flodl_b200 import ops
+    from flodl_b200.ops import core
+    monkeypatch.setitem(core._EAGER, "min_numel", 0)      # the native kernels at every size, as in a captured step
+    torch.manual_seed(V)
+    x = torch.randn(rows, K, device="cuda").bfloat16().requires_grad_()
+    w = (torch.randn(V, K, device="cuda") * 0.05).bfloat16().requires_grad_()
+    b = torch.randn(V, device="cuda").requires_grad_()
+    t = torch.randint(0, V, (rows,), device="cuda")
+    if sparse:
+        t[torch.rand(rows, device="cuda") < 0.85] = -100
+    w._fb_grad, b._fb_grad = torch.zeros(V, K, device="cuda"), torch.zeros(V, device="cuda")
+    (3.0 * ops.linear_cross_entropy(x, w, b, t, -100, sparse)).backward()
+    xd, wd, bd = (v.detach().double().requires_grad_() for v in (x, w, b))
+    (3.0 * F.cross_entropy(xd @ wd.t() + bd, t, ignore_index=-100)).backward()
+    for got, want in ((x.grad, xd.grad), (w._fb_grad, wd.grad), (b._fb_grad, bd.grad)):
+        assert (got.double() - want).norm() <= 0.01 * want.norm()
+    assert sparse is False or (x.grad[t == -100] == 0).all()
+
+
 def test_linear_gradients_in_one_launch_are_refused_where_they_do_not_fit(C):
     dy, w, x = (torch.randn(s, device="cuda").bfloat16() for s in ((2048, 1024), (1024, 1024), (2048, 1024)))
     dx, dw, db = torch.zeros_like(x), torch.zeros(1024, 1024, device="cuda"), torch.zeros(1028, device="cuda")
