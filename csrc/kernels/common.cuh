@@ -110,14 +110,20 @@ __device__ __forceinline__ uint4 philox4x32(uint2 key, uint4 ctr) {
   return ctr;
 }
 
+// A value is kept where u = (w >> 8) / 2^24 >= p, that is where w >= ceil(p 2^24) 2^8 (2^32, which no word reaches, from p = 1 on): compared as it
+// is, a word costs neither the conversion to float, which the special-function unit does, nor a product.
+__device__ __forceinline__ bool dropout_keeps(uint32_t w, float p) {
+  const float t = ceilf(p * 16777216.f);
+  return t < 16777216.f && w >= (static_cast<uint32_t>(fmaxf(t, 0.f)) << 8);
+}
+
 // Keep-mask for element `idx` of a dropout site: deterministic in (seed, idx), so forward and
 // backward agree without storing the mask. Returns 1/(1-p) for kept elements, 0 for dropped.
 __device__ __forceinline__ float dropout_scale(uint64_t seed, uint64_t idx, float p, float inv_keep) {
   uint4 r = philox4x32(make_uint2(static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32)),
                        make_uint4(static_cast<uint32_t>(idx >> 2), static_cast<uint32_t>(idx >> 34), 0u, 0u));
   const uint32_t w = (idx & 3) == 0 ? r.x : (idx & 3) == 1 ? r.y : (idx & 3) == 2 ? r.z : r.w;
-  const float u = (w >> 8) * (1.0f / 16777216.0f);
-  return u >= p ? inv_keep : 0.f;
+  return dropout_keeps(w, p) ? inv_keep : 0.f;
 }
 // Four consecutive elements starting at a multiple of 4.
 __device__ __forceinline__ void dropout_scale4(uint64_t seed, uint64_t idx4, float p, float inv_keep, float (&s)[4]) {
@@ -125,7 +131,7 @@ __device__ __forceinline__ void dropout_scale4(uint64_t seed, uint64_t idx4, flo
                        make_uint4(static_cast<uint32_t>(idx4 >> 2), static_cast<uint32_t>(idx4 >> 34), 0u, 0u));
   const uint32_t w[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
-  for (int i = 0; i < 4; ++i) s[i] = ((w[i] >> 8) * (1.0f / 16777216.0f)) >= p ? inv_keep : 0.f;
+  for (int i = 0; i < 4; ++i) s[i] = dropout_keeps(w[i], p) ? inv_keep : 0.f;
 }
 
 

@@ -150,6 +150,17 @@ def test_linear_gradients_in_one_launch(C, rows, n, k, epi, bias):
         assert ((db.double() - want_db).abs() <= 2.0 ** -20 * (dy.double().abs().sum(0) + 8)).all()
 
 
+def test_dropout_keeps_what_its_threshold_says(C):
+    """One draw per value: what a larger p keeps, a smaller one keeps too, in shares of 1 - p (within six standard deviations), also at the ends."""
+    x, n = torch.ones(1 << 22, device="cuda"), 1 << 22
+    kept = {p: C.dropout(x, p, 11, None) != 0 for p in (0.0, 1e-8, 2.0 ** -24, 0.1, 0.5, 0.9, 1 - 2.0 ** -24)}
+    ps = sorted(kept)
+    for a, b in zip(ps, ps[1:]):
+        assert not (kept[b] & ~kept[a]).any()
+    for p in ps:
+        assert abs(kept[p].sum().item() - n * (1 - p)) <= 6 * math.sqrt(n * p * (1 - p)) + 1
+
+
 @pytest.mark.parametrize("rows,V,K,sparse", [(1024, 4104, 200, True), (4096, 8200, 768, True), (1500, 3000, 264, False), (4096, 8200, 264, False)])
 def test_linear_cross_entropy_gradients_with_few_rows(monkeypatch, rows, V, K, sparse):
     """The projection's dX, whose reduction over the vocabulary is split where rows make few tiles, and its dW and db. dX is rounded to bf16 once from
