@@ -3,7 +3,7 @@
 //
 // Backward: one CTA per (key block of 128 rows, head, batch) walks the query blocks that see it. K, V and the dK / dV
 // accumulators stay put; Q and dO stream through a three-stage TMA ring. Roles: 16 softmax warps (thread = one query row x
-// 32 keys), 4 warps that drain dQ, one that adds it to the scratch, one MMA issuer, one TMA producer. S and dP of the next query
+// 32 keys), 4 warps that drain dQ, two that add it to the scratch in turn, one MMA issuer, one producer (TMA and row statistics). S and dP of the next query
 // block are issued as soon as the softmax warps have loaded this block's into registers, so the tensor cores work under the exponentials.
 // A query block's dQ is a sum over key blocks, i.e. over CTAs: it is added into an fp32 scratch with bulk reductions, in the order of
 // the key blocks, so that two calls give the same bits. The scratch is not row-major: within the 32 rows a warp owns, 16-byte chunk c of
@@ -13,9 +13,9 @@
 // What bounds it: the chain scores -> exponentials -> P and dS in shared memory -> products of one tile, with the shared-memory
 // pipe (P and dS are written once and read by three products) as its slowest part. The fixed order costs a causal head's first CTAs, which start
 // together, about 4 us for each block between them (from the end of one's additions to the start of the next one's).
-// Forward + backward, bf16, us; in brackets the backward with additions in order of arrival: B 2 x H 12 x S 4096 causal 99 + 275 (252), full
-// 204 + 490 (496), B 4 x H 8 x S 1024 causal 20 + 45 (37), B 6 x H 12 x S 509 causal 13 + 33 (31), B 32 x H 8 x S 256 causal 14 + 46 (47),
-// B 64 x H 12 x S 384 78 + 275 (262). Eight softmax warps, reductions from registers and persistent CTAs took 338 at 4096 causal.
+// Backward, bf16, us; in brackets with one adding thread, the row statistics behind the dQ staging area and one value per instruction: B 2 x H 12 x
+// S 4096 causal 205 (276), full 358 (496), B 4 x H 8 x S 1024 causal 40 (47), B 6 x H 12 x S 509 with a mask 38 (43), B 32 x H 8 x S 256 causal 44 (47),
+// B 64 x H 12 x S 384 with a mask 255 (280).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -38,7 +38,7 @@ namespace {
 
 constexpr int kBwdStages = 3;
 constexpr int kBwdSoftmaxWarps = 16;
-constexpr int kBwdThreads = 32 * (kBwdSoftmaxWarps + 4 + 3);
+constexpr int kBwdThreads = 32 * (kBwdSoftmaxWarps + 4 + 4);
 
 struct BwdLong {
   static constexpr int Q = 0;                                   // kBwdStages x 16 KB
@@ -172,8 +172,8 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint64_t* dq_full = grads_full + 1;             // [2] the same event, per dQ buffer, for the draining warps
   uint64_t* dq_free = dq_full + 2;                // [2] the buffer has been read
   uint64_t* stat_full = dq_free + 2;              // [2] lse and D of a query block are in shared memory
-  uint64_t* staged = stat_full + 2;               // dQ of a query block is in shared memory
-  uint64_t* stage_free = staged + 1;              // ... and has been read from there
+  uint64_t* staged = stat_full + 2;               // [2] dQ of a query block is in shared memory
+  uint64_t* stage_free = staged + 2;              // ... and has been read from there
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stage_free + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* item = abort_flag + 1;            // key block, head, batch: reloaded where needed, the softmax warps have no registers to spare
@@ -199,8 +199,7 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     mbar_init(sdp_free, kBwdSoftmaxWarps);
     mbar_init(pds_ready, kBwdSoftmaxWarps);
     mbar_init(grads_full, 1);
-    for (int s = 0; s < 2; ++s) { mbar_init(&dq_full[s], 1); mbar_init(&dq_free[s], 4); mbar_init(&stat_full[s], 4); }
-    mbar_init(staged, 4);
+    for (int s = 0; s < 2; ++s) { mbar_init(&dq_full[s], 1); mbar_init(&dq_free[s], 4); mbar_init(&stat_full[s], 1); mbar_init(&staged[s], 4); }
     mbar_init(stage_free, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -229,15 +228,38 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tma_load_4d(smem + L::V, &tmV, kv_full, 0, j * kBlk, h, b);
     }
     __syncwarp();
-    for (int it = 0; it < n; ++it) {
+    // The row statistics go with them, a block later: their two buffers are free when the ring has a stage again, which block it - 3 left. (Where the
+    // warps that drain dQ loaded them, behind the staging area that frees up with the additions, they reached the softmax warps 2000 cycles late.)
+    const long long bh = static_cast<long long>(b) * p.H + h;
+    float2 ahead[4];
+    for (int it = 0; it <= n; ++it) {
       const int st = it % kBwdStages;
       if (!warp_wait(&q_empty[st], ((it / kBwdStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitEmpty)) break;
-      if (elect_one()) {
+      if (it < n && elect_one()) {
         mbar_expect_tx(&q_full[st], 32768);
         tma_load_4d(smem + L::Q + st * 16384, &tmQ, &q_full[st], 0, query_block(it) * kBlk, h, b);
         tma_load_4d(smem + L::DO + st * 16384, &tmDO, &q_full[st], 0, query_block(it) * kBlk, h, b);
       }
       __syncwarp();
+      if (it > 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {      // (the arithmetic here: next to the loads it would wait for them)
+          // a row beyond S, or one that no key takes part in, gets +inf: every probability of it is then 2^-inf = 0
+          const float l = ahead[i].x == -INFINITY ? INFINITY : ahead[i].x * kLog2e;
+          stats[((it - 1) & 1) * 128 + i * 32 + lane] = make_float2(l, ahead[i].y * p.scale);
+        }
+        arrive_warp(&stat_full[(it - 1) & 1], lane);
+      }
+      if (it == n) break;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int q = query_block(it) * kBlk + i * 32 + lane;
+        ahead[i] = make_float2(-INFINITY, 0.f);
+        if (q < p.S) {
+          ahead[i].x = __ldg(lse + bh * p.S + q);
+          ahead[i].y = __ldcg(&reinterpret_cast<const DqSlot*>(dq + b * p.gsb + h * p.gsh + q * p.gss)->D);
+        }
+      }
     }
   } else if (warp == kBwdSoftmaxWarps + 4) {
     // ------------------------------------------------------------------ MMA issuer
@@ -294,18 +316,19 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       __syncwarp();
     }
-  } else if (warp == kBwdSoftmaxWarps + 6) {
+  } else if (warp >= kBwdSoftmaxWarps + 6) {
     // ------------------------------------------------------------------ dQ into the scratch
-    // One thread adds a query block's 128 rows at once. A sum of three or more depends on its order, so the third and later key blocks wait
+    // One thread adds a query block's 128 rows at once; two of them take turns, so that one block's additions, which the next key block waits for the
+    // end of, do not hold up the next block's. A sum of three or more depends on its order, so the third and later key blocks wait
     // for the ones before them; the first two may come either way round, 0 + a + b being 0 + b + a.
     if (lane == 0) {
       const int j = item[0], h = item[1], b = item[2];
       const uint32_t src = smem_u32(smem + L::DQ);
-      for (int it = 0; it < n; ++it) {
+      for (int it = warp - kBwdSoftmaxWarps - 6; it < n; it += 2) {
         const int qblk = query_block(it), row0 = qblk * kBlk, adders = p.causal ? qblk + 1 : nblk;
         unsigned int* added = &reinterpret_cast<DqSlot*>(dq + b * p.gsb + h * p.gsh + row0 * p.gss)->added;
-        if (!mbar_wait(staged, it & 1, abort_flag, p.status, kStatusWaitAccum)) break;
         if (j >= 2 && !wait_added(added, static_cast<unsigned int>(j), abort_flag, p.status)) break;
+        if (!mbar_wait(&staged[it & 1], (it >> 1) & 1, abort_flag, p.status, kStatusWaitAccum)) break;
         bulk_add(dq_accum + ((static_cast<long long>(b) * p.H + h) * p.S + row0) * kHD, src, min(kBlk, p.S - row0) * kHD * 4);
         tma_store_commit();
         tma_store_wait_read();
@@ -318,51 +341,31 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
     }
   } else if (warp >= kBwdSoftmaxWarps) {
-    // ------------------------------------------------------------------ row statistics in, dQ out
-    const int quarter = warp & 3, t = quarter * 32 + lane, h = item[1], b = item[2];
-    const long long bh = static_cast<long long>(b) * p.H + h;
-    auto load_stats = [&](int it) {
-      const int q = query_block(it) * kBlk + t;
-      // a row beyond S, or one that no key takes part in, gets +inf: every probability of it is then 2^-inf = 0
-      float l = INFINITY, D = 0.f;
-      if (q < p.S) {
-        l = __ldg(lse + bh * p.S + q);
-        l = l == -INFINITY ? INFINITY : l * kLog2e;
-        D = __ldcg(&reinterpret_cast<const DqSlot*>(dq + b * p.gsb + h * p.gsh + q * p.gss)->D);
-      }
-      return make_float2(l, D);
-    };
-    auto put_stats = [&](int it, float2 ld) {
-      stats[(it & 1) * 128 + t] = ld;
-      arrive_warp(&stat_full[it & 1], lane);
-    };
-    put_stats(0, load_stats(0));
-    if (n > 1) put_stats(1, load_stats(1));
+    // ------------------------------------------------------------------ dQ out
+    const int quarter = warp & 3;
     const uint32_t stage = smem_u32(smem + L::DQ) + quarter * 8192;
     for (int it = 0; it < n; ++it) {
       const int qb = it & 1;
-      const float2 ahead = it + 2 < n ? load_stats(it + 2) : make_float2(0.f, 0.f);
       bool ok = mbar_wait(&dq_full[qb], (it >> 1) & 1, abort_flag, p.status, kStatusWaitAccum);
-      ok = ok && (it == 0 || mbar_wait(stage_free, (it - 1) & 1, abort_flag, p.status, kStatusWaitEpi));
       if (!__all_sync(0xffffffffu, ok)) break;
       tc_fence_after_sync();
-      // 16-byte chunk c of this warp's row r at (c * rows + r) * 16, as in the scratch
-      const int nr = min(32, p.S - query_block(it) * kBlk - quarter * 32);
-#pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        uint32_t v[32];
-        tmem_ld32(tDQ + qb * 64 + half * 32 + (static_cast<uint32_t>(quarter * 32) << 16), v);
-        tmem_ld_wait();
-        if (lane < nr) {
-#pragma unroll
-          for (int c = 0; c < 8; ++c) st_shared_v4(stage + ((half * 8 + c) * nr + lane) * 16, make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]));
-        }
-      }
+      // out of TMEM before the staging area is free: the next but one block's products need not wait for that
+      uint32_t v[2][32];
+      tmem_ld64_sync(tDQ + qb * 64 + (static_cast<uint32_t>(quarter * 32) << 16), v[0], v[1]);
       tc_fence_before_sync();
       arrive_warp(&dq_free[qb], lane);
+      if (it > 0 && !warp_wait(stage_free, (it - 1) & 1, abort_flag, p.status, kStatusWaitEpi)) break;
+      // 16-byte chunk c of this warp's row r at (c * rows + r) * 16, as in the scratch
+      const int nr = min(32, p.S - query_block(it) * kBlk - quarter * 32);
+      if (lane < nr) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            st_shared_v4(stage + ((half * 8 + c) * nr + lane) * 16, make_uint4(v[half][4 * c], v[half][4 * c + 1], v[half][4 * c + 2], v[half][4 * c + 3]));
+      }
       fence_proxy_async_smem();
-      arrive_warp(staged, lane);
-      if (it + 2 < n) put_stats(it + 2, ahead);   // every softmax thread has read buffer it & 1: its P and dS went into these products
+      arrive_warp(&staged[it & 1], lane);
     }
   } else {
     // ------------------------------------------------------------------ softmax: thread = query row t x 32 keys
@@ -403,7 +406,12 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
       } else {
 #pragma unroll
-        for (int e = 0; e < 32; ++e) sv[e] = __float_as_uint(ex2_approx(__uint_as_float(sv[e]) * sc - ld.x));
+        for (int e = 0; e < 32; e += 2) {
+          float lo, hi;
+          f2_get(f2_fma(f2_make(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), f2_splat(sc), f2_splat(-ld.x)), lo, hi);
+          sv[e] = __float_as_uint(ex2_approx(lo));
+          sv[e + 1] = __float_as_uint(ex2_approx(hi));
+        }
       }
       if (diagonal) {
 #pragma unroll
@@ -421,13 +429,26 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const float pe = __uint_as_float(sv[e + k]);
-            dpv[e + k] = __float_as_uint(pe * (__uint_as_float(dpv[e + k]) * z[k] - ld.y) * p.scale);
+            dpv[e + k] = __float_as_uint(pe * fmaf(__uint_as_float(dpv[e + k]) * z[k], p.scale, -ld.y));
             sv[e + k] = __float_as_uint(pe * z[k]);
           }
         }
       } else {
 #pragma unroll
-        for (int e = 0; e < 32; ++e) dpv[e] = __float_as_uint(__uint_as_float(sv[e]) * (__uint_as_float(dpv[e]) - ld.y) * p.scale);
+        for (int e = 0; e < 32; e += 2) {
+          const F2 d = f2_fma(f2_make(__uint_as_float(dpv[e]), __uint_as_float(dpv[e + 1])), f2_splat(p.scale), f2_splat(-ld.y));
+          float lo, hi;
+          f2_get(f2_mul(f2_make(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), d), lo, hi);
+          dpv[e] = __float_as_uint(lo);
+          dpv[e + 1] = __float_as_uint(hi);
+        }
+      }
+      // As they are stored, before the wait: the compiler would leave the arithmetic behind it, where nothing overlaps it.
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        sv[e] = pack2(__uint_as_float(sv[2 * e]), __uint_as_float(sv[2 * e + 1]));
+        dpv[e] = pack2(__uint_as_float(dpv[2 * e]), __uint_as_float(dpv[2 * e + 1]));
+        asm volatile("" : "+r"(sv[e]), "+r"(dpv[e]));
       }
       if (it > 0) {        // the previous block's products have read P and dS
         ok = __all_sync(0xffffffffu, mbar_wait(grads_full, (it - 1) & 1, abort_flag, p.status, kStatusWaitAccum));
@@ -435,11 +456,8 @@ attn_bwd_long_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
 #pragma unroll
       for (int g8 = 0; g8 < 4; ++g8) {
-        float pr[8], ds[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) { pr[e] = __uint_as_float(sv[8 * g8 + e]); ds[e] = __uint_as_float(dpv[8 * g8 + e]); }
-        st_shared_v4(swz_chunk(pp, t, (part & 1) * 4 + g8), pack8(pr));
-        st_shared_v4(swz_chunk(dp, t, (part & 1) * 4 + g8), pack8(ds));
+        st_shared_v4(swz_chunk(pp, t, (part & 1) * 4 + g8), make_uint4(sv[4 * g8], sv[4 * g8 + 1], sv[4 * g8 + 2], sv[4 * g8 + 3]));
+        st_shared_v4(swz_chunk(dp, t, (part & 1) * 4 + g8), make_uint4(dpv[4 * g8], dpv[4 * g8 + 1], dpv[4 * g8 + 2], dpv[4 * g8 + 3]));
       }
       fence_proxy_async_smem();
       arrive_warp(pds_ready, lane);
