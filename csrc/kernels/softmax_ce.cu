@@ -41,20 +41,39 @@ struct RowSplit {
 };
 
 // Maximum and sum of exponentials relative to it, over a stream of values; -inf values (and rows of nothing else) add nothing.
+// exp(v - base) of two values: the difference first, then the power of two, as for one.
+__device__ __forceinline__ F2 f2_exp_from(F2 v, F2 minus_base) {
+  float lo, hi;
+  f2_get(f2_mul(f2_add(v, minus_base), f2_splat(1.4426950408889634f)), lo, hi);
+  return f2_make(ex2_approx(lo), ex2_approx(hi));
+}
 struct OnlineSum {
-  float m = -INFINITY, s = 0.f;
+  float m = -INFINITY;
+  F2 s2 = f2_splat(0.f);
+  __device__ __forceinline__ void reach(float vm) {
+    if (vm > m) {
+      s2 = f2_mul(s2, f2_splat(__expf(m - vm)));
+      m = vm;
+    }
+  }
   template <int N>
   __device__ __forceinline__ void add(const float (&v)[N]) {
     float vm = v[0];
 #pragma unroll
     for (int j = 1; j < N; ++j) vm = fmaxf(vm, v[j]);
-    if (vm > m) {
-      s *= __expf(m - vm);
-      m = vm;
-    }
-    const float base = m == -INFINITY ? 0.f : m;
+    reach(vm);
+    const F2 minus = f2_splat(m == -INFINITY ? 0.f : -m);
 #pragma unroll
-    for (int j = 0; j < N; ++j) s += __expf(v[j] - base);
+    for (int j = 0; j < N; j += 2) s2 = f2_add(s2, f2_exp_from(f2_make(v[j], v[j + 1]), minus));
+  }
+  __device__ __forceinline__ void add(float v) {
+    reach(v);
+    s2 = f2_add(s2, f2_make(__expf(v - (m == -INFINITY ? 0.f : m)), 0.f));
+  }
+  __device__ __forceinline__ float sum() const {
+    float lo, hi;
+    f2_get(s2, lo, hi);
+    return lo + hi;
   }
 };
 // A sum without a maximum is 0, or NaN if all its values were NaN, and stays what it is.
@@ -63,10 +82,10 @@ __device__ __forceinline__ float sum_rebased(float s, float m, float to) { retur
 // One row per block or, for short rows, per warp. The row is read twice, for the statistics and for the gradient, and written once. What bounds it is
 // HBM where the second read finds the row in L2, so that a row's threads times the resident blocks' rows decide: few threads to a row keep the
 // barrier and the exponentials of one row behind the loads of others, but put more rows in flight; long rows then leave L2 between their reads.
-// us for a mean loss with its gradient; in brackets a 256-thread block per row that takes rows off a 16-byte boundary value by value, and
-// 512-thread (up to 64 KB 256-thread) blocks striding over the rows:
-//   bf16 4843 x 392 9.9 (13.3, 10.4), 4000 x 3000 18.9 (19.8, 19.0), 8192 x 8000 73.5 (72.7, 88.5), 8192 x 32000 238 (266, 255), 4096 x 50304 in place
-//   199 (214, 206), 2048 x 128000 256 (294, 266); fp32 8192 x 4000 55.5 (64.0, 75.8), 2094 x 23544 79 (107, 88), 4096 x 30522 187 (396, 220).
+// Exponentials (two a value) and issue slots are not far behind, so the arithmetic goes two values an instruction and the target is looked for once
+// per vector. us for a mean loss with its gradient; in brackets one value an instruction, before that a 256-thread block per row:
+//   bf16 4000 x 3000 17.5 (20.3, 19.8), 8192 x 8000 64.5 (74.2, 72.7), 4096 x 32000 114 (126), 8192 x 32000 219 (238, 266), 2048 x 50304 88 (103);
+//   fp32 8192 x 4000 57.1 (56.6, 64.0), 2094 x 23544 81 (81, 107), 4096 x 30522 181 (187, 396).
 // kUnroll vectors in flight per thread, kBlocks blocks of kThreads on an SM.
 template <typename T, bool kWarpRow, int kThreads, int kBlocks, int kUnroll>
 __global__ void __launch_bounds__(kThreads, kBlocks)
@@ -106,8 +125,8 @@ ce_fwd_kernel(const T* __restrict__ logits, long long ld, const long long* __res
   if constexpr (kWarpRow) __syncwarp();
 
   OnlineSum acc;
-  for (int k = me; k < sp.head; k += step) { const float v[1] = {VecIO<T>::get(lr + k)}; acc.add(v); }
-  for (int k = sp.tail + me; k < V; k += step) { const float v[1] = {VecIO<T>::get(lr + k)}; acc.add(v); }
+  for (int k = me; k < sp.head; k += step) acc.add(VecIO<T>::get(lr + k));
+  for (int k = sp.tail + me; k < V; k += step) acc.add(VecIO<T>::get(lr + k));
   const T* body = lr + sp.head;
   int i = me;
   for (; i + (kUnroll - 1) * step < sp.nvec; i += kUnroll * step) {
@@ -123,7 +142,7 @@ ce_fwd_kernel(const T* __restrict__ logits, long long ld, const long long* __res
     acc.add(v);
   }
   float gmax = warp_max(acc.m);
-  float gsum = warp_sum(sum_rebased(acc.s, acc.m, gmax));
+  float gsum = warp_sum(sum_rebased(acc.sum(), acc.m, gmax));
   if constexpr (!kWarpRow) {
     __shared__ float red_m[kWarps], red_s[kWarps];
     if (lane == 0) { red_m[warp] = gmax; red_s[warp] = gsum; }
@@ -138,6 +157,24 @@ ce_fwd_kernel(const T* __restrict__ logits, long long ld, const long long* __res
   const float inv_n = count_inv ? count_inv[1] : 1.f, inv_sum = 1.f / gsum;
   T* dbody = dr + sp.head;
   auto grad = [&](float x, int k) { return (__expf(x - gmax) * inv_sum - (k == t ? 1.f : 0.f)) * inv_n; };
+  // a vector's: two values an instruction, and the target looked for once per vector
+  const F2 minus = f2_splat(-gmax), scale = f2_splat(inv_sum * inv_n);
+  const int t_vec = t >= sp.head && t < sp.tail ? static_cast<int>(t - sp.head) / VEC : -1, t_at = static_cast<int>(t - sp.head) % VEC;
+  auto grads = [&](float (&v)[VEC], int vec) {
+    float x_target = 0.f;
+    if (vec == t_vec) {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j)
+        if (j == t_at) x_target = v[j];
+    }
+#pragma unroll
+    for (int j = 0; j < VEC; j += 2) f2_get(f2_mul(f2_exp_from(f2_make(v[j], v[j + 1]), minus), scale), v[j], v[j + 1]);
+    if (vec == t_vec) {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j)
+        if (j == t_at) v[j] = (__expf(x_target - gmax) * inv_sum - 1.f) * inv_n;
+    }
+  };
   for (int k = me; k < sp.head; k += step) VecIO<T>::put(dr + k, grad(VecIO<T>::get(lr + k), k));
   for (int k = sp.tail + me; k < V; k += step) VecIO<T>::put(dr + k, grad(VecIO<T>::get(lr + k), k));
   i = me;
@@ -147,16 +184,14 @@ ce_fwd_kernel(const T* __restrict__ logits, long long ld, const long long* __res
     for (int u = 0; u < kUnroll; ++u) VecIO<T>::load(body + static_cast<long long>(i + u * step) * VEC, v[u]);
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
-#pragma unroll
-      for (int j = 0; j < VEC; ++j) v[u][j] = grad(v[u][j], sp.head + (i + u * step) * VEC + j);
+      grads(v[u], i + u * step);
       VecIO<T>::store(dbody + static_cast<long long>(i + u * step) * VEC, v[u]);
     }
   }
   for (; i < sp.nvec; i += step) {
     float v[VEC];
     VecIO<T>::load(body + static_cast<long long>(i) * VEC, v);
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) v[j] = grad(v[j], sp.head + i * VEC + j);
+    grads(v, i);
     VecIO<T>::store(dbody + static_cast<long long>(i) * VEC, v);
   }
 }
