@@ -40,13 +40,13 @@ struct RowSplit {
   }
 };
 
-// Maximum and sum of exponentials relative to it, over a stream of values; -inf values (and rows of nothing else) add nothing.
 // exp(v - base) of two values: the difference first, then the power of two, as for one.
 __device__ __forceinline__ F2 f2_exp_from(F2 v, F2 minus_base) {
   float lo, hi;
   f2_get(f2_mul(f2_add(v, minus_base), f2_splat(1.4426950408889634f)), lo, hi);
   return f2_make(ex2_approx(lo), ex2_approx(hi));
 }
+// Maximum and sum of exponentials relative to it, over a stream of values; -inf values (and rows of nothing else) add nothing.
 struct OnlineSum {
   float m = -INFINITY;
   F2 s2 = f2_splat(0.f);
