@@ -38,27 +38,40 @@ __device__ __forceinline__ void load_f32_vec(const float* __restrict__ p, int of
   }
 }
 
-// The same for bf16 parameters (a model cast to bf16 for inference): one conversion here instead of a cast launch per parameter.
+// N consecutive parameters as they are in memory, fp32 or bf16 (a model cast to bf16 for inference): loaded, and converted where they are used, so that
+// a warp has all its loads in flight. A parameter off the alignment of a vector is read value by value; a missing one is `fill`.
+template <typename P, int N>
+struct Param;
 template <int N>
-__device__ __forceinline__ void load_f32_vec(const __nv_bfloat16* __restrict__ p, int off, float fill, float (&out)[N]) {
+struct Param<float, N> {
+  float v[N];
+  __device__ __forceinline__ void load(const float* __restrict__ p, int off, float fill) { load_f32_vec<N>(p, off, fill, v); }
+  __device__ __forceinline__ float get(int j) const { return v[j]; }
+};
+template <int N>
+struct Param<__nv_bfloat16, N> {
   static_assert(N == 4 || N == 8, "");
-  if (!p) {
+  uint32_t h[N / 2];
+  __device__ __forceinline__ void load(const __nv_bfloat16* __restrict__ p, int off, float fill) {
+    if (!p) {
 #pragma unroll
-    for (int j = 0; j < N; ++j) out[j] = fill;
-  } else if ((reinterpret_cast<uintptr_t>(p) & (2 * N - 1)) == 0) {
-    if constexpr (N == 8) {
-      const uint4 q = __ldg(reinterpret_cast<const uint4*>(p + off));
-      VecIO<__nv_bfloat16>::unpack(q, out);
+      for (int j = 0; j < N / 2; ++j) h[j] = __float_as_uint(fill) >> 16 | (__float_as_uint(fill) & 0xffff0000u);
+    } else if ((reinterpret_cast<uintptr_t>(p) & (2 * N - 1)) == 0) {
+      if constexpr (N == 8) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(p + off));
+        h[0] = q.x; h[1] = q.y; h[2] = q.z; h[3] = q.w;
+      } else {
+        const uint2 q = __ldg(reinterpret_cast<const uint2*>(p + off));
+        h[0] = q.x; h[1] = q.y;
+      }
     } else {
-      const uint2 q = __ldg(reinterpret_cast<const uint2*>(p + off));
-      const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.y));
-      out[0] = a.x; out[1] = a.y; out[2] = b.x; out[3] = b.y;
-    }
-  } else {
+      const uint16_t* u = reinterpret_cast<const uint16_t*>(p + off);
 #pragma unroll
-    for (int j = 0; j < N; ++j) out[j] = __bfloat162float(p[off + j]);
+      for (int j = 0; j < N / 2; ++j) h[j] = static_cast<uint32_t>(__ldg(u + 2 * j)) | static_cast<uint32_t>(__ldg(u + 2 * j + 1)) << 16;
+    }
   }
-}
+  __device__ __forceinline__ float get(int j) const { return __uint_as_float(j & 1 ? h[j / 2] & 0xffff0000u : h[j / 2] << 16); }
+};
 
 // Blocks per SM: of one row of `size`-byte values in the forward pass (one more for fp32 makes a whole wave of 4096 rows: 1024 wide 6.2 us, with six 9.0),
 // and in the backward pass what `values` columns per lane and two rows in flight leave registers for.
@@ -70,12 +83,23 @@ constexpr int ln_bwd_blocks(int values) { return values <= 16 ? 4 : values <= 24
 // us, plain / with residual, in brackets a load where it is used, and one wave of warps that walk the rows with the next row's loads in flight:
 // bf16 65536 x 768 49 / 61 (60 / 81, 50 / 65), 4096 x 768 5.0 / 5.6 (5.6 / 6.0, 6.2 / 6.5), 65536 x 256 20 / 25 (21 / 30, 31 / 36), 4096 x 1024 6.2 / 6.9
 // (6.4 / 6.8, 7.8 / 8.4), fp32 4096 x 1024 6.2 / 8.7 (7.3 / 9.3, 10.9 / 11.2), 65536 x 1024 95 / 166 (110 / 165, 119 / 156).
-template <typename T, int VPL, typename P>
-__global__ void __launch_bounds__(kLnWarps * 32, ln_fwd_blocks(sizeof(T)))
+// kFew, for as many rows as two blocks on each SM take: such a launch is one chain of latencies, so that gamma and beta are brought to L2 while the
+// previous kernel still runs and loaded along with the row instead of after its sums, in registers that many rows need for more warps. bf16 768 wide,
+// residual, pre kept: 77 rows 2.0 us (2.6), 1184 rows 2.6 (3.1), 2368 rows 4.2 against 3.7; an encoder of bf16 parameters, cold: 5.0 -> 3.0 a launch, of
+// which half is the parameters' conversion, which had made each of six loads wait for the one before.
+template <typename T, int VPL, typename P, bool kFew>
+__global__ void __launch_bounds__(kLnWarps * 32, kFew ? 2 : ln_fwd_blocks(sizeof(T)))
 ln_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const P* __restrict__ gamma,
               const P* __restrict__ beta, T* __restrict__ y, T* __restrict__ pre_out,
               float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols, float eps,
               float p_drop, uint64_t seed_in, const unsigned long long* __restrict__ seed_dev) {
+  if constexpr (kFew) {
+    const int at = threadIdx.x * (128 / static_cast<int>(sizeof(P)));
+    if (at < cols) {
+      if (gamma) asm volatile("prefetch.global.L2 [%0];" ::"l"(gamma + at));
+      if (beta) asm volatile("prefetch.global.L2 [%0];" ::"l"(beta + at));
+    }
+  }
   pdl_entry();
   constexpr int V = VecIO<T>::kVec;
   const uint64_t seed = seed_in + (seed_dev ? *seed_dev : 0ull);
@@ -95,6 +119,17 @@ ln_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const P* 
     if (vi < nvec) {
       nx[i] = xr[vi];
       if (residual) nr[i] = rr[vi];
+    }
+  }
+  Param<P, V> g[VPL], b[VPL];
+  if constexpr (kFew) {
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      const int vi = lane + i * 32;
+      if (vi < nvec) {
+        g[i].load(gamma, vi * V, 1.f);
+        b[i].load(beta, vi * V, 0.f);
+      }
     }
   }
   float v[VPL][V];
@@ -152,11 +187,13 @@ ln_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual, const P* 
   for (int i = 0; i < VPL; ++i) {
     const int vi = lane + i * 32;
     if (vi < nvec) {
-      float o[V], g[V], b[V];
-      load_f32_vec<V>(gamma, vi * V, 1.f, g);
-      load_f32_vec<V>(beta, vi * V, 0.f, b);
+      float o[V];
+      if constexpr (!kFew) {
+        g[i].load(gamma, vi * V, 1.f);
+        b[i].load(beta, vi * V, 0.f);
+      }
 #pragma unroll
-      for (int j = 0; j < V; ++j) o[j] = fmaf((v[i][j] - mean) * rstd, g[j], b[j]);
+      for (int j = 0; j < V; ++j) o[j] = fmaf((v[i][j] - mean) * rstd, g[i].get(j), b[i].get(j));
       VecIO<T>::store(y + static_cast<long long>(row) * cols + vi * V, o);
     }
   }
@@ -349,8 +386,13 @@ template <typename T, int VPL, typename P>
 static int ln_fwd_launch(const void* x, const void* res, const P* gamma, const P* beta, void* y,
                          void* pre, float* mean, float* rstd, int rows, int cols, float eps, float p,
                          uint64_t seed, const unsigned long long* seed_dev, cudaStream_t st) {
-  launch_pdl(ln_fwd_kernel<T, VPL, P>, dim3((rows + kLnWarps - 1) / kLnWarps), dim3(kLnWarps * 32), 0, st, static_cast<const T*>(x), static_cast<const T*>(res), gamma, beta, static_cast<T*>(y),
-      static_cast<T*>(pre), mean, rstd, rows, cols, eps, p, seed, seed_dev);
+  const int blocks = (rows + kLnWarps - 1) / kLnWarps;
+  auto go = [&](auto kern) {
+    launch_pdl(kern, dim3(blocks), dim3(kLnWarps * 32), 0, st, static_cast<const T*>(x), static_cast<const T*>(res), gamma, beta, static_cast<T*>(y),
+               static_cast<T*>(pre), mean, rstd, rows, cols, eps, p, seed, seed_dev);
+  };
+  if (blocks <= 2 * sm_count()) go(ln_fwd_kernel<T, VPL, P, true>);
+  else go(ln_fwd_kernel<T, VPL, P, false>);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -359,6 +359,22 @@ def test_layernorm_backward_grids(C, dtype, rows, cols):
     test_layernorm_rows_per_warp(C, dtype, rows, cols)
 
 
+@pytest.mark.parametrize("dtype,cols", [(torch.bfloat16, 768), (torch.bfloat16, 264), (torch.float32, 1024), (torch.float32, 36)])
+@pytest.mark.parametrize("param", [torch.float32, torch.bfloat16])
+def test_layernorm_parameters_around_few_rows(C, dtype, cols, param):
+    """Either side of the row count (eight to an SM) up to which the parameters are loaded with the row; parameters of both types, on and off the
+    alignment of a vector, and absent. 32-bit arithmetic, one rounding to the type of the result."""
+    torch.manual_seed(15)
+    few = 8 * torch.cuda.get_device_properties(0).multi_processor_count
+    hold = torch.randn(2, cols + 1, device="cuda").to(param)
+    for rows in (1, few, few + 1):
+        x = torch.randn(rows, cols, device="cuda").to(dtype)
+        for g, b in ((hold[0, :cols].clone(), hold[1, :cols].clone()), (hold[0, 1:], hold[1, 1:].clone()), (hold[0, :cols].clone(), hold[1, 1:]), (None, None)):
+            y = C.layernorm_fwd(x, None, g, b, 1e-5, 0.0, 0, False)[0]
+            ref = torch.nn.functional.layer_norm(x.double(), (cols,), None if g is None else g.double(), None if b is None else b.double(), 1e-5)
+            assert ((y.double() - ref).norm() / ref.norm()).item() < (2 ** -8 if dtype == torch.bfloat16 else 2 ** -18)
+
+
 @pytest.mark.parametrize("dtype,V", [(torch.bfloat16, 4104), (torch.bfloat16, 32768), (torch.bfloat16, 32776), (torch.float32, 16384), (torch.float32, 16388)])
 def test_softmax_ce_block_sizes(C, dtype, V):
     """Either side of the row length at which a block's size changes, with more rows than resident blocks. The gradient carries one rounding to its
