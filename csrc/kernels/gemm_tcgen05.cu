@@ -1297,6 +1297,19 @@ static bool backward_in_one(int rows, int n, int tiles0, long long chain, long l
   return rows >= 256 && (n < 2304 || tiles0 > 12) && (n < 6400 || chain * 4 <= share * 5);
 }
 
+// Whether they go out in 128 x 64 tiles of one CTA instead of 256 x 256 tiles of a pair. A small layer has less than a tile for each pair, and then the time
+// is that of one tile's chain (its loads, its products, its epilogue of 256 columns), of which a 64-wide tile has a third. That holds as long as dX's tiles
+// leave SMs to dW; beyond, and where an SM has more than some 50 K blocks to go through, the wide tiles' fewer bytes per product count. Below 65 rows
+// there is nothing to sum in dW. Us against pair tiles: 256 x 128 x 128 4.1 (6.2), 512 x 512 x 128 4.7 (7.1), 512 x 128 x 512 with GELU' 5.6 (8.9),
+// 512 x 512 x 512 4.7 (7.8), 512 x 768 x 768 6.2 (8.4), 1024 x 2048 x 512 9.8 (14.6), 4096 x 1024 x 256 10.8 (12.9); 1536 x 768 x 768, whose dX has 144 tiles,
+// 9.5 (9.2), 512 x 768 x 3072 with GELU', 192 tiles, 16.5 (13.8). Against dX beside dW and db, where pair tiles are not taken: 77 x 768 x 768 5.5 (6.5), 200 x 512 x 512
+// 4.6 (6.5), 512 x 3072 x 768 13.8 (18.7), 768 x 3072 x 768 15.7 (22.2); 16 x 768 x 768 8.0 (5.9), 1024 x 3072 x 768, 62 blocks an SM, 19.2 (18.0).
+static bool backward_narrow(int rows, int n, int k) {
+  const long long tiles0 = static_cast<long long>((rows + BM - 1) / BM) * ((k + 63) / 64), tiles1 = static_cast<long long>((n + BM - 1) / BM) * ((k + 63) / 64);
+  const int kb0 = (n + BK - 1) / BK, kb1 = (rows + BK - 1) / BK, sms = sm_count();
+  return rows > 64 && tiles0 * 8 <= sms * 7 && kb0 <= 50 && tiles0 * kb0 + tiles1 * kb1 <= 50 * sms;
+}
+
 static cudaLaunchConfig_t split_config(int M, int N, cudaLaunchAttribute* attr, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(4, (M + 2 * BM - 1) / (2 * BM), (N + 255) / 256);
@@ -1526,16 +1539,19 @@ extern "C" int fb_gemm_backward(const void* dY, const void* W, const void* X, vo
   if (db && ((reinterpret_cast<uintptr_t>(db) & 15) || n % 8)) return -7;
   const bool dgelu = epi == FB_EPI_DGELU_ERF || epi == FB_EPI_DGELU_TANH;
   if (dgelu ? !aux || !aligned(aux, ldaux, 2) : epi != FB_EPI_NONE) return -7;
-  int pairs = sm_count() / 2;
-  const int tiles0 = ((rows + 255) / 256) * ((k + 255) / 256), tiles1 = ((n + 255) / 256) * ((k + 255) / 256);
   const int kb0 = (n + BK - 1) / BK, kb1 = (rows + BK - 1) / BK;
+  const bool narrow = backward_narrow(rows, n, k);
+  const int tm = narrow ? BM : 2 * BM, tn = narrow ? 64 : 256;
+  const int tiles0 = ((rows + tm - 1) / tm) * ((k + tn - 1) / tn), tiles1 = ((n + tm - 1) / tm) * ((k + tn - 1) / tn);
+  int groups = narrow ? sm_count() : sm_count() / 2;
   // Work is counted in K blocks of 64, which a pair's products take 530 cycles for; a tile of dX costs its epilogue on top, or that alone where it is
   // the longer.
-  const int cost = (dgelu ? (kb0 > 15 ? kb0 : 15) : kb0) + 3;
-  if (!backward_in_one(rows, n, tiles0, static_cast<long long>((tiles0 + pairs - 1) / pairs) * cost, (static_cast<long long>(tiles0) * cost + static_cast<long long>(tiles1) * kb1) / pairs))
+  const int cost = (dgelu && !narrow ? (kb0 > 15 ? kb0 : 15) : kb0) + 3;
+  if (!narrow && !backward_in_one(rows, n, tiles0, static_cast<long long>((tiles0 + groups - 1) / groups) * cost,
+                                  (static_cast<long long>(tiles0) * cost + static_cast<long long>(tiles1) * kb1) / groups))
     return -7;
   if (tiles1 * static_cast<long long>(kb1) > (1 << 22)) return -7;       // shares are counted in 1/256 of a block
-  if (const int most = tiles0 + tiles1 * kb1 / 4; most < pairs) pairs = most > 0 ? most : 1;
+  if (const int most = tiles0 + tiles1 * kb1 / 4; most < groups) groups = most > 0 ? most : 1;
 
   GemmLaunch<2> g;
   std::memset(&g, 0, sizeof(g));
@@ -1544,20 +1560,22 @@ extern "C" int fb_gemm_backward(const void* dY, const void* W, const void* X, vo
       (r = make_tmap_bf16_2d(&g.a[1], dY, n, rows, ldy, 64, BK)) || (r = make_tmap_bf16_2d(&g.b[1], X, k, rows, ldx, 64, BK)) ||
       (r = make_tmap_out(&g.c[0], dX, k, rows, lddx, false)) || (r = make_tmap_out(&g.c[1], dW, k, n, lddw, true)))
     return r;
-  if (dgelu && (r = make_tmap_out(&g.aux, aux, k, rows, ldaux, false))) return r;
+  if (dgelu && !narrow && (r = make_tmap_out(&g.aux, aux, k, rows, ldaux, false))) return r;
   GemmParams& p = g.p[0];
   p.M = rows; p.N = k; p.K = n; p.a_mn = 0; p.b_mn = 1; p.C = dX; p.ldc = lddx; p.epi = epi; p.aux = const_cast<void*>(aux); p.ldaux = ldaux;
-  p.split_k = 1; p.c_mode = 1; p.aux_tma = dgelu ? 2 : 0; p.kind = !dgelu ? kEpiPlain : epi == FB_EPI_DGELU_ERF ? kEpiDgelu : kEpiDgeluTanh;
-  p.band = band_of(k, 256); p.status = status; p.alpha = alpha;
+  p.split_k = 1; p.c_mode = narrow ? 0 : 1; p.aux_tma = dgelu && !narrow ? 2 : 0;
+  p.kind = narrow ? kEpiDirect : !dgelu ? kEpiPlain : epi == FB_EPI_DGELU_ERF ? kEpiDgelu : kEpiDgeluTanh;
+  p.band = band_of(k, tn); p.status = status; p.alpha = alpha;
   GemmParams& q = g.p[1];
   q.alpha = alpha;
-  q.M = n; q.N = k; q.K = rows; q.a_mn = 1; q.b_mn = 1; q.C = dW; q.ldc = lddw; q.c_fp32 = 1; q.accumulate = 1; q.split_k = 1; q.c_mode = 2;
-  q.kind = kEpiF32; q.band = band_of(k, 256); q.status = status;
+  q.M = n; q.N = k; q.K = rows; q.a_mn = 1; q.b_mn = 1; q.C = dW; q.ldc = lddw; q.c_fp32 = 1; q.accumulate = 1; q.split_k = 1; q.c_mode = narrow ? 0 : 2;
+  q.kind = narrow ? kEpiDirect : kEpiF32; q.band = band_of(k, tn); q.status = status;
   const long long total = static_cast<long long>(tiles1) * kb1;
-  g.ahead = tiles0 % pairs;
-  const long long rest = pairs - g.ahead, level = g.ahead ? cost : 0;
-  g.share_ahead = total > rest * level ? static_cast<int>((total - rest * level) * 256 / pairs) : 0;
+  g.ahead = tiles0 % groups;
+  const long long rest = groups - g.ahead, level = g.ahead ? cost : 0;
+  g.share_ahead = total > rest * level ? static_cast<int>((total - rest * level) * 256 / groups) : 0;
   g.share = static_cast<int>((total * 256 - static_cast<long long>(g.ahead) * g.share_ahead) / rest);
   g.sum_x = static_cast<const __nv_bfloat16*>(dY); g.sum_out = db; g.sum_rows = rows; g.sum_cols = n; g.sum_ld = ldy;
-  return launch_gemm<2, 256, 2>(g, pairs, static_cast<cudaStream_t>(stream_));
+  if (narrow) return launch_gemm<1, 64, 2>(g, groups, static_cast<cudaStream_t>(stream_));
+  return launch_gemm<2, 256, 2>(g, groups, static_cast<cudaStream_t>(stream_));
 }

@@ -124,7 +124,8 @@ def test_gemm_staged_epilogues(C, config, M, N, K, pad, bias):
 
 
 @pytest.mark.parametrize("rows,n,k,epi,bias", [(4096, 768, 768, 0, True), (3054, 768, 3072, 2, True), (2500, 2304, 768, 0, False), (8192, 520, 1032, 4, True),
-                                               (20000, 264, 256, 0, True), (1030, 2056, 264, 0, True), (3400, 2312, 264, 0, True), (256, 8, 8, 0, True)])
+                                               (20000, 264, 256, 0, True), (1030, 2056, 264, 0, True), (3400, 2312, 264, 0, True), (256, 8, 8, 0, True),
+                                               (65, 72, 40, 2, True), (77, 768, 768, 0, True), (130, 3072, 104, 4, False), (2000, 136, 520, 2, True)])
 def test_linear_gradients_in_one_launch(C, rows, n, k, epi, bias):
     """dX, dW and db from one launch where tiles are ragged and the pairs' shares of dW start anywhere in a tile. dX is rounded to bf16 once (and the
     activation's derivative takes the hardware's tanh: 3e-4); dW and db are fp32 sums of exact products."""
