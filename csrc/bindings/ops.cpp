@@ -320,6 +320,33 @@ void gather_rows(const Tensor& x, const Tensor& idx, const Tensor& counts, Tenso
                        (int)x.size(1), is_bf16(x), stream_of(x)),
         "fb_gather_rows");
 }
+// dst[i].copy_(src[i]) for all i as one launch, where each is a plain copy within one device; false, and nothing done, where one is not.
+bool copy_buffers(const std::vector<Tensor>& dst, const std::vector<Tensor>& src) {
+  const size_t n = dst.size();
+  if (n == 0 || n != src.size() || n > FB_MAX_COPIES) return false;
+  const void* from[FB_MAX_COPIES];
+  void* to[FB_MAX_COPIES];
+  long long bytes[FB_MAX_COPIES];
+  const auto apart = [](const void* a, long long na, const void* b, long long nb) {
+    return static_cast<const char*>(a) + na <= static_cast<const char*>(b) || static_cast<const char*>(b) + nb <= static_cast<const char*>(a);
+  };
+  for (size_t i = 0; i < n; ++i) {
+    const Tensor &d = dst[i], &s = src[i];
+    for (const Tensor* t : {&d, &s})
+      if (!t->is_cuda() || t->layout() != at::kStrided || !t->is_contiguous() || t->is_conj() || t->is_neg() || t->requires_grad()) return false;
+    if (s.get_device() != d.get_device() || d.get_device() != dst[0].get_device() || s.scalar_type() != d.scalar_type() || s.sizes() != d.sizes()) return false;
+    from[i] = s.data_ptr();
+    to[i] = d.data_ptr();
+    bytes[i] = static_cast<long long>(d.nbytes());
+  }
+  for (size_t i = 0; i < n; ++i)
+    for (size_t j = 0; j < n; ++j)
+      if (!apart(from[i], bytes[i], to[j], bytes[j]) || (i != j && !apart(to[i], bytes[i], to[j], bytes[j]))) return false;
+  c10::cuda::CUDAGuard guard(dst[0].device());
+  check(fb_copy_buffers(from, to, bytes, static_cast<int>(n), stream_of(dst[0])), "fb_copy_buffers");
+  return true;
+}
+
 void scatter_rows(const Tensor& dxc, const Tensor& idx, const Tensor& counts, Tensor& dx) {
   want_float_kind(dxc, "dxc");
   c10::cuda::CUDAGuard guard(dxc.device());
@@ -710,6 +737,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("colsum", &colsum, py::arg("x"), py::arg("out"), py::arg("rows_dyn") = py::none());
   m.def("compact_targets", &compact_targets);
   m.def("gather_rows", &gather_rows);
+  m.def("copy_buffers", &copy_buffers);
   m.def("scatter_rows", &scatter_rows);
   m.def("cast_into", &cast_into);
   m.def("embedding_bwd", &embedding_bwd);

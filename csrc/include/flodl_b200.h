@@ -125,6 +125,9 @@ int fb_compact_targets(const long long* targets, int rows, long long ignore_inde
 /* xc[i] = x[idx[i]] for i < counts[0], zero rows up to counts[1], later rows untouched (bf16 or fp32 rows of `cols`). */
 int fb_gather_rows(const void* x, long long ld, const int* idx, const int* counts, void* xc, long long ldc, int rows,
                    int cols, int is_bf16, void* stream);
+/* bytes[i] bytes from src[i] to dst[i], i < n, in one launch; no source may overlap a destination, nor two destinations each other. */
+#define FB_MAX_COPIES 8
+int fb_copy_buffers(const void* const* src, void* const* dst, const long long* bytes, int n, void* stream);
 /* dx[idx[i]] = dxc[i] for i < counts[0]; dx must be zeroed by the caller. */
 int fb_scatter_rows_f32(const float* dxc, long long ldc, const int* idx, const int* counts, void* dx, long long ld, int rows, int cols,
                         void* stream);   /* fp32 rows to bf16 ones; widths and strides multiples of 8 */

@@ -524,4 +524,57 @@ extern "C" int fb_scatter_rows(const void* dxc, long long ldc, const int* idx, c
   return static_cast<int>(cudaGetLastError());
 }
 
+// Up to FB_MAX_COPIES buffers copied by one launch: 16 KB to a block, four 16-byte loads in flight per thread. What bounds it is the launch: the five
+// inputs of a step (2 KB to 32 KB) one after the other took 1.5 us each and a gap of as much, together 1.6; a two-layer encoder's step 228 -> 220 us, ResNet-20 of 128 images 1015.5 -> 1012.
+namespace {
+struct Copies {
+  const unsigned char* src[FB_MAX_COPIES];
+  unsigned char* dst[FB_MAX_COPIES];
+  long long bytes[FB_MAX_COPIES];
+  int first[FB_MAX_COPIES + 1];      // the first block of each
+};
+constexpr int kCopyThreads = 256, kCopyBytes = kCopyThreads * 64;
+}  // namespace
+__global__ void __launch_bounds__(kCopyThreads) copy_buffers_kernel(const __grid_constant__ Copies c, int n) {
+  fb::pdl_entry();
+  int i = 0;
+  while (i + 1 < n && static_cast<int>(blockIdx.x) >= c.first[i + 1]) ++i;
+  const long long at = static_cast<long long>(blockIdx.x - c.first[i]) * kCopyBytes;
+  const unsigned char* src = c.src[i] + at;
+  unsigned char* dst = c.dst[i] + at;
+  const int bytes = static_cast<int>(min(static_cast<long long>(kCopyBytes), c.bytes[i] - at));
+  int done = 0;
+  if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
+    const int vecs = bytes / 16;
+    uint4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (const int at_vec = threadIdx.x + k * kCopyThreads; at_vec < vecs) v[k] = reinterpret_cast<const uint4*>(src)[at_vec];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (const int at_vec = threadIdx.x + k * kCopyThreads; at_vec < vecs) reinterpret_cast<uint4*>(dst)[at_vec] = v[k];
+    done = vecs * 16;
+  }
+  for (int b = done + threadIdx.x; b < bytes; b += kCopyThreads) dst[b] = src[b];
+}
+extern "C" int fb_copy_buffers(const void* const* src, void* const* dst, const long long* bytes, int n, void* stream) {
+  if (n < 0 || n > FB_MAX_COPIES) return -2;
+  Copies c = {};
+  int m = 0;
+  long long blocks = 0;
+  for (int i = 0; i < n; ++i) {
+    if (bytes[i] <= 0) continue;
+    c.src[m] = static_cast<const unsigned char*>(src[i]);
+    c.dst[m] = static_cast<unsigned char*>(dst[i]);
+    c.bytes[m] = bytes[i];
+    c.first[m] = static_cast<int>(blocks);
+    blocks += (bytes[i] + kCopyBytes - 1) / kCopyBytes;
+    if (blocks > 0x7fffffff) return -2;
+    c.first[++m] = static_cast<int>(blocks);
+  }
+  if (!m) return 0;
+  fb::launch_pdl(copy_buffers_kernel, dim3(static_cast<unsigned>(blocks)), dim3(kCopyThreads), 0, static_cast<cudaStream_t>(stream), c, m);
+  return static_cast<int>(cudaGetLastError());
+}
+
 FB_BOUNDS_ATTACH(elementwise)

@@ -270,8 +270,12 @@ class TrainEngine:
             raise TensorError("replay() before capture()")
         if self.sync.symm is not None:
             self.sync.symm.check_async()
-        for dst, src in zip(self._static_in, inputs):
-            dst.copy_(src, non_blocking=True)
+        pairs = list(zip(self._static_in, inputs))
+        # one launch for all, unless one comes from the host, in another type, shape or stride, or as a tensor with ways of its own
+        if not (all(type(src) is torch.Tensor for _, src in pairs) and _ops.native_enabled()
+                and _ext.require().copy_buffers([dst for dst, _ in pairs], [src for _, src in pairs])):
+            for dst, src in pairs:
+                dst.copy_(src, non_blocking=True)
         self._pre()
         self._graph.replay()
         self.steps += 1

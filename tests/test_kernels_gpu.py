@@ -151,6 +151,20 @@ def test_linear_gradients_in_one_launch(C, rows, n, k, epi, bias):
         assert ((db.double() - want_db).abs() <= 2.0 ** -20 * (dy.double().abs().sum(0) + 8)).all()
 
 
+def test_copy_buffers(C):
+    """Bytes arrive as they are at every length and alignment; what is not a plain copy on one device is refused, with nothing done."""
+    src = [torch.randint(0, 256, (n,), device="cuda", dtype=torch.uint8) for n in (1, 15, 16, 16383, 16384, 16385, 100003)] + [torch.randn(3, 0, device="cuda")]
+    dst = [torch.zeros_like(s) for s in src]
+    assert C.copy_buffers(dst, src) and all(torch.equal(d, s) for d, s in zip(dst, src))
+    odd = [torch.zeros(40001, device="cuda", dtype=torch.uint8)[1:], torch.zeros(5003, device="cuda", dtype=torch.float32)[3:]]
+    new = [torch.randint(0, 256, (40000,), device="cuda", dtype=torch.uint8), torch.randn(5000, device="cuda")]
+    assert C.copy_buffers(odd, new) and all(torch.equal(d, s) for d, s in zip(odd, new))
+    a, b = torch.zeros(8, 8, device="cuda"), torch.ones(8, 8, device="cuda")
+    for d, s in ((a, b.cpu()), (a, b.t()), (a, b[:1]), (a, b.double()), (a, a), (a.view(-1)[:60], a.view(-1)[4:]), (a, b.clone().requires_grad_())):
+        assert not C.copy_buffers([d], [s])
+    assert not C.copy_buffers([a, a], [b, b]) and not C.copy_buffers([a] * 9, [b] * 9) and not a.any()
+
+
 def test_dropout_keeps_what_its_threshold_says(C):
     """One draw per value: what a larger p keeps, a smaller one keeps too, in shares of 1 - p (within six standard deviations), also at the ends."""
     x, n = torch.ones(1 << 22, device="cuda"), 1 << 22
