@@ -590,8 +590,8 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmW, const HaloParams p)
   float* stat_smem = reinterpret_cast<float*>(smem + p.bars_off + 512);   // [4 warps][2][Nout]
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
-  // Consecutive MMAs into one accumulator wait for each other (about 0.1 us each, measured), so the
-  // nine taps of a tile are spread round-robin over `groups` accumulators that the epilogue adds up.
+  // Consecutive MMAs into one accumulator wait for each other, so the nine taps of a tile are spread
+  // round-robin over `groups` accumulators that the epilogue adds up.
   const int groups = p.groups;
   const int acc_cols = groups * p.Nout;            // columns of one buffer (two buffers)
 

@@ -7,8 +7,8 @@
 // Shape of the kernel
 //   * persistent: one CTA (or one CTA pair) per SM walks a list of output tiles;
 //   * warp 0 feeds a multi-stage shared-memory ring with TMA (`cp.async.bulk.tensor`, 128-byte
-//     swizzle), warp 1 issues `tcgen05.mma` from one elected thread, warps 2..9 drain the
-//     accumulator from TMEM with `tcgen05.ld` and run the epilogue;
+//     swizzle), warp 1 issues `tcgen05.mma` (both run their loops whole, one elected lane issues), warps 2..9
+//     drain the accumulator from TMEM with `tcgen05.ld` and run the epilogue;
 //   * two accumulator buffers in TMEM, so the epilogue of tile i overlaps the main loop of
 //     tile i+1;
 //   * `kCG == 2` pairs two CTAs of a cluster on one 256-row tile (`cta_group::2`): each CTA loads
@@ -17,7 +17,9 @@
 //   * operands may be K-major (row = M/N index) or MN-major (row = K index); the second form is
 //     what dX = dY * W and dW = dY^T * X need, so no transposes are materialised.
 //   * epilogue: optional alpha (device scalar), bias, GELU (erf or tanh; pre-activation saved to
-//     `aux`), GELU' (multiply by gelu'(aux)), accumulate into C, split-K via fp32 atomics.
+//     `aux`), GELU' (multiply by gelu'(aux)), accumulate into C, split-K added to memory in fp32;
+//   * the gradients of a linear layer as one launch: dX's tiles, then dW's reduction cut where the tiles of dX leave time, and
+//     two more warps for the bias gradient (`fb_gemm_backward`).
 //
 // All waits are bounded (see ptx_sm100.cuh); a give-up is reported through `status`.
 #include <cuda.h>

@@ -203,7 +203,8 @@ def _pick_dw_plan(m_out: int, n_out: int, k_red: int):
 
 
 # ---- weight gradients beside the data gradient ------------------------------------------------------
-# dX and dW of a linear layer are independent products of the same upstream gradient. Issued on two
+# dX, dW and db of a linear layer go out as one launch where the kernel takes the sizes (`_backward_in_one`). Otherwise:
+# dX and dW are independent products of the same upstream gradient. Issued on two
 # streams they share the GPU: the blocks of one fill the SMs the other leaves idle in its last
 # (partial) wave and behind its fixed latencies, and the small bias-gradient column sums vanish
 # behind the GEMMs. The side stream forks from the current stream and is joined before backward()
