@@ -664,6 +664,13 @@ def test_attention_fwd_bwd(C, B, H, S, causal, use_mask):
         assert err < 0.06 * max(1.0, g.abs().max().item()), (i, err, g.abs().max().item())
 
 
+@pytest.mark.parametrize("S", [18, 32, 33, 64, 65, 96, 97])
+def test_attention_up_to_the_end_of_a_short_sequence(C, S):
+    """Either side of the lengths at which thirty-two keys more are worked on; bounds as above."""
+    for causal, use_mask in ((False, True), (True, False)):
+        test_attention_fwd_bwd(C, 2, 3, S, causal, use_mask)
+
+
 @pytest.mark.parametrize("B,H,S,causal,use_mask", [(1, 1, 129, True, False), (2, 3, 131, False, True), (1, 2, 255, True, True), (3, 1, 257, False, False),
                                                    (1, 4, 509, False, True), (2, 2, 641, True, False), (9, 20, 129, False, False), (1, 1, 2050, True, False)])
 def test_attention_several_key_blocks(C, B, H, S, causal, use_mask):
