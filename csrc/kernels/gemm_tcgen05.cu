@@ -568,6 +568,14 @@ struct alignas(64) GemmLaunch {
   long long sum_ld;
 };
 
+// A reduction of `blocks` K blocks in at most `parts` equal ones: as many as hold a block. One without would add an accumulator that no product has
+// written (17 blocks each for 500 in 31 parts: the last two would start behind the end).
+__host__ __device__ constexpr int parts_with_blocks(int blocks, int parts) {
+  if (blocks <= 0 || parts <= 1) return 1;
+  const int per = (blocks + parts - 1) / parts;
+  return (blocks + per - 1) / per;
+}
+
 // What a pair (or CTA) works on next: K blocks [kb0, kb1) of a tile.
 struct Segment {
   int prob, tm, tn, kb0, kb1, ks;
@@ -575,7 +583,7 @@ struct Segment {
 template <int kCG, int kBN, int kProblems>
 struct Worklist {
   const GemmLaunch<kProblems>& g;
-  int step, num_m, num_n, num_kb, kb_per, units, u;      // the first product: whole tiles, or their K splits
+  int step, num_m, num_n, num_kb, split, kb_per, units, u;      // the first product: whole tiles, or their K splits
   int num_m1, num_n1, num_kb1, at, end;                  // the second: a stretch of its K blocks
 
   __device__ __forceinline__ Worklist(const GemmLaunch<kProblems>& g_, int group, int groups, int m_eff, int k_eff) : g(g_), step(groups), u(group) {
@@ -583,8 +591,9 @@ struct Worklist {
     num_m = (m_eff + BM * kCG - 1) / (BM * kCG);
     num_n = (p.N + kBN - 1) / kBN;
     num_kb = (k_eff + BK - 1) / BK;
-    kb_per = (num_kb + p.split_k - 1) / p.split_k;
-    units = num_kb > 0 ? num_m * num_n * p.split_k : 0;
+    split = parts_with_blocks(num_kb, p.split_k);          // (again: a reduction of dynamic length may have fewer blocks than parts were asked for)
+    kb_per = (num_kb + split - 1) / split;
+    units = num_kb > 0 ? num_m * num_n * split : 0;
     if constexpr (kProblems == 2) {
       const GemmParams& q = g.p[1];
       num_m1 = (q.M + BM * kCG - 1) / (BM * kCG);
@@ -604,9 +613,9 @@ struct Worklist {
     if (u < units) {
       int t = u;
       s.ks = 0;
-      if (kProblems == 1 && g.p[0].split_k > 1) {
-        t = u / g.p[0].split_k;
-        s.ks = u - t * g.p[0].split_k;
+      if (kProblems == 1 && split > 1) {
+        t = u / split;
+        s.ks = u - t * split;
       }
       tile_of(t, num_m, num_n, g.p[0].band, s.tm, s.tn);
       s.prob = 0;
@@ -896,10 +905,11 @@ gemm_bf16_kernel(const __grid_constant__ GemmLaunch<kProblems> g) {
     // Thread i of the four warps of a half keeps column i's bias of the tile to come.
     const bool staged_bias = kStaged && kProblems == 1 && p.bias != nullptr && p.kind != kEpiDirect;
     const auto bias_of = [&](int u) -> float {
+      if (u >= work.units) return 0.f;
       int tm, tn;
-      tile_of(u / p.split_k, work.num_m, work.num_n, p.band, tm, tn);
+      tile_of(u / work.split, work.num_m, work.num_n, p.band, tm, tn);
       const int c = q * 32 + lane, col = tn * kBN + half * kSplit + c;
-      if (u >= work.units || c >= cols || col >= p.N) return 0.f;
+      if (c >= cols || col >= p.N) return 0.f;
       return p.bias_fp32 ? __ldg(static_cast<const float*>(p.bias) + col) : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col]);
     };
     float next_bias = staged_bias ? bias_of(group) : 0.f;
@@ -1427,6 +1437,8 @@ extern "C" int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, in
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (split_k < 1) split_k = 1;
   if (split_k > 1 && !c_fp32) return -2;
+  if (split_k > 1 && !accumulate) accumulate = 1;          // parts are added to what the caller has zeroed, also if only one of them holds a block
+  split_k = parts_with_blocks((K + BK - 1) / BK, split_k);
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
   bool over_pairs = false;       // the reduction split over two pairs of a cluster
   if (config < 0) {

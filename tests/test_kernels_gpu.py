@@ -199,6 +199,35 @@ def test_linear_cross_entropy_gradients_with_few_rows(monkeypatch, rows, V, K, s
     assert sparse is False or (x.grad[t == -100] == 0).all()
 
 
+@pytest.mark.parametrize("config", [0, 1, 2, 3, 4, 5])
+@pytest.mark.parametrize("blocks,parts", [(33, 16), (500, 31), (5, 4), (3, 7), (1, 2)])
+def test_gemm_split_into_more_parts_than_hold_a_block(C, config, blocks, parts):
+    """Equal parts of a reduction, rounded up to whole K blocks, may be over before the last part starts, on the host's sizes or on the device's. fp32 sums of
+    exact products: a few ulp of the sum of magnitudes. What an earlier product left in the accumulators must not come in."""
+    torch.manual_seed(blocks)
+    M, N, K = 300, 328, blocks * 64
+    big = torch.full((4096, 64), 1e4, device="cuda").bfloat16()
+    a, b, bias = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16(), torch.randn(N, device="cuda")
+    C.clear_status(0)
+    for k_dyn in (None, 64 * max(1, blocks // 9)):
+        k = K if k_dyn is None else k_dyn
+        ad, bd = a[:, :k].double(), b[:, :k].double()
+        C.gemm(big, big, torch.empty(4096, 4096, device="cuda", dtype=torch.bfloat16), config=config)
+        out = torch.ones(M, N, device="cuda")
+        C.gemm(a, b, out, bias=bias, accumulate=True, split_k=parts, config=config, k_dyn=None if k_dyn is None else torch.tensor([k], device="cuda", dtype=torch.int32))
+        assert C.read_status(0) == 0
+        assert ((out.double() - 1 - bias.double() - ad @ bd.t()).abs() <= 2.0 ** -20 * (ad.abs() @ bd.abs().t() + 8)).all()
+
+
+@pytest.mark.parametrize("rows,V,K,sparse", [(256, 32000, 512, False), (64, 32000, 128, False), (256, 18440, 256, False), (200, 50257, 512, False), (128, 28996, 256, False),
+                                             (1024, 32000, 512, True), (1024, 25000, 768, True), (1024, 50257, 512, True)])
+def test_linear_cross_entropy_gradients_over_large_vocabularies(C, monkeypatch, rows, V, K, sparse):
+    """As above at vocabularies whose K blocks the parts do not divide."""
+    big = torch.full((4096, 64), 1e4, device="cuda").bfloat16()
+    C.gemm(big, big, torch.empty(4096, 4096, device="cuda", dtype=torch.bfloat16), config=0)
+    test_linear_cross_entropy_gradients_with_few_rows(monkeypatch, rows, V, K, sparse)
+
+
 def test_linear_gradients_in_one_launch_are_refused_where_they_do_not_fit(C):
     dy, w, x = (torch.randn(s, device="cuda").bfloat16() for s in ((2048, 1024), (1024, 1024), (2048, 1024)))
     dx, dw, db = torch.zeros_like(x), torch.zeros(1024, 1024, device="cuda"), torch.zeros(1028, device="cuda")
