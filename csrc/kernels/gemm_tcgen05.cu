@@ -1484,7 +1484,8 @@ extern "C" int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, in
     else c_mode = 0;
   }
   if (epi == FB_EPI_DGELU_ERF || epi == FB_EPI_DGELU_TANH) {
-    if (c_mode == 1 && !c_fp32 && (reinterpret_cast<uintptr_t>(aux) & 15) == 0 && (ldaux * 2) % 16 == 0) aux_tma = 2;
+    if (over_pairs) {                          // that kernel reads the pre-activations itself, at any alignment, and stores C through its tensor map
+    } else if (c_mode == 1 && !c_fp32 && (reinterpret_cast<uintptr_t>(aux) & 15) == 0 && (ldaux * 2) % 16 == 0) aux_tma = 2;
     else c_mode = 0;
   }
   CUtensorMap tc, tx;

@@ -345,6 +345,23 @@ def test_gemm_two_pairs(C, M, N, K, b_mn, epi):
     test_gemm_few_tiles(C, M, N, K, b_mn, epi, pad=8)
 
 
+@pytest.mark.parametrize("M,N,K", [(1800, 1000, 1352), (4096, 512, 2048)])
+@pytest.mark.parametrize("pad,at", [(1, 0), (4, 0), (8, 1), (8, 4)])
+def test_gemm_two_pairs_takes_pre_activations_at_any_alignment(C, M, N, K, pad, at):
+    """GELU' over two pairs of a cluster where rows of the pre-activations are off a 16-byte boundary. Bounds as above."""
+    torch.manual_seed(16)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(K, N, device="cuda") / math.sqrt(K)).bfloat16()
+    aux = torch.randn(M, N + pad, device="cuda").bfloat16()[:, at:at + N]
+    out = torch.zeros(M, N, device="cuda").bfloat16()
+    for epi, approximate in ((2, "none"), (4, "tanh")):
+        C.clear_status(0)
+        C.gemm(a, b, out, False, True, epi=epi, aux=aux)
+        assert C.read_status(0) == 0
+        x = aux.double().requires_grad_(True)
+        torch.nn.functional.gelu(x, approximate=approximate).backward(a.double() @ b.double())
+        assert ((out.double() - x.grad).norm() / x.grad.norm()).item() < 2 ** -8
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("cols", [768, 512, 16 * 8, 1024])
 def test_layernorm_fwd_bwd(C, dtype, cols):
