@@ -524,8 +524,11 @@ extern "C" int fb_scatter_rows(const void* dxc, long long ldc, const int* idx, c
   return static_cast<int>(cudaGetLastError());
 }
 
-// Up to FB_MAX_COPIES buffers copied by one launch: 16 KB to a block, four 16-byte loads in flight per thread. What bounds it is the launch: the five
-// inputs of a step (2 KB to 32 KB) one after the other took 1.5 us each and a gap of as much, together 1.6; a two-layer encoder's step 228 -> 220 us, ResNet-20 of 128 images 1015.5 -> 1012.
+// Up to FB_MAX_COPIES buffers copied by one launch: 16 KB to a block, in the widest vectors that both ends are aligned to, 4 to 16 of them in flight per
+// thread. What bounds it is the launch: the five inputs of a step (2 KB to 32 KB) one after the other took 1.5 us each and a gap of as much, together 1.6; a
+// two-layer encoder's step 228 -> 220 us, ResNet-20 of 128 images 1015.5 -> 1012.
+// 64 MB, us at offsets of 0, 8, 4, 2 and 1 byte, in brackets one copy_ of the library: 19, 19, 21, 27, 36 (25, 25, 25, 47, 47); at no size from 16 KB to
+// 256 MB slower than that. Byte by byte whatever is off a 16-byte boundary took 120.
 namespace {
 struct Copies {
   const unsigned char* src[FB_MAX_COPIES];
@@ -534,6 +537,23 @@ struct Copies {
   int first[FB_MAX_COPIES + 1];      // the first block of each
 };
 constexpr int kCopyThreads = 256, kCopyBytes = kCopyThreads * 64;
+
+// `bytes` of at most kCopyBytes, both ends aligned to V.
+template <typename V>
+__device__ __forceinline__ void copy_chunk(const unsigned char* src, unsigned char* dst, int bytes) {
+  constexpr int kInFlight = sizeof(V) >= 4 ? 64 / sizeof(V) : 16;
+  const int n = bytes / static_cast<int>(sizeof(V));
+  for (int at = threadIdx.x; at < n; at += kInFlight * kCopyThreads) {
+    V v[kInFlight];
+#pragma unroll
+    for (int k = 0; k < kInFlight; ++k)
+      if (at + k * kCopyThreads < n) v[k] = reinterpret_cast<const V*>(src)[at + k * kCopyThreads];
+#pragma unroll
+    for (int k = 0; k < kInFlight; ++k)
+      if (at + k * kCopyThreads < n) reinterpret_cast<V*>(dst)[at + k * kCopyThreads] = v[k];
+  }
+  for (int b = n * static_cast<int>(sizeof(V)) + threadIdx.x; b < bytes; b += kCopyThreads) dst[b] = src[b];
+}
 }  // namespace
 __global__ void __launch_bounds__(kCopyThreads) copy_buffers_kernel(const __grid_constant__ Copies c, int n) {
   fb::pdl_entry();
@@ -543,19 +563,12 @@ __global__ void __launch_bounds__(kCopyThreads) copy_buffers_kernel(const __grid
   const unsigned char* src = c.src[i] + at;
   unsigned char* dst = c.dst[i] + at;
   const int bytes = static_cast<int>(min(static_cast<long long>(kCopyBytes), c.bytes[i] - at));
-  int done = 0;
-  if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
-    const int vecs = bytes / 16;
-    uint4 v[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (const int at_vec = threadIdx.x + k * kCopyThreads; at_vec < vecs) v[k] = reinterpret_cast<const uint4*>(src)[at_vec];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (const int at_vec = threadIdx.x + k * kCopyThreads; at_vec < vecs) reinterpret_cast<uint4*>(dst)[at_vec] = v[k];
-    done = vecs * 16;
-  }
-  for (int b = done + threadIdx.x; b < bytes; b += kCopyThreads) dst[b] = src[b];
+  const uintptr_t off = reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst);
+  if ((off & 15) == 0) copy_chunk<uint4>(src, dst, bytes);
+  else if ((off & 7) == 0) copy_chunk<uint2>(src, dst, bytes);
+  else if ((off & 3) == 0) copy_chunk<uint32_t>(src, dst, bytes);
+  else if ((off & 1) == 0) copy_chunk<uint16_t>(src, dst, bytes);
+  else copy_chunk<uint8_t>(src, dst, bytes);
 }
 extern "C" int fb_copy_buffers(const void* const* src, void* const* dst, const long long* bytes, int n, void* stream) {
   if (n < 0 || n > FB_MAX_COPIES) return -2;

@@ -165,6 +165,35 @@ def test_copy_buffers(C):
     assert not C.copy_buffers([a, a], [b, b]) and not C.copy_buffers([a] * 9, [b] * 9) and not a.any()
 
 
+@pytest.mark.parametrize("src_at", [0, 1, 2, 4, 6, 8, 12, 16])
+@pytest.mark.parametrize("dst_at", [0, 1, 2, 4, 8])
+def test_copy_buffers_at_every_alignment(C, src_at, dst_at):
+    """Each width of vector, alone and with a rest, around the sizes of a block; bytes before and behind stay."""
+    for n in (1, 3, 255, 4099, 16383, 16384, 16385, 65551):
+        src, dst = torch.randint(0, 256, (n + 64,), device="cuda", dtype=torch.uint8), torch.full((n + 64,), 7, device="cuda", dtype=torch.uint8)
+        assert C.copy_buffers([dst[dst_at:dst_at + n]], [src[src_at:src_at + n]])
+        assert torch.equal(dst[dst_at:dst_at + n], src[src_at:src_at + n]) and (dst[:dst_at] == 7).all() and (dst[dst_at + n:] == 7).all()
+
+
+def test_a_copy_off_alignment_takes_no_longer_than_the_librarys(C):
+    """64 MB from an address off a 16-byte boundary, as a slice of a larger tensor has it: as fast as `copy_` within the noise of a shared GPU (byte by byte it was 5 times as long)."""
+    n = 64 << 20
+    src, dst = torch.zeros(n + 16, device="cuda", dtype=torch.uint8), torch.zeros(n, device="cuda", dtype=torch.uint8)
+
+    def us(call):
+        best = float("inf")
+        for _ in range(10):
+            a, b = torch.cuda.Event(True), torch.cuda.Event(True)
+            a.record()
+            call()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3)
+        return best
+    for at in (8, 4, 2, 1):
+        assert us(lambda: C.copy_buffers([dst], [src[at:at + n]])) < 1.5 * us(lambda: dst.copy_(src[at:at + n])), at
+
+
 def test_dropout_keeps_what_its_threshold_says(C):
     """One draw per value: what a larger p keeps, a smaller one keeps too, in shares of 1 - p (within six standard deviations), also at the ends."""
     x, n = torch.ones(1 << 22, device="cuda"), 1 << 22
