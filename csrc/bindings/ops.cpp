@@ -151,6 +151,28 @@ bool gemm_backward(const Tensor& dy, const Tensor& w, const Tensor& x, Tensor& d
   return true;
 }
 
+// dx = alpha dy w with the reduction in parts (rows idx[i] of dx for i < counts[0]; the others are the caller's); false: not taken, nothing done.
+bool gemm_in_parts(const Tensor& dy, const Tensor& w, Tensor& dx, const Tensor& alpha, const OptTensor& idx, const OptTensor& counts) {
+  want_cuda(dy, "dy");
+  c10::cuda::CUDAGuard guard(dy.device());
+  for (const Tensor* t : {&dy, &w, static_cast<const Tensor*>(&dx)})
+    TORCH_CHECK(t->is_cuda() && is_bf16(*t) && t->dim() == 2 && t->stride(1) == 1, "bf16 [rows, cols] with unit inner stride");
+  const int64_t M = dy.size(0), K = dy.size(1), N = w.size(1);
+  TORCH_CHECK(w.size(0) == K && dx.size(0) == M && dx.size(1) == N, "shapes do not fit together");
+  TORCH_CHECK(alpha.is_cuda() && alpha.scalar_type() == at::kFloat && alpha.numel() == 1, "alpha must be one fp32");
+  TORCH_CHECK(idx.has_value() == counts.has_value(), "idx and counts go together");
+  if (idx.has_value())
+    TORCH_CHECK(idx->is_cuda() && idx->scalar_type() == at::kInt && idx->is_contiguous() && idx->numel() == M && counts->is_cuda() && counts->scalar_type() == at::kInt &&
+                counts->is_contiguous() && counts->numel() == 2, "idx must be int32 [rows], counts int32 [2]");
+  const int64_t rows = fb_gemm_parts_apply((int)M, (int)N, (int)K, counts.has_value());
+  if (rows == 0) return false;
+  const Tensor scratch = torch::empty({rows, N}, dy.options().dtype(at::kFloat));
+  check(fb_gemm_parts(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), scratch.data_ptr<float>(), (int)M, (int)N, (int)K, dy.stride(0), w.stride(0), dx.stride(0),
+                      alpha.data_ptr<float>(), ptr<const int>(idx), ptr<const int>(counts), status_word(dy.get_device()).data_ptr<int>(), stream_of(dy)),
+        "fb_gemm_parts");
+  return true;
+}
+
 int gemm_pick_config(int M, int N, int K, int split_k) { return fb_gemm_pick_config(M, N, K, split_k); }
 
 // Bounds-check record of the debug build (FLODL_BOUNDS_CHECK): one host-mapped int[4] = {site, index, limit, 0}.
@@ -162,6 +184,7 @@ int* bounds_word(bool create) {
     host[0] = host[1] = host[2] = host[3] = 0;
     TORCH_CHECK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&dev), host, 0) == cudaSuccess, "cudaHostGetDevicePointer");
     check(fb_bounds_attach_elementwise(dev), "fb_bounds_attach_elementwise");
+    check(fb_bounds_attach_gemm(dev), "fb_bounds_attach_gemm");
     check(fb_bounds_attach_softmax_ce(dev), "fb_bounds_attach_softmax_ce");
   }
   return host;
@@ -350,15 +373,8 @@ bool copy_buffers(const std::vector<Tensor>& dst, const std::vector<Tensor>& src
 void scatter_rows(const Tensor& dxc, const Tensor& idx, const Tensor& counts, Tensor& dx) {
   want_float_kind(dxc, "dxc");
   c10::cuda::CUDAGuard guard(dxc.device());
-  TORCH_CHECK(dx.dim() == 2 && dxc.dim() == 2 && dx.stride(1) == 1 && dxc.stride(1) == 1 && dx.sizes() == dxc.sizes());
-  TORCH_CHECK(dx.scalar_type() == dxc.scalar_type() || (is_bf16(dx) && dxc.scalar_type() == at::kFloat), "scatter_rows: rows of one type, or fp32 to bf16");
+  TORCH_CHECK(dx.dim() == 2 && dxc.dim() == 2 && dx.stride(1) == 1 && dxc.stride(1) == 1 && dx.sizes() == dxc.sizes() && dx.scalar_type() == dxc.scalar_type());
   TORCH_CHECK(idx.scalar_type() == at::kInt && idx.numel() == dx.size(0) && counts.scalar_type() == at::kInt && counts.numel() == 2);
-  if (dx.scalar_type() != dxc.scalar_type()) {
-    check(fb_scatter_rows_f32(dxc.data_ptr<float>(), dxc.stride(0), idx.data_ptr<int>(), counts.data_ptr<int>(), dx.data_ptr(), dx.stride(0), (int)dx.size(0),
-                              (int)dx.size(1), stream_of(dx)),
-          "fb_scatter_rows_f32");
-    return;
-  }
   check(fb_scatter_rows(dxc.data_ptr(), dxc.stride(0), idx.data_ptr<int>(), counts.data_ptr<int>(), dx.data_ptr(), dx.stride(0), (int)dx.size(0),
                         (int)dx.size(1), is_bf16(dx), stream_of(dx)),
         "fb_scatter_rows");
@@ -734,6 +750,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dropout", &dropout, py::arg("x"), py::arg("p"), py::arg("seed"), py::arg("seed_dev") = py::none());
   m.def("gemm_backward", &gemm_backward, py::arg("dy"), py::arg("w"), py::arg("x"), py::arg("dx"), py::arg("dw"), py::arg("db") = py::none(),
         py::arg("epi") = 0, py::arg("aux") = py::none(), py::arg("alpha") = py::none());
+  m.def("gemm_in_parts", &gemm_in_parts, py::arg("dy"), py::arg("w"), py::arg("dx"), py::arg("alpha"), py::arg("idx") = py::none(), py::arg("counts") = py::none());
+  m.def("gemm_part_count", &fb_gemm_part_count);
+  m.def("gemm_part_rows", &fb_gemm_part_rows);
   m.def("colsum", &colsum, py::arg("x"), py::arg("out"), py::arg("rows_dyn") = py::none());
   m.def("compact_targets", &compact_targets);
   m.def("gather_rows", &gather_rows);

@@ -113,6 +113,14 @@ int fb_dropout(const void* x, void* y, long long n, float p, unsigned long long 
  * of dY (db may be null), all times *alpha (may be null). bf16 operands and dX, fp32 dW and db. -7: not taken (size or alignment), nothing launched. */
 int fb_gemm_backward(const void* dY, const void* W, const void* X, void* dX, float* dW, float* db, int rows, int n, int k, long long ldy, long long ldw,
                      long long ldx, long long lddx, long long lddw, int epi, const void* aux, long long ldaux, const float* alpha, int* status, void* stream);
+/* dX = alpha dY W ([M, K] x [K, N], bf16) with the reduction in parts, summed in their order. With `counts`, the first counts[0] rows alone, row i to row
+ * idx[i] of dX. `scratch`: fb_gemm_parts_apply rows of N fp32; that is 0 where one product serves better. */
+long long fb_gemm_parts_apply(int M, int N, int K, int counted);
+int fb_gemm_parts(const void* dY, const void* W, void* dX, float* scratch, int M, int N, int K, long long ldy, long long ldw, long long ldx, const float* alpha,
+                  const int* idx, const int* counts, int* status, void* stream);
+/* How many parts M rows make for `groups` pairs of SMs, and the rows of scratch that any count up to M needs. */
+int fb_gemm_part_count(int M, int N, int K, int groups);
+long long fb_gemm_part_rows(int M, int N, int K, int counted, int groups);
 /* out[c] += sum over rows of x[r][c] (the caller zeroes `out`, or passes a gradient slot to accumulate into). */
 int fb_colsum(const void* x, float* out, int rows, int cols, long long ld, int is_bf16, void* stream);
 /* As fb_colsum over the first min(rows, *rows_dyn) rows (device-side count). */
@@ -129,8 +137,6 @@ int fb_gather_rows(const void* x, long long ld, const int* idx, const int* count
 #define FB_MAX_COPIES 8
 int fb_copy_buffers(const void* const* src, void* const* dst, const long long* bytes, int n, void* stream);
 /* dx[idx[i]] = dxc[i] for i < counts[0]; dx must be zeroed by the caller. */
-int fb_scatter_rows_f32(const float* dxc, long long ldc, const int* idx, const int* counts, void* dx, long long ld, int rows, int cols,
-                        void* stream);   /* fp32 rows to bf16 ones; widths and strides multiples of 8 */
 int fb_scatter_rows(const void* dxc, long long ldc, const int* idx, const int* counts, void* dx, long long ld, int rows,
                     int cols, int is_bf16, void* stream);
 int fb_embedding_bwd(const void* dy, const long long* ids, float* dw, long long tokens, int dim, long long vocab,
@@ -222,6 +228,7 @@ long long fb_grad_norm_noalloc_max(void);
  * device-visible int[4] (host-mapped memory works); attach it once per translation unit. In a
  * regular build the attach functions do nothing. */
 int fb_bounds_attach_elementwise(int* dev_word);
+int fb_bounds_attach_gemm(int* dev_word);
 int fb_bounds_attach_softmax_ce(int* dev_word);
 
 /* ---- collectives over peer-mapped buffers ---------------------------------------------------- */

@@ -491,27 +491,6 @@ extern "C" int fb_gather_rows(const void* x, long long ld, const int* idx, const
   return static_cast<int>(cudaGetLastError());
 }
 
-// The same from fp32 sums to bf16 rows. cols, ld and ldc multiples of 8, both bases 16-byte aligned.
-__global__ void scatter_rows_f32_kernel(const float* __restrict__ dxc, long long ldc, const int* __restrict__ idx, const int* __restrict__ counts,
-                                        __nv_bfloat16* __restrict__ dx, long long ld, int cols) {
-  fb::pdl_entry();
-  const int i = blockIdx.x;
-  if (i >= counts[0]) return;
-  if (!FB_INDEX_OK(counts[0], static_cast<long long>(gridDim.x) + 1, 105) || !FB_INDEX_OK(idx[i], gridDim.x, 106)) return;
-  const float* src = dxc + static_cast<long long>(i) * ldc;
-  __nv_bfloat16* dst = dx + static_cast<long long>(idx[i]) * ld;
-  for (int c = threadIdx.x * 8; c < cols; c += blockDim.x * 8) {
-    const float4 a = *reinterpret_cast<const float4*>(src + c), b = *reinterpret_cast<const float4*>(src + c + 4);
-    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    fb::VecIO<__nv_bfloat16>::store(dst + c, v);
-  }
-}
-extern "C" int fb_scatter_rows_f32(const float* dxc, long long ldc, const int* idx, const int* counts, void* dx, long long ld, int rows, int cols, void* stream) {
-  if (rows <= 0 || cols <= 0) return 0;
-  if (cols % 8 || ld % 8 || ldc % 8 || (reinterpret_cast<uintptr_t>(dxc) & 15) || (reinterpret_cast<uintptr_t>(dx) & 15)) return -3;
-  fb::launch_pdl(scatter_rows_f32_kernel, dim3(rows), dim3(128), 0, static_cast<cudaStream_t>(stream), dxc, ldc, idx, counts, static_cast<__nv_bfloat16*>(dx), ld, cols);
-  return static_cast<int>(cudaGetLastError());
-}
 extern "C" int fb_scatter_rows(const void* dxc, long long ldc, const int* idx, const int* counts, void* dx, long long ld, int rows,
                                int cols, int is_bf16, void* stream) {
   if (rows <= 0 || cols <= 0) return 0;

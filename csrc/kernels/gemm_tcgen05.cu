@@ -75,6 +75,8 @@ struct GemmParams {
   int accumulate;
   int split_k;
   int c_mode;      // 0 = per-thread global stores, 1 = staged TMA store, 2 = staged TMA reduce-add (fp32)
+  int part_groups; // not 0: the device cuts K for as many pairs (parts_for); C is [parts][rows of whole tiles][N] fp32, written and not added to, or
+                   // with one part [M][N] bf16 through the map `aux`
   int kind;        // EpiKind: what the epilogue does
   int band;        // column tiles per band of the tile order (tile_of)
   int aux_tma;     // 1: the GELU pre-activation goes out through its own staged TMA store; 2: GELU' takes it in through TMA loads
@@ -576,6 +578,15 @@ __host__ __device__ constexpr int parts_with_blocks(int blocks, int parts) {
   return (blocks + per - 1) / per;
 }
 
+// Parts to cut a reduction into for `groups` pairs that have `tiles` tiles: a part for every pair, none shorter than kPartBlocks, whose addition or
+// storing would cost more than it spreads. The kernel that sums the parts asks again, with the same row count from the device.
+constexpr int kPartBlocks = 16;
+__host__ __device__ constexpr int parts_for(int tiles, int blocks, int groups) {
+  if (tiles <= 0) return 1;
+  const int spread = groups / tiles, most = blocks / kPartBlocks;
+  return parts_with_blocks(blocks, spread < most ? spread : most);
+}
+
 // What a pair (or CTA) works on next: K blocks [kb0, kb1) of a tile.
 struct Segment {
   int prob, tm, tn, kb0, kb1, ks;
@@ -591,7 +602,7 @@ struct Worklist {
     num_m = (m_eff + BM * kCG - 1) / (BM * kCG);
     num_n = (p.N + kBN - 1) / kBN;
     num_kb = (k_eff + BK - 1) / BK;
-    split = parts_with_blocks(num_kb, p.split_k);          // (again: a reduction of dynamic length may have fewer blocks than parts were asked for)
+    split = kProblems == 1 && p.part_groups ? parts_for(num_m * num_n, num_kb, p.part_groups) : parts_with_blocks(num_kb, p.split_k);   // (again: a reduction of dynamic length may have fewer blocks than parts were asked for)
     kb_per = (num_kb + split - 1) / split;
     units = num_kb > 0 ? num_m * num_n * split : 0;
     if constexpr (kProblems == 2) {
@@ -918,7 +929,7 @@ gemm_bf16_kernel(const __grid_constant__ GemmLaunch<kProblems> g) {
     for (; work.next(seg); ++it) {
       const GemmParams& pp = g.p[kProblems == 1 ? 0 : seg.prob];
       const CUtensorMap& tmC = g.c[kProblems == 1 ? 0 : seg.prob];
-      const int row0 = seg.tm * BM * kCG + static_cast<int>(rank) * BM + q * 32;
+      const int row0 = (seg.tm + (kProblems == 1 && p.part_groups ? seg.ks * work.num_m : 0)) * BM * kCG + static_cast<int>(rank) * BM + q * 32;
       const int ncol0 = seg.tn * kBN + half * kSplit;
       const int acc = it & 1;
       uint32_t bias = 0;
@@ -946,13 +957,16 @@ gemm_bf16_kernel(const __grid_constant__ GemmLaunch<kProblems> g) {
         }
       };
       if constexpr (kStaged) {
-        const int chunks = ncol0 >= pp.N ? 0 : (min(cols, pp.N - ncol0) + 63) / 64;
+        // (of a part, whose rows reach to the end of its last tile, only those that are read)
+        const bool unread = kProblems == 1 && p.part_groups && seg.tm * BM * kCG + static_cast<int>(rank) * BM + q * 32 >= m_eff;
+        const int chunks = ncol0 >= pp.N || unread ? 0 : (min(cols, pp.N - ncol0) + 63) / 64;
+        const bool whole = kProblems == 1 && p.part_groups && work.split == 1;
         const auto run = [&](auto kind) {
-          ok = epilogue_tile<decltype(kind)::value>(pp, tmC, g.aux, w, taddr, ncol0, row0, chunks, bias, abort_flag, hand_back, load_aux);
+          ok = epilogue_tile<decltype(kind)::value>(pp, whole ? g.aux : tmC, g.aux, w, taddr, ncol0, row0, chunks, bias, abort_flag, hand_back, load_aux);
         };
         if (pp.kind != kEpiDirect) {
           if (chunks == 0) hand_back();
-          else if (pp.kind == kEpiPlain) run(std::integral_constant<int, kEpiPlain>());
+          else if (pp.kind == kEpiPlain || whole) run(std::integral_constant<int, kEpiPlain>());
           else if (pp.kind == kEpiF32) epilogue_tile_f32(pp, tmC, w, taddr, ncol0, row0, min(cols, pp.N - ncol0), bias, hand_back);
           else if (pp.kind == kEpiGelu) run(std::integral_constant<int, kEpiGelu>());
           else if (pp.kind == kEpiGeluAux) run(std::integral_constant<int, kEpiGeluAux>());
@@ -1500,7 +1514,7 @@ extern "C" int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, in
   p.M = M; p.N = N; p.K = K; p.a_mn = a_mn; p.b_mn = b_mn; p.C = C; p.ldc = ldc; p.c_fp32 = c_fp32;
   p.bias = bias; p.bias_fp32 = bias_fp32; p.epi = epi; p.aux = aux; p.ldaux = ldaux; p.alpha = alpha;
   p.accumulate = accumulate; p.split_k = split_k; p.status = status; p.ts = ts;
-  p.m_dyn = m_dyn; p.k_dyn = k_dyn;
+  p.m_dyn = m_dyn; p.k_dyn = k_dyn; p.part_groups = 0;
   p.band = band_of(N, bn);
   if (over_pairs) return launch_split(ta, tb, tc, tx, p, stream);
   switch (config) {
@@ -1594,3 +1608,128 @@ extern "C" int fb_gemm_backward(const void* dY, const void* W, const void* X, vo
   if (narrow) return launch_gemm<1, 64, 2>(g, groups, static_cast<cudaStream_t>(stream_));
   return launch_gemm<2, 256, 2>(g, groups, static_cast<cudaStream_t>(stream_));
 }
+
+// dX = alpha dY W where few rows make few tiles of a long reduction: the parts into which it is cut go to a scratch, in fp32, and are summed from there
+// in their order, so that two calls give the same bits (added to one buffer as they came, three parts and more did not).
+// With `counts`, only the first counts[0] rows take part, and row i's sum goes to row idx[i] of dX.
+namespace fb {
+namespace {
+constexpr int kPartTile = 256;
+
+__host__ __device__ constexpr int tiles_of(int n) { return (n + kPartTile - 1) / kPartTile; }
+
+// Rows of the scratch for up to M rows: tiles * parts is at most what there are pairs, unless there is one part.
+long long part_rows(int M, int N, int K, bool counted, int groups) {
+  const int num_m = tiles_of(M), num_n = tiles_of(N), num_kb = (K + BK - 1) / BK;
+  if (!counted) return static_cast<long long>(parts_for(num_m * num_n, num_kb, groups)) * num_m * kPartTile;
+  const long long spread = groups / num_n, most = static_cast<long long>(num_m) * (num_kb / kPartBlocks);
+  const long long parted = spread < most ? spread : most;
+  return (parted > num_m ? parted : num_m) * kPartTile;
+}
+
+// Four columns a thread, up to eight parts in flight. Where that leaves threads without work, four of them take every fourth part each and meet in
+// shared memory, in their order. One part is bf16 already and only goes to its place.
+// A chain of latencies: the grid is what two waves hold, so that many rows are walked and few are shared. The whole of fb_gemm_parts, us, a block for every
+// 64 quads instead: 2048 x 768 x 8200 26.5 (45.5), 4096 x 768 x 30522 with 614 rows 38.0 (63.3); without the four lanes 64 x 768 x 50257 20.6 (27.8).
+constexpr int kSumThreads = 256, kSumLanes = 4, kSumBlocks = 8;
+__global__ void __launch_bounds__(kSumThreads, 4) sum_parts_kernel(const float* __restrict__ parts, int rows, int cols, int num_kb, int groups,
+                                                                            const int* __restrict__ idx, const int* __restrict__ counts,
+                                                                            __nv_bfloat16* __restrict__ dx, long long ld) {
+  __shared__ float4 meet[kSumLanes - 1][kSumThreads / kSumLanes];
+  pdl_entry();
+  if (counts) (void)FB_INDEX_OK(counts[0], static_cast<long long>(rows) + 1, 107);
+  const int m = counts ? max(0, min(rows, counts[0])) : rows, quads = cols / 4, num_m = tiles_of(m), n = parts_for(num_m * tiles_of(cols), num_kb, groups);
+  const long long stride = static_cast<long long>(num_m) * kPartTile * cols, items = static_cast<long long>(m) * quads;
+  const auto put = [&](long long item, uint2 v) {
+    const long long row = item / quads, to = idx ? idx[row] : row;
+    if (FB_INDEX_OK(to, rows, 108)) *reinterpret_cast<uint2*>(dx + to * ld + (item - row * quads) * 4) = v;
+  };
+  const auto sum_of = [&](long long item, int first, int step) {
+    const float4* p = reinterpret_cast<const float4*>(parts + item * 4);
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = first; i < n; i += 8 * step) {
+      float4 v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (i + j * step < n) v[j] = p[(i + j * step) * (stride / 4)];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (i + j * step < n) { sum.x += v[j].x; sum.y += v[j].y; sum.z += v[j].z; sum.w += v[j].w; }
+    }
+    return sum;
+  };
+  const auto pack = [](float4 v) { return make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w)); };
+  if (n == 1 || items * kSumLanes > static_cast<long long>(gridDim.x) * kSumThreads) {
+    for (long long item = static_cast<long long>(blockIdx.x) * kSumThreads + threadIdx.x; item < items; item += static_cast<long long>(gridDim.x) * kSumThreads)
+      put(item, n == 1 ? reinterpret_cast<const uint2*>(parts)[item] : pack(sum_of(item, 0, 1)));
+    return;
+  }
+  const int quad = threadIdx.x % (kSumThreads / kSumLanes), lane = threadIdx.x / (kSumThreads / kSumLanes);
+  const long long item = static_cast<long long>(blockIdx.x) * (kSumThreads / kSumLanes) + quad;
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (item < items) sum = sum_of(item, lane, kSumLanes);
+  if (lane) meet[lane - 1][quad] = sum;
+  __syncthreads();
+  if (lane || item >= items) return;
+#pragma unroll
+  for (int j = 0; j < kSumLanes - 1; ++j) {
+    const float4 v = meet[j][quad];
+    sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+  }
+  put(item, pack(sum));
+}
+}  // namespace
+}  // namespace fb
+
+extern "C" int fb_gemm_part_count(int M, int N, int K, int groups) {
+  using namespace fb;
+  return parts_for(tiles_of(M) * tiles_of(N), (K + BK - 1) / BK, groups);
+}
+
+extern "C" long long fb_gemm_part_rows(int M, int N, int K, int counted, int groups) { return fb::part_rows(M, N, K, counted != 0, groups); }
+
+// Rows of scratch for a reduction in parts, 0 where one product serves better. Parts save K blocks that run one after the other, `chain` in the kernel
+// that would take the product otherwise, and cost the scratch and a launch, about the time of 20 blocks; a cluster of two pairs saves as much as two parts.
+// us against one product, rows x columns x reduction: 64 x 128 x 18440 11.5 (13.6), 256 x 512 x 32000 16.1 (23.6), 512 x 512 x 32000 23.7 (40.3),
+// 1024 x 512 x 32000 34.1 (77.6), 2048 x 512 x 32000 56.7 (93.4), 2048 x 768 x 8200 26.6 (27.0); left: 256 x 512 x 8200 13.3 (12.7), 512 x 512 x 8200 14.1 (14.8),
+// 64 x 512 x 2056 12.4 (4.9). Counted rows are taken for a sixth of M here (a masked-LM batch has about that many labels); the device then cuts for what it
+// counts, so that a wrong guess costs little. With the zero fill and the scatter, 4096 x 768 x 30522 of which 614 38.0 (147.5), all 158.5 (157.3); 8192 x
+// 768 x 30522, 1228 57.8 (154), all 329 (330); 24576 x 512 x 32000, 3686 106.7 (184), all 588 (605); 1024 x 512 x 2056, 153 rows, left, 16.8 (14.4).
+extern "C" long long fb_gemm_parts_apply(int M, int N, int K, int counted) {
+  using namespace fb;
+  if (M <= 0 || N <= 0 || K <= 0 || N % 8) return 0;
+  const int groups = sm_count() / 2, num_kb = (K + BK - 1) / BK;
+  const int parts = fb_gemm_part_count(counted ? (M + 5) / 6 : M, N, K, groups), small = counted ? 0 : gemm_small_split(M, N, K);
+  const int chain = small ? (num_kb + small - 1) / small : !counted && split_applies(M, N, K) ? (num_kb + 1) / 2 : num_kb;
+  if (parts < (counted ? 2 : 3) || chain - num_kb / parts < 20) return 0;
+  return part_rows(M, N, K, counted != 0, groups);
+}
+
+extern "C" int fb_gemm_parts(const void* dY, const void* W, void* dX, float* scratch, int M, int N, int K, long long ldy, long long ldw, long long ldx, const float* alpha,
+                             const int* idx, const int* counts, int* status, void* stream_) {
+  using namespace fb;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (ldy % 8 || ldw % 8 || N % 8 || ldx % 4 || (reinterpret_cast<uintptr_t>(dY) & 15) || (reinterpret_cast<uintptr_t>(W) & 15) || (reinterpret_cast<uintptr_t>(dX) & 7) ||
+      (reinterpret_cast<uintptr_t>(scratch) & 15) || !idx != !counts)
+    return -3;
+  const int groups = sm_count() / 2, num_kb = (K + BK - 1) / BK;
+  const long long quads = (static_cast<long long>(M) * (N / 4) + kSumThreads / kSumLanes - 1) / (kSumThreads / kSumLanes);
+  const int blocks = quads < kSumBlocks * sm_count() ? static_cast<int>(quads) : kSumBlocks * sm_count();
+  GemmLaunch<1> g;
+  std::memset(&g, 0, sizeof(g));
+  int r;
+  if ((r = make_tmap_bf16_2d(&g.a[0], dY, K, M, ldy, BK, BM)) || (r = make_tmap_bf16_2d(&g.b[0], W, N, K, ldw, 64, BK)) ||
+      (r = make_tmap_out(&g.c[0], scratch, N, part_rows(M, N, K, counts != nullptr, groups), N, true)) || (r = make_tmap_out(&g.aux, scratch, N, M, N, false)))
+    return r;
+  GemmParams& p = g.p[0];
+  p.M = M; p.N = N; p.K = K; p.b_mn = 1; p.C = scratch; p.ldc = N; p.c_fp32 = 1; p.alpha = alpha; p.split_k = 1; p.part_groups = groups; p.c_mode = 1; p.kind = kEpiF32;
+  p.band = band_of(N, kPartTile); p.status = status; p.m_dyn = counts;
+  const long long units = static_cast<long long>(tiles_of(M)) * tiles_of(N) * (counts ? groups : parts_for(tiles_of(M) * tiles_of(N), num_kb, groups));
+  if ((r = launch_gemm<2, 256, 1>(g, units < groups ? static_cast<int>(units) : groups, stream))) return r;
+  launch_pdl(sum_parts_kernel, dim3(blocks), dim3(kSumThreads), 0, stream, scratch, M, N, num_kb, groups, idx, counts,
+             static_cast<__nv_bfloat16*>(dX), ldx);
+  return static_cast<int>(cudaGetLastError());
+}
+
+FB_BOUNDS_ATTACH(gemm)

@@ -720,24 +720,17 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
                 db = _bias_grad(dl, b, alpha=alpha, rows_dyn=n_dyn)
         if ctx.needs_input_grad[0]:
             rows, K = x2.shape
-            # Few rows (of a masked-LM batch about a sixth is labelled) make few tiles and the vocabulary a long reduction: that is split until every
-            # pair of SMs has a part, summed in fp32.
-            tiles = math.ceil((rows if counts is None else max(1, rows // 6)) / 256) * math.ceil(K / 256)
-            split = min(74 // tiles, dl.shape[1] // 1024)
-            if split > 1:
-                dx2 = torch.zeros(rows, K, dtype=torch.float32, device=dl.device)
-                C.gemm(dl, w16, dx2, False, True, alpha=alpha, accumulate=True, split_k=split, config=0, m_dyn=n_dyn)
+            dx2 = _new_rows(rows, K, BF16, dl.device) if counts is None else torch.zeros(rows, K, dtype=BF16, device=dl.device)
+            if C.gemm_in_parts(dl, w16, dx2, alpha, idx, counts):
+                _launched(2 if counts is None else 3)
+            elif counts is None:
+                C.gemm(dl, w16, dx2, False, True, alpha=alpha)
+                _launched()
             else:
-                dx2 = _new_rows(rows, K, BF16, dl.device)
-                C.gemm(dl, w16, dx2, False, True, alpha=alpha, m_dyn=n_dyn)
-            _launched()
-            if counts is not None:
-                full = torch.zeros(rows, K, dtype=BF16, device=dl.device)
-                C.scatter_rows(dx2, idx, counts, full)
-                _launched(2)
-                dx2 = full
-            elif split > 1:
-                dx2 = dx2.to(BF16)
+                dxc = _new_rows(rows, K, BF16, dl.device)
+                C.gemm(dl, w16, dxc, False, True, alpha=alpha, m_dyn=n_dyn)
+                C.scatter_rows(dxc, idx, counts, dx2)
+                _launched(3)
             dx = dx2.view(ctx.xshape)
         fork.join()
         return dx, dw, db, None, None, None

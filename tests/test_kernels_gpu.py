@@ -257,6 +257,63 @@ def test_linear_cross_entropy_gradients_over_large_vocabularies(C, monkeypatch, 
     test_linear_cross_entropy_gradients_with_few_rows(monkeypatch, rows, V, K, sparse)
 
 
+@pytest.mark.parametrize("M,N,K,counts", [(256, 512, 32000, None), (300, 136, 20000, None), (513, 768, 30522, None), (1, 8, 50257, None), (2048, 264, 18440, None),
+                                          (1500, 768, 30522, (0, 1, 255, 256, 257, 600, 1500)), (4096, 136, 8200, (1, 256, 2500, 4096)), (6000, 512, 32000, (37, 6000))])
+def test_product_in_parts(C, M, N, K, counts):
+    """dX = alpha dY W with its reduction in parts of a number that, with `counts`, only the device knows: ragged sizes, rows that take no part, memory that
+    held NaN before. One rounding to bf16 (2^-8) of fp32 sums of exact products; the same bits again."""
+    torch.manual_seed(N)
+    dy = (torch.randn(M, (K + 7) // 8 * 8, device="cuda") * 0.1).bfloat16()[:, :K]
+    w, alpha = torch.randn(K, N, device="cuda").bfloat16(), torch.tensor([-3.0], device="cuda")
+    lin, size = -3.0 * (dy.double() @ w.double()), 3.0 * (dy.double().abs() @ w.double().abs())
+
+    def run(*rows):
+        torch.full((80 * 256 * 256,), float("nan"), device="cuda")     # freed: the scratch may take its place
+        dx = torch.full((M, N), 7.0, device="cuda", dtype=torch.bfloat16)
+        assert C.gemm_in_parts(dy, w, dx, alpha, *rows)
+        assert C.read_status(0) == 0
+        return dx
+
+    C.clear_status(0)
+    for m in counts or (None,):
+        idx = torch.randperm(M, device="cuda")[:M].int()
+        rows = () if m is None else (idx, torch.tensor([m, M], device="cuda", dtype=torch.int32))
+        dx, again = run(*rows), run(*rows)
+        assert torch.equal(dx, again)
+        to = torch.arange(M, device="cuda") if m is None else idx[:m].long()
+        n = M if m is None else m
+        assert ((dx[to].double() - lin[:n]).abs() <= lin[:n].abs() * 2.0 ** -8 + 2.0 ** -20 * (size[:n] + 8)).all()
+        left = torch.ones(M, dtype=torch.bool, device="cuda")
+        left[to] = False
+        assert (dx[left] == 7).all()
+
+
+def test_product_in_parts_is_left_where_one_serves_better(C):
+    for M, N, K, counted in ((256, 512, 2056, False), (256, 512, 8200, False), (8192, 512, 32000, False), (24576, 768, 30522, True), (4096, 768, 1000, True)):
+        dy, w = torch.zeros(M, (K + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, :K], torch.zeros(K, N, device="cuda", dtype=torch.bfloat16)
+        dx = torch.ones(M, N, device="cuda", dtype=torch.bfloat16)
+        rows = (torch.arange(M, device="cuda").int(), torch.tensor([M, M], device="cuda", dtype=torch.int32)) if counted else ()
+        assert not C.gemm_in_parts(dy, w, dx, torch.ones(1, device="cuda"), *rows) and (dx == 1).all()
+
+
+@pytest.mark.parametrize("rows,V,K,sparse", [(256, 32000, 512, False), (4096, 30522, 768, True), (1024, 8200, 256, True)])
+def test_linear_cross_entropy_gives_dx_the_same_bits_again(C, monkeypatch, rows, V, K, sparse):
+    from flodl_b200 import ops
+    from flodl_b200.ops import core
+    monkeypatch.setitem(core._EAGER, "min_numel", 0)
+    torch.manual_seed(K)
+    x, w = torch.randn(rows, K, device="cuda").bfloat16(), (torch.randn(V, K, device="cuda") * 0.05).bfloat16()
+    t = torch.randint(0, V, (rows,), device="cuda")
+    if sparse:
+        t[torch.rand(rows, device="cuda") < 0.85] = -100
+    grads = []
+    for _ in range(4):
+        xg = x.clone().requires_grad_()
+        ops.linear_cross_entropy(xg, w, None, t, -100, sparse).backward()
+        grads.append(xg.grad)
+    assert all(torch.equal(grads[0], g) for g in grads[1:])
+
+
 def test_linear_gradients_in_one_launch_are_refused_where_they_do_not_fit(C):
     dy, w, x = (torch.randn(s, device="cuda").bfloat16() for s in ((2048, 1024), (1024, 1024), (2048, 1024)))
     dx, dw, db = torch.zeros_like(x), torch.zeros(1024, 1024, device="cuda"), torch.zeros(1028, device="cuda")

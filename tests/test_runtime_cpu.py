@@ -245,3 +245,19 @@ def test_eager_dispatch_threshold_is_process_wide_and_cpu_never_native():
         assert not core._native_ok(torch.zeros(4))  # CPU tensors never take the native path
     finally:
         core.set_eager_min_numel(old)
+
+
+@pytest.mark.parametrize("pairs", [1, 7, 66, 74])
+def test_parts_of_a_reduction_hold_blocks_and_fit_their_scratch(pairs):
+    """Every part of a product's split reduction has a K block, tiles times parts is at most what there are pairs of SMs, and the scratch that is sized for
+    any row count up to `M` holds the parts of each."""
+    for N, K in ((8, 64), (128, 2056), (256, 18440), (512, 32000), (768, 30522), (1024, 50257), (4096, 151936)):
+        blocks = -(-K // 64)
+        for M in (1, 255, 256, 257, 1500, 4096, 24576):
+            rows = C.gemm_part_rows(M, N, K, True, pairs)
+            for m in {0, 1, 255, 256, 257, M // 6, M // 2, M - 1, M} & set(range(M + 1)):
+                tiles_m, tiles_n = -(-m // 256), -(-N // 256)
+                n = C.gemm_part_count(m, N, K, pairs)
+                assert n >= 1 and (n - 1) * -(-blocks // n) < blocks and (n == 1 or (n * tiles_m * tiles_n <= pairs and blocks // n >= 16))
+                assert n * tiles_m * 256 <= rows
+            assert C.gemm_part_rows(M, N, K, False, pairs) == C.gemm_part_count(M, N, K, pairs) * -(-M // 256) * 256
