@@ -75,8 +75,8 @@ struct GemmParams {
   int accumulate;
   int split_k;
   int c_mode;      // 0 = per-thread global stores, 1 = staged TMA store, 2 = staged TMA reduce-add (fp32)
-  int part_groups; // not 0: the device cuts K for as many pairs (parts_for); C is [parts][rows of whole tiles][N] fp32, written and not added to, or
-                   // with one part [M][N] bf16 through the map `aux`
+  int part_groups; // of kernels with kParts: the device cuts K for as many pairs (parts_for); C is [parts][rows of whole tiles][N] fp32, written and not
+                   // added to, or with one part [M][N] bf16 through the map `aux`
   int kind;        // EpiKind: what the epilogue does
   int band;        // column tiles per band of the tile order (tile_of)
   int aux_tma;     // 1: the GELU pre-activation goes out through its own staged TMA store; 2: GELU' takes it in through TMA loads
@@ -591,7 +591,7 @@ __host__ __device__ constexpr int parts_for(int tiles, int blocks, int groups) {
 struct Segment {
   int prob, tm, tn, kb0, kb1, ks;
 };
-template <int kCG, int kBN, int kProblems>
+template <int kCG, int kBN, int kProblems, bool kParts>
 struct Worklist {
   const GemmLaunch<kProblems>& g;
   int step, num_m, num_n, num_kb, split, kb_per, units, u;      // the first product: whole tiles, or their K splits
@@ -602,9 +602,9 @@ struct Worklist {
     num_m = (m_eff + BM * kCG - 1) / (BM * kCG);
     num_n = (p.N + kBN - 1) / kBN;
     num_kb = (k_eff + BK - 1) / BK;
-    split = kProblems == 1 && p.part_groups ? parts_for(num_m * num_n, num_kb, p.part_groups) : parts_with_blocks(num_kb, p.split_k);   // (again: a reduction of dynamic length may have fewer blocks than parts were asked for)
-    kb_per = (num_kb + split - 1) / split;
-    units = num_kb > 0 ? num_m * num_n * split : 0;
+    if (kParts) split = parts_for(num_m * num_n, num_kb, p.part_groups);
+    kb_per = (num_kb + parts() - 1) / parts();
+    units = num_kb > 0 ? num_m * num_n * parts() : 0;
     if constexpr (kProblems == 2) {
       const GemmParams& q = g.p[1];
       num_m1 = (q.M + BM * kCG - 1) / (BM * kCG);
@@ -620,13 +620,15 @@ struct Worklist {
       end = group + 1 < groups ? start(group + 1) : total;
     }
   }
+  // Each has a block: parts_for says so, or the host, which does not split a length that it does not know.
+  __device__ __forceinline__ int parts() const { return kParts ? split : g.p[0].split_k; }
   __device__ __forceinline__ bool next(Segment& s) {
     if (u < units) {
       int t = u;
       s.ks = 0;
-      if (kProblems == 1 && split > 1) {
-        t = u / split;
-        s.ks = u - t * split;
+      if (kProblems == 1 && parts() > 1) {
+        t = u / parts();
+        s.ks = u - t * parts();
       }
       tile_of(t, num_m, num_n, g.p[0].band, s.tm, s.tn);
       s.prob = 0;
@@ -688,7 +690,8 @@ __device__ __forceinline__ void column_sums(const GemmLaunch<kProblems>& g, int 
 
 constexpr int gemm_threads(int problems) { return kGemmThreads + (problems == 2 ? 64 : 0); }
 
-template <int kCG, int kBN, int kProblems>
+// kParts: a kernel of its own for the reduction in parts; the choices below cost the others' epilogue (8192 x 2048 x 512 with GELU 23.8 -> 24.8 us).
+template <int kCG, int kBN, int kProblems, bool kParts>
 __global__ void __launch_bounds__(gemm_threads(kProblems), 1)
 gemm_bf16_kernel(const __grid_constant__ GemmLaunch<kProblems> g) {
   const GemmParams& p = g.p[0];
@@ -785,7 +788,7 @@ gemm_bf16_kernel(const __grid_constant__ GemmLaunch<kProblems> g) {
   int m_eff = p.M, k_eff = p.K;
   if (kProblems == 1 && p.m_dyn) m_eff = max(0, min(p.M, *p.m_dyn));
   if (kProblems == 1 && p.k_dyn) k_eff = max(0, min(p.K, *p.k_dyn));
-  Worklist<kCG, kBN, kProblems> work(g, group, num_groups, m_eff, k_eff);
+  Worklist<kCG, kBN, kProblems, kParts> work(g, group, num_groups, m_eff, k_eff);
   Segment seg;
 
   if (warp == 0) {
@@ -918,7 +921,7 @@ gemm_bf16_kernel(const __grid_constant__ GemmLaunch<kProblems> g) {
     const auto bias_of = [&](int u) -> float {
       if (u >= work.units) return 0.f;
       int tm, tn;
-      tile_of(u / work.split, work.num_m, work.num_n, p.band, tm, tn);
+      tile_of(u / work.parts(), work.num_m, work.num_n, p.band, tm, tn);
       const int c = q * 32 + lane, col = tn * kBN + half * kSplit + c;
       if (c >= cols || col >= p.N) return 0.f;
       return p.bias_fp32 ? __ldg(static_cast<const float*>(p.bias) + col) : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col]);
@@ -929,7 +932,7 @@ gemm_bf16_kernel(const __grid_constant__ GemmLaunch<kProblems> g) {
     for (; work.next(seg); ++it) {
       const GemmParams& pp = g.p[kProblems == 1 ? 0 : seg.prob];
       const CUtensorMap& tmC = g.c[kProblems == 1 ? 0 : seg.prob];
-      const int row0 = (seg.tm + (kProblems == 1 && p.part_groups ? seg.ks * work.num_m : 0)) * BM * kCG + static_cast<int>(rank) * BM + q * 32;
+      const int row0 = (kParts ? seg.tm + seg.ks * work.num_m : seg.tm) * BM * kCG + static_cast<int>(rank) * BM + q * 32;
       const int ncol0 = seg.tn * kBN + half * kSplit;
       const int acc = it & 1;
       uint32_t bias = 0;
@@ -958,15 +961,20 @@ gemm_bf16_kernel(const __grid_constant__ GemmLaunch<kProblems> g) {
       };
       if constexpr (kStaged) {
         // (of a part, whose rows reach to the end of its last tile, only those that are read)
-        const bool unread = kProblems == 1 && p.part_groups && seg.tm * BM * kCG + static_cast<int>(rank) * BM + q * 32 >= m_eff;
+        const bool unread = kParts && seg.tm * BM * kCG + static_cast<int>(rank) * BM + q * 32 >= m_eff;
         const int chunks = ncol0 >= pp.N || unread ? 0 : (min(cols, pp.N - ncol0) + 63) / 64;
-        const bool whole = kProblems == 1 && p.part_groups && work.split == 1;
         const auto run = [&](auto kind) {
-          ok = epilogue_tile<decltype(kind)::value>(pp, whole ? g.aux : tmC, g.aux, w, taddr, ncol0, row0, chunks, bias, abort_flag, hand_back, load_aux);
+          ok = epilogue_tile<decltype(kind)::value>(pp, kParts ? g.aux : tmC, g.aux, w, taddr, ncol0, row0, chunks, bias, abort_flag, hand_back, load_aux);
         };
+        if constexpr (kParts) {
+          if (chunks == 0) hand_back();
+          else if (work.split == 1) run(std::integral_constant<int, kEpiPlain>());
+          else epilogue_tile_f32(pp, tmC, w, taddr, ncol0, row0, min(cols, pp.N - ncol0), bias, hand_back);
+          continue;
+        }
         if (pp.kind != kEpiDirect) {
           if (chunks == 0) hand_back();
-          else if (pp.kind == kEpiPlain || whole) run(std::integral_constant<int, kEpiPlain>());
+          else if (pp.kind == kEpiPlain) run(std::integral_constant<int, kEpiPlain>());
           else if (pp.kind == kEpiF32) epilogue_tile_f32(pp, tmC, w, taddr, ncol0, row0, min(cols, pp.N - ncol0), bias, hand_back);
           else if (pp.kind == kEpiGelu) run(std::integral_constant<int, kEpiGelu>());
           else if (pp.kind == kEpiGeluAux) run(std::integral_constant<int, kEpiGeluAux>());
@@ -1272,11 +1280,11 @@ static int make_tmap_out(CUtensorMap* out, const void* base, uint64_t cols, uint
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
-template <int kCG, int kBN, int kProblems>
+template <int kCG, int kBN, int kProblems, bool kParts = false>
 static int launch_gemm(const GemmLaunch<kProblems>& g, int groups, cudaStream_t stream) {
   using Cfg = GemmCfg<kCG, kBN>;
-  auto kern = gemm_bf16_kernel<kCG, kBN, kProblems>;
-  if (const cudaError_t e = allow_smem<gemm_bf16_kernel<kCG, kBN, kProblems>>(Cfg::SMEM_BYTES)) return static_cast<int>(e);
+  auto kern = gemm_bf16_kernel<kCG, kBN, kProblems, kParts>;
+  if (const cudaError_t e = allow_smem<gemm_bf16_kernel<kCG, kBN, kProblems, kParts>>(Cfg::SMEM_BYTES)) return static_cast<int>(e);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(groups * kCG, 1, 1);
   cfg.blockDim = dim3(gemm_threads(kProblems), 1, 1);
@@ -1452,7 +1460,7 @@ extern "C" int fb_gemm_bf16_dyn(const void* A, const void* B, void* C, int M, in
   if (split_k < 1) split_k = 1;
   if (split_k > 1 && !c_fp32) return -2;
   if (split_k > 1 && !accumulate) accumulate = 1;          // parts are added to what the caller has zeroed, also if only one of them holds a block
-  split_k = parts_with_blocks((K + BK - 1) / BK, split_k);
+  split_k = k_dyn ? 1 : parts_with_blocks((K + BK - 1) / BK, split_k);
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
   bool over_pairs = false;       // the reduction split over two pairs of a cluster
   if (config < 0) {
@@ -1726,7 +1734,7 @@ extern "C" int fb_gemm_parts(const void* dY, const void* W, void* dX, float* scr
   p.M = M; p.N = N; p.K = K; p.b_mn = 1; p.C = scratch; p.ldc = N; p.c_fp32 = 1; p.alpha = alpha; p.split_k = 1; p.part_groups = groups; p.c_mode = 1; p.kind = kEpiF32;
   p.band = band_of(N, kPartTile); p.status = status; p.m_dyn = counts;
   const long long units = static_cast<long long>(tiles_of(M)) * tiles_of(N) * (counts ? groups : parts_for(tiles_of(M) * tiles_of(N), num_kb, groups));
-  if ((r = launch_gemm<2, 256, 1>(g, units < groups ? static_cast<int>(units) : groups, stream))) return r;
+  if ((r = launch_gemm<2, 256, 1, true>(g, units < groups ? static_cast<int>(units) : groups, stream))) return r;
   launch_pdl(sum_parts_kernel, dim3(blocks), dim3(kSumThreads), 0, stream, scratch, M, N, num_kb, groups, idx, counts,
              static_cast<__nv_bfloat16*>(dX), ldx);
   return static_cast<int>(cudaGetLastError());
