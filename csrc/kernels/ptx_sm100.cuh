@@ -115,7 +115,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   *abort_flag = 1;
   set_status(status, code);
   return false;
-}// A warp that loads or issues runs its loop whole and lets one elected lane issue: waits and indices are then the same for all its lanes, also to
+}
+
+// A warp that loads or issues runs its loop whole and lets one elected lane issue: waits and indices are then the same for all its lanes, also to
 // the compiler, and the operands of TMA loads and tcgen05.mma stay in the uniform registers that these take them from. In a branch of lane 0
 // each one is moved there first, which cost a 64-wide K step of a 128 x 128 GEMM tile 660 cycles instead of 460.
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
